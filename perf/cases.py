@@ -145,15 +145,19 @@ def _reads(g, n, L, genome, err, err_end, n_rate, paired, gc, repeats):
     for a in range(0, n, step):
         k = min(step, n - a)
         if paired:
-            ins = (torch.randn(k // 2, generator=g, device="cuda") * 50 + 400).round().clamp(min=L, max=seq.numel() // 2)
+            ins = (torch.randn(k // 2, generator=g, device="cuda") * 50 + 400).round().long()
+            ins = ins.clamp(min=L, max=seq.numel() // 2)
+            # whole numbers and 64-bit products: a float32 genome length would round past the end
             first = (torch.rand(k // 2, generator=g, device="cuda", dtype=torch.float64)
                      * (seq.numel() - ins + 1)).long()
-            start = torch.stack([first, first + ins.long() - L], 1)
+            first = torch.minimum(first, seq.numel() - ins)
+            start = torch.stack([first, first + ins - L], 1)
             flip = torch.rand(k // 2, 1, generator=g, device="cuda") < 0.5  # fragment from the reverse strand
             start = torch.where(flip, start.flip(1), start).reshape(-1)
             rc = torch.cat([flip, ~flip], 1).reshape(-1)
         else:
             start = (torch.rand(k, generator=g, device="cuda", dtype=torch.float64) * (seq.numel() - L + 1)).long()
+            start = start.clamp(max=seq.numel() - L)
             rc = torch.rand(k, generator=g, device="cuda") < 0.5
         # a reverse-complemented read walks its window backwards
         at = torch.where(rc, start + L - 1, start)[:, None] + torch.where(rc, -1, 1)[:, None] * cols
