@@ -34,6 +34,9 @@
 #ifndef ABS
 #define ABS std::abs
 #endif
+#ifdef CURC_NO_CODERS
+#include "no_coders.hpp"
+#else
 #include <fast-lzma2/fast-lzma2.h>
 #include <lzma/Alloc.h>
 #include <lzma/LzmaEnc.h>
@@ -41,6 +44,7 @@
 #include <lzma/VarLenDNACoder/LzmaLib.h>
 #include <range_coder/clr.cdr>
 #include <range_coder/simple_model.h>
+#endif
 
 #include "../../../include/curc_b200.h"
 #include "host.hpp"

@@ -32,11 +32,15 @@
 #include <string>
 #include <vector>
 
+#ifdef CURC_NO_CODERS
+#include "no_coders.hpp"
+#else
 #include <fast-lzma2/fast-lzma2.h>
 #include <lzma/Alloc.h>
 #include <lzma/LzmaDec.h>
 #include <lzma/Ppmd7.h>
 #include <lzma/VarLenDNACoder/LzmaLib.h>
+#endif
 
 #include "../../../include/curc_b200.h"
 #include "host.hpp"

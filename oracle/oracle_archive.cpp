@@ -5,6 +5,7 @@
 // The entropy coders are the reference's vendored third-party libraries,
 // linked from oracle/_ref/libcurc_coders.a; the strand stream goes through
 // the reference's `bsc` executable exactly as compress.cu does (util.cuh:527).
+#include <algorithm>
 #include <sys/stat.h>
 #include <unistd.h>
 
@@ -23,6 +24,9 @@
 #ifndef ABS
 #define ABS std::abs
 #endif
+#ifdef CURC_NO_CODERS
+#include "../curc_b200/csrc/host/no_coders.hpp"
+#else
 #include <lzma/VarLenDNACoder/LzmaLib.h>
 #include <range_coder/clr.cdr>
 #include <range_coder/simple_model.h>
@@ -30,6 +34,7 @@
 namespace lzma2 {
 void lzma2_compress(const char* infile, const char* outfile, int level, int thread_num);
 }
+#endif
 
 namespace oracle {
 namespace {
@@ -548,9 +553,11 @@ int oracle_compress_files(const char* f1, const char* f2, const char* working_di
 }
 }
 
+#ifndef CURC_NO_CODERS
 namespace lzma2 {
 void lzma2_decompress(const char* infile, const char* outfile);
 }
+#endif
 
 extern "C" {
 
