@@ -102,6 +102,13 @@ __device__ __forceinline__ uint64_t revcomp_kmer(uint64_t kmer, int k) {
     return kmer >> (64 - 2 * k);
 }
 
+// The 32 2-bit groups of a word in reverse order: nb bases held in the low
+// 2 nb bits come out reversed and left-aligned, zero padded.
+__device__ __forceinline__ uint64_t reverse_bases(uint64_t x) {
+    x = __brevll(x);
+    return ((x & 0x5555555555555555ULL) << 1) | ((x >> 1) & 0x5555555555555555ULL);
+}
+
 // Number of differing bases between two packed words (util.cuh:228-232).
 __device__ __forceinline__ int base_mismatches(uint64_t a, uint64_t b) {
     uint64_t x = a ^ b;

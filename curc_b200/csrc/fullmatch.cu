@@ -9,11 +9,26 @@
 // runs one sequential two-pointer merge per bucket.  Inside a bucket the
 // merge pairs, in order, the suffixes and prefixes of each run of equal
 // strings (with a rotation when a read meets itself), so here the work is
-// organised per run of equal suffix strings instead: no fixed 4^10 cost,
-// and one thread per run executes the reference's merge steps for that run.
+// organised per run of equal suffix strings instead.
 //
-// (1) is done as a tree of parallel stable pairwise merges of the
-// per-symbol runs (merge path).
+// Which suffix meets which prefixes does not depend on the links made: only
+// on the two lists.  So the meetings are listed first, for many offsets at
+// once, and then only they are walked, offset by offset
+// (full_match_events).  The walk needs the suffixes of a run in the
+// reference's order.  Its stable merges order suffixes that share
+// read[off, L) by the symbols before off, read backwards: by off-1, then
+// off-2, and so on.  Since the shared part is a common prefix of the reversed
+// reads, that order is at every offset the order of the whole reversed
+// reads.  One sort of the suffix list by reversed reads therefore makes each
+// run contiguous and ordered at every offset.
+//
+// The launch-per-kernel form that re-sorts at every offset
+// (full_match_passes) remains for reads with symbols other than A, C, G, N
+// and T, whose partition classes do not follow their byte order, and as
+// tune.fm_loop 0.  There (1) is a tree of parallel stable pairwise merges
+// of the per-symbol runs (merge path).
+#include <algorithm>
+
 #include "compact.cuh"
 #include "stages.cuh"
 
@@ -34,6 +49,18 @@ struct PackedAcc {
     __device__ __forceinline__ uint64_t key(uint32_t a, int pos) const {
         const int nb = L - pos < KS ? L - pos : KS;
         return word_at(db + uint64_t(a) * W, uint32_t(pos), nb) << (64 - SB * nb);
+    }
+    // word k of the reversed read: 32 symbols backwards from L-1 - 32 k,
+    // left-aligned, zero padded
+    __device__ __forceinline__ uint64_t rword(uint32_t a, int k) const {
+        const int end = L - KS * k, nb = end < KS ? end : KS;
+        return reverse_bases(word_at(db + uint64_t(a) * W, uint32_t(end - nb), nb));
+    }
+    __device__ __forceinline__ int rwords() const { return W; }
+    // hash of the FK <= FK_MAX symbols from pos
+    static constexpr int FK_MAX = 32;
+    __device__ __forceinline__ uint64_t fhash(uint32_t a, int pos, int fk) const {
+        return murmur64(word_at(db + uint64_t(a) * W, uint32_t(pos), fk));
     }
 };
 
@@ -65,6 +92,22 @@ struct AsciiAcc {
         for (int b = 0; b < KS; ++b) v = (v << 8) | (pos + b < L ? x[pos + b] : 0);
         return v;
     }
+    __device__ __forceinline__ uint64_t rword(uint32_t a, int k) const {
+        const uint8_t* x = r + uint64_t(a) * L;
+        uint64_t v = 0;
+        for (int b = 0; b < KS; ++b) {
+            const int pos = L - 1 - KS * k - b;
+            v = (v << 8) | (pos >= 0 ? x[pos] : 0);
+        }
+        return v;
+    }
+    __device__ __forceinline__ int rwords() const { return (L + KS - 1) / KS; }
+    static constexpr int FK_MAX = 16;
+    __device__ __forceinline__ uint64_t fhash(uint32_t a, int pos, int fk) const {
+        const uint64_t k0 = key(a, pos);
+        if (fk <= KS) return murmur64(k0 >> (64 - SB * fk));
+        return murmur64(murmur64(k0) ^ (key(a, pos + KS) >> (64 - SB * (fk - KS))));
+    }
 };
 
 // Comparison of read a from aoff with read b from boff over len symbols,
@@ -82,14 +125,6 @@ __device__ __forceinline__ int cmp_keyed(const Acc& acc, uint64_t ka, uint32_t a
     if (len <= Acc::KS) return 0;
     return acc.cmp(a, aoff + Acc::KS, b, boff + Acc::KS, len - Acc::KS);
 }
-
-// The pass's offset: a kernel argument when the host queues the passes,
-// read from device memory when the passes replay from a graph.
-struct FmOff {
-    int v;
-    const int* p;
-    __device__ __forceinline__ int get() const { return p ? *p : v; }
-};
 
 // Keys of the list entries [t0, m) step ts at offset off.  With sym_count
 // (2-bit reads only), also how many entries have each base at off-1: the
@@ -118,10 +153,9 @@ __device__ __forceinline__ void list_keys_range(const Acc& acc, const uint32_t* 
 // list's length).
 template <class Acc>
 __global__ void list_keys_kernel(Acc acc, const uint32_t* __restrict__ ids, const uint32_t* __restrict__ m_dev,
-                                 FmOff fo, uint64_t* __restrict__ key, uint32_t* __restrict__ sym_count,
+                                 int off, uint64_t* __restrict__ key, uint32_t* __restrict__ sym_count,
                                  const uint32_t* __restrict__ mp_dev, unsigned long long* __restrict__ tally) {
     const uint32_t m = *m_dev;
-    const int off = fo.get();
     if (tally && blockIdx.x == 0 && threadIdx.x == 0) {
         const uint32_t mp = *mp_dev;
         if (m && mp) {
@@ -183,9 +217,9 @@ __device__ __forceinline__ void run_bounds_block(const Acc& acc, const uint32_t*
 
 template <class Acc>
 __global__ void __launch_bounds__(256) run_bounds_kernel(Acc acc, const uint32_t* __restrict__ suf,
-                                                         const uint32_t* __restrict__ m_dev, FmOff fo,
+                                                         const uint32_t* __restrict__ m_dev, int off,
                                                          uint32_t* __restrict__ bounds) {
-    run_bounds_block(acc, suf, *m_dev, fo.get(), bounds);
+    run_bounds_block(acc, suf, *m_dev, off, bounds);
 }
 
 // Stable merge of the symbol runs by read[off, L), as a tree of pairwise
@@ -259,11 +293,11 @@ __device__ __forceinline__ void merge_level_range(const Acc& acc, int off, const
 // bounds: the run bounds (ALPHA + 1 entries), or with `counts` the number of
 // entries per symbol, from which the bounds are summed.
 template <class Acc>
-__global__ void merge_level_kernel(Acc acc, FmOff fo, const uint32_t* __restrict__ in, const uint64_t* __restrict__ ink,
+__global__ void merge_level_kernel(Acc acc, int off, const uint32_t* __restrict__ in, const uint64_t* __restrict__ ink,
                                    uint32_t* __restrict__ out, uint64_t* __restrict__ outk,
                                    const uint32_t* __restrict__ bounds, bool counts, const uint32_t* __restrict__ m_dev,
                                    int width) {
-    merge_level_range(acc, fo.get(), in, ink, out, outk, bounds, counts, *m_dev, width,
+    merge_level_range(acc, off, in, ink, out, outk, bounds, counts, *m_dev, width,
                       uint64_t(blockIdx.x) * blockDim.x + threadIdx.x, uint64_t(gridDim.x) * blockDim.x);
 }
 
@@ -337,230 +371,12 @@ __device__ __forceinline__ void group_one(const Acc& acc, uint32_t* pre, uint64_
 template <class Acc>
 __global__ void merge_groups_kernel(Acc acc, uint32_t* pre, uint64_t* pk, const uint32_t* __restrict__ mp_dev,
                                     const uint32_t* __restrict__ suf, const uint64_t* __restrict__ sk,
-                                    const uint32_t* __restrict__ ms_dev, FmOff fo, uint32_t* next, uint32_t* prev,
+                                    const uint32_t* __restrict__ ms_dev, int off, uint32_t* next, uint32_t* prev,
                                     uint16_t* offset) {
     const uint32_t mp = *mp_dev, ms = *ms_dev;
     if (mp == 0) return;
-    const int off = fo.get();
     for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < ms; j += gridDim.x * blockDim.x)
         group_one(acc, pre, pk, mp, suf, sk, ms, off, j, next, prev, offset);
-}
-
-// ---------------------------------------------------------------- persistent form
-//
-// One cooperative launch runs every pass: the phases of a pass (keys and
-// run bounds, the merge levels, the pairing, a two-phase compaction of both
-// lists) are separated by grid-wide barriers instead of kernel boundaries,
-// and the lists' lengths are read from device memory at the top of each
-// pass, so neither launches nor host reads separate the passes.  Every block
-// is resident (cooperative launch), which the barriers need.  The results
-// are those of the launch-per-kernel form: the same device functions do the
-// work, and the compaction keeps both lists in order (chunks in block order,
-// entries in index order inside a chunk).
-constexpr int FM_THREADS = 256;
-constexpr uint32_t FM_BARRIER_LIMIT = 1u << 22;  // ~0.3 s of 64 ns sleeps; a barrier takes microseconds
-
-// Grid-wide barrier with a bounded wait (cooperative launch: every block
-// resident).  word[0] counts arrivals, word[1] is the generation, word[2]
-// the error flag.  Block writes before the barrier are visible to every
-// block after it (block barrier, then a device-scope fence by the arriving
-// thread, and one after the wait).  Returns false once any block's wait
-// has run out: the caller leaves the loop, so no block waits for ever.
-__device__ __forceinline__ bool fm_grid_barrier(uint32_t* word, uint32_t nblocks) {
-    __shared__ uint32_t s_ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        volatile uint32_t* gen = word + 1;
-        volatile uint32_t* err = word + 2;
-        const uint32_t g = *gen;
-        __threadfence();
-        bool ok = *err == 0;
-        if (ok) {
-            if (atomicAdd(word, 1u) == nblocks - 1) {
-                word[0] = 0;
-                __threadfence();
-                atomicAdd(word + 1, 1u);
-            } else {
-                uint32_t spins = 0;
-                while (*gen == g) {
-                    if (*err != 0 || ++spins > FM_BARRIER_LIMIT) {
-                        atomicExch(word + 2, 1u);
-                        ok = false;
-                        break;
-                    }
-                    __nanosleep(64);
-                }
-            }
-        }
-        __threadfence();
-        s_ok = ok ? 1u : 0u;
-    }
-    __syncthreads();
-    return s_ok != 0;
-}
-
-struct FmPersist {
-    uint32_t *pre, *tmp, *suf, *suf2, *mtmp;
-    uint64_t *pk, *tk, *sk, *sk2, *mk2;
-    uint32_t* bounds;             // run bounds, or base counts (2-bit reads; zero at launch)
-    uint32_t* len;                // [0] prefixes, [1] suffixes in the lists
-    uint32_t* bcnt;               // per block: kept prefixes, then kept suffixes (2 x gridDim)
-    uint32_t *next, *prev;
-    uint16_t* offset;
-    unsigned long long* tally;    // optional: passes, suffix and prefix entries
-    uint32_t* passes;             // passes run
-    uint32_t* barrier;            // fm_grid_barrier words (3; zero at launch)
-};
-
-// Block-wide exclusive scan of one value per thread (FM_THREADS threads);
-// returns the thread's exclusive prefix, *total the block's sum.
-__device__ __forceinline__ uint32_t fm_block_scan(uint32_t v, uint32_t* s_warp, uint32_t* total) {
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    uint32_t incl = v;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t u = __shfl_up_sync(0xFFFFFFFFu, incl, d);
-        if (lane >= uint32_t(d)) incl += u;
-    }
-    if (lane == 31) s_warp[warp] = incl;
-    __syncthreads();
-    uint32_t before = 0, all = 0;
-#pragma unroll
-    for (int w = 0; w < FM_THREADS / 32; ++w) {
-        const uint32_t c = s_warp[w];
-        before += w < int(warp) ? c : 0;
-        all += c;
-    }
-    __syncthreads();  // s_warp is reused by the next call
-    *total = all;
-    return before + incl - v;
-}
-
-// Block-wide sum (FM_THREADS threads).
-__device__ __forceinline__ uint32_t fm_block_sum(uint32_t v, uint32_t* s_warp) {
-    uint32_t t;
-    fm_block_scan(v, s_warp, &t);
-    return t;
-}
-
-template <class Acc>
-__global__ void __launch_bounds__(FM_THREADS) fm_persistent_kernel(Acc acc, FmPersist st) {
-    __shared__ uint32_t s_warp[FM_THREADS / 32];
-    auto sync = [&] { return fm_grid_barrier(st.barrier, gridDim.x); };
-    constexpr bool by_count = Acc::ALPHA == 4;
-    int levels = 0;
-    while ((1 << levels) < Acc::ALPHA) ++levels;
-    const uint32_t G = gridDim.x;
-    const uint64_t gt = uint64_t(blockIdx.x) * FM_THREADS + threadIdx.x, gs = uint64_t(G) * FM_THREADS;
-    uint32_t* pre = st.pre;
-    uint32_t* tmp = st.tmp;
-    uint64_t* pk = st.pk;
-    uint64_t* tk = st.tk;
-    uint32_t passes = 0;
-    for (int off = 1; off < acc.L; ++off) {
-        // the lengths were written before the last barrier; read past L1 so
-        // that every block sees the same values and takes the same barriers
-        const uint32_t mp = *reinterpret_cast<volatile const uint32_t*>(st.len);
-        const uint32_t ms = *reinterpret_cast<volatile const uint32_t*>(st.len + 1);
-        if (mp == 0 || ms == 0) break;
-        ++passes;
-        if (gt == 0 && st.tally) {
-            st.tally[0] += 1;
-            st.tally[1] += ms;
-            st.tally[2] += mp;
-        }
-        // keys of the suffixes at off (and, 2-bit reads, their base counts at off-1)
-        list_keys_range(acc, st.suf, ms, off, st.sk, by_count ? st.bounds : nullptr, uint32_t(gt), uint32_t(gs));
-        if (!by_count && blockIdx.x == 0) run_bounds_block(acc, st.suf, ms, off, st.bounds);
-        if (!sync()) break;
-        // merge levels: the last one writes suf2/sk2
-        bool alive = true;
-        {
-            const uint32_t* src = st.suf;
-            const uint64_t* srck = st.sk;
-            for (int l = 0; l < levels && alive; ++l) {
-                const bool last = l + 1 == levels;
-                uint32_t* dst = last ? st.suf2 : (l % 2 == 0 ? st.mtmp : st.suf);
-                uint64_t* dstk = last ? st.sk2 : (l % 2 == 0 ? st.mk2 : st.sk);
-                merge_level_range(acc, off, src, srck, dst, dstk, st.bounds, by_count, ms, 1 << l, gt, gs);
-                alive = sync();
-                src = dst;
-                srck = dstk;
-            }
-        }
-        if (!alive) break;
-        // pairing, one thread per run of equal suffix strings
-        for (uint64_t j = gt; j < ms; j += gs)
-            group_one(acc, pre, pk, mp, st.suf2, st.sk2, ms, off, uint32_t(j), st.next, st.prev, st.offset);
-        if (by_count && gt < 4) st.bounds[gt] = 0;  // counts of the next pass (the merges are done)
-        if (!sync()) break;
-        // compaction, phase 1: kept entries of this block's chunk of each list
-        const uint32_t cp = (mp + G - 1) / G, cs = (ms + G - 1) / G;
-        const uint32_t p0 = min(mp, blockIdx.x * cp), p1 = min(mp, p0 + cp);
-        const uint32_t s0 = min(ms, blockIdx.x * cs), s1 = min(ms, s0 + cs);
-        {
-            uint32_t kp = 0, ks = 0;
-            for (uint32_t i = p0 + threadIdx.x; i < p1; i += FM_THREADS) kp += st.prev[pre[i]] == INVALID;
-            for (uint32_t i = s0 + threadIdx.x; i < s1; i += FM_THREADS) ks += st.next[st.suf2[i]] == INVALID;
-            kp = fm_block_sum(kp, s_warp);
-            ks = fm_block_sum(ks, s_warp);
-            if (threadIdx.x == 0) {
-                st.bcnt[blockIdx.x] = kp;
-                st.bcnt[G + blockIdx.x] = ks;
-            }
-        }
-        if (!sync()) break;
-        // phase 2: this chunk's place from the chunks before it, then the
-        // kept entries in order
-        {
-            uint32_t bp = 0, bs = 0, tp = 0, ts = 0;
-            const volatile uint32_t* bc = st.bcnt;  // other blocks' counts, from L2
-            for (uint32_t b = threadIdx.x; b < G; b += FM_THREADS) {
-                const uint32_t a = bc[b], c = bc[G + b];
-                tp += a;
-                ts += c;
-                if (b < blockIdx.x) {
-                    bp += a;
-                    bs += c;
-                }
-            }
-            bp = fm_block_sum(bp, s_warp);
-            bs = fm_block_sum(bs, s_warp);
-            tp = fm_block_sum(tp, s_warp);
-            ts = fm_block_sum(ts, s_warp);
-            for (uint32_t i0 = p0; i0 < p1; i0 += FM_THREADS) {
-                const uint32_t i = i0 + threadIdx.x;
-                const bool keep = i < p1 && st.prev[pre[i]] == INVALID;
-                uint32_t tile;
-                const uint32_t r = fm_block_scan(keep ? 1u : 0u, s_warp, &tile);
-                if (keep) {
-                    tmp[bp + r] = pre[i];
-                    tk[bp + r] = pk[i];
-                }
-                bp += tile;
-            }
-            for (uint32_t i0 = s0; i0 < s1; i0 += FM_THREADS) {
-                const uint32_t i = i0 + threadIdx.x;
-                const bool keep = i < s1 && st.next[st.suf2[i]] == INVALID;
-                uint32_t tile;
-                const uint32_t r = fm_block_scan(keep ? 1u : 0u, s_warp, &tile);
-                if (keep) st.suf[bs + r] = st.suf2[i];
-                bs += tile;
-            }
-            if (gt == 0) {
-                st.len[0] = tp;
-                st.len[1] = ts;
-            }
-        }
-        uint32_t* t32 = pre;
-        pre = tmp;
-        tmp = t32;
-        uint64_t* t64 = pk;
-        pk = tk;
-        tk = t64;
-        if (!sync()) break;
-    }
-    if (gt == 0) *st.passes = passes;
 }
 
 // Compaction functors: keep the list entries whose link is still free.
@@ -585,52 +401,16 @@ struct MoveIdKey {
     }
 };
 
-__global__ void fm_zero4_kernel(uint32_t* p) { p[threadIdx.x] = 0; }
 
-// Graph form of the pass loop.  After the first pass of a replayed pair the
-// offset advances; past the last offset the second pass's list lengths are
-// zeroed, so its launches find no work.
-__global__ void fm_step_kernel(int* offp, uint32_t* next_len, int L) {
-    const int o = ++*offp;
-    if (o >= L) {
-        next_len[0] = 0;
-        next_len[1] = 0;
-    }
-}
-
-// After the second pass: the device loop goes on while offsets remain and
-// both lists hold entries.  The offset grows by two per iteration, so the
-// loop ends after at most L / 2 iterations whatever the lists hold; the
-// iteration count is capped at L as well, independently of the offset.
-__global__ void fm_cond_kernel(cudaGraphConditionalHandle h, int* offp, const uint32_t* len, int L,
-                               uint32_t* iters) {
-    const int o = ++*offp;
-    const uint32_t it = ++*iters;
-    cudaGraphSetConditional(h, (o < L && it < uint32_t(L) && len[0] != 0 && len[1] != 0) ? 1u : 0u);
-}
-
-// The passes run without a host round trip: list lengths stay on the
-// device (two slots per list, read by one pass and written by its
-// compaction) and kernels walk them with resident grids.  Three forms, with
-// the same results (tune.fm_loop): 0, one launch per kernel from the host,
-// which looks at the lengths every few passes to stop early (and times the
-// sub-stages); 1, a graph whose conditional `while` node replays a pair of
-// passes, the offset and the stop test on the device, so one graph launch
-// runs the whole loop; 2, one persistent cooperative kernel whose phases
-// are separated by grid-wide barriers (fm_persistent_kernel).
+// ---------------------------------------------------------------- pass form
+//
+// One launch per kernel and offset, queued by the host: list lengths stay on
+// the device (two slots per list, read by one pass and written by its
+// compaction), kernels walk the lists with resident grids, and the host looks
+// at the lengths every few passes to stop early.
 template <class Acc>
-void full_match_loop(const Acc& acc, uint32_t* pre, uint32_t* suf, uint32_t cnt, uint32_t* next, uint32_t* prev,
-                     uint16_t* offset, int mode, unsigned long long* tally, Arena& a, cudaStream_t s) {
-    // nothing to link without ends; a single prefix and a single suffix can
-    // still link when they are different reads (the head and the tail of one
-    // chain, which then closes into a cycle, as the reference's merge does)
-    if (cnt == 0 || acc.L < 2) return;
-    if (cnt == 1) {  // one end of each kind: nothing links when both are the same read
-        uint32_t ends[2];
-        read_small(ends, pre, 4, s);
-        read_small(ends + 1, suf, 4, s);
-        if (ends[0] == ends[1]) return;
-    }
+void full_match_passes(const Acc& acc, uint32_t* pre, uint32_t* suf, uint32_t cnt, uint32_t* next, uint32_t* prev,
+                       uint16_t* offset, unsigned long long* tally, Arena& a, cudaStream_t s) {
     auto mk = a.mark();
     uint32_t* suf2 = a.alloc<uint32_t>(cnt);
     uint32_t* tmp = a.alloc<uint32_t>(cnt);
@@ -644,38 +424,30 @@ void full_match_loop(const Acc& acc, uint32_t* pre, uint32_t* suf, uint32_t cnt,
     uint64_t* mk2 = a.alloc<uint64_t>(cnt);
     uint32_t* bounds = a.alloc<uint32_t>(8);
     uint32_t* len = a.alloc<uint32_t>(4);  // mp, ms for even passes, then for odd passes
-    int* offp = a.alloc<int>(2);           // graph form: [0] the pass's offset, [1] iterations
     const uint32_t init[4] = {cnt, cnt, 0, 0};
     CURC_CHECK(cudaMemcpyAsync(len, init, sizeof(init), cudaMemcpyHostToDevice, s));
     Compactor cp(cnt, a, s);
     const int gk = resident_grid(list_keys_kernel<Acc>, 256, cnt);
     const int gm = resident_grid(merge_level_kernel<Acc>, 256, div_up(cnt, MP_ITEMS));
     const int gg = resident_grid(merge_groups_kernel<Acc>, 128, cnt);
-    list_keys_kernel<Acc><<<gk, 256, 0, s>>>(acc, pre, len, FmOff{0, nullptr}, pk, nullptr, nullptr, nullptr);
+    list_keys_kernel<Acc><<<gk, 256, 0, s>>>(acc, pre, len, 0, pk, nullptr, nullptr, nullptr);
     CURC_LAUNCH_CHECK();
     // 2-bit reads: the base runs' bounds come from counts taken with the keys
     constexpr bool by_count = Acc::ALPHA == 4;
-
-    // One pass over the lists in slots `par`, at offset fo.
-    auto pass = [&](FmOff fo, int par, bool graph) {
+    constexpr int CHECK_EVERY = 8;
+    int par = 0;
+    for (int off = 1; off < acc.L; ++off, par ^= 1) {
         uint32_t* mp_in = len + 2 * par;
         uint32_t* ms_in = mp_in + 1;
         uint32_t* mp_out = len + 2 * (par ^ 1);
         uint32_t* ms_out = mp_out + 1;
-        SubStage sp_merge("full_match.resort", !graph);
         if (by_count) {
-            if (graph) {  // a kernel node rather than a memset node in the loop body
-                fm_zero4_kernel<<<1, 4, 0, s>>>(bounds);
-                CURC_LAUNCH_CHECK();
-            } else {
-                CURC_CHECK(cudaMemsetAsync(bounds, 0, 4 * sizeof(uint32_t), s));
-            }
+            CURC_CHECK(cudaMemsetAsync(bounds, 0, 4 * sizeof(uint32_t), s));
         } else {
-            run_bounds_kernel<Acc><<<1, 256, 0, s>>>(acc, suf, ms_in, fo, bounds);
+            run_bounds_kernel<Acc><<<1, 256, 0, s>>>(acc, suf, ms_in, off, bounds);
             CURC_LAUNCH_CHECK();
         }
-        list_keys_kernel<Acc><<<gk, 256, 0, s>>>(acc, suf, ms_in, fo, sk, by_count ? bounds : nullptr, mp_in,
-                                                  tally);
+        list_keys_kernel<Acc><<<gk, 256, 0, s>>>(acc, suf, ms_in, off, sk, by_count ? bounds : nullptr, mp_in, tally);
         CURC_LAUNCH_CHECK();
         {
             // levels: runs merged in pairs, then pairs of pairs, ...; the last
@@ -688,121 +460,649 @@ void full_match_loop(const Acc& acc, uint32_t* pre, uint32_t* suf, uint32_t cnt,
                 const bool last = l + 1 == levels;
                 uint32_t* dst = last ? suf2 : (l % 2 == 0 ? mtmp : suf);
                 uint64_t* dstk = last ? sk2 : (l % 2 == 0 ? mk2 : sk);
-                merge_level_kernel<Acc><<<gm, 256, 0, s>>>(acc, fo, src, srck, dst, dstk, bounds, by_count, ms_in,
+                merge_level_kernel<Acc><<<gm, 256, 0, s>>>(acc, off, src, srck, dst, dstk, bounds, by_count, ms_in,
                                                             1 << l);
                 CURC_LAUNCH_CHECK();
                 src = dst;
                 srck = dstk;
             }
         }
-        sp_merge.stop();
-        SubStage sp_groups("full_match.groups", !graph);
-        merge_groups_kernel<Acc><<<gg, 128, 0, s>>>(acc, pre, pk, mp_in, suf2, sk2, ms_in, fo, next, prev, offset);
+        merge_groups_kernel<Acc><<<gg, 128, 0, s>>>(acc, pre, pk, mp_in, suf2, sk2, ms_in, off, next, prev, offset);
         CURC_LAUNCH_CHECK();
-        sp_groups.stop();
-        SubStage sp_comp("full_match.compact", !graph);
-        if (graph) {
-            cp.run_replayable(mp_in, cnt, mp_out, FreeLink{pre, prev}, MoveIdKey{pre, pk, tmp, tk});
-            cp.run_replayable(ms_in, cnt, ms_out, FreeLink{suf2, next}, MoveId{suf2, suf});
-        } else {
-            cp.run(mp_in, cnt, mp_out, FreeLink{pre, prev}, MoveIdKey{pre, pk, tmp, tk});
-            cp.run(ms_in, cnt, ms_out, FreeLink{suf2, next}, MoveId{suf2, suf});
-        }
+        cp.run(mp_in, cnt, mp_out, FreeLink{pre, prev}, MoveIdKey{pre, pk, tmp, tk});
+        cp.run(ms_in, cnt, ms_out, FreeLink{suf2, next}, MoveId{suf2, suf});
         std::swap(pre, tmp);
         std::swap(pk, tk);
-        sp_comp.stop();
-    };
-
-    if (mode == 2) {
-        SubStage sp_loop("full_match.persistent");
-        int dev = 0, sms = 0, per_sm = 0;
-        CURC_CHECK(cudaGetDevice(&dev));
-        CURC_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-        CURC_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fm_persistent_kernel<Acc>, FM_THREADS, 0));
-        if (per_sm < 1) throw std::runtime_error("full match: the persistent kernel does not fit on an SM");
-        const int grid = sms * per_sm;  // every block resident: the barriers need it
-        uint32_t* bcnt = a.alloc<uint32_t>(2 * size_t(grid));
-        uint32_t* barrier = a.alloc<uint32_t>(4);
-        CURC_CHECK(cudaMemsetAsync(bounds, 0, 8 * sizeof(uint32_t), s));
-        CURC_CHECK(cudaMemsetAsync(barrier, 0, 4 * sizeof(uint32_t), s));
-        FmPersist fp{pre,  tmp,  suf,  suf2,   mtmp,  pk,    tk,                                  sk,
-                     sk2,  mk2,  bounds, len,  bcnt,  next,  prev,                                offset,
-                     tally, reinterpret_cast<uint32_t*>(offp), barrier};
-        Acc acc_arg = acc;
-        void* args[] = {&acc_arg, &fp};
-        CURC_CHECK(cudaLaunchCooperativeKernel(reinterpret_cast<void*>(fm_persistent_kernel<Acc>), grid, FM_THREADS,
-                                               args, 0, s));
-        CURC_LAUNCH_CHECK();
-        sp_loop.stop();
-        uint32_t err = 0;
-        read_small(&err, barrier + 2, 4, s);
-        if (err) throw std::runtime_error("full match: a grid barrier wait of the persistent kernel ran out");
-    } else if (mode == 0) {
-        constexpr int CHECK_EVERY = 8;
-        int par = 0;
-        for (int off = 1; off < acc.L; ++off, par ^= 1) {
-            pass(FmOff{off, nullptr}, par, false);
-            if (off % CHECK_EVERY == 0) {
-                uint32_t h[2];
-                read_small(h, len + 2 * (par ^ 1), 8, s);
-                if (h[0] == 0 || h[1] == 0) break;
-            }
+        if (off % CHECK_EVERY == 0) {
+            uint32_t h[2];
+            read_small(h, len + 2 * (par ^ 1), 8, s);
+            if (h[0] == 0 || h[1] == 0) break;
         }
-        cp.check();
-    } else {
-        SubStage sp_loop("full_match.graph");
-        const int init_off[2] = {1, 0};
-        CURC_CHECK(cudaMemcpyAsync(offp, init_off, sizeof(init_off), cudaMemcpyHostToDevice, s));
-        cudaGraph_t g = nullptr, body = nullptr;
-        cudaGraphExec_t ge = nullptr;
-        uint64_t body_launches = 0;
-        try {
-            CURC_CHECK(cudaGraphCreate(&g, 0));
-            cudaGraphConditionalHandle h;
-            CURC_CHECK(cudaGraphConditionalHandleCreate(&h, g, 1, cudaGraphCondAssignDefault));
-            cudaGraphNodeParams np = {};
-            np.type = cudaGraphNodeTypeConditional;
-            np.conditional.handle = h;
-            np.conditional.type = cudaGraphCondTypeWhile;
-            np.conditional.size = 1;
-            cudaGraphNode_t node;
-            CURC_CHECK(cudaGraphAddNode(&node, g, nullptr, 0, &np));
-            body = np.conditional.phGraph_out[0];
-            CURC_CHECK(cudaStreamBeginCaptureToGraph(s, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-            try {
-                pass(FmOff{0, offp}, 0, true);
-                fm_step_kernel<<<1, 1, 0, s>>>(offp, len + 2, acc.L);
-                CURC_LAUNCH_CHECK();
-                pass(FmOff{0, offp}, 1, true);
-                fm_cond_kernel<<<1, 1, 0, s>>>(h, offp, len, acc.L, reinterpret_cast<uint32_t*>(offp + 1));
-                CURC_LAUNCH_CHECK();
-            } catch (...) {
-                cudaGraph_t dummy = nullptr;
-                cudaStreamEndCapture(s, &dummy);
-                if (dummy && dummy != body) cudaGraphDestroy(dummy);
-                throw;
-            }
-            CURC_CHECK(cudaStreamEndCapture(s, &body));
-            size_t nodes = 0;  // every node of the body is a kernel
-            CURC_CHECK(cudaGraphGetNodes(body, nullptr, &nodes));
-            body_launches = nodes;
-            CURC_CHECK(cudaGraphInstantiate(&ge, g, 0));
-            CURC_CHECK(cudaGraphLaunch(ge, s));
-        } catch (...) {
-            if (ge) cudaGraphExecDestroy(ge);
-            if (g) cudaGraphDestroy(g);
-            throw;
-        }
-        sp_loop.stop();
-        cp.check();  // synchronises: the graph has run
-        uint32_t iters = 0;
-        read_small(&iters, offp + 1, 4, s);
-        CURC_CHECK(cudaGraphExecDestroy(ge));
-        CURC_CHECK(cudaGraphDestroy(g));
-        // the captured launches were counted once; the device replayed them
-        if (iters > 1) count_launches(body_launches * (iters - 1));
     }
+    cp.check();
     a.release(mk);
+}
+
+// ---------------------------------------------------------------- event form
+
+// Meeting of a suffix (id s) with the prefixes [lo, hi) of the list, p the
+// first one's id.
+struct __align__(16) FmItem {
+    uint32_t s, lo, hi, p;
+};
+
+template <class Acc>
+__global__ void fm_prefix_kernel(Acc acc, const uint32_t* __restrict__ pre, uint32_t m, uint64_t* __restrict__ pk,
+                                 int fk, uint32_t* __restrict__ bits, uint32_t bmask) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= m) return;
+    const uint32_t id = pre[i];
+    pk[i] = acc.key(id, 0);
+    const uint32_t h = uint32_t(acc.fhash(id, 0, fk)) & bmask;
+    atomicOr(&bits[h >> 5], 1u << (h & 31));
+}
+
+// The prefixes of the list that start with s[off, L): [lo, hi), by binary
+// search; false when there is none.
+template <class Acc>
+__device__ __forceinline__ bool fm_run(const Acc& acc, const uint32_t* pre, const uint64_t* pk, uint32_t mp,
+                                       uint32_t s, int off, uint32_t& lo_out, uint32_t& hi_out) {
+    const int len = acc.L - off;
+    const uint64_t k = acc.key(s, off);
+    auto pcmp = [&](uint32_t i) { return cmp_keyed(acc, pk[i], pre[i], 0, k, s, off, len); };
+    uint32_t lo = 0, count = mp;
+    int at_lo = 1;  // the comparison of the entry the search ends on
+    while (count > 0) {
+        const uint32_t step = count / 2, it = lo + step;
+        const int r = pcmp(it);
+        if (r < 0) {
+            lo = it + 1;
+            count -= step + 1;
+        } else {
+            count = step;
+            at_lo = r;
+        }
+    }
+    if (lo >= mp || at_lo != 0) return false;
+    uint32_t hi = lo + 1;
+    if (hi < mp && pcmp(hi) == 0) {
+        uint32_t c = mp - hi;
+        while (c > 0) {
+            const uint32_t step = c / 2, it = hi + step;
+            if (pcmp(it) <= 0) {
+                hi = it + 1;
+                c -= step + 1;
+            } else {
+                c = step;
+            }
+        }
+    }
+    lo_out = lo;
+    hi_out = hi;
+    return true;
+}
+
+// Lists the meetings of the suffixes at offsets [off0, off0 + noffs): one
+// thread takes one suffix and 32 offsets (blockIdx.y), tests the 32 strings
+// in the prefixes' presence bitmap (loads in flight together), reserves room
+// for those that pass and searches the prefix list for each.  hits holds the
+// runs found, in no order; word w of suffix j has its meeting offsets in
+// em[w * ms + j] and the first of its runs at ub[w * ms + j].  *used counts
+// the room asked for; when it passes cap the caller repeats with fewer
+// offsets.
+template <class Acc>
+__global__ void __launch_bounds__(256) fm_meet_kernel(Acc acc, const uint32_t* __restrict__ suf, uint32_t ms,
+                                                      const uint32_t* __restrict__ pre,
+                                                      const uint64_t* __restrict__ pk, uint32_t mp,
+                                                      const uint32_t* __restrict__ bits, uint32_t bmask, int fk,
+                                                      int off0, int noffs, uint2* __restrict__ hits, uint32_t cap,
+                                                      unsigned long long* __restrict__ used,
+                                                      uint32_t* __restrict__ em, uint32_t* __restrict__ ub) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    const int w = blockIdx.y;
+    const uint32_t s = j < ms ? suf[j] : 0;
+    uint32_t maybe = 0;
+    if (j < ms) {
+#pragma unroll
+        for (int b = 0; b < 32; ++b) {
+            if (w * 32 + b < noffs) {
+                const uint32_t h = uint32_t(acc.fhash(s, off0 + w * 32 + b, fk)) & bmask;
+                maybe |= ((bits[h >> 5] >> (h & 31)) & 1u) << b;
+            }
+        }
+    }
+    const uint32_t lane = threadIdx.x & 31u, want = __popc(maybe);
+    uint32_t incl = want;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+        if (lane >= uint32_t(d)) incl += v;
+    }
+    unsigned long long base = 0;
+    if (lane == 31 && incl) base = atomicAdd(used, static_cast<unsigned long long>(incl));
+    base = __shfl_sync(0xFFFFFFFFu, base, 31) + (incl - want);
+    if (j >= ms) return;
+    uint32_t exact = 0, n = 0;
+    if (base + want <= cap) {
+        while (maybe) {
+            const int b = __ffs(maybe) - 1;
+            maybe &= maybe - 1;
+            uint32_t lo, hi;
+            if (fm_run(acc, pre, pk, mp, s, off0 + w * 32 + b, lo, hi)) {
+                hits[base + n++] = make_uint2(lo, hi);
+                exact |= 1u << b;
+            }
+        }
+    }
+    em[uint64_t(w) * ms + j] = exact;
+    ub[uint64_t(w) * ms + j] = uint32_t(base);
+}
+
+// Meetings per offset and warp of 32 suffixes: count[o * nw + warp].
+__global__ void __launch_bounds__(256) fm_count_kernel(const uint32_t* __restrict__ em, uint32_t ms, uint32_t nw,
+                                                       uint32_t* __restrict__ count) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x, warp = j >> 5, lane = threadIdx.x & 31u;
+    const uint32_t m = j < ms ? em[uint64_t(blockIdx.y) * ms + j] : 0;
+    uint32_t mine = 0;
+#pragma unroll
+    for (int b = 0; b < 32; ++b) {
+        const uint32_t bal = __ballot_sync(0xFFFFFFFFu, (m >> b) & 1u);
+        if (lane == uint32_t(b)) mine = __popc(bal);
+    }
+    if (warp < nw) count[(uint64_t(blockIdx.y) * 32 + lane) * nw + warp] = mine;
+}
+
+// Meetings in order of (offset, suffix): first = the exclusive scan of the
+// counts.
+__global__ void __launch_bounds__(256) fm_place_kernel(const uint32_t* __restrict__ suf, uint32_t ms, uint32_t nw,
+                                                       const uint32_t* __restrict__ pre,
+                                                       const uint2* __restrict__ hits,
+                                                       const uint32_t* __restrict__ em,
+                                                       const uint32_t* __restrict__ ub,
+                                                       const uint32_t* __restrict__ first, FmItem* __restrict__ item) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x, warp = j >> 5, lane = threadIdx.x & 31u;
+    const bool on = j < ms;
+    const uint32_t m = on ? em[uint64_t(blockIdx.y) * ms + j] : 0;
+    const uint32_t s = on ? suf[j] : 0;
+    uint32_t u = on ? ub[uint64_t(blockIdx.y) * ms + j] : 0;
+    if (!__any_sync(0xFFFFFFFFu, m != 0)) return;
+    const uint32_t at = first[(uint64_t(blockIdx.y) * 32 + lane) * nw + warp];  // of offset `lane` of this word
+    const uint32_t lt = (1u << lane) - 1u;
+    for (int b = 0; b < 32; ++b) {
+        const uint32_t bal = __ballot_sync(0xFFFFFFFFu, (m >> b) & 1u);
+        const uint32_t base = __shfl_sync(0xFFFFFFFFu, at, b);
+        if ((m >> b) & 1u) {
+            const uint2 h = hits[u++];
+            item[base + __popc(bal & lt)] = FmItem{s, h.x, h.y, pre[h.x]};
+        }
+    }
+}
+
+__device__ __forceinline__ uint32_t ld_l2(const uint32_t* p) { return __ldcg(p); }
+
+// The suffixes of one run (items [i, e) with the same lo, in order) each take
+// the first free prefix that is not themselves, as the reference's merge of
+// the run does (its rotation puts a prefix that meets itself back in front).
+// One thread.
+__device__ __forceinline__ void fm_walk(const FmItem* __restrict__ item, uint32_t i, uint32_t e,
+                                        const uint32_t* __restrict__ pre, uint32_t q0, uint32_t hi, int off,
+                                        uint32_t* next, uint32_t* prev, uint16_t* offset) {
+    const uint32_t lo = item[i].lo;
+    for (; i < e && item[i].lo == lo; ++i) {
+        const uint32_t s = item[i].s;
+        if (ld_l2(next + s) != INVALID) continue;
+        bool any = false;  // a free prefix was left
+        for (uint32_t q = q0; q < hi; ++q) {
+            const uint32_t p = pre[q];
+            if (ld_l2(prev + p) != INVALID) {
+                if (!any) q0 = q + 1;
+                continue;
+            }
+            any = true;
+            if (p == s) continue;
+            next[s] = p;
+            prev[p] = s;
+            offset[s] = uint16_t(off);
+            break;
+        }
+        if (!any) return;
+    }
+}
+
+// The same by a whole warp, for long runs: free suffixes and free prefixes
+// are taken 32 at a time and paired in order; where a read would meet itself
+// the rest of the run is walked by one lane.
+__device__ void fm_walk_warp(const FmItem* __restrict__ item, uint32_t i, uint32_t e, const uint32_t* __restrict__ pre,
+                             uint32_t q, uint32_t hi, int off, uint32_t* next, uint32_t* prev, uint16_t* offset) {
+    const uint32_t lane = threadIdx.x & 31u;
+    const uint32_t lo = item[i].lo;
+    uint32_t sm = 0, pm = 0;          // free entries of the current 32 items / prefixes
+    uint32_t ib = i, qb = q;          // where the next 32 start
+    uint32_t s = 0, p = 0;            // this lane's entries
+    bool more_s = true;
+    for (;;) {
+        while (sm == 0) {
+            if (!more_s) return;
+            const uint32_t t = ib + lane;
+            const bool in = t < e && item[t].lo == lo;
+            const uint32_t all = __ballot_sync(0xFFFFFFFFu, in);
+            s = in ? item[t].s : 0;
+            sm = __ballot_sync(0xFFFFFFFFu, in && ld_l2(next + s) == INVALID);
+            ib += 32;
+            more_s = all == 0xFFFFFFFFu;
+        }
+        while (pm == 0) {
+            if (qb >= hi) return;
+            const uint32_t t = qb + lane;
+            const bool in = t < hi;
+            p = in ? pre[t] : 0;
+            pm = __ballot_sync(0xFFFFFFFFu, in && ld_l2(prev + p) == INVALID);
+            qb += 32;
+        }
+        const int n = min(__popc(sm), __popc(pm));
+        // lane k < n pairs the k-th free suffix with the k-th free prefix
+        const int ks = int(lane) < n ? int(__fns(sm, 0, int(lane) + 1)) : 0;
+        const int kp = int(lane) < n ? int(__fns(pm, 0, int(lane) + 1)) : 0;
+        const uint32_t S = __shfl_sync(0xFFFFFFFFu, s, ks), P = __shfl_sync(0xFFFFFFFFu, p, kp);
+        const uint32_t self = __ballot_sync(0xFFFFFFFFu, int(lane) < n && S == P);
+        const int good = self ? __ffs(self) - 1 : n;
+        if (int(lane) < good) {
+            next[S] = P;
+            prev[P] = S;
+            offset[S] = uint16_t(off);
+        }
+        __syncwarp();
+        if (self) {
+            if (lane == 0) fm_walk(item, ib - 32, e, pre, qb - 32, hi, off, next, prev, offset);
+            __syncwarp();
+            return;
+        }
+        for (int k = 0; k < n; ++k) {  // the n lowest of each are used up
+            sm &= sm - 1;
+            pm &= pm - 1;
+        }
+    }
+}
+
+constexpr int FM_WALK_THREADS = 512;
+constexpr int FM_MAX_OFFS = 512;
+
+// The walk: offset after offset, one thread per run of equal suffix strings
+// (long runs: a warp).  Runs of one offset share no read, so an offset's runs
+// are independent; a barrier over the cluster separates the offsets.  One
+// cluster suffices: an offset has few meetings (thousands at most where a
+// list has 400,000 entries), and its time is the latency of two dependent
+// loads and the barrier.
+__global__ void __launch_bounds__(FM_WALK_THREADS) fm_walk_kernel(const FmItem* __restrict__ item,
+                                                                  const uint32_t* __restrict__ first, uint32_t nw,
+                                                                  const uint32_t* __restrict__ total, int off0,
+                                                                  int noffs, const uint32_t* __restrict__ pre,
+                                                                  const unsigned long long* __restrict__ used,
+                                                                  uint32_t cap, uint32_t* next, uint32_t* prev,
+                                                                  uint16_t* offset,
+                                                                  unsigned long long* __restrict__ tally) {
+    __shared__ uint32_t start[FM_MAX_OFFS + 1];
+    if (*used > cap) return;  // the listing is incomplete: the caller repeats it
+    for (int o = threadIdx.x; o <= noffs; o += FM_WALK_THREADS)
+        start[o] = o < noffs ? first[uint64_t(o) * nw] : *total;
+    __syncthreads();
+    const uint32_t threads = gridDim.x * FM_WALK_THREADS, me = blockIdx.x * FM_WALK_THREADS + threadIdx.x;
+    if (tally && me == 0) {
+        tally[0] += uint32_t(noffs);
+        tally[1] += start[noffs];
+        tally[2] += start[noffs];
+    }
+    for (int o = 0; o < noffs; ++o) {
+        const uint32_t a = start[o], e = start[o + 1];
+        if (a == e) continue;
+        const int off = off0 + o;
+        for (uint32_t i0 = a; i0 < e; i0 += threads) {  // the same trip count for a whole warp
+            const uint32_t i = i0 + me;
+            bool long_run = false;
+            FmItem it = {0, 0, 0, 0};
+            if (i < e) {
+                it = item[i];
+                const bool lead = i == a || item[i - 1].lo != it.lo;
+                const bool alone = i + 1 == e || item[i + 1].lo != it.lo;
+                if (lead) {
+                    if (alone && it.hi == it.lo + 1) {
+                        if (it.p != it.s) {
+                            const uint32_t nx = ld_l2(next + it.s), pv = ld_l2(prev + it.p);
+                            if (nx == INVALID && pv == INVALID) {
+                                next[it.s] = it.p;
+                                prev[it.p] = it.s;
+                                offset[it.s] = uint16_t(off);
+                            }
+                        }
+                    } else {
+                        // more than a few members or prefixes: by the whole warp
+                        long_run = it.hi - it.lo > 8 || (i + 8 < e && item[i + 8].lo == it.lo);
+                        if (!long_run) fm_walk(item, i, e, pre, it.lo, it.hi, off, next, prev, offset);
+                    }
+                }
+            }
+            uint32_t todo = __ballot_sync(0xFFFFFFFFu, long_run);
+            while (todo) {
+                const int l = __ffs(todo) - 1;
+                todo &= todo - 1;
+                const uint32_t ii = __shfl_sync(0xFFFFFFFFu, i, l), lo = __shfl_sync(0xFFFFFFFFu, it.lo, l),
+                               hi = __shfl_sync(0xFFFFFFFFu, it.hi, l);
+                fm_walk_warp(item, ii, e, pre, lo, hi, off, next, prev, offset);
+            }
+        }
+        if (gridDim.x > 1) {
+            asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        } else {
+            __syncthreads();
+        }
+    }
+}
+
+// Every offset from off0 on of two short lists, by one block: keys, runs and
+// link states in shared memory, two barriers per offset.  suf in the order
+// of the reversed reads when `ordered`, else it is ordered here (each thread
+// ranks its suffix against all).
+constexpr uint32_t FM_SMALL = 1024;
+template <class Acc>
+__global__ void __launch_bounds__(FM_SMALL) fm_small_kernel(Acc acc, const uint32_t* __restrict__ pre_in,
+                                                            const uint32_t* __restrict__ suf_in, uint32_t n, int off0,
+                                                            bool ordered, uint32_t* next, uint32_t* prev,
+                                                            uint16_t* offset, unsigned long long* __restrict__ tally) {
+    __shared__ uint64_t pk[FM_SMALL], rk[FM_SMALL];
+    __shared__ uint32_t pre[FM_SMALL], suf[FM_SMALL], run[FM_SMALL];
+    __shared__ uint8_t sdone[FM_SMALL], pdone[FM_SMALL];
+    __shared__ uint32_t s_left;
+    const uint32_t t = threadIdx.x;
+    if (t == 0) s_left = n;
+    uint32_t me = 0;
+    if (t < n) {
+        pre[t] = pre_in[t];
+        pk[t] = acc.key(pre[t], 0);
+        me = suf_in[t];
+        suf[t] = me;
+        rk[t] = acc.rword(me, 0);
+        sdone[t] = pdone[t] = 0;
+    }
+    __syncthreads();
+    if (!ordered) {
+        uint32_t rank = 0;
+        if (t < n) {
+            const uint64_t mine = rk[t];
+            const int nw = acc.rwords();
+            for (uint32_t j = 0; j < n; ++j) {
+                const uint64_t o = rk[j];
+                bool before = o < mine;
+                if (o == mine && j != t) {
+                    int k = 1;
+                    uint64_t x = 0, y = 0;
+                    for (; k < nw; ++k) {
+                        x = acc.rword(suf[j], k);
+                        y = acc.rword(me, k);
+                        if (x != y) break;
+                    }
+                    before = k < nw ? x < y : j < t;
+                }
+                rank += before;
+            }
+        }
+        __syncthreads();
+        if (t < n) suf[rank] = me;
+        __syncthreads();
+        if (t < n) me = suf[t];
+    }
+    int passes = 0;
+    for (int off = off0; off < acc.L; ++off) {
+        ++passes;
+        uint32_t lo = INVALID;
+        if (t < n) {
+            // (the upper end of the run is found as it is walked)
+            const int len = acc.L - off;
+            const uint64_t k = acc.key(me, off);
+            uint32_t b = 0, c = n;
+            int at = 1;
+            while (c > 0) {
+                const uint32_t step = c / 2, it = b + step;
+                const int r = cmp_keyed(acc, pk[it], pre[it], 0, k, me, off, len);
+                if (r < 0) {
+                    b = it + 1;
+                    c -= step + 1;
+                } else {
+                    c = step;
+                    at = r;
+                }
+            }
+            if (b < n && at == 0) lo = b;
+            run[t] = lo;
+        }
+        if (!__syncthreads_or(lo != INVALID)) continue;
+        if (t < n && lo != INVALID && (t == 0 || run[t - 1] != lo)) {
+            const int len = acc.L - off;
+            const uint64_t k = acc.key(me, off);
+            uint32_t q0 = lo;
+            bool left = true;
+            for (uint32_t i = t; left && i < n && run[i] == lo; ++i) {
+                if (sdone[i]) continue;
+                const uint32_t S = suf[i];
+                left = false;
+                for (uint32_t q = q0; q < n; ++q) {
+                    if (q > lo && cmp_keyed(acc, pk[q], pre[q], 0, k, me, off, len) != 0) break;
+                    if (pdone[q]) {
+                        if (!left) q0 = q + 1;
+                        continue;
+                    }
+                    left = true;
+                    const uint32_t P = pre[q];
+                    if (P == S) continue;
+                    next[S] = P;
+                    prev[P] = S;
+                    offset[S] = uint16_t(off);
+                    sdone[i] = pdone[q] = 1;
+                    atomicSub(&s_left, 1u);
+                    break;
+                }
+            }
+        }
+        __syncthreads();
+        if (s_left == 0) break;
+    }
+    if (tally && t == 0) {
+        tally[0] += uint32_t(passes);
+        tally[1] += uint64_t(passes) * n;
+        tally[2] += uint64_t(passes) * n;
+    }
+}
+
+// Reversed reads of a list as rows for the read sort, with their positions.
+__global__ void fm_reversed_kernel(PackedAcc acc, const uint32_t* __restrict__ suf, uint32_t m,
+                                   uint64_t* __restrict__ rows, uint32_t* __restrict__ idx) {
+    const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t >= uint64_t(m) * acc.W) return;
+    const uint32_t i = uint32_t(t / acc.W), w = uint32_t(t - uint64_t(i) * acc.W);
+    rows[t] = acc.rword(suf[i], int(w));
+    if (w == 0) idx[i] = i;
+}
+__global__ void fm_reversed_ascii_kernel(AsciiAcc acc, const uint32_t* __restrict__ suf, uint32_t m,
+                                         uint8_t* __restrict__ rows, uint32_t* __restrict__ idx) {
+    const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t >= uint64_t(m) * acc.L) return;
+    const uint32_t i = uint32_t(t / acc.L), b = uint32_t(t - uint64_t(i) * acc.L);
+    rows[t] = acc.r[uint64_t(suf[i]) * acc.L + acc.L - 1 - b];
+    if (b == 0) idx[i] = i;
+}
+__global__ void fm_permute_kernel(const uint32_t* __restrict__ suf, const uint32_t* __restrict__ idx, uint32_t m,
+                                  uint32_t* __restrict__ out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < m) out[i] = suf[idx[i]];
+}
+
+// out = suf in the order of the reversed reads (ties in list order).
+void fm_reverse_order(const PackedAcc& acc, const uint32_t* suf, uint32_t m, uint32_t* out, Arena& a, cudaStream_t s) {
+    auto mk = a.mark();
+    uint64_t* rows = a.alloc<uint64_t>(size_t(m) * acc.W);
+    uint32_t* idx = a.alloc<uint32_t>(m);
+    fm_reversed_kernel<<<grid_for(uint64_t(m) * acc.W, 256), 256, 0, s>>>(acc, suf, m, rows, idx);
+    CURC_LAUNCH_CHECK();
+    sort_ids_by_reads(rows, acc.W, acc.L, idx, m, a, s);
+    fm_permute_kernel<<<grid_for(m, 256), 256, 0, s>>>(suf, idx, m, out);
+    CURC_LAUNCH_CHECK();
+    a.release(mk);
+}
+void fm_reverse_order(const AsciiAcc& acc, const uint32_t* suf, uint32_t m, uint32_t* out, Arena& a, cudaStream_t s) {
+    auto mk = a.mark();
+    uint8_t* rows = a.alloc<uint8_t>(size_t(m) * acc.L);
+    uint32_t* idx = a.alloc<uint32_t>(m);
+    fm_reversed_ascii_kernel<<<grid_for(uint64_t(m) * acc.L, 256), 256, 0, s>>>(acc, suf, m, rows, idx);
+    CURC_LAUNCH_CHECK();
+    sort_ids_by_ascii(rows, acc.L, idx, m, a, s);
+    fm_permute_kernel<<<grid_for(m, 256), 256, 0, s>>>(suf, idx, m, out);
+    CURC_LAUNCH_CHECK();
+    a.release(mk);
+}
+
+// The lowest string length of the next stage, whose highest is hi: long
+// strings (16 and more) are met rarely and are all listed at once; below, a
+// random list of m entries meets almost every string of ceil(log4 m) symbols,
+// so a stage stops where its runs would hold 32 entries on average and the
+// lists are compacted before the next one.
+int fm_stage_low(int hi, uint32_t m) {
+    int base = 1;
+    while (base < 16 && (uint64_t(32) << (2 * base)) < m) ++base;
+    return std::min(hi, hi > 16 ? std::max(16, base) : base);
+}
+
+// What bounds the match is the serial chain of offsets, not bytes: as a
+// conditional graph of ten small launches an offset cost 33 us whatever the
+// lists held.  Listed at once, the offsets share a handful of launches, and
+// the walk costs a barrier and two dependent loads per offset that has a
+// meeting.  Measured on B200, the full match of the pseudogenome: 2,000 reads
+// of 100 bp (113 ends) 3.3 -> 0.19 ms, 8M reads of 250 bp (371,000 ends)
+// 18.5 -> 3.7 ms, 10M pairs of 150 bp (436,000 ends) 10.5 -> 3.5 ms.  Lists
+// of up to FM_SMALL ends take the one-block form: below that the launches of
+// a stage (12, and a read back) cost more than the block's two barriers per
+// offset.
+template <class Acc>
+void full_match_events(const Acc& acc, uint32_t* pre, uint32_t* suf, uint32_t cnt, uint32_t* next, uint32_t* prev,
+                       uint16_t* offset, unsigned long long* tally, Arena& a, cudaStream_t s) {
+    auto small = [&](const uint32_t* pl, const uint32_t* sl, uint32_t n, int off, bool ordered) {
+        const uint32_t threads = std::max(64u, uint32_t(div_up(n, 32)) * 32);
+        fm_small_kernel<Acc><<<1, threads, 0, s>>>(acc, pl, sl, n, off, ordered, next, prev, offset, tally);
+        CURC_LAUNCH_CHECK();
+    };
+    if (cnt <= FM_SMALL) {
+        small(pre, suf, cnt, 1, false);
+        return;
+    }
+    auto mk = a.mark();
+    uint32_t* suf_o = a.alloc<uint32_t>(cnt);
+    fm_reverse_order(acc, suf, cnt, suf_o, a, s);
+    uint32_t* pl = pre;
+    uint32_t* sl = suf_o;
+    uint32_t* pl2 = a.alloc<uint32_t>(cnt);
+    uint32_t* sl2 = suf;
+    uint64_t* pk = a.alloc<uint64_t>(cnt);
+    // room for the runs of one stage's meetings, and false ones
+    const uint32_t cap = uint32_t(std::min<uint64_t>(0xF0000000ull, std::max<uint64_t>(uint64_t(4) << 20, uint64_t(cnt) * 6)));
+    uint2* hits = a.alloc<uint2>(cap);
+    FmItem* item = a.alloc<FmItem>(cap);
+    struct State {
+        unsigned long long used;
+        uint32_t total, len_in, len_out[2];
+    };
+    State* st = a.alloc<State>(1);
+    Compactor cp(cnt, a, s);
+    uint32_t m = cnt;
+    int hi = acc.L - 1;
+    int fewer = acc.L;  // at most this many offsets per stage (lowered when a listing ran out of room)
+    while (hi >= 1 && m > FM_SMALL) {
+        auto mk2 = a.mark();
+        const int low = std::max(fm_stage_low(hi, m), hi - std::min(fewer, FM_MAX_OFFS) + 1);
+        const int noffs = hi - low + 1, off0 = acc.L - hi, words = (noffs + 31) / 32;
+        const int fk = std::min(low, int(Acc::FK_MAX));
+        // presence bitmap of the prefixes' first fk symbols: 32 bits per
+        // prefix, so that 3% of the strings that meet none pass
+        int bbits = 15;
+        while (bbits < 32 && (1ull << bbits) < uint64_t(m) * 32) ++bbits;
+        uint32_t* bits = a.alloc<uint32_t>((1ull << bbits) / 32);
+        const uint32_t bmask = uint32_t((1ull << bbits) - 1);
+        const uint32_t nw = uint32_t(div_up(m, 32));
+        uint32_t* em = a.alloc<uint32_t>(size_t(words) * m);
+        uint32_t* ub = a.alloc<uint32_t>(size_t(words) * m);
+        uint32_t* count = a.alloc<uint32_t>(size_t(words) * 32 * nw);
+        CURC_CHECK(cudaMemsetAsync(bits, 0, (1ull << bbits) / 8, s));
+        const State init{0, 0, m, {0, 0}};
+        CURC_CHECK(cudaMemcpyAsync(st, &init, sizeof(init), cudaMemcpyHostToDevice, s));
+        fm_prefix_kernel<Acc><<<grid_for(m, 256), 256, 0, s>>>(acc, pl, m, pk, fk, bits, bmask);
+        CURC_LAUNCH_CHECK();
+        const dim3 grid(unsigned(div_up(m, 256)), unsigned(words));
+        fm_meet_kernel<Acc><<<grid, 256, 0, s>>>(acc, sl, m, pl, pk, m, bits, bmask, fk, off0, noffs, hits, cap,
+                                                  &st->used, em, ub);
+        CURC_LAUNCH_CHECK();
+        fm_count_kernel<<<grid, 256, 0, s>>>(em, m, nw, count);
+        CURC_LAUNCH_CHECK();
+        exclusive_scan<uint32_t>(count, count, size_t(words) * 32 * nw, &st->total, a, s);
+        fm_place_kernel<<<grid, 256, 0, s>>>(sl, m, nw, pl, hits, em, ub, count, item);
+        CURC_LAUNCH_CHECK();
+        {
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute at;
+            at.id = cudaLaunchAttributeClusterDimension;
+            // short lists meet a few hundred at a time: one block, whose
+            // barrier is cheaper than the cluster's
+            const unsigned blocks = m > 16384 ? 8 : 1;
+            at.val.clusterDim = {blocks, 1, 1};
+            cfg.gridDim = dim3(blocks);
+            cfg.blockDim = dim3(FM_WALK_THREADS);
+            cfg.stream = s;
+            cfg.attrs = &at;
+            cfg.numAttrs = 1;
+            const uint32_t* first = count;
+            const uint32_t* total = &st->total;
+            const uint32_t* plc = pl;
+            const unsigned long long* used = &st->used;
+            const FmItem* items = item;
+            CURC_CHECK(cudaLaunchKernelEx(&cfg, fm_walk_kernel, items, first, nw, total, off0, noffs, plc, used, cap,
+                                          next, prev, offset, tally));
+            CURC_LAUNCH_CHECK();
+        }
+        cp.run(&st->len_in, m, &st->len_out[0], FreeLink{pl, prev}, MoveId{pl, pl2});
+        cp.run(&st->len_in, m, &st->len_out[1], FreeLink{sl, next}, MoveId{sl, sl2});
+        State h;
+        read_small(&h, st, sizeof(h), s);
+        a.release(mk2);
+        if (h.used > cap) {
+            fewer = std::max(1, noffs / 2);
+            continue;  // nothing was linked; the lists are as they were
+        }
+        std::swap(pl, pl2);
+        std::swap(sl, sl2);
+        m = h.len_out[0];
+        hi = low - 1;
+    }
+    cp.check();
+    if (hi >= 1 && m > 0) small(pl, sl, m, acc.L - hi, true);
+    a.release(mk);
+}
+
+// nothing to link without ends
+template <class Acc>
+void full_match_loop(const Acc& acc, uint32_t* pre, uint32_t* suf, uint32_t cnt, uint32_t* next, uint32_t* prev,
+                     uint16_t* offset, bool passes, unsigned long long* tally, Arena& a, cudaStream_t s) {
+    if (cnt == 0 || acc.L < 2) return;
+    if (passes)
+        full_match_passes(acc, pre, suf, cnt, next, prev, offset, tally, a, s);
+    else
+        full_match_events(acc, pre, suf, cnt, next, prev, offset, tally, a, s);
+}
+
+// *other = 1 when a listed read holds a byte other than A, C, G, N and T.
+__global__ void other_symbols_kernel(const uint8_t* __restrict__ r, int L, const uint32_t* __restrict__ ids,
+                                     uint32_t m, uint32_t* __restrict__ other) {
+    for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < uint64_t(m) * L;
+         t += uint64_t(gridDim.x) * blockDim.x) {
+        const uint32_t i = uint32_t(t / L), b = uint32_t(t - uint64_t(i) * L);
+        const uint8_t c = r[uint64_t(ids[i]) * L + b];
+        if (c != 'A' && c != 'C' && c != 'G' && c != 'N' && c != 'T') *other = 1;
+    }
 }
 
 __global__ void ascii_chunk_kernel(const uint8_t* __restrict__ r, int L, const uint32_t* __restrict__ ids, uint32_t m,
@@ -842,7 +1142,7 @@ __global__ void ends_flags_kernel(const uint32_t* __restrict__ ids, uint32_t m, 
 void full_match_packed(const BlockParams& p, const uint64_t* db, uint32_t* pre, uint32_t* suf, uint32_t cnt,
                        uint32_t* next, uint32_t* prev, uint16_t* offset, Arena& a, cudaStream_t s,
                        unsigned long long* tally) {
-    full_match_loop(PackedAcc{db, p.W, p.L}, pre, suf, cnt, next, prev, offset, p.tune.fm_loop, tally, a, s);
+    full_match_loop(PackedAcc{db, p.W, p.L}, pre, suf, cnt, next, prev, offset, p.tune.fm_loop == 0, tally, a, s);
 }
 
 void sort_ids_by_ascii(const uint8_t* reads, int L, uint32_t* ids, uint32_t m, Arena& a, cudaStream_t s) {
@@ -879,11 +1179,17 @@ void full_match_ascii(const BlockParams& p, const uint8_t* reads, uint32_t* ids,
     CURC_LAUNCH_CHECK();
     uint32_t* pre = a.alloc<uint32_t>(m);
     uint32_t* suf = a.alloc<uint32_t>(m);
-    uint32_t* counts = a.alloc<uint32_t>(2);
+    uint32_t* counts = a.alloc<uint32_t>(3);  // ends of each kind, other symbols seen
+    CURC_CHECK(cudaMemsetAsync(counts + 2, 0, 4, s));
+    other_symbols_kernel<<<resident_grid(other_symbols_kernel, 256, uint64_t(m) * p.L), 256, 0, s>>>(reads, p.L, ids, m,
+                                                                                                  counts + 2);
+    CURC_LAUNCH_CHECK();
     select_flagged(ids, pf, pre, m, counts + 0, a, s);
     select_flagged(ids, sf, suf, m, counts + 1, a, s);
-    const uint32_t cnt = read_scalar(counts + 0, s);
-    full_match_loop(AsciiAcc{reads, 0, p.L}, pre, suf, cnt, next, prev, offset, p.tune.fm_loop, nullptr, a, s);
+    uint32_t h[3];
+    read_small(h, counts, 12, s);
+    full_match_loop(AsciiAcc{reads, 0, p.L}, pre, suf, h[0], next, prev, offset, p.tune.fm_loop == 0 || h[2] != 0,
+                    nullptr, a, s);
     a.release(mk);
 }
 

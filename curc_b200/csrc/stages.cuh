@@ -20,7 +20,7 @@ std::string& ctxless_error();
 // threads per block of the mapping kernel (one warp per read).
 struct Tuning {
     int table_factor = 4, bitmap_bits = 16, check_every = 8, map_threads = 128;
-    int fm_loop = 1;  // full-match pass loop: 0 a launch per kernel, 1 one graph, 2 one persistent kernel
+    int fm_loop = 1;  // full match: 0 a pass of launches per offset, 1 and 2 meetings listed at once
 };
 
 // Autotuner cache key of a block: read length and read count rounded down
@@ -87,8 +87,8 @@ void chain_filter(uint32_t n, const uint32_t* sorted, uint32_t m, uint32_t* next
 
 // ---- a6/a7 (fullmatch.cu)
 // Packed reads: prefix/suffix lists are consumed (scratch).  tally (device,
-// 3 counters, optional): passes with both lists non-empty, and their summed
-// suffix and prefix list lengths.
+// 3 counters, optional): offsets passed, and the suffix and prefix list
+// entries examined there (in the listed form: the meetings).
 void full_match_packed(const BlockParams& p, const uint64_t* db, uint32_t* pre, uint32_t* suf, uint32_t cnt,
                        uint32_t* next, uint32_t* prev, uint16_t* offset, Arena& a, cudaStream_t s,
                        unsigned long long* tally = nullptr);
