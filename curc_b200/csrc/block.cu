@@ -191,8 +191,12 @@ void Block::run(const uint8_t* d_seq, uint64_t n_reads, int L, bool po, bool pe)
 
     emit(T);
     CURC_CHECK(cudaEventRecord(ev1, s));
+    // the one-pass kernels' error word comes with the streams
+    uint8_t* waits = pinned.alloc(sizeof(uint32_t));
+    CURC_CHECK(cudaMemcpyAsync(waits, arena.wait_error(), sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
     T.collect(stage_ms);
     CURC_CHECK(cudaStreamSynchronize(s));
+    arena.check_waits(waits, s);
     float total = 0;
     CURC_CHECK(cudaEventElapsedTime(&total, ev0, ev1));
     stage_ms["total"] = total;

@@ -828,11 +828,17 @@ __global__ void __launch_bounds__(FM_SMALL) fm_small_kernel(Acc acc, const uint3
         uint32_t rank = 0;
         if (t < n) {
             const uint64_t mine = rk[t];
-            const int nw = acc.rwords();
+            uint32_t equal = 0;
+#pragma unroll 8
             for (uint32_t j = 0; j < n; ++j) {
                 const uint64_t o = rk[j];
-                bool before = o < mine;
-                if (o == mine && j != t) {
+                rank += o < mine;
+                equal += o == mine;
+            }
+            if (equal > 1) {
+                const int nw = acc.rwords();
+                for (uint32_t j = 0; j < n; ++j) {
+                    if (rk[j] != mine || j == t) continue;
                     int k = 1;
                     uint64_t x = 0, y = 0;
                     for (; k < nw; ++k) {
@@ -840,9 +846,8 @@ __global__ void __launch_bounds__(FM_SMALL) fm_small_kernel(Acc acc, const uint3
                         y = acc.rword(me, k);
                         if (x != y) break;
                     }
-                    before = k < nw ? x < y : j < t;
+                    rank += k < nw ? x < y : j < t;
                 }
-                rank += before;
             }
         }
         __syncthreads();
@@ -913,21 +918,14 @@ __global__ void __launch_bounds__(FM_SMALL) fm_small_kernel(Acc acc, const uint3
 }
 
 // Reversed reads of a list as rows for the read sort, with their positions.
-__global__ void fm_reversed_kernel(PackedAcc acc, const uint32_t* __restrict__ suf, uint32_t m,
+template <class Acc>
+__global__ void fm_reversed_kernel(Acc acc, const uint32_t* __restrict__ suf, uint32_t m, int W,
                                    uint64_t* __restrict__ rows, uint32_t* __restrict__ idx) {
     const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= uint64_t(m) * acc.W) return;
-    const uint32_t i = uint32_t(t / acc.W), w = uint32_t(t - uint64_t(i) * acc.W);
+    if (t >= uint64_t(m) * W) return;
+    const uint32_t i = uint32_t(t / W), w = uint32_t(t - uint64_t(i) * W);
     rows[t] = acc.rword(suf[i], int(w));
     if (w == 0) idx[i] = i;
-}
-__global__ void fm_reversed_ascii_kernel(AsciiAcc acc, const uint32_t* __restrict__ suf, uint32_t m,
-                                         uint8_t* __restrict__ rows, uint32_t* __restrict__ idx) {
-    const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= uint64_t(m) * acc.L) return;
-    const uint32_t i = uint32_t(t / acc.L), b = uint32_t(t - uint64_t(i) * acc.L);
-    rows[t] = acc.r[uint64_t(suf[i]) * acc.L + acc.L - 1 - b];
-    if (b == 0) idx[i] = i;
 }
 __global__ void fm_permute_kernel(const uint32_t* __restrict__ suf, const uint32_t* __restrict__ idx, uint32_t m,
                                   uint32_t* __restrict__ out) {
@@ -936,24 +934,15 @@ __global__ void fm_permute_kernel(const uint32_t* __restrict__ suf, const uint32
 }
 
 // out = suf in the order of the reversed reads (ties in list order).
-void fm_reverse_order(const PackedAcc& acc, const uint32_t* suf, uint32_t m, uint32_t* out, Arena& a, cudaStream_t s) {
+template <class Acc>
+void fm_reverse_order(const Acc& acc, const uint32_t* suf, uint32_t m, uint32_t* out, Arena& a, cudaStream_t s) {
     auto mk = a.mark();
-    uint64_t* rows = a.alloc<uint64_t>(size_t(m) * acc.W);
+    const int W = int(div_up(uint64_t(acc.L), Acc::KS));
+    uint64_t* rows = a.alloc<uint64_t>(size_t(m) * W);
     uint32_t* idx = a.alloc<uint32_t>(m);
-    fm_reversed_kernel<<<grid_for(uint64_t(m) * acc.W, 256), 256, 0, s>>>(acc, suf, m, rows, idx);
+    fm_reversed_kernel<Acc><<<grid_for(uint64_t(m) * W, 256), 256, 0, s>>>(acc, suf, m, W, rows, idx);
     CURC_LAUNCH_CHECK();
-    sort_ids_by_reads(rows, acc.W, acc.L, idx, m, a, s);
-    fm_permute_kernel<<<grid_for(m, 256), 256, 0, s>>>(suf, idx, m, out);
-    CURC_LAUNCH_CHECK();
-    a.release(mk);
-}
-void fm_reverse_order(const AsciiAcc& acc, const uint32_t* suf, uint32_t m, uint32_t* out, Arena& a, cudaStream_t s) {
-    auto mk = a.mark();
-    uint8_t* rows = a.alloc<uint8_t>(size_t(m) * acc.L);
-    uint32_t* idx = a.alloc<uint32_t>(m);
-    fm_reversed_ascii_kernel<<<grid_for(uint64_t(m) * acc.L, 256), 256, 0, s>>>(acc, suf, m, rows, idx);
-    CURC_LAUNCH_CHECK();
-    sort_ids_by_ascii(rows, acc.L, idx, m, a, s);
+    sort_rows(rows, W, Acc::SB * (acc.L - Acc::KS * (W - 1)), idx, m, a, s);
     fm_permute_kernel<<<grid_for(m, 256), 256, 0, s>>>(suf, idx, m, out);
     CURC_LAUNCH_CHECK();
     a.release(mk);
@@ -1105,14 +1094,18 @@ __global__ void other_symbols_kernel(const uint8_t* __restrict__ r, int L, const
     }
 }
 
-__global__ void ascii_chunk_kernel(const uint8_t* __restrict__ r, int L, const uint32_t* __restrict__ ids, uint32_t m,
-                                   int chunk, uint64_t* __restrict__ key) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m) return;
-    const uint8_t* p = r + uint64_t(ids[i]) * L + chunk * 8;
+// ASCII reads as rows of big-endian words, zero padded (word order is
+// memcmp order).
+__global__ void ascii_rows_kernel(const uint8_t* __restrict__ r, int L, const uint32_t* __restrict__ ids, uint32_t m,
+                                  int W, uint64_t* __restrict__ rows, uint32_t* __restrict__ idx) {
+    const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t >= uint64_t(m) * W) return;
+    const uint32_t i = uint32_t(t / W), w = uint32_t(t - uint64_t(i) * W);
+    const uint8_t* p = r + uint64_t(ids[i]) * L + w * 8;
     uint64_t v = 0;
-    for (int b = 0; b < 8; ++b) v = (v << 8) | (chunk * 8 + b < L ? p[b] : 0);
-    key[i] = v;
+    for (int b = 0; b < 8; ++b) v = (v << 8) | (int(w * 8) + b < L ? p[b] : 0);
+    rows[t] = v;
+    if (w == 0) idx[i] = i;
 }
 
 __global__ void ascii_dedupe_kernel(const uint8_t* __restrict__ r, int L, const uint32_t* __restrict__ ids, uint32_t m,
@@ -1146,17 +1139,19 @@ void full_match_packed(const BlockParams& p, const uint64_t* db, uint32_t* pre, 
 }
 
 void sort_ids_by_ascii(const uint8_t* reads, int L, uint32_t* ids, uint32_t m, Arena& a, cudaStream_t s) {
-    // stable lexicographic (memcmp) order: LSD over 8-byte big-endian chunks
+    // stable lexicographic (memcmp) order
     if (m <= 1) return;
     auto mk = a.mark();
-    uint64_t* key = a.alloc<uint64_t>(m);
-    const int chunks = (L + 7) / 8;
-    for (int c = chunks - 1; c >= 0; --c) {
-        ascii_chunk_kernel<<<grid_for(m, 256), 256, 0, s>>>(reads, L, ids, m, c, key);
-        CURC_LAUNCH_CHECK();
-        const int lo = (c == chunks - 1) ? 8 * (8 * chunks - L) : 0;
-        radix_sort_pairs<uint64_t, uint32_t>(key, ids, m, lo, 64, a, s);
-    }
+    const int W = (L + 7) / 8;
+    uint64_t* rows = a.alloc<uint64_t>(size_t(m) * W);
+    uint32_t* idx = a.alloc<uint32_t>(m);
+    uint32_t* in = a.alloc<uint32_t>(m);
+    CURC_CHECK(cudaMemcpyAsync(in, ids, size_t(m) * 4, cudaMemcpyDeviceToDevice, s));
+    ascii_rows_kernel<<<grid_for(uint64_t(m) * W, 256), 256, 0, s>>>(reads, L, ids, m, W, rows, idx);
+    CURC_LAUNCH_CHECK();
+    sort_rows(rows, W, 8 * (L - 8 * (W - 1)), idx, m, a, s);
+    fm_permute_kernel<<<grid_for(m, 256), 256, 0, s>>>(in, idx, m, ids);
+    CURC_LAUNCH_CHECK();
     a.release(mk);
 }
 

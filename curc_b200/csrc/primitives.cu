@@ -22,6 +22,23 @@ uint64_t launches() { return g_launches.load(); }
 
 Arena::~Arena() {
     for (auto& c : chunks_) cudaFree(c.base);
+    if (wait_error_) cudaFree(wait_error_);
+}
+
+uint32_t* Arena::wait_error() {
+    if (!wait_error_) {
+        CURC_CHECK(cudaMalloc(&wait_error_, sizeof(uint32_t)));
+        CURC_CHECK(cudaMemset(wait_error_, 0, sizeof(uint32_t)));
+    }
+    return wait_error_;
+}
+
+void Arena::check_waits(const void* copy, cudaStream_t s) {
+    uint32_t e;
+    std::memcpy(&e, copy, sizeof(e));
+    if (!e) return;
+    CURC_CHECK(cudaMemsetAsync(wait_error(), 0, sizeof(uint32_t), s));
+    throw std::runtime_error("a tile's bounded wait ran out");
 }
 
 void* Arena::alloc_bytes(size_t bytes) {
@@ -230,7 +247,7 @@ StageTimer*& active_timer() {
 // ---------------------------------------------------------------- scan
 
 namespace {
-constexpr int SCAN_THREADS = 256, SCAN_ITEMS = 8, SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
+constexpr int SCAN_THREADS = 256, SCAN_ITEMS = 16, SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
 template <class T>
 __device__ T block_exclusive_sum(T v, T* block_total) {
@@ -260,26 +277,67 @@ __device__ T block_exclusive_sum(T v, T* block_total) {
     return warp_prefix + x - v;
 }
 
-template <class T>
-__global__ void __launch_bounds__(SCAN_THREADS) scan_reduce_kernel(const T* __restrict__ in, size_t n,
-                                                                   T* __restrict__ sums) {
-    const size_t base = size_t(blockIdx.x) * SCAN_TILE;
-    T s = 0;
-#pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; ++i) {
-        size_t idx = base + size_t(i) * SCAN_THREADS + threadIdx.x;
-        if (idx < n) s += in[idx];
+// One-pass scans: tiles are taken in order from a counter, publish their
+// sum, and find the sum before them by looking back over the tiles before
+// (whose blocks have started, since the counter is in order).  A state is a
+// 62-bit value under two flag bits: 1, the tile's own sum; 2, the sum up to
+// and with the tile.  Waits are bounded: one that runs out sets *err, which
+// the block run checks before it returns results (Arena::check_waits).
+constexpr uint32_t LOOK_WAIT_LIMIT = 1u << 22;
+constexpr uint64_t LOOK_SUM = 1ull << 62, LOOK_INCL = 2ull << 62, LOOK_VALUE = LOOK_SUM - 1;
+
+__device__ __forceinline__ uint64_t look_wait(unsigned long long* st, uint32_t* err) {
+    uint64_t v;
+    uint32_t spins = 0;
+    for (;;) {
+        v = *reinterpret_cast<volatile unsigned long long*>(st);
+        if (v >> 62) return v;
+        if (++spins >= LOOK_WAIT_LIMIT) {
+            atomicExch(err, 1u);
+            return LOOK_INCL;  // void, and *err says so; no later tile waits on this one
+        }
+        __nanosleep(32);
     }
-    T total;
-    block_exclusive_sum(s, &total);
-    if (threadIdx.x == 0) sums[blockIdx.x] = total;
 }
 
+// Warp 0, all lanes: publishes the tile's sum and returns the sum of the
+// tiles before it (32 predecessors per step).
+__device__ __forceinline__ uint64_t look_back(unsigned long long* st, uint32_t tile, uint64_t sum, uint32_t* err) {
+    const uint32_t lane = threadIdx.x & 31u;
+    if (tile == 0) {
+        if (lane == 0) atomicExch(&st[0], LOOK_INCL | (sum & LOOK_VALUE));
+        return 0;
+    }
+    if (lane == 0) atomicExch(&st[tile], LOOK_SUM | (sum & LOOK_VALUE));
+    uint64_t before = 0;
+    for (int64_t top = int64_t(tile) - 1;; top -= 32) {
+        const int64_t j = top - int64_t(lane);
+        const uint64_t v = j >= 0 ? look_wait(&st[j], err) : LOOK_INCL;
+        __syncwarp();
+        // the nearest lane with an inclusive sum ends the search
+        const uint32_t inc = __ballot_sync(0xFFFFFFFFu, (v >> 62) == 2);
+        const int stop = inc ? __ffs(inc) - 1 : 32;
+        uint64_t add = int(lane) <= stop ? v & LOOK_VALUE : 0;
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) add += __shfl_xor_sync(0xFFFFFFFFu, add, d);
+        before += add;
+        if (inc) break;
+    }
+    if (lane == 0) atomicExch(&st[tile], LOOK_INCL | ((before + sum) & LOOK_VALUE));
+    return before;
+}
+
+// st: one state per tile and, behind them, the tile counter (all zero).
 template <class T>
-__global__ void __launch_bounds__(SCAN_THREADS) scan_apply_kernel(const T* in, T* out, size_t n,
-                                                                  const T* __restrict__ offsets, T* total) {
+__global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(const T* in, T* out, size_t n, T* total,
+                                                            unsigned long long* st, uint32_t tiles, uint32_t* err) {
     __shared__ T sm[SCAN_TILE];
-    const size_t base = size_t(blockIdx.x) * SCAN_TILE;
+    __shared__ uint32_t s_tile;
+    __shared__ uint64_t s_before;
+    if (threadIdx.x == 0) s_tile = tiles > 1 ? uint32_t(atomicAdd(&st[tiles], 1ull)) : 0;
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    const size_t base = size_t(tile) * SCAN_TILE;
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; ++i) {
         size_t idx = base + size_t(i) * SCAN_THREADS + threadIdx.x;
@@ -295,20 +353,34 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_apply_kernel(const T* in, T
     }
     T btotal;
     T run = block_exclusive_sum(tsum, &btotal);
-    if (offsets) run += offsets[blockIdx.x];
+    if (tiles > 1) {
+        if (threadIdx.x < 32) {
+            const uint64_t before = look_back(st, tile, uint64_t(btotal), err);
+            if (threadIdx.x == 0) s_before = before;
+        }
+        __syncthreads();
+        run += T(s_before);
+    }
+    if (total && tile + 1 == tiles && threadIdx.x == 0) *total = btotal + (tiles > 1 ? T(s_before) : T(0));
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; ++i) {
         T t = local[i];
         sm[threadIdx.x * SCAN_ITEMS + i] = run;
         run += t;
     }
-    if (total && gridDim.x == 1 && threadIdx.x == 0) *total = btotal;
     __syncthreads();
 #pragma unroll
     for (int i = 0; i < SCAN_ITEMS; ++i) {
         size_t idx = base + size_t(i) * SCAN_THREADS + threadIdx.x;
         if (idx < n) out[idx] = sm[i * SCAN_THREADS + threadIdx.x];
     }
+}
+
+// Zeroed tile states and counter of a one-pass kernel.
+unsigned long long* look_states(size_t tiles, Arena& a, cudaStream_t s) {
+    unsigned long long* st = a.alloc<unsigned long long>(tiles + 1);
+    CURC_CHECK(cudaMemsetAsync(st, 0, (tiles + 1) * sizeof(unsigned long long), s));
+    return st;
 }
 }  // namespace
 
@@ -319,17 +391,10 @@ void exclusive_scan(const T* in, T* out, size_t n, T* total, Arena& a, cudaStrea
         return;
     }
     const size_t tiles = div_up(n, SCAN_TILE);
-    if (tiles == 1) {
-        scan_apply_kernel<T><<<1, SCAN_THREADS, 0, s>>>(in, out, n, nullptr, total);
-        CURC_LAUNCH_CHECK();
-        return;
-    }
     auto m = a.mark();
-    T* sums = a.alloc<T>(tiles);
-    scan_reduce_kernel<T><<<unsigned(tiles), SCAN_THREADS, 0, s>>>(in, n, sums);
-    CURC_LAUNCH_CHECK();
-    exclusive_scan<T>(sums, sums, tiles, total, a, s);
-    scan_apply_kernel<T><<<unsigned(tiles), SCAN_THREADS, 0, s>>>(in, out, n, sums, nullptr);
+    unsigned long long* st = tiles > 1 ? look_states(tiles, a, s) : nullptr;
+    scan_kernel<T><<<unsigned(tiles), SCAN_THREADS, 0, s>>>(in, out, n, total, st, uint32_t(tiles),
+                                                            tiles > 1 ? a.wait_error() : nullptr);
     CURC_LAUNCH_CHECK();
     a.release(m);
 }
@@ -340,45 +405,49 @@ template void exclusive_scan<uint64_t>(const uint64_t*, uint64_t*, size_t, uint6
 // ---------------------------------------------------------------- compaction
 
 namespace {
-constexpr int SEL_THREADS = 256, SEL_ITEMS = 8, SEL_TILE = SEL_THREADS * SEL_ITEMS;
+constexpr int SEL_THREADS = 256, SEL_ITEMS = 16, SEL_TILE = SEL_THREADS * SEL_ITEMS;
+static_assert(SEL_THREADS == SCAN_THREADS, "block_exclusive_sum");
 
-__global__ void __launch_bounds__(SEL_THREADS) count_flags_kernel(const uint8_t* __restrict__ flags, size_t n,
-                                                                  uint32_t* __restrict__ counts) {
-    const size_t base = size_t(blockIdx.x) * SEL_TILE;
-    uint32_t c = 0;
-#pragma unroll
-    for (int i = 0; i < SEL_ITEMS; ++i) {
-        size_t idx = base + size_t(i) * SEL_THREADS + threadIdx.x;
-        if (idx < n) c += flags[idx] != 0;
-    }
-    uint32_t total;
-    block_exclusive_sum<uint32_t>(c, &total);
-    if (threadIdx.x == 0) counts[blockIdx.x] = total;
-}
-
+// One-pass stable compaction (tile states as in scan_kernel); thread t owns
+// the tile's items [16 t, 16 t + 16).
 template <class T, bool kIndices>
 __global__ void __launch_bounds__(SEL_THREADS) select_kernel(const T* __restrict__ in, const uint8_t* __restrict__ flags,
-                                                             size_t n, const uint32_t* __restrict__ offsets,
-                                                             T* __restrict__ out) {
-    // blocked arrangement: thread t owns tile items [t*ITEMS, (t+1)*ITEMS)
-    const size_t base = size_t(blockIdx.x) * SEL_TILE + size_t(threadIdx.x) * SEL_ITEMS;
-    uint8_t f[SEL_ITEMS];
-    uint32_t c = 0;
+                                                             size_t n, T* __restrict__ out, uint32_t* __restrict__ count,
+                                                             unsigned long long* st, uint32_t tiles, uint32_t* err) {
+    __shared__ uint32_t s_tile;
+    __shared__ uint64_t s_before;
+    if (threadIdx.x == 0) s_tile = tiles > 1 ? uint32_t(atomicAdd(&st[tiles], 1ull)) : 0;
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    const size_t base = size_t(tile) * SEL_TILE + size_t(threadIdx.x) * SEL_ITEMS;
+    uint32_t keep = 0;  // bit i: item base + i
+    if (base + SEL_ITEMS <= n && (reinterpret_cast<uintptr_t>(flags) & 15) == 0) {
+        const uint4 f = *reinterpret_cast<const uint4*>(flags + base);
+        const uint32_t w[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
-    for (int i = 0; i < SEL_ITEMS; ++i) {
-        size_t idx = base + i;
-        f[i] = idx < n ? flags[idx] != 0 : 0;
-        c += f[i];
+        for (int i = 0; i < SEL_ITEMS; ++i) keep |= uint32_t(((w[i / 4] >> (8 * (i % 4))) & 0xFFu) != 0) << i;
+    } else {
+#pragma unroll
+        for (int i = 0; i < SEL_ITEMS; ++i)
+            if (base + i < n && flags[base + i]) keep |= 1u << i;
     }
     uint32_t total;
-    uint32_t pos = block_exclusive_sum<uint32_t>(c, &total) + offsets[blockIdx.x];
-#pragma unroll
-    for (int i = 0; i < SEL_ITEMS; ++i) {
-        if (f[i]) {
-            if constexpr (kIndices) out[pos] = T(base + i);
-            else out[pos] = in[base + i];
-            ++pos;
+    uint64_t pos = block_exclusive_sum<uint32_t>(__popc(keep), &total);
+    if (tiles > 1) {
+        if (threadIdx.x < 32) {
+            const uint64_t before = look_back(st, tile, total, err);
+            if (threadIdx.x == 0) s_before = before;
         }
+        __syncthreads();
+        pos += s_before;
+    }
+    if (tile + 1 == tiles && threadIdx.x == 0) *count = total + (tiles > 1 ? uint32_t(s_before) : 0u);
+    while (keep) {
+        const int i = __ffs(keep) - 1;
+        keep &= keep - 1;
+        if constexpr (kIndices) out[pos] = T(base + i);
+        else out[pos] = in[base + i];
+        ++pos;
     }
 }
 
@@ -390,11 +459,9 @@ void select_impl(const T* in, const uint8_t* flags, T* out, size_t n, uint32_t* 
     }
     auto m = a.mark();
     const size_t tiles = div_up(n, SEL_TILE);
-    uint32_t* off = a.alloc<uint32_t>(tiles);
-    count_flags_kernel<<<unsigned(tiles), SEL_THREADS, 0, s>>>(flags, n, off);
-    CURC_LAUNCH_CHECK();
-    exclusive_scan<uint32_t>(off, off, tiles, count, a, s);
-    select_kernel<T, kIndices><<<unsigned(tiles), SEL_THREADS, 0, s>>>(in, flags, n, off, out);
+    unsigned long long* st = tiles > 1 ? look_states(tiles, a, s) : nullptr;
+    select_kernel<T, kIndices><<<unsigned(tiles), SEL_THREADS, 0, s>>>(in, flags, n, out, count, st, uint32_t(tiles),
+                                                                       tiles > 1 ? a.wait_error() : nullptr);
     CURC_LAUNCH_CHECK();
     a.release(m);
 }
@@ -423,127 +490,219 @@ __device__ __forceinline__ uint32_t digit_of(K k, int shift, uint32_t mask) {
     return uint32_t(k >> shift) & mask;
 }
 
+constexpr int RS_PASSES = 8;  // digits of a 64-bit key
+
+// The digits of a sort: `passes` of them from begin_bit on, 8 bits each (the
+// last one what is left).
+struct RsDigits {
+    int begin, end;
+    __host__ __device__ int passes() const { return (end - begin + 7) / 8; }
+    __host__ __device__ int shift(int p) const { return begin + 8 * p; }
+    __host__ __device__ uint32_t mask(int p) const {
+        const int left = end - shift(p);
+        return left >= 8 ? 0xFFu : (1u << left) - 1u;
+    }
+};
+
+// Counts of every digit of every pass in one read of the keys:
+// hist[pass * 256 + digit].
 template <class K>
-__global__ void __launch_bounds__(RS_THREADS) rs_hist_kernel(const K* __restrict__ keys, size_t n, int shift,
-                                                             uint32_t mask, uint32_t* __restrict__ hist,
-                                                             uint32_t tiles) {
-    __shared__ uint32_t h[256];
-    h[threadIdx.x] = 0;
+__global__ void __launch_bounds__(RS_THREADS) rs_hist_kernel(const K* __restrict__ keys, size_t n, RsDigits dg,
+                                                             uint32_t* __restrict__ hist) {
+    __shared__ uint32_t h[RS_PASSES][256];
+    const int np = dg.passes();
+    for (int p = 0; p < np; ++p) h[p][threadIdx.x] = 0;
     __syncthreads();
-    const size_t base = size_t(blockIdx.x) * RS_TILE;
-#pragma unroll 4
-    for (int r = 0; r < RS_ROUNDS; ++r) {
-        size_t idx = base + size_t(r) * RS_THREADS + threadIdx.x;
-        if (idx < n) atomicAdd(&h[digit_of(keys[idx], shift, mask)], 1u);
+    for (size_t i = size_t(blockIdx.x) * RS_THREADS + threadIdx.x; i < n; i += size_t(gridDim.x) * RS_THREADS) {
+        const K k = keys[i];
+        for (int p = 0; p < np; ++p) atomicAdd(&h[p][digit_of(k, dg.shift(p), dg.mask(p))], 1u);
     }
     __syncthreads();
-    hist[size_t(threadIdx.x) * tiles + blockIdx.x] = h[threadIdx.x];
+    for (int p = 0; p < np; ++p)
+        if (h[p][threadIdx.x]) atomicAdd(&hist[p * 256 + threadIdx.x], h[p][threadIdx.x]);
 }
 
-// Stable scatter: items are ranked in index order.  Warp w takes the
-// tile's items [512 w, 512 w + 512) in 16 rounds of 32 consecutive ones,
-// keeping them in registers, and ranks each among the warp's earlier items
-// of its digit with match_any and warp-private digit counters (no block
-// barrier inside); the warps' counts are then scanned per digit, and the
-// tile is reordered by digit in shared memory (its digit counts come from
-// the scanned histogram: the difference of consecutive offsets) and written
-// out in that order, so that items of one digit leave as one contiguous run
-// and the stores coalesce.
-template <class K, class V>
-__global__ void __launch_bounds__(RS_THREADS) rs_scatter_kernel(const K* __restrict__ kin, const V* __restrict__ vin,
-                                                                K* __restrict__ kout, V* __restrict__ vout, size_t n,
-                                                                int shift, uint32_t mask,
-                                                                const uint32_t* __restrict__ offsets, uint32_t tiles) {
-    extern __shared__ __align__(16) uint8_t rs_smem[];
-    K* sk = reinterpret_cast<K*>(rs_smem);
-    V* sv = reinterpret_cast<V*>(rs_smem + sizeof(K) * RS_TILE);
-    __shared__ uint32_t gbase[256];
-    __shared__ uint32_t tstart[256];
-    __shared__ uint32_t wcnt[RS_WARPS][256];
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    {
-        // this tile's count of digit tid, from the exclusive scan over
-        // (digit, tile): the next flattened entry minus this one
-        const size_t fi = size_t(tid) * tiles + blockIdx.x;
-        const uint32_t g = offsets[fi];
-        const uint32_t nx = fi + 1 < size_t(256) * tiles ? offsets[fi + 1] : uint32_t(n);
-        gbase[tid] = g;
-        tstart[tid] = nx - g;
-    }
+// Exclusive scan over the block's 256 threads.
+__device__ __forceinline__ uint32_t rs_scan256(uint32_t v, uint32_t* wsum) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t x = v;
 #pragma unroll
-    for (int w = 0; w < RS_WARPS; ++w) wcnt[w][tid] = 0;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
+    }
+    __syncthreads();  // wsum may still be read from an earlier call
+    if (lane == 31) wsum[warp] = x;
     __syncthreads();
-    // exclusive scan of the tile's digit counts (256 entries, one per thread)
-    {
-        __shared__ uint32_t wsum[RS_WARPS];
-        const uint32_t v = tstart[tid];
-        uint32_t x = v;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
-            if (lane >= o) x += y;
-        }
-        if (lane == 31) wsum[warp] = x;
-        __syncthreads();
-        uint32_t wbase = 0;
-        for (int w = 0; w < warp; ++w) wbase += wsum[w];
-        tstart[tid] = wbase + x - v;
-    }
-    const uint32_t lt_mask = (1u << lane) - 1u;
-    const size_t base = size_t(blockIdx.x) * RS_TILE;
-    const uint32_t items = uint32_t(min(size_t(RS_TILE), n - base));
-    // this warp's items, ranked within the warp
-    const size_t wb = base + size_t(warp) * (RS_TILE / RS_WARPS);
-    uint32_t* cnt = wcnt[warp];
+    uint32_t before = 0;
+    for (int w = 0; w < warp; ++w) before += wsum[w];
+    return before + x - v;
+}
+
+// Items of one tile in registers, 16 rounds of 32 consecutive items per warp,
+// each ranked among the warp's earlier items of its digit with match_any and
+// warp-private digit counters (no block barrier inside).
+template <class K, class V>
+struct RsTile {
     K k[RS_ROUNDS];
     V v[RS_ROUNDS];
     uint32_t rk[RS_ROUNDS];
+    __device__ __forceinline__ void rank(uint32_t items, int shift, uint32_t mask, uint32_t* cnt) {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        const uint32_t lt_mask = (1u << lane) - 1u;
 #pragma unroll
-    for (int r = 0; r < RS_ROUNDS; ++r) {
-        const size_t idx = wb + size_t(r) * 32 + lane;
-        const bool valid = idx < n;
-        k[r] = valid ? kin[idx] : K{};
-        v[r] = (valid && vin) ? vin[idx] : V{};
-        const uint32_t d = valid ? digit_of(k[r], shift, mask) : 256u;
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
-        const uint32_t before = __popc(peers & lt_mask);
-        uint32_t c0 = 0;
-        if (valid) c0 = cnt[d];  // the warp's earlier items of digit d
-        __syncwarp();
-        if (valid && before == 0) cnt[d] = c0 + __popc(peers);
-        __syncwarp();
-        rk[r] = c0 + before;
-    }
-    __syncthreads();
-    // per digit: the items of earlier warps come first
-    {
-        uint32_t acc = 0;
-#pragma unroll
-        for (int w = 0; w < RS_WARPS; ++w) {
-            const uint32_t c = wcnt[w][tid];
-            wcnt[w][tid] = acc;
-            acc += c;
+        for (int r = 0; r < RS_ROUNDS; ++r) {
+            const uint32_t t = uint32_t(warp) * (RS_TILE / RS_WARPS) + r * 32 + lane;
+            const bool valid = t < items;
+            const uint32_t d = valid ? digit_of(k[r], shift, mask) : 256u;
+            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
+            const uint32_t before = __popc(peers & lt_mask);
+            uint32_t c0 = 0;
+            if (valid) c0 = cnt[d];  // the warp's earlier items of digit d
+            __syncwarp();
+            if (valid && before == 0) cnt[d] = c0 + __popc(peers);
+            __syncwarp();
+            rk[r] = c0 + before;
         }
     }
+};
+
+// One pass: tiles are taken in order from a counter; each ranks its items,
+// publishes its count of every digit, reorders itself by digit in shared
+// memory and, thread d for digit d, looks back over the tiles before it for
+// the items of its digit that precede (one state per tile and digit, as in
+// look_back).  The start of a digit comes from the counts of the whole input.
+// Items of one digit leave the tile as one contiguous run, so the stores
+// coalesce.  One launch and one read and write of the items per pass; with a
+// histogram, a scan and a scatter launch per pass a sort of a few thousand
+// items took 360 us, all of it launches (B200, 64-bit keys).
+template <class K, class V>
+__global__ void __launch_bounds__(RS_THREADS) rs_pass_kernel(const K* __restrict__ kin, const V* __restrict__ vin,
+                                                             K* __restrict__ kout, V* __restrict__ vout, size_t n,
+                                                             int shift, uint32_t mask,
+                                                             const uint32_t* __restrict__ hist,
+                                                             unsigned long long* __restrict__ st, uint32_t tiles,
+                                                             uint32_t* __restrict__ err) {
+    extern __shared__ __align__(16) uint8_t rs_smem[];
+    K* sk = reinterpret_cast<K*>(rs_smem);
+    V* sv = reinterpret_cast<V*>(rs_smem + sizeof(K) * RS_TILE);
+    __shared__ uint32_t gbase[256], tstart[256];
+    __shared__ uint32_t wcnt[RS_WARPS][256];
+    __shared__ uint32_t wsum[RS_WARPS], s_tile;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    if (tid == 0) s_tile = uint32_t(atomicAdd(&st[size_t(tiles) * 256], 1ull));
+#pragma unroll
+    for (int w = 0; w < RS_WARPS; ++w) wcnt[w][tid] = 0;
+    const uint32_t digit_start = rs_scan256(hist[tid], wsum);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    const size_t base = size_t(tile) * RS_TILE;
+    const uint32_t items = uint32_t(min(size_t(RS_TILE), n - base));
+    RsTile<K, V> T;
+#pragma unroll
+    for (int r = 0; r < RS_ROUNDS; ++r) {
+        const uint32_t t = uint32_t(warp) * (RS_TILE / RS_WARPS) + r * 32 + lane;
+        T.k[r] = t < items ? kin[base + t] : K{};
+        T.v[r] = (t < items && vin) ? vin[base + t] : V{};
+    }
+    T.rank(items, shift, mask, wcnt[warp]);
+    __syncthreads();
+    // per digit: this tile's count, the items of earlier warps first
+    uint32_t mine = 0;
+#pragma unroll
+    for (int w = 0; w < RS_WARPS; ++w) {
+        const uint32_t c = wcnt[w][tid];
+        wcnt[w][tid] = mine;
+        mine += c;
+    }
+    unsigned long long* state = st + size_t(tile) * 256 + tid;
+    atomicExch(state, (tile == 0 ? LOOK_INCL : LOOK_SUM) | mine);
+    tstart[tid] = rs_scan256(mine, wsum);
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < RS_ROUNDS; ++r) {
-        const size_t idx = wb + size_t(r) * 32 + lane;
-        if (idx < n) {
-            const uint32_t d = digit_of(k[r], shift, mask);
-            const uint32_t lp = tstart[d] + cnt[d] + rk[r];
-            sk[lp] = k[r];
-            if (vin) sv[lp] = v[r];
+        const uint32_t t = uint32_t(warp) * (RS_TILE / RS_WARPS) + r * 32 + lane;
+        if (t < items) {
+            const uint32_t d = digit_of(T.k[r], shift, mask);
+            const uint32_t lp = tstart[d] + wcnt[warp][d] + T.rk[r];
+            sk[lp] = T.k[r];
+            if (vin) sv[lp] = T.v[r];
         }
     }
+    // items of digit tid in the tiles before this one
+    uint64_t before = 0;
+    if (tile > 0) {
+        unsigned long long* p = state;
+        for (uint32_t j = tile; j > 0; --j) {
+            p -= 256;
+            const uint64_t v = look_wait(p, err);
+            before += v & LOOK_VALUE;
+            if ((v >> 62) == 2) break;
+        }
+        atomicExch(state, LOOK_INCL | (before + mine));
+    }
+    gbase[tid] = digit_start + uint32_t(before) - tstart[tid];
     __syncthreads();
     // the tile in digit order: runs of one digit go to consecutive places
     for (uint32_t p = tid; p < items; p += RS_THREADS) {
         const K kk = sk[p];
-        const uint32_t d = digit_of(kk, shift, mask);
-        const uint32_t gpos = gbase[d] + (p - tstart[d]);
+        const uint32_t gpos = gbase[digit_of(kk, shift, mask)] + p;
         kout[gpos] = kk;
         if (vout) vout[gpos] = sv[p];
+    }
+}
+
+// Every pass of a sort of at most one tile, in place, by one block.
+template <class K, class V>
+__global__ void __launch_bounds__(RS_THREADS) rs_single_kernel(K* __restrict__ keys, V* __restrict__ vals, uint32_t n,
+                                                               RsDigits dg) {
+    extern __shared__ __align__(16) uint8_t rs_smem[];
+    K* sk = reinterpret_cast<K*>(rs_smem);
+    V* sv = reinterpret_cast<V*>(rs_smem + sizeof(K) * RS_TILE);
+    __shared__ uint32_t tstart[256];
+    __shared__ uint32_t wcnt[RS_WARPS][256];
+    __shared__ uint32_t wsum[RS_WARPS];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    RsTile<K, V> T;
+    const int np = dg.passes();
+    for (int p = 0; p < np; ++p) {
+        const int shift = dg.shift(p);
+        const uint32_t mask = dg.mask(p);
+#pragma unroll
+        for (int w = 0; w < RS_WARPS; ++w) wcnt[w][tid] = 0;
+#pragma unroll
+        for (int r = 0; r < RS_ROUNDS; ++r) {
+            const uint32_t t = uint32_t(warp) * (RS_TILE / RS_WARPS) + r * 32 + lane;
+            T.k[r] = t < n ? (p ? sk[t] : keys[t]) : K{};
+            T.v[r] = (t < n && vals) ? (p ? sv[t] : vals[t]) : V{};
+        }
+        __syncthreads();
+        T.rank(n, shift, mask, wcnt[warp]);
+        __syncthreads();
+        uint32_t mine = 0;
+#pragma unroll
+        for (int w = 0; w < RS_WARPS; ++w) {
+            const uint32_t c = wcnt[w][tid];
+            wcnt[w][tid] = mine;
+            mine += c;
+        }
+        tstart[tid] = rs_scan256(mine, wsum);
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < RS_ROUNDS; ++r) {
+            const uint32_t t = uint32_t(warp) * (RS_TILE / RS_WARPS) + r * 32 + lane;
+            if (t < n) {
+                const uint32_t d = digit_of(T.k[r], shift, mask);
+                const uint32_t lp = tstart[d] + wcnt[warp][d] + T.rk[r];
+                sk[lp] = T.k[r];
+                if (vals) sv[lp] = T.v[r];
+            }
+        }
+        __syncthreads();
+    }
+    for (uint32_t t = tid; t < n; t += RS_THREADS) {
+        keys[t] = sk[t];
+        if (vals) vals[t] = sv[t];
     }
 }
 
@@ -552,7 +711,7 @@ constexpr size_t rs_smem_bytes() {
     return (sizeof(K) + sizeof(V)) * size_t(RS_TILE);
 }
 
-// The scatter kernel's dynamic shared-memory limit, raised once per device.
+// The kernels' dynamic shared-memory limit, raised once per device.
 template <class K, class V>
 void rs_prepare() {
     static std::mutex mu;
@@ -562,7 +721,9 @@ void rs_prepare() {
     if (dev < 0 || dev >= 64) throw std::runtime_error("device ordinal out of range");
     std::lock_guard<std::mutex> g(mu);
     if (!done[dev]) {
-        CURC_CHECK(cudaFuncSetAttribute(rs_scatter_kernel<K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        CURC_CHECK(cudaFuncSetAttribute(rs_pass_kernel<K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        int(rs_smem_bytes<K, V>())));
+        CURC_CHECK(cudaFuncSetAttribute(rs_single_kernel<K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         int(rs_smem_bytes<K, V>())));
         done[dev] = true;
     }
@@ -573,24 +734,33 @@ template <class K, class V>
 void radix_sort_pairs(K* keys, V* vals, size_t n, int begin_bit, int end_bit, Arena& a, cudaStream_t s) {
     if (n <= 1 || end_bit <= begin_bit) return;
     if (n > 0xFFFFFFFFull) throw std::runtime_error("radix_sort_pairs: more than 2^32 items");
+    rs_prepare<K, V>();
+    const RsDigits dg{begin_bit, end_bit};
+    if (n <= size_t(RS_TILE)) {
+        rs_single_kernel<K, V><<<1, RS_THREADS, rs_smem_bytes<K, V>(), s>>>(keys, vals, uint32_t(n), dg);
+        CURC_LAUNCH_CHECK();
+        return;
+    }
     auto m = a.mark();
     K* kalt = a.alloc<K>(n);
     V* valt = vals ? a.alloc<V>(n) : nullptr;
     const uint32_t tiles = uint32_t(div_up(n, RS_TILE));
-    uint32_t* hist = a.alloc<uint32_t>(size_t(256) * tiles);
+    const int np = dg.passes();
+    // per pass: 256 states per tile and the tile counter; then the counts
+    const size_t pass_words = size_t(tiles) * 256 + 1;
+    unsigned long long* st = a.alloc<unsigned long long>(pass_words * np + size_t(np) * 128);
+    uint32_t* hist = reinterpret_cast<uint32_t*>(st + pass_words * np);
+    CURC_CHECK(cudaMemsetAsync(st, 0, (pass_words * np + size_t(np) * 128) * sizeof(unsigned long long), s));
+    rs_hist_kernel<K><<<unsigned(std::min<size_t>(div_up(n, RS_THREADS * 8), size_t(SM_COUNT_B200) * 8)), RS_THREADS, 0,
+                        s>>>(keys, n, dg, hist);
+    CURC_LAUNCH_CHECK();
     K* kc = keys;
     V* vc = vals;
-    rs_prepare<K, V>();
-    for (int shift = begin_bit; shift < end_bit; shift += 8) {
-        const int bits = std::min(8, end_bit - shift);
-        const uint32_t mask = (1u << bits) - 1u;
-        rs_hist_kernel<K><<<tiles, RS_THREADS, 0, s>>>(kc, n, shift, mask, hist, tiles);
-        CURC_LAUNCH_CHECK();
-        exclusive_scan<uint32_t>(hist, hist, size_t(256) * tiles, nullptr, a, s);
+    for (int p = 0; p < np; ++p) {
         K* ko = (kc == keys) ? kalt : keys;
         V* vo = vals ? ((vc == vals) ? valt : vals) : nullptr;
-        rs_scatter_kernel<K, V><<<tiles, RS_THREADS, rs_smem_bytes<K, V>(), s>>>(kc, vc, ko, vo, n, shift, mask,
-                                                                                 hist, tiles);
+        rs_pass_kernel<K, V><<<tiles, RS_THREADS, rs_smem_bytes<K, V>(), s>>>(
+            kc, vc, ko, vo, n, dg.shift(p), dg.mask(p), hist + p * 256, st + pass_words * p, tiles, a.wait_error());
         CURC_LAUNCH_CHECK();
         kc = ko;
         vc = vo;
@@ -657,14 +827,6 @@ void iota(uint32_t* p, size_t n, cudaStream_t s) {
 }
 
 namespace {
-// Marks elements that share their first word with a neighbour (tie runs).
-__global__ void tie_flags_kernel(const uint64_t* __restrict__ k0, size_t n, uint8_t* __restrict__ tie) {
-    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint64_t v = k0[i];
-    tie[i] = (i > 0 && k0[i - 1] == v) || (i + 1 < n && k0[i + 1] == v);
-}
-
 // 1 where a tie element starts a new run (its predecessor in the tie list
 // is not its neighbour or has another first word).
 __global__ void run_starts_kernel(const uint32_t* __restrict__ pos, const uint64_t* __restrict__ k0, uint32_t m,
@@ -681,55 +843,153 @@ __global__ void run_number_kernel(const uint32_t* __restrict__ excl, const uint3
     if (t < m) out[t] = uint64_t(excl[t]) + start[t];
 }
 
-__global__ void run_starts8_kernel(const uint32_t* __restrict__ pos, const uint64_t* __restrict__ k0, uint32_t m,
-                                   uint8_t* __restrict__ start) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= m) return;
-    start[t] = t == 0 || pos[t - 1] + 1 != pos[t] || k0[pos[t - 1]] != k0[pos[t]];
-}
-
-// One warp per run of reads sharing their first word: runs of up to 32
-// reads are ordered in place by their remaining words, ties by position
-// (stable), each lane ranking its read against the others' words by
-// shuffles.  Longer runs are flagged for the radix path.
-__global__ void small_runs_kernel(const uint64_t* __restrict__ db, int W, uint32_t* __restrict__ ids,
-                                  const uint32_t* __restrict__ pos, const uint32_t* __restrict__ rb, uint32_t R,
-                                  uint32_t m, uint8_t* __restrict__ large) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < R; r += warps) {
-        const uint32_t b = rb[r], e = r + 1 < R ? rb[r + 1] : m, len = e - b;
-        if (len > 32) {
-            for (uint32_t k = lane; k < len; k += 32) large[b + k] = 1;
-            continue;
+// Runs of rows that share their first word (k0, sorted), ordered in place by
+// their remaining words, ties by position (stable).  The thread at a run's
+// start orders runs of up to RUN_THREAD rows by insertion; a warp orders
+// runs of up to 32, each lane ranking its row against the others' words by
+// shuffles (rows of up to 16 words) or loads; longer runs are flagged for
+// the radix path, and *any_large counts their rows.  Most runs have two or
+// three rows (reads that start at one place), so a warp per run left most
+// lanes idle.
+constexpr uint32_t RUN_THREAD = 4;
+__global__ void __launch_bounds__(256) order_runs_kernel(const uint64_t* __restrict__ db, int W,
+                                                         uint32_t* __restrict__ ids,
+                                                         const uint64_t* __restrict__ k0, uint32_t n,
+                                                         uint8_t* __restrict__ large, uint32_t* __restrict__ any_large) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    uint32_t len = 0;  // of the run that starts here (up to 33), else 0
+    if (i + 1 < n) {
+        const uint64_t v = k0[i];
+        if (k0[i + 1] == v && (i == 0 || k0[i - 1] != v)) {
+            len = 2;
+            while (len <= 32 && i + len < n && k0[i + len] == v) ++len;
         }
-        const uint32_t p0 = pos[b];
-        uint32_t id = 0;
-        uint64_t w[15];
+    }
+    if (len >= 2 && len <= RUN_THREAD) {
+        uint32_t id[RUN_THREAD];
 #pragma unroll
-        for (int k = 0; k < 15; ++k) w[k] = 0;
-        if (lane < len) {
-            id = ids[p0 + lane];
+        for (uint32_t t = 0; t < RUN_THREAD; ++t) id[t] = t < len ? ids[i + t] : 0;
+        auto before = [&](uint32_t x, uint32_t y) {  // row x strictly before row y
+            for (int w = 1; w < W; ++w) {
+                const uint64_t p = db[uint64_t(x) * W + w], q = db[uint64_t(y) * W + w];
+                if (p != q) return p < q;
+            }
+            return false;
+        };
 #pragma unroll
-            for (int k = 0; k < 15; ++k)
-                if (k + 1 < W) w[k] = db[uint64_t(id) * W + k + 1];
-        }
-        uint32_t rank = 0;
-        for (uint32_t j = 0; j < len; ++j) {
-            int c = 0;  // lane j's read against mine
+        for (uint32_t t = 1; t < RUN_THREAD; ++t) {
+            if (t < len) {
+                bool go = true;
 #pragma unroll
-            for (int k = 0; k < 15; ++k) {
-                if (k + 1 < W) {
-                    const uint64_t o = __shfl_sync(0xFFFFFFFFu, w[k], int(j));
-                    if (c == 0 && o != w[k]) c = o < w[k] ? -1 : 1;
+                for (uint32_t u = t; u > 0; --u) {
+                    if (go && before(id[u], id[u - 1])) {
+                        const uint32_t x = id[u];
+                        id[u] = id[u - 1];
+                        id[u - 1] = x;
+                    } else {
+                        go = false;
+                    }
                 }
             }
-            rank += (c < 0 || (c == 0 && j < lane)) ? 1u : 0u;
+        }
+#pragma unroll
+        for (uint32_t t = 0; t < RUN_THREAD; ++t)
+            if (t < len) ids[i + t] = id[t];
+    }
+    uint32_t todo = __ballot_sync(0xFFFFFFFFu, len > RUN_THREAD);
+    while (todo) {
+        const int l = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const uint32_t p0 = __shfl_sync(0xFFFFFFFFu, i, l), m = __shfl_sync(0xFFFFFFFFu, len, l);
+        if (m > 32) {  // flag the whole run
+            const uint64_t v = k0[p0];
+            uint32_t rows = 0;
+            for (uint32_t t = p0 + lane;; t += 32) {
+                const bool in = t < n && k0[t] == v;
+                if (in) large[t] = 1;
+                const uint32_t c = __popc(__ballot_sync(0xFFFFFFFFu, in));
+                rows += c;
+                if (c < 32) break;
+            }
+            if (lane == 0) atomicAdd(any_large, rows);
+            continue;
+        }
+        const uint32_t id = lane < m ? ids[p0 + lane] : 0;
+        uint32_t rank = 0;
+        if (W <= 16) {
+            uint64_t w[15];
+#pragma unroll
+            for (int k = 0; k < 15; ++k) w[k] = (lane < m && k + 1 < W) ? db[uint64_t(id) * W + k + 1] : 0;
+            for (uint32_t j = 0; j < m; ++j) {
+                int c = 0;  // lane j's row against mine
+#pragma unroll
+                for (int k = 0; k < 15; ++k) {
+                    if (k + 1 < W) {
+                        const uint64_t o = __shfl_sync(0xFFFFFFFFu, w[k], int(j));
+                        if (c == 0 && o != w[k]) c = o < w[k] ? -1 : 1;
+                    }
+                }
+                rank += (c < 0 || (c == 0 && j < lane)) ? 1u : 0u;
+            }
+        } else {
+            for (uint32_t j = 0; j < m; ++j) {
+                const uint32_t o = __shfl_sync(0xFFFFFFFFu, id, int(j));
+                int c = 0;
+                if (lane < m)
+                    for (int k = 1; k < W && c == 0; ++k) {
+                        const uint64_t x = db[uint64_t(o) * W + k], y = db[uint64_t(id) * W + k];
+                        if (x != y) c = x < y ? -1 : 1;
+                    }
+                rank += (c < 0 || (c == 0 && j < lane)) ? 1u : 0u;
+            }
         }
         __syncwarp();
-        if (lane < len) ids[p0 + rank] = id;
+        if (lane < m) ids[p0 + rank] = id;
         __syncwarp();
     }
+}
+
+// Up to ROWS_SMALL rows in one launch: eight lanes rank a row against all, by
+// the first word (every block holds all of them in shared memory) and, where
+// that is equal, by the others, ties by position.  out[rank] = id.
+constexpr uint32_t ROWS_SMALL = 4096;
+__global__ void __launch_bounds__(256) sort_rows_small_kernel(const uint64_t* __restrict__ db, int W,
+                                                              const uint32_t* __restrict__ ids, uint32_t n,
+                                                              uint32_t* __restrict__ out) {
+    __shared__ uint64_t k0[ROWS_SMALL];
+    for (uint32_t t = threadIdx.x; t < n; t += blockDim.x) k0[t] = db[uint64_t(ids[t]) * W];
+    __syncthreads();
+    const uint32_t t = blockIdx.x * 32 + (threadIdx.x >> 3), sub = threadIdx.x & 7u;
+    const uint64_t mine = t < n ? k0[t] : 0;
+    uint32_t rank = 0, equal = 0;
+    if (t < n) {
+#pragma unroll 8
+        for (uint32_t j = sub; j < n; j += 8) {
+            const uint64_t o = k0[j];
+            rank += o < mine;
+            equal += o == mine;
+        }
+    }
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) equal += __shfl_xor_sync(0xFFFFFFFFu, equal, d);
+    if (t < n && equal > 1) {
+        const uint64_t* me = db + uint64_t(ids[t]) * W;
+        for (uint32_t j = sub; j < n; j += 8) {
+            if (k0[j] != mine || j == t) continue;
+            const uint64_t* other = db + uint64_t(ids[j]) * W;
+            int w = 1;
+            uint64_t x = 0, y = 0;
+            for (; w < W; ++w) {
+                x = other[w];
+                y = me[w];
+                if (x != y) break;
+            }
+            rank += w < W ? x < y : j < t;
+        }
+    }
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) rank += __shfl_xor_sync(0xFFFFFFFFu, rank, d);
+    if (t < n && sub == 0) out[rank] = ids[t];
 }
 
 __global__ void gather_ids_kernel(const uint32_t* __restrict__ ids, const uint32_t* __restrict__ pos, uint32_t m,
@@ -745,54 +1005,43 @@ __global__ void scatter_ids_kernel(const uint32_t* __restrict__ vals, const uint
 }
 }  // namespace
 
-void sort_ids_by_reads(const uint64_t* db, int W, int L, uint32_t* ids, size_t n, Arena& a, cudaStream_t s) {
-    // Stable lexicographic order of the reads (compress.cu:1400-1407 under a
+void sort_rows(const uint64_t* db, int W, int last_bits, uint32_t* ids, size_t n, Arena& a, cudaStream_t s) {
+    // Stable lexicographic order of the rows (compress.cu:1400-1407 under a
     // stable comparison sort; ties keep input order).  First by the first
-    // 32 bases; then only the runs of reads that share them are ordered by
-    // the remaining words: runs of up to 32 reads by one warp each, longer
-    // runs by radix passes over the remaining words, least significant first,
-    // and finally by run so that every run returns to its place.
+    // word; then only the runs of rows that share it are ordered by the
+    // remaining words: runs of up to 32 rows by a thread or a warp each,
+    // longer runs by radix passes over the remaining words, least significant
+    // first, and finally by run so that every run returns to its place.
     if (n <= 1) return;
     auto mk = a.mark();
+    if (n <= ROWS_SMALL) {
+        // two launches and no read back (the general path takes a dozen and one)
+        uint32_t* out = a.alloc<uint32_t>(n);
+        sort_rows_small_kernel<<<grid_for(n, 32), 256, 0, s>>>(db, W, ids, uint32_t(n), out);
+        CURC_LAUNCH_CHECK();
+        CURC_CHECK(cudaMemcpyAsync(ids, out, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
+        a.release(mk);
+        return;
+    }
     uint64_t* k0 = a.alloc<uint64_t>(n);
     {
-        // the first-word sort alone (the tie runs below read counts back to the host)
+        // the first-word sort alone (the tie runs below read a count back to the host)
         SubStage sp("sort_dedupe.first_word");
         gather_words(db, ids, n, W, 0, k0, s);
-        const int lo0 = W == 1 ? 64 - 2 * L : 0;
-        radix_sort_pairs<uint64_t, uint32_t>(k0, ids, n, lo0, 64, a, s);
+        radix_sort_pairs<uint64_t, uint32_t>(k0, ids, n, W == 1 ? 64 - last_bits : 0, 64, a, s);
     }
     if (W > 1) {
-        uint8_t* tie = a.alloc<uint8_t>(n);
-        tie_flags_kernel<<<grid_for(n, 256), 256, 0, s>>>(k0, n, tie);
+        uint8_t* large = a.alloc<uint8_t>(n);
+        uint32_t* cnt = a.alloc<uint32_t>(2);
+        CURC_CHECK(cudaMemsetAsync(large, 0, n, s));
+        CURC_CHECK(cudaMemsetAsync(cnt, 0, 8, s));
+        order_runs_kernel<<<grid_for(n, 256), 256, 0, s>>>(db, W, ids, k0, uint32_t(n), large, cnt);
         CURC_LAUNCH_CHECK();
-        uint32_t* pos = a.alloc<uint32_t>(n);
-        uint32_t* cnt = a.alloc<uint32_t>(1);
-        select_indices(tie, pos, n, cnt, a, s);
-        const uint32_t m0 = read_scalar(cnt, s);
-        uint32_t m = 0;
-        if (m0) {
-            // runs of up to 32 reads: one warp each; longer runs: radix below
-            uint8_t* st8 = a.alloc<uint8_t>(m0);
-            run_starts8_kernel<<<grid_for(m0, 256), 256, 0, s>>>(pos, k0, m0, st8);
-            CURC_LAUNCH_CHECK();
-            uint32_t* rb = a.alloc<uint32_t>(m0);
-            uint32_t* rc = a.alloc<uint32_t>(2);
-            select_indices(st8, rb, m0, rc, a, s);
-            const uint32_t R = read_scalar(rc, s);
-            uint8_t* large = a.alloc<uint8_t>(m0);
-            CURC_CHECK(cudaMemsetAsync(large, 0, m0, s));
-            small_runs_kernel<<<grid_for(uint64_t(R) * 32, 256), 256, 0, s>>>(db, W, ids, pos, rb, R, m0, large);
-            CURC_LAUNCH_CHECK();
-            uint32_t* li = a.alloc<uint32_t>(m0);
-            select_indices(large, li, m0, rc + 1, a, s);
-            m = read_scalar(rc + 1, s);
-            if (m) {
-                uint32_t* lp = a.alloc<uint32_t>(m);
-                gather_ids_kernel<<<grid_for(m, 256), 256, 0, s>>>(pos, li, m, lp);
-                CURC_LAUNCH_CHECK();
-                pos = lp;
-            }
+        const uint32_t m = read_scalar(cnt, s);
+        uint32_t* pos = nullptr;
+        if (m) {
+            pos = a.alloc<uint32_t>(m);
+            select_indices(large, pos, n, cnt + 1, a, s);
         }
         if (m) {
             uint32_t* sub = a.alloc<uint32_t>(m);
@@ -819,7 +1068,7 @@ void sort_ids_by_reads(const uint64_t* db, int W, int L, uint32_t* ids, size_t n
                 gather_ids_kernel<<<grid_for(m, 256), 256, 0, s>>>(sub, perm, m, tmp);  // current order's ids
                 CURC_LAUNCH_CHECK();
                 gather_words(db, tmp, m, W, w, key, s);
-                const int lo = w == W - 1 ? 64 - 2 * (L - 32 * (W - 1)) : 0;
+                const int lo = w == W - 1 ? 64 - last_bits : 0;
                 radix_sort_pairs<uint64_t, uint32_t>(key, perm, m, lo, 64, a, s);
             }
             // stable by run number (ascending with position)
@@ -835,6 +1084,10 @@ void sort_ids_by_reads(const uint64_t* db, int W, int L, uint32_t* ids, size_t n
         }
     }
     a.release(mk);
+}
+
+void sort_ids_by_reads(const uint64_t* db, int W, int L, uint32_t* ids, size_t n, Arena& a, cudaStream_t s) {
+    sort_rows(db, W, 2 * (L - 32 * (W - 1)), ids, n, a, s);
 }
 
 }  // namespace curc

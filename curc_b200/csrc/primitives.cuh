@@ -33,6 +33,11 @@ public:
     // Frees every chunk (nothing may be in use: the stream work that used
     // them must have completed; cudaFree waits for the device).
     void trim();
+    // Device error word of the one-pass kernels that take their scratch here
+    // (a wait on another tile that ran out), zero unless one did.
+    uint32_t* wait_error();
+    // Throws when a host copy of it (4 bytes) is set, and clears it.
+    void check_waits(const void* copy, cudaStream_t s);
     size_t high_water() const { return high_water_; }
     size_t in_use() const;
 
@@ -47,6 +52,7 @@ private:
     size_t cur_ = 0;
     size_t chunk_;
     size_t high_water_ = 0;
+    uint32_t* wait_error_ = nullptr;
 };
 
 // Growable pinned host memory, bump allocated, reset per block; results are
@@ -136,6 +142,9 @@ void radix_sort_pairs(K* keys, V* vals, size_t n, int begin_bit, int end_bit, Ar
 // Stable sort of ids by packed read content (W words per read, lexicographic
 // over all words): ids is permuted in place.
 void sort_ids_by_reads(const uint64_t* db, int W, int L, uint32_t* ids, size_t n, Arena& a, cudaStream_t s);
+
+// The same for rows of W words of which the last one's top last_bits count.
+void sort_rows(const uint64_t* rows, int W, int last_bits, uint32_t* ids, size_t n, Arena& a, cudaStream_t s);
 
 // Gather 64-bit words: out[i] = src[idx[i] * stride + word].
 void gather_words(const uint64_t* src, const uint32_t* idx, size_t n, int stride, int word, uint64_t* out,
