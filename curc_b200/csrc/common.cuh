@@ -78,6 +78,24 @@ __device__ __forceinline__ uint64_t word_at(const uint64_t* __restrict__ r, uint
     return v >> (64 - 2 * nb);
 }
 
+// The 64 bases of a packed read from base p0 on (zeros past its W words) in
+// registers: three loads serve the k-mers at 32 consecutive positions, where
+// word_at() loads two words for each, 32 cache lines a warp.
+struct BaseWindow {
+    uint64_t x0, x1;
+    __device__ __forceinline__ BaseWindow(const uint64_t* __restrict__ row, int W, int p0) {
+        const int w = p0 >> 5, sh = 2 * (p0 & 31);
+        const uint64_t a = w < W ? row[w] : 0, b = w + 1 < W ? row[w + 1] : 0, c = w + 2 < W ? row[w + 2] : 0;
+        x0 = sh ? (a << sh) | (b >> (64 - sh)) : a;
+        x1 = sh ? (b << sh) | (c >> (64 - sh)) : b;
+    }
+    // the nb <= 32 bases from p0 + b on, 0 <= b < 32, as word_at() gives them
+    __device__ __forceinline__ uint64_t at(int b, int nb) const {
+        const uint64_t v = b ? (x0 << (2 * b)) | (x1 >> (64 - 2 * b)) : x0;
+        return v >> (64 - 2 * nb);
+    }
+};
+
 // Same over a padded contiguous bit string (one zero word after the last
 // base); util.cuh:189-195.
 __device__ __forceinline__ uint64_t word_unaligned(const uint64_t* __restrict__ r, uint64_t off, int nb) {

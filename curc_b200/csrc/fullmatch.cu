@@ -31,6 +31,7 @@
 
 #include "compact.cuh"
 #include "stages.cuh"
+#include "walk.cuh"
 
 namespace curc {
 
@@ -62,6 +63,13 @@ struct PackedAcc {
     __device__ __forceinline__ uint64_t fhash(uint32_t a, int pos, int fk) const {
         return murmur64(word_at(db + uint64_t(a) * W, uint32_t(pos), fk));
     }
+    // the same for 32 consecutive positions
+    struct Hasher {
+        BaseWindow w;
+        __device__ __forceinline__ Hasher(const PackedAcc& acc, uint32_t a, int pos)
+            : w(acc.db + uint64_t(a) * acc.W, acc.W, pos) {}
+        __device__ __forceinline__ uint64_t at(int b, int fk) const { return murmur64(w.at(b, fk)); }
+    };
 };
 
 struct AsciiAcc {
@@ -108,6 +116,13 @@ struct AsciiAcc {
         if (fk <= KS) return murmur64(k0 >> (64 - SB * fk));
         return murmur64(murmur64(k0) ^ (key(a, pos + KS) >> (64 - SB * (fk - KS))));
     }
+    struct Hasher {
+        const AsciiAcc& acc;
+        uint32_t a;
+        int pos;
+        __device__ __forceinline__ Hasher(const AsciiAcc& acc_, uint32_t a_, int pos_) : acc(acc_), a(a_), pos(pos_) {}
+        __device__ __forceinline__ uint64_t at(int b, int fk) const { return acc.fhash(a, pos + b, fk); }
+    };
 };
 
 // Comparison of read a from aoff with read b from boff over len symbols,
@@ -379,17 +394,7 @@ __global__ void merge_groups_kernel(Acc acc, uint32_t* pre, uint64_t* pk, const 
         group_one(acc, pre, pk, mp, suf, sk, ms, off, j, next, prev, offset);
 }
 
-// Compaction functors: keep the list entries whose link is still free.
-struct FreeLink {
-    const uint32_t* ids;
-    const uint32_t* link;
-    __device__ bool operator()(uint32_t i) const { return link[ids[i]] == INVALID; }
-};
-struct MoveId {
-    const uint32_t* in;
-    uint32_t* out;
-    __device__ void operator()(uint32_t i, uint32_t d) const { out[d] = in[i]; }
-};
+// Compaction functor: ids with their keys.
 struct MoveIdKey {
     const uint32_t* in;
     const uint64_t* ink;
@@ -485,12 +490,6 @@ void full_match_passes(const Acc& acc, uint32_t* pre, uint32_t* suf, uint32_t cn
 
 // ---------------------------------------------------------------- event form
 
-// Meeting of a suffix (id s) with the prefixes [lo, hi) of the list, p the
-// first one's id.
-struct __align__(16) FmItem {
-    uint32_t s, lo, hi, p;
-};
-
 template <class Acc>
 __global__ void fm_prefix_kernel(Acc acc, const uint32_t* __restrict__ pre, uint32_t m, uint64_t* __restrict__ pk,
                                  int fk, uint32_t* __restrict__ bits, uint32_t bmask) {
@@ -563,10 +562,11 @@ __global__ void __launch_bounds__(256) fm_meet_kernel(Acc acc, const uint32_t* _
     const uint32_t s = j < ms ? suf[j] : 0;
     uint32_t maybe = 0;
     if (j < ms) {
+        const typename Acc::Hasher hash(acc, s, off0 + w * 32);
 #pragma unroll
         for (int b = 0; b < 32; ++b) {
             if (w * 32 + b < noffs) {
-                const uint32_t h = uint32_t(acc.fhash(s, off0 + w * 32 + b, fk)) & bmask;
+                const uint32_t h = uint32_t(hash.at(b, fk)) & bmask;
                 maybe |= ((bits[h >> 5] >> (h & 31)) & 1u) << b;
             }
         }
@@ -619,7 +619,7 @@ __global__ void __launch_bounds__(256) fm_place_kernel(const uint32_t* __restric
                                                        const uint2* __restrict__ hits,
                                                        const uint32_t* __restrict__ em,
                                                        const uint32_t* __restrict__ ub,
-                                                       const uint32_t* __restrict__ first, FmItem* __restrict__ item) {
+                                                       const uint32_t* __restrict__ first, Meeting* __restrict__ item) {
     const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x, warp = j >> 5, lane = threadIdx.x & 31u;
     const bool on = j < ms;
     const uint32_t m = on ? em[uint64_t(blockIdx.y) * ms + j] : 0;
@@ -633,169 +633,16 @@ __global__ void __launch_bounds__(256) fm_place_kernel(const uint32_t* __restric
         const uint32_t base = __shfl_sync(0xFFFFFFFFu, at, b);
         if ((m >> b) & 1u) {
             const uint2 h = hits[u++];
-            item[base + __popc(bal & lt)] = FmItem{s, h.x, h.y, pre[h.x]};
+            item[base + __popc(bal & lt)] = Meeting{s, h.x, h.y, pre[h.x]};
         }
     }
 }
 
-__device__ __forceinline__ uint32_t ld_l2(const uint32_t* p) { return __ldcg(p); }
-
-// The suffixes of one run (items [i, e) with the same lo, in order) each take
-// the first free prefix that is not themselves, as the reference's merge of
-// the run does (its rotation puts a prefix that meets itself back in front).
-// One thread.
-__device__ __forceinline__ void fm_walk(const FmItem* __restrict__ item, uint32_t i, uint32_t e,
-                                        const uint32_t* __restrict__ pre, uint32_t q0, uint32_t hi, int off,
-                                        uint32_t* next, uint32_t* prev, uint16_t* offset) {
-    const uint32_t lo = item[i].lo;
-    for (; i < e && item[i].lo == lo; ++i) {
-        const uint32_t s = item[i].s;
-        if (ld_l2(next + s) != INVALID) continue;
-        bool any = false;  // a free prefix was left
-        for (uint32_t q = q0; q < hi; ++q) {
-            const uint32_t p = pre[q];
-            if (ld_l2(prev + p) != INVALID) {
-                if (!any) q0 = q + 1;
-                continue;
-            }
-            any = true;
-            if (p == s) continue;
-            next[s] = p;
-            prev[p] = s;
-            offset[s] = uint16_t(off);
-            break;
-        }
-        if (!any) return;
-    }
-}
-
-// The same by a whole warp, for long runs: free suffixes and free prefixes
-// are taken 32 at a time and paired in order; where a read would meet itself
-// the rest of the run is walked by one lane.
-__device__ void fm_walk_warp(const FmItem* __restrict__ item, uint32_t i, uint32_t e, const uint32_t* __restrict__ pre,
-                             uint32_t q, uint32_t hi, int off, uint32_t* next, uint32_t* prev, uint16_t* offset) {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t lo = item[i].lo;
-    uint32_t sm = 0, pm = 0;          // free entries of the current 32 items / prefixes
-    uint32_t ib = i, qb = q;          // where the next 32 start
-    uint32_t s = 0, p = 0;            // this lane's entries
-    bool more_s = true;
-    for (;;) {
-        while (sm == 0) {
-            if (!more_s) return;
-            const uint32_t t = ib + lane;
-            const bool in = t < e && item[t].lo == lo;
-            const uint32_t all = __ballot_sync(0xFFFFFFFFu, in);
-            s = in ? item[t].s : 0;
-            sm = __ballot_sync(0xFFFFFFFFu, in && ld_l2(next + s) == INVALID);
-            ib += 32;
-            more_s = all == 0xFFFFFFFFu;
-        }
-        while (pm == 0) {
-            if (qb >= hi) return;
-            const uint32_t t = qb + lane;
-            const bool in = t < hi;
-            p = in ? pre[t] : 0;
-            pm = __ballot_sync(0xFFFFFFFFu, in && ld_l2(prev + p) == INVALID);
-            qb += 32;
-        }
-        const int n = min(__popc(sm), __popc(pm));
-        // lane k < n pairs the k-th free suffix with the k-th free prefix
-        const int ks = int(lane) < n ? int(__fns(sm, 0, int(lane) + 1)) : 0;
-        const int kp = int(lane) < n ? int(__fns(pm, 0, int(lane) + 1)) : 0;
-        const uint32_t S = __shfl_sync(0xFFFFFFFFu, s, ks), P = __shfl_sync(0xFFFFFFFFu, p, kp);
-        const uint32_t self = __ballot_sync(0xFFFFFFFFu, int(lane) < n && S == P);
-        const int good = self ? __ffs(self) - 1 : n;
-        if (int(lane) < good) {
-            next[S] = P;
-            prev[P] = S;
-            offset[S] = uint16_t(off);
-        }
-        __syncwarp();
-        if (self) {
-            if (lane == 0) fm_walk(item, ib - 32, e, pre, qb - 32, hi, off, next, prev, offset);
-            __syncwarp();
-            return;
-        }
-        for (int k = 0; k < n; ++k) {  // the n lowest of each are used up
-            sm &= sm - 1;
-            pm &= pm - 1;
-        }
-    }
-}
-
-constexpr int FM_WALK_THREADS = 512;
-constexpr int FM_MAX_OFFS = 512;
-
-// The walk: offset after offset, one thread per run of equal suffix strings
-// (long runs: a warp).  Runs of one offset share no read, so an offset's runs
-// are independent; a barrier over the cluster separates the offsets.  One
-// cluster suffices: an offset has few meetings (thousands at most where a
-// list has 400,000 entries), and its time is the latency of two dependent
-// loads and the barrier.
-__global__ void __launch_bounds__(FM_WALK_THREADS) fm_walk_kernel(const FmItem* __restrict__ item,
-                                                                  const uint32_t* __restrict__ first, uint32_t nw,
-                                                                  const uint32_t* __restrict__ total, int off0,
-                                                                  int noffs, const uint32_t* __restrict__ pre,
-                                                                  const unsigned long long* __restrict__ used,
-                                                                  uint32_t cap, uint32_t* next, uint32_t* prev,
-                                                                  uint16_t* offset,
-                                                                  unsigned long long* __restrict__ tally) {
-    __shared__ uint32_t start[FM_MAX_OFFS + 1];
-    if (*used > cap) return;  // the listing is incomplete: the caller repeats it
-    for (int o = threadIdx.x; o <= noffs; o += FM_WALK_THREADS)
+// First meeting of each offset, and the end of the last.
+__global__ void fm_starts_kernel(const uint32_t* __restrict__ first, uint32_t nw, const uint32_t* __restrict__ total,
+                                 int noffs, uint32_t* __restrict__ start) {
+    for (int o = threadIdx.x; o <= noffs; o += blockDim.x)
         start[o] = o < noffs ? first[uint64_t(o) * nw] : *total;
-    __syncthreads();
-    const uint32_t threads = gridDim.x * FM_WALK_THREADS, me = blockIdx.x * FM_WALK_THREADS + threadIdx.x;
-    if (tally && me == 0) {
-        tally[0] += uint32_t(noffs);
-        tally[1] += start[noffs];
-        tally[2] += start[noffs];
-    }
-    for (int o = 0; o < noffs; ++o) {
-        const uint32_t a = start[o], e = start[o + 1];
-        if (a == e) continue;
-        const int off = off0 + o;
-        for (uint32_t i0 = a; i0 < e; i0 += threads) {  // the same trip count for a whole warp
-            const uint32_t i = i0 + me;
-            bool long_run = false;
-            FmItem it = {0, 0, 0, 0};
-            if (i < e) {
-                it = item[i];
-                const bool lead = i == a || item[i - 1].lo != it.lo;
-                const bool alone = i + 1 == e || item[i + 1].lo != it.lo;
-                if (lead) {
-                    if (alone && it.hi == it.lo + 1) {
-                        if (it.p != it.s) {
-                            const uint32_t nx = ld_l2(next + it.s), pv = ld_l2(prev + it.p);
-                            if (nx == INVALID && pv == INVALID) {
-                                next[it.s] = it.p;
-                                prev[it.p] = it.s;
-                                offset[it.s] = uint16_t(off);
-                            }
-                        }
-                    } else {
-                        // more than a few members or prefixes: by the whole warp
-                        long_run = it.hi - it.lo > 8 || (i + 8 < e && item[i + 8].lo == it.lo);
-                        if (!long_run) fm_walk(item, i, e, pre, it.lo, it.hi, off, next, prev, offset);
-                    }
-                }
-            }
-            uint32_t todo = __ballot_sync(0xFFFFFFFFu, long_run);
-            while (todo) {
-                const int l = __ffs(todo) - 1;
-                todo &= todo - 1;
-                const uint32_t ii = __shfl_sync(0xFFFFFFFFu, i, l), lo = __shfl_sync(0xFFFFFFFFu, it.lo, l),
-                               hi = __shfl_sync(0xFFFFFFFFu, it.hi, l);
-                fm_walk_warp(item, ii, e, pre, lo, hi, off, next, prev, offset);
-            }
-        }
-        if (gridDim.x > 1) {
-            asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-        } else {
-            __syncthreads();
-        }
-    }
 }
 
 // Every offset from off0 on of two short lists, by one block: keys, runs and
@@ -992,19 +839,20 @@ void full_match_events(const Acc& acc, uint32_t* pre, uint32_t* suf, uint32_t cn
     // room for the runs of one stage's meetings, and false ones
     const uint32_t cap = uint32_t(std::min<uint64_t>(0xF0000000ull, std::max<uint64_t>(uint64_t(4) << 20, uint64_t(cnt) * 6)));
     uint2* hits = a.alloc<uint2>(cap);
-    FmItem* item = a.alloc<FmItem>(cap);
+    Meeting* item = a.alloc<Meeting>(cap);
     struct State {
         unsigned long long used;
         uint32_t total, len_in, len_out[2];
     };
     State* st = a.alloc<State>(1);
+    uint32_t* start = a.alloc<uint32_t>(WALK_MAX_OFFS + 1);
     Compactor cp(cnt, a, s);
     uint32_t m = cnt;
     int hi = acc.L - 1;
     int fewer = acc.L;  // at most this many offsets per stage (lowered when a listing ran out of room)
     while (hi >= 1 && m > FM_SMALL) {
         auto mk2 = a.mark();
-        const int low = std::max(fm_stage_low(hi, m), hi - std::min(fewer, FM_MAX_OFFS) + 1);
+        const int low = std::max(fm_stage_low(hi, m), hi - std::min(fewer, WALK_MAX_OFFS) + 1);
         const int noffs = hi - low + 1, off0 = acc.L - hi, words = (noffs + 31) / 32;
         const int fk = std::min(low, int(Acc::FK_MAX));
         // presence bitmap of the prefixes' first fk symbols: 32 bits per
@@ -1031,28 +879,9 @@ void full_match_events(const Acc& acc, uint32_t* pre, uint32_t* suf, uint32_t cn
         exclusive_scan<uint32_t>(count, count, size_t(words) * 32 * nw, &st->total, a, s);
         fm_place_kernel<<<grid, 256, 0, s>>>(sl, m, nw, pl, hits, em, ub, count, item);
         CURC_LAUNCH_CHECK();
-        {
-            cudaLaunchConfig_t cfg = {};
-            cudaLaunchAttribute at;
-            at.id = cudaLaunchAttributeClusterDimension;
-            // short lists meet a few hundred at a time: one block, whose
-            // barrier is cheaper than the cluster's
-            const unsigned blocks = m > 16384 ? 8 : 1;
-            at.val.clusterDim = {blocks, 1, 1};
-            cfg.gridDim = dim3(blocks);
-            cfg.blockDim = dim3(FM_WALK_THREADS);
-            cfg.stream = s;
-            cfg.attrs = &at;
-            cfg.numAttrs = 1;
-            const uint32_t* first = count;
-            const uint32_t* total = &st->total;
-            const uint32_t* plc = pl;
-            const unsigned long long* used = &st->used;
-            const FmItem* items = item;
-            CURC_CHECK(cudaLaunchKernelEx(&cfg, fm_walk_kernel, items, first, nw, total, off0, noffs, plc, used, cap,
-                                          next, prev, offset, tally));
-            CURC_LAUNCH_CHECK();
-        }
+        fm_starts_kernel<<<1, 256, 0, s>>>(count, nw, &st->total, noffs, start);
+        CURC_LAUNCH_CHECK();
+        walk_meetings(item, start, off0, noffs, pl, &st->used, cap, m, next, prev, offset, tally, s);
         cp.run(&st->len_in, m, &st->len_out[0], FreeLink{pl, prev}, MoveId{pl, pl2});
         cp.run(&st->len_in, m, &st->len_out[1], FreeLink{sl, next}, MoveId{sl, sl2});
         State h;

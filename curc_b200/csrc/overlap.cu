@@ -7,11 +7,15 @@
 // Determinism.  The reference links with atomicCAS, so which suffix wins a
 // contested prefix depends on scheduling.  Here the result is defined as the
 // sequential loop over suffixes in list order, and computed in parallel
-// exactly: every suffix whose equal-prefix run is claimed by it alone links
-// directly (runs of different suffix strings are disjoint); suffixes that
-// share a run are resolved by one thread per run, in list order.
+// exactly.  Which suffix meets which prefixes at which offset does not depend
+// on the links, so the meetings of several offsets are listed at once; then
+// they are walked offset by offset, one thread per run of equal prefixes
+// (runs of different strings are disjoint), its suffixes in list order.
+#include <algorithm>
+
 #include "compact.cuh"
 #include "stages.cuh"
+#include "walk.cuh"
 
 namespace curc {
 
@@ -41,370 +45,255 @@ __global__ void link_flags_kernel(const uint32_t* __restrict__ sorted, uint32_t 
     suf_f[i] = next[id] == INVALID;
 }
 
-__global__ void prefix_hash_kernel(const uint64_t* __restrict__ db, int W, int kip, int k, uint32_t mask,
-                                   uint32_t bmask, const uint32_t* __restrict__ pre, uint32_t m,
-                                   uint32_t* __restrict__ keys, uint32_t* __restrict__ present) {
+// The k-mer index of the prefixes of a stage.  A prefix that a suffix meets
+// holds the suffix's k-mer at kmer_index_pos, and its other k-mers too; the
+// further k-mers (positions qpos, lengths qlen, as far as the overlap
+// reaches) only filter.
+constexpr int OV_MAX_Q = 16;
+struct OverlapIndex {
+    const uint64_t* db;
+    int W, L, k, kip;
+    uint32_t mask;            // buckets - 1
+    uint32_t* present;        // bitmap of the prefixes' k-mer hashes (high 32 bits)
+    uint32_t bmask;
+    uint32_t* extra;          // one bitmap per further k-mer
+    uint32_t xmask;
+    int nq;
+    int16_t qpos[OV_MAX_Q], qlen[OV_MAX_Q];
+    const uint32_t* va;       // prefix ids sorted by (bucket, read)
+    const uint32_t* kr;       // bucket ranges
+};
+
+__device__ __forceinline__ uint32_t extra_bit(const OverlapIndex& c, const uint64_t* row, int at, int q) {
+    return uint32_t(murmur64(word_at(row, uint32_t(at + c.qpos[q]), c.qlen[q]))) & c.xmask;
+}
+
+__global__ void __launch_bounds__(256) prefix_index_kernel(OverlapIndex c, const uint32_t* __restrict__ pre, uint32_t m,
+                                                           uint32_t* __restrict__ keys, uint32_t* __restrict__ va) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m) return;
-    const uint64_t hv = murmur64(word_at(db + uint64_t(pre[i]) * W, kip, k));
-    keys[i] = uint32_t(hv & mask);
-    const uint32_t bit = uint32_t(hv >> 32) & bmask;
-    atomicOr(&present[bit >> 5], 1u << (bit & 31));
+    const uint32_t id = pre[i];
+    const uint64_t* row = c.db + uint64_t(id) * c.W;
+    const uint64_t hv = murmur64(word_at(row, c.kip, c.k));
+    const uint32_t h = uint32_t(hv) & c.mask;
+    keys[i] = h;
+    va[i] = id;
+    const uint32_t bit = uint32_t(hv >> 32) & c.bmask;
+    atomicOr(&c.present[bit >> 5], 1u << (bit & 31));
+    for (int q = 0; q < c.nq; ++q) {
+        const uint32_t x = extra_bit(c, row, 0, q);
+        atomicOr(&c.extra[uint64_t(q) * (uint64_t(c.xmask) + 1) / 32 + (x >> 5)], 1u << (x & 31));
+    }
 }
 
-__global__ void gather_rows_kernel(const uint64_t* __restrict__ db, int W, const uint32_t* __restrict__ ids,
-                                   uint32_t m, uint64_t* __restrict__ out) {
-    const uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (t >= uint64_t(m) * W) return;
-    const uint32_t i = uint32_t(t / W), w = uint32_t(t - uint64_t(i) * W);
-    out[t] = db[uint64_t(ids[i]) * W + w];
-}
-
-// keep flag of each suffix (not linked) as a 0/1 count for the scan
-__global__ void keep_count_kernel(const uint8_t* __restrict__ linked, uint32_t ms, uint32_t* __restrict__ keep) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < ms) keep[j] = !linked[j];
-}
-
-// moves the kept suffixes (id, packed words, offset mask) to their
-// compacted slots, preserving list order
-__global__ void compact_rows_kernel(const uint32_t* __restrict__ suf, const uint64_t* __restrict__ sufw, int W,
-                                    const uint32_t* __restrict__ mask, int mw, uint32_t ms, uint32_t ms2,
-                                    const uint32_t* __restrict__ keep, const uint32_t* __restrict__ pos,
-                                    uint32_t* __restrict__ suf2, uint64_t* __restrict__ sufw2,
-                                    uint32_t* __restrict__ mask2) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= ms || !keep[j]) return;
-    const uint32_t q = pos[j];
-    for (int w = 0; w < W; ++w) sufw2[uint64_t(q) * W + w] = sufw[uint64_t(j) * W + w];
-    for (int w = 0; w < mw; ++w) mask2[uint64_t(w) * ms2 + q] = mask[uint64_t(w) * ms + j];
-    suf2[q] = suf[j];
-}
-
+// (Keys sorted: neighbours count in the same sectors.)
 __global__ void bucket_count_kernel(const uint32_t* __restrict__ keys, uint32_t m, uint32_t* __restrict__ kr) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < m) atomicAdd(&kr[keys[i]], 1u);
 }
 
-// bit h of bfree: bucket h still holds a prefix without a predecessor
-__global__ void bucket_free_bits_kernel(const uint32_t* __restrict__ cnt, uint32_t words, uint32_t* __restrict__ bfree) {
-    for (uint32_t w = blockIdx.x * blockDim.x + threadIdx.x; w < words; w += gridDim.x * blockDim.x) {
-        uint32_t v = 0;
-        const uint4* c4 = reinterpret_cast<const uint4*>(cnt + uint64_t(w) * 32);
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const uint4 c = c4[q];
-            v |= uint32_t(c.x != 0) << (4 * q) | uint32_t(c.y != 0) << (4 * q + 1) | uint32_t(c.z != 0) << (4 * q + 2) |
-                 uint32_t(c.w != 0) << (4 * q + 3);
-        }
-        bfree[w] = v;
-    }
-}
-
-// Per prefix slot, while a pass runs: how many suffixes met the run that
-// starts there, the lowest of their list indices, and the head of the list
-// of their indices (one sector for the three).
-struct __align__(16) RunSlot {
-    uint32_t claim, lead, head, pad;
-};
-
-struct OverlapCtx {
-    const uint64_t* db;
-    int W, L, k, kip;
-    uint32_t mask;
-    const uint32_t* present;  // bitmap of prefix k-mer hashes (high 32 bits)
-    uint32_t bmask;
-    const uint32_t* va;  // prefix ids sorted by (bucket, read)
-    const uint32_t* kr;  // bucket ranges
-    uint32_t* free_cnt;  // per bucket: prefixes without a predecessor
-    uint32_t* bfree;     // per bucket: free_cnt != 0 (one bit, stays in L2)
-    uint32_t* next;
-    uint32_t* prev;
-    uint16_t* offset;
-};
-
-// First free non-self prefix of the equal run starting at lo, if equal;
-// sr = the suffix read's packed words.
-__device__ __forceinline__ bool link_first_free(const OverlapCtx& c, uint32_t s, const uint64_t* sr, uint32_t lo,
-                                                uint32_t e, int off) {
+// compress.cu:1476-1501: the prefixes of the suffix's bucket that equal
+// suffix[off, L) in [0, L - off): [lo, hi), false when there is none.
+__device__ __forceinline__ bool overlap_run(const OverlapIndex& c, const uint64_t* sr, int off, uint32_t& lo_out,
+                                            uint32_t& hi_out, uint32_t& compares) {
     const int cl = c.L - off;
-    for (uint32_t q = lo; q < e; ++q) {
-        const uint32_t pr = c.va[q];
-        if (pr == s || c.prev[pr] != INVALID) continue;
-        // the probe found prefix lo equal; later entries need the comparison
-        if (q == lo || cmp_span(c.db + uint64_t(pr) * c.W, 0, sr, off, cl) == 0) {
-            c.prev[pr] = s;
-            c.next[s] = pr;
-            c.offset[s] = uint16_t(off);
-            return true;
-        }
-        return false;
-    }
-    return false;
-}
-
-// A prefix of bucket h got its predecessor: the bucket's free count drops,
-// and its bit clears with the last one.
-__device__ __forceinline__ void take_from_bucket(const OverlapCtx& c, uint32_t h) {
-    if (atomicSub(&c.free_cnt[h], 1u) == 1u) atomicAnd(&c.bfree[h >> 5], ~(1u << (h & 31)));
-}
-
-// Offsets at which a suffix can meet a prefix at all: bit off of the
-// suffix's mask (word off/32 of the list's masks, stored word-major so a
-// pass reads one coalesced u32 per suffix) is set when the k-mer at kmer_index_pos+off is in the
-// presence bitmap of prefix k-mers.  The prefix set is fixed for the whole
-// stage, so this is computed once, with the suffix's words in registers.
-// Word wi of the masks (offsets 32 wi .. 32 wi + 31).  Words after the
-// first are computed only when the passes reach them, for the suffixes
-// still unlinked then.
-__global__ void offset_mask_kernel(OverlapCtx c, const uint64_t* __restrict__ sufw, uint32_t ms, int max_off, int wi,
-                                   uint32_t* __restrict__ mask) {
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= ms) return;
-    const uint64_t* sr = sufw + uint64_t(j) * c.W;
-    // 32 independent bitmap lookups in flight per thread
-    uint32_t word = 0;
-#pragma unroll
-    for (int b = 0; b < 32; ++b) {
-        const int off = wi * 32 + b;
-        if (off > 0 && off < max_off) {
-            const uint64_t hv = murmur64(word_at(sr, c.kip + off, c.k));
-            const uint32_t bit = uint32_t(hv >> 32) & c.bmask;
-            word |= ((c.present[bit >> 5] >> (bit & 31)) & 1u) << b;
-        }
-    }
-    mask[uint64_t(wi) * ms + j] = word;
-}
-
-// The suffixes probed in a pass: not yet linked, and with a prefix k-mer
-// present at this offset (mask bit).  Listing them first lets the probe and
-// resolve kernels give every thread real work, instead of warps that wait on
-// the few lanes whose suffix probes.
-struct ProbeFilter {
-    const uint8_t* linked;
-    const uint32_t* mrow;  // mask word off/32 of every suffix
-    uint32_t bit;
-    __device__ bool operator()(uint32_t j) const { return !linked[j] && ((mrow[j] >> bit) & 1u); }
-};
-struct ProbeListMove {
-    uint32_t* plist;
-    __device__ void operator()(uint32_t j, uint32_t d) const { plist[d] = j; }
-};
-
-// Three-way compare of prefix entry `it` ([0, cl)) with the suffix's
-// [off, off + cl); every comparison reads the prefix's row (counted in
-// `rows`).  Prefixes of one bucket share the indexed k-mer and, for true
-// overlaps, their first bases too, so a stored first word decided only a
-// quarter of the comparisons and cost more than it saved.
-__device__ __forceinline__ int cmp_prefix(const OverlapCtx& c, uint32_t it, const uint64_t* sr, int off, int cl,
-                                          uint32_t& rows) {
-    ++rows;
-    return cmp_span(c.db + uint64_t(c.va[it]) * c.W, 0, sr, off, cl);
-}
-
-// compress.cu:1476-1501, the part after the hash: lower bound of
-// suffix[off, L) among the prefix[0, L-off) of bucket h (whose free bit was
-// set).  Returns whether an equal prefix exists; then the hit (list index,
-// run start, bucket end, bucket) is set and the suffix joins the run's
-// claimers.
-__device__ __forceinline__ bool search_bucket(const OverlapCtx& c, const uint64_t* __restrict__ sufw, uint32_t j,
-                                              uint32_t h, int off, RunSlot* __restrict__ run,
-                                              uint32_t* __restrict__ gnext, uint4& hitrec, uint32_t& searched,
-                                              uint32_t& compares, uint32_t& rows) {
-    const int cl = c.L - off;
-    const uint64_t* sr = sufw + uint64_t(j) * c.W;
+    const uint32_t h = uint32_t(murmur64(word_at(sr, c.kip + off, c.k))) & c.mask;
     uint32_t lo = c.kr[h];
     const uint32_t e = c.kr[h + 1];
     uint32_t count = e - lo;
-    ++searched;
+    auto cmp = [&](uint32_t it) {
+        ++compares;
+        return cmp_span(c.db + uint64_t(c.va[it]) * c.W, 0, sr, off, cl);
+    };
     // lower bound; the entry it ends on (if below e) is the last one that
     // compared >= 0, so its comparison decides equality without a re-read
-    int at_hi = 1;
+    int at_lo = 1;
     while (count > 0) {
-        ++compares;
         const uint32_t step = count / 2, it = lo + step;
-        const int r = cmp_prefix(c, it, sr, off, cl, rows);
+        const int r = cmp(it);
         if (r < 0) {
             lo = it + 1;
             count -= step + 1;
         } else {
             count = step;
-            at_hi = r;
+            at_lo = r;
         }
     }
-    if (lo >= e || at_hi != 0) return false;
-    // run membership: count, lowest list index, and a list of members
-    atomicAdd(&run[lo].claim, 1u);
-    atomicMin(&run[lo].lead, j);
-    gnext[j] = atomicExch(&run[lo].head, j);
-    hitrec = make_uint4(j, lo, e, h);
+    if (lo >= e || at_lo != 0) return false;
+    uint32_t hi = lo + 1;
+    if (hi < e && cmp(hi) == 0) {
+        uint32_t n = e - ++hi;
+        while (n > 0) {
+            const uint32_t step = n / 2, it = hi + step;
+            if (cmp(it) <= 0) {
+                hi = it + 1;
+                n -= step + 1;
+            } else {
+                n = step;
+            }
+        }
+    }
+    lo_out = lo;
+    hi_out = hi;
     return true;
 }
 
-constexpr uint32_t PROBE_THREADS = 512;
+// Lists the meetings of the suffixes at offsets [off0, off0 + noffs).  One
+// thread takes one suffix and 32 offsets at a time (words_each times): the 32
+// k-mers are looked up in the presence bitmap with their loads in flight
+// together.  Every lane's lookup is a cache line of its own, which is what
+// bounds the kernel (a line a clock and SM), so the read itself lies in shared
+// memory: with two loads of the read per k-mer it ran at a third of the rate
+// (8M reads of 250 bp, 1.2e9 k-mers: 13.3 ms).  The k-mers
+// found are tested against the further k-mers' bitmaps (a read pair with an
+// error in the overlap fails there: of the 250 bp reads with rising errors
+// 4 in 100 of the first lookup's finds are meetings), and what is left is
+// searched in its bucket.  Room for the runs is reserved per warp; *used
+// counts the room asked for, and past cap the caller repeats with fewer
+// offsets.  Word w of suffix j has its meeting offsets in em[w * ms + j] and
+// the first of its runs at ub[w * ms + j].  tally: [0] k-mers found, [1]
+// buckets searched, [2] prefix rows compared.
+__global__ void __launch_bounds__(256) meet_kernel(OverlapIndex c, const uint32_t* __restrict__ suf, uint32_t ms,
+                                                   int off0, int noffs, int words_each, uint2* __restrict__ hits,
+                                                   uint32_t cap, unsigned long long* __restrict__ used,
+                                                   uint32_t* __restrict__ em, uint32_t* __restrict__ ub,
+                                                   unsigned long long* __restrict__ tally) {
+    extern __shared__ uint64_t s_rows[];
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
+    uint64_t* sr = s_rows + threadIdx.x * (c.W | 1);  // odd stride: few bank conflicts
+    if (j < ms) {
+        const uint64_t* row = c.db + uint64_t(suf[j]) * c.W;
+        for (int w = 0; w < c.W; ++w) sr[w] = row[w];
+    }
+    uint32_t found = 0, wanted = 0, compares = 0;
+    for (int w = blockIdx.y * words_each; w < int(blockIdx.y + 1) * words_each && w * 32 < noffs; ++w) {
+        const int o0 = off0 + w * 32, no = min(32, noffs - w * 32);
+        uint32_t maybe = 0;
+        if (j < ms) {
+            const BaseWindow win(sr, c.W, c.kip + o0);
+#pragma unroll
+            for (int b = 0; b < 32; ++b) {
+                if (b < no) {
+                    const uint32_t bit = uint32_t(murmur64(win.at(b, c.k)) >> 32) & c.bmask;
+                    maybe |= ((c.present[bit >> 5] >> (bit & 31)) & 1u) << b;
+                }
+            }
+            found += __popc(maybe);
+            for (uint32_t rest = maybe; rest; rest &= rest - 1) {
+                const int b = __ffs(rest) - 1, off = o0 + b;
+                for (int q = 0; q < c.nq; ++q) {
+                    if (c.qpos[q] + c.qlen[q] > c.L - off) break;
+                    const uint32_t x = extra_bit(c, sr, off, q);
+                    if (!((c.extra[uint64_t(q) * (uint64_t(c.xmask) + 1) / 32 + (x >> 5)] >> (x & 31)) & 1u)) {
+                        maybe &= ~(1u << b);
+                        break;
+                    }
+                }
+            }
+        }
+        const uint32_t want = __popc(maybe);
+        wanted += want;
+        uint32_t incl = want;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+            if (lane >= uint32_t(d)) incl += v;
+        }
+        unsigned long long base = 0;
+        if (lane == 31 && incl) base = atomicAdd(used, static_cast<unsigned long long>(incl));
+        base = __shfl_sync(0xFFFFFFFFu, base, 31) + (incl - want);
+        if (j < ms) {
+            uint32_t exact = 0, n = 0;
+            if (base + want <= cap) {
+                while (maybe) {
+                    const int b = __ffs(maybe) - 1;
+                    maybe &= maybe - 1;
+                    uint32_t lo, hi;
+                    if (overlap_run(c, sr, o0 + b, lo, hi, compares)) {
+                        hits[base + n++] = make_uint2(lo, hi);
+                        exact |= 1u << b;
+                    }
+                }
+            }
+            em[uint64_t(w) * ms + j] = exact;
+            ub[uint64_t(w) * ms + j] = uint32_t(base);
+        }
+    }
+    block_tally<unsigned long long>(found, &tally[0]);
+    block_tally<unsigned long long>(wanted, &tally[1]);
+    block_tally<unsigned long long>(compares, &tally[2]);
+}
 
-// Probes every listed suffix and lists the hits (hlist, *hcount; their
-// order is immaterial to the resolution).  Two phases per block, so that
-// the dependent loads of the bucket search run with full warps: every
-// thread hashes one listed suffix and tests its bucket's free bit (most
-// buckets have none left after the first passes), the suffixes that pass
-// are queued in shared memory (one slot range per warp, from a ballot),
-// and whenever a block's worth is queued, and at the end, each thread
-// searches the bucket of one queued suffix.  Which thread searches which
-// suffix does not change any result: a probe reads only the index and the
-// free bits, which no probe of the pass writes, and the run's claim count,
-// lowest member and member set do not depend on the order of the claims.
-// tally[0] counts probes, tally[1] hits, tally[4] probes that searched a
-// bucket, tally[5] prefix comparisons, tally[6] prefix rows read (for the
-// algorithmic bytes of the pass).
-__global__ void __launch_bounds__(PROBE_THREADS) probe_kernel(OverlapCtx c, const uint64_t* __restrict__ sufw,
-                                                              const uint32_t* __restrict__ plist,
-                                                              const uint32_t* __restrict__ pcount, int off,
-                                                              RunSlot* __restrict__ run, uint32_t* __restrict__ gnext,
-                                                              uint4* __restrict__ hlist, uint32_t* __restrict__ hcount,
-                                                              unsigned long long* __restrict__ tally) {
-    __shared__ uint4 s_hits[PROBE_THREADS];
-    // queued (suffix, bucket) pairs: fewer than PROBE_THREADS are left
-    // after a search round, and one round of hashing adds at most
-    // PROBE_THREADS
-    __shared__ uint2 s_q[2 * PROBE_THREADS];
-    __shared__ uint32_t s_n, s_base, s_qn;
-    uint32_t probes = 0, hits = 0, searched = 0, compares = 0, rows = 0;
-    const uint32_t np = *pcount;
-    const uint32_t lane = threadIdx.x & 31u;
-    if (threadIdx.x == 0) s_qn = 0;
+// Meetings per suffix and per offset.
+__global__ void __launch_bounds__(256) meet_count_kernel(const uint32_t* __restrict__ em, uint32_t ms, int words,
+                                                         uint32_t* __restrict__ per_suffix,
+                                                         uint32_t* __restrict__ per_off) {
+    __shared__ uint32_t h[WALK_MAX_OFFS];
+    for (int o = threadIdx.x; o < words * 32; o += 256) h[o] = 0;
     __syncthreads();
-    for (uint64_t b0 = uint64_t(blockIdx.x) * PROBE_THREADS;; b0 += uint64_t(gridDim.x) * PROBE_THREADS) {
-        const bool more = b0 < np;  // the same for the whole block
-        if (more) {
-            const uint64_t q = b0 + threadIdx.x;
-            bool keep = false;
-            uint32_t j = 0, h = 0;
-            if (q < np) {
-                ++probes;
-                j = plist[q];
-                const uint64_t* sr = sufw + uint64_t(j) * c.W;
-                h = uint32_t(murmur64(word_at(sr, c.kip + off, c.k)) & c.mask);
-                // every prefix of the bucket has a predecessor already: no
-                // link is possible for any suffix that meets it, so none
-                // needs to claim it
-                keep = (c.bfree[h >> 5] >> (h & 31)) & 1u;
-            }
-            const uint32_t bal = __ballot_sync(0xffffffffu, keep);
-            uint32_t slot = 0;
-            if (lane == 0 && bal) slot = atomicAdd(&s_qn, uint32_t(__popc(bal)));
-            slot = __shfl_sync(0xffffffffu, slot, 0);
-            if (keep) s_q[slot + uint32_t(__popc(bal & ((1u << lane) - 1u)))] = make_uint2(j, h);
-            __syncthreads();
+    for (uint32_t j = blockIdx.x * 256 + threadIdx.x; j < ms; j += gridDim.x * 256) {
+        uint32_t c = 0;
+        for (int w = 0; w < words; ++w) {
+            uint32_t m = em[uint64_t(w) * ms + j];
+            c += __popc(m);
+            for (; m; m &= m - 1) atomicAdd(&h[w * 32 + __ffs(m) - 1], 1u);
         }
-        const uint32_t qn = s_qn;  // the same for the whole block (read after a barrier)
-        if (qn >= PROBE_THREADS || (!more && qn > 0)) {
-            // search the last `take` queued suffixes; the rest stay in place
-            const uint32_t take = qn < PROBE_THREADS ? qn : PROBE_THREADS;
-            bool hit = false;
-            uint4 rec;
-            if (threadIdx.x < take) {
-                const uint2 e = s_q[qn - take + threadIdx.x];
-                hit = search_bucket(c, sufw, e.x, e.y, off, run, gnext, rec, searched, compares, rows);
-                hits += hit;
-            }
-            if (threadIdx.x == 0) s_n = 0;
-            __syncthreads();
-            if (threadIdx.x == 0) s_qn = qn - take;
-            if (hit) s_hits[atomicAdd(&s_n, 1u)] = rec;
-            __syncthreads();
-            if (threadIdx.x == 0 && s_n) s_base = atomicAdd(hcount, s_n);
-            __syncthreads();
-            if (threadIdx.x < s_n) hlist[s_base + threadIdx.x] = s_hits[threadIdx.x];
-            __syncthreads();
-        }
-        if (!more) break;
+        per_suffix[j] = c;
     }
-    block_tally<unsigned long long>(probes, &tally[0]);
-    block_tally<unsigned long long>(hits, &tally[1]);
-    block_tally<unsigned long long>(searched, &tally[4]);
-    block_tally<unsigned long long>(compares, &tally[5]);
-    block_tally<unsigned long long>(rows, &tally[6]);
+    __syncthreads();
+    for (int o = threadIdx.x; o < words * 32; o += 256)
+        if (h[o]) atomicAdd(&per_off[o], h[o]);
 }
 
-constexpr uint32_t RESOLVE_BATCH = 16;
-
-// A suffix alone on its run links directly.  A run claimed by several
-// suffixes is resolved by its lowest-index member, which visits the members
-// in list order (ascending index, in sorted batches from one walk of the
-// member list each) and gives each the first free non-self prefix, exactly
-// the sequential loop of compress.cu:1474.  The run's bookkeeping is reset
-// for the next pass by the thread that used it.  tally[2] counts links,
-// tally[3] the members of contested runs.
-
-__global__ void __launch_bounds__(512) resolve_kernel(OverlapCtx c, const uint32_t* __restrict__ suf,
-                                                      const uint64_t* __restrict__ sufw,
-                                                      const uint4* __restrict__ hlist,
-                                                      const uint32_t* __restrict__ hcount, int off,
-                                                      RunSlot* __restrict__ run, const uint32_t* __restrict__ gnext,
-                                                      uint8_t* __restrict__ linked,
-                                                      unsigned long long* __restrict__ tally) {
-    uint32_t links = 0, contested = 0;
-    const uint32_t nh = *hcount;
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < nh; q += gridDim.x * blockDim.x) {
-        // members of a run share its start, bucket end and bucket
-        const uint4 hr = hlist[q];
-        const uint32_t j = hr.x, lo = hr.y, e = hr.z, h = hr.w;
-        const RunSlot rs = run[lo];
-        const uint32_t n = rs.claim;
-        if (n == 1) {
-            if (link_first_free(c, suf[j], sufw + uint64_t(j) * c.W, lo, e, off)) {
-                linked[j] = 1;
-                ++links;
-                take_from_bucket(c, h);
-            }
-        } else if (rs.lead == j) {
-            // members in ascending list index: each walk of the run's member
-            // list keeps the RESOLVE_BATCH smallest above the last one
-            // handled, in order, so a run of n members takes
-            // ceil(n / RESOLVE_BATCH) walks instead of n
-            contested += n;
-            uint32_t buf[RESOLVE_BATCH];
-            uint32_t last = 0;
-            bool first = true;
-            for (;;) {
-                uint32_t cnt = 0;
-                for (uint32_t m = rs.head; m != INVALID; m = gnext[m]) {
-                    if (!first && m <= last) continue;
-                    if (cnt == RESOLVE_BATCH && m >= buf[RESOLVE_BATCH - 1]) continue;
-                    uint32_t t = cnt < RESOLVE_BATCH ? cnt++ : RESOLVE_BATCH - 1;
-                    while (t > 0 && buf[t - 1] > m) {
-                        buf[t] = buf[t - 1];
-                        --t;
-                    }
-                    buf[t] = m;
-                }
-                for (uint32_t t = 0; t < cnt; ++t) {
-                    const uint32_t best = buf[t];
-                    if (link_first_free(c, suf[best], sufw + uint64_t(best) * c.W, lo, e, off)) {
-                        linked[best] = 1;
-                        ++links;
-                        take_from_bucket(c, h);
-                    }
-                }
-                if (cnt < RESOLVE_BATCH) break;
-                last = buf[RESOLVE_BATCH - 1];
-                first = false;
-            }
-        } else {
-            continue;  // the run's lowest member resolves it
-        }
-        run[lo] = RunSlot{0, INVALID, INVALID, 0};
+// start[o] = meetings of the offsets before o (one block; noffs <= 512).
+__global__ void __launch_bounds__(512) meet_starts_kernel(const uint32_t* __restrict__ per_off, int noffs,
+                                                          uint32_t* __restrict__ start) {
+    __shared__ uint32_t s[512];
+    const int t = threadIdx.x;
+    s[t] = t < noffs ? per_off[t] : 0;
+    __syncthreads();
+    for (int d = 1; d < 512; d <<= 1) {
+        const uint32_t v = t >= d ? s[t - d] : 0;
+        __syncthreads();
+        s[t] += v;
+        __syncthreads();
     }
-    block_tally<unsigned long long>(links, &tally[2]);
-    block_tally<unsigned long long>(contested, &tally[3]);
+    if (t < noffs) start[t + 1] = s[t];
+    if (t == 0) start[0] = 0;
 }
 
-__global__ void set_u32_kernel(uint32_t* p, uint32_t v) { *p = v; }
+// Meetings in suffix order with their sort keys (offset, run).
+template <class K>
+__global__ void __launch_bounds__(256) meet_place_kernel(const uint32_t* __restrict__ suf, uint32_t ms, int words,
+                                                         const uint32_t* __restrict__ em,
+                                                         const uint32_t* __restrict__ ub,
+                                                         const uint2* __restrict__ hits,
+                                                         const uint32_t* __restrict__ first,
+                                                         const uint32_t* __restrict__ va, int run_bits,
+                                                         Meeting* __restrict__ item, K* __restrict__ key,
+                                                         uint32_t* __restrict__ idx) {
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= ms) return;
+    uint32_t at = first[j];
+    const uint32_t s = suf[j];
+    for (int w = 0; w < words; ++w) {
+        uint32_t m = em[uint64_t(w) * ms + j];
+        if (!m) continue;
+        uint32_t u = ub[uint64_t(w) * ms + j];
+        for (; m; m &= m - 1) {
+            const uint2 h = hits[u++];
+            item[at] = Meeting{s, h.x, h.y, va[h.x]};
+            key[at] = K(w * 32 + __ffs(m) - 1) << run_bits | h.x;
+            idx[at] = at;
+            ++at;
+        }
+    }
+}
 
-__global__ void run_slots_init_kernel(RunSlot* run, uint32_t n) {
+__global__ void gather_meetings_kernel(const Meeting* __restrict__ in, const uint32_t* __restrict__ idx, uint32_t n,
+                                       Meeting* __restrict__ out) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) run[i] = RunSlot{0, INVALID, INVALID, 0};
+    if (i < n) out[i] = in[idx[i]];
 }
 
 __global__ void chain_res_kernel(uint32_t n, const uint32_t* __restrict__ next, const uint32_t* __restrict__ prev,
@@ -445,12 +334,6 @@ __global__ void gather_flags_kernel(const uint32_t* __restrict__ ids, uint32_t m
     nf[i] = !v;
 }
 
-inline int log2_exact(uint32_t x) {
-    int b = 0;
-    while ((1u << b) < x) ++b;
-    return b;
-}
-
 }  // namespace
 
 void dedupe_links(const uint64_t* db, int W, const uint32_t* sorted, uint32_t m, uint32_t* next, uint32_t* prev,
@@ -460,6 +343,36 @@ void dedupe_links(const uint64_t* db, int W, const uint32_t* sorted, uint32_t m,
     CURC_LAUNCH_CHECK();
 }
 
+namespace {
+// Meetings sorted by (offset, run); inside a run in list order.
+template <class K>
+Meeting* sorted_meetings(const uint32_t* suf, uint32_t ms, int words, const uint32_t* em, const uint32_t* ub,
+                         const uint2* hits, const uint32_t* first, const uint32_t* va, int run_bits, int bits,
+                         uint32_t n, Arena& a, cudaStream_t s) {
+    Meeting* item = a.alloc<Meeting>(n);
+    Meeting* out = a.alloc<Meeting>(n);
+    K* key = a.alloc<K>(n);
+    uint32_t* idx = a.alloc<uint32_t>(n);
+    meet_place_kernel<K><<<grid_for(ms, 256), 256, 0, s>>>(suf, ms, words, em, ub, hits, first, va, run_bits, item, key,
+                                                           idx);
+    CURC_LAUNCH_CHECK();
+    radix_sort_pairs<K, uint32_t>(key, idx, n, 0, bits, a, s);
+    gather_meetings_kernel<<<grid_for(n, 256), 256, 0, s>>>(item, idx, n, out);
+    CURC_LAUNCH_CHECK();
+    return out;
+}
+}  // namespace
+
+// Links the suffixes offset after offset (compress.cu:1473-1532), in stages
+// of several offsets: index the free prefixes, list every meeting of the
+// unlinked suffixes with them, sort the meetings and walk them.  A list of up
+// to OV_ALL suffixes takes all offsets in one stage: its time was that of
+// three launches per offset (39 us an offset, 3.2 ms for 2,000 reads).
+// Longer lists take tune.check_every offsets first and twice as many in each
+// next stage, since most suffixes link in the first offsets and what has
+// linked is not listed again.
+constexpr uint32_t OV_ALL = 1u << 19;
+constexpr uint64_t OV_BITMAPS = 80ull << 20;  // bytes, of 126 MB of L2
 void overlap_link(const BlockParams& p, const uint64_t* db, const uint32_t* sorted, uint32_t m, uint32_t* next,
                   uint32_t* prev, uint16_t* offset, Arena& a, cudaStream_t s, OverlapStats* st) {
     if (m == 0) return;
@@ -470,173 +383,169 @@ void overlap_link(const BlockParams& p, const uint64_t* db, const uint32_t* sort
     CURC_LAUNCH_CHECK();
     uint32_t* pre = a.alloc<uint32_t>(m);
     uint32_t* suf = a.alloc<uint32_t>(m);
-    uint32_t* suf2 = a.alloc<uint32_t>(m);
-    uint32_t* counts = a.alloc<uint32_t>(4);
-    select_flagged(sorted, pre_f, pre, m, counts + 0, a, s);
-    select_flagged(sorted, suf_f, suf, m, counts + 1, a, s);
-    uint32_t hc[2];
-    read_small(hc, counts, 8, s);
-    const uint32_t mp = hc[0];
-    uint32_t ms = hc[1];
-
-    SubStage sp_index("overlap.index");
-    // index: stable sort of prefixes by bucket (compress.cu:1440-1471)
-    // The table size does not change which prefixes a suffix meets: equal
-    // strings share a bucket whatever its size, and other bucket entries are
-    // rejected by the comparison.  The reference sizes it to the prefix count
-    // (get_hash_size); four times that keeps most probes of unlinkable
-    // suffixes at one empty bucket instead of a binary search.
-    const uint32_t hs = hash_size_for(uint64_t(mp) * uint64_t(p.tune.table_factor));
-    // presence bitmap, 16 bits per prefix (2^20..2^32 bits): a test that stays
-    // in L2 rejects most suffixes without touching the bucket table
-    int bbits = 20;
-    while (bbits < 32 && (1ull << bbits) < uint64_t(mp) * uint64_t(p.tune.bitmap_bits)) ++bbits;
-    const uint64_t bwords = (1ull << bbits) / 32;
-    uint32_t* present = a.alloc<uint32_t>(bwords);
-    CURC_CHECK(cudaMemsetAsync(present, 0, bwords * 4, s));
-    OverlapCtx c{db, p.W, p.L, p.k, p.kip, hs - 1, present, uint32_t((1ull << bbits) - 1), pre, nullptr, nullptr,
-                 nullptr, next, prev, offset};
-    uint32_t* keys = a.alloc<uint32_t>(mp ? mp : 1);
-    SubStage sp_sort("overlap.index_sort");
-    if (mp) {
-        prefix_hash_kernel<<<grid_for(mp, 256), 256, 0, s>>>(db, p.W, p.kip, p.k, c.mask, c.bmask, pre, mp, keys,
-                                                             present);
-        CURC_LAUNCH_CHECK();
-        radix_sort_pairs<uint32_t, uint32_t>(keys, pre, mp, 0, log2_exact(hs), a, s);
-    }
-    uint32_t* kr = a.alloc<uint32_t>(size_t(hs) + 2);
-    CURC_CHECK(cudaMemsetAsync(kr, 0, (size_t(hs) + 2) * sizeof(uint32_t), s));
-    if (mp) {
-        bucket_count_kernel<<<grid_for(mp, 256), 256, 0, s>>>(keys, mp, kr);
-        CURC_LAUNCH_CHECK();
-    }
-    uint32_t* free_cnt = a.alloc<uint32_t>(size_t(hs) + 32);
-    uint32_t* bfree = a.alloc<uint32_t>(hs / 32 + 1);
-    CURC_CHECK(cudaMemcpyAsync(free_cnt, kr, size_t(hs) * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
-    bucket_free_bits_kernel<<<grid_for(hs / 32, 256), 256, 0, s>>>(free_cnt, hs / 32, bfree);
-    CURC_LAUNCH_CHECK();
-    c.free_cnt = free_cnt;
-    c.bfree = bfree;
-    exclusive_scan<uint32_t>(kr, kr, size_t(hs) + 2, nullptr, a, s);
-    c.kr = kr;
-    sp_sort.stop();
-
-    // per prefix slot: run claim count, lowest claimer, member list head
-    RunSlot* run = a.alloc<RunSlot>(mp ? mp : 1);
-    run_slots_init_kernel<<<grid_for(mp ? mp : 1, 256), 256, 0, s>>>(run, mp ? mp : 1);
-    CURC_LAUNCH_CHECK();
-    uint32_t* gnext = a.alloc<uint32_t>(ms ? ms : 1);
-    uint32_t* keepc = a.alloc<uint32_t>(ms ? ms : 1);
-    uint32_t* kpos = a.alloc<uint32_t>(ms ? ms : 1);
-    // suffix reads and offset masks in list order
-    const int W = p.W, mw = (p.max_off + 31) / 32;
-    uint64_t* sufw = a.alloc<uint64_t>(size_t(ms ? ms : 1) * W);
-    uint64_t* sufw2 = a.alloc<uint64_t>(size_t(ms ? ms : 1) * W);
-    uint32_t* mask = a.alloc<uint32_t>(size_t(ms ? ms : 1) * mw);
-    uint32_t* mask2 = a.alloc<uint32_t>(size_t(ms ? ms : 1) * mw);
-    uint8_t* linked = a.alloc<uint8_t>(ms ? ms : 1);
-    CURC_CHECK(cudaMemsetAsync(linked, 0, ms ? ms : 1, s));
-    SubStage sp_mask("overlap.index_mask");
-    if (ms) {
-        gather_rows_kernel<<<grid_for(uint64_t(ms) * W, 256), 256, 0, s>>>(db, W, suf, ms, sufw);
-        CURC_LAUNCH_CHECK();
-        if (mp) {
-            offset_mask_kernel<<<grid_for(ms, 256), 256, 0, s>>>(c, sufw, ms, p.max_off, 0, mask);
-            CURC_LAUNCH_CHECK();
-        }
-    }
-    sp_mask.stop();
-    // probes, probes that met a prefix, links, contested members
-    unsigned long long* tally = a.alloc<unsigned long long>(7);
-    CURC_CHECK(cudaMemsetAsync(tally, 0, 56, s));
-    sp_index.stop();
-
-    // List of size ms, of which `active` are unlinked; compacted once half
-    // of it has linked.  Passes are queued without a host round trip; the
-    // host reads the link count every few passes to compact or stop.
-    uint32_t* plist = a.alloc<uint32_t>(ms ? ms : 1);
-    uint4* hlist = a.alloc<uint4>(ms ? ms : 1);
-    uint32_t* hcount = a.alloc<uint32_t>(p.max_off + 1);  // one per pass
-    CURC_CHECK(cudaMemsetAsync(hcount, 0, size_t(p.max_off + 1) * 4, s));
-    uint32_t* dcount = a.alloc<uint32_t>(2);  // [0] list size, [1] listed probes
-    set_u32_kernel<<<1, 1, 0, s>>>(dcount, ms);
-    CURC_LAUNCH_CHECK();
-    Compactor cp(ms, a, s);
-    const int gp = resident_grid(probe_kernel, PROBE_THREADS, ms ? ms : 1);
-    const int gr = resident_grid(resolve_kernel, 512, ms ? ms : 1);
-    const int CHECK_EVERY = p.tune.check_every;
-    uint32_t passes = 0, active = ms;
-    uint64_t links_seen = 0, active_sum = 0;
-    const uint32_t ms0 = ms;
-    int words = 1;  // mask words computed so far
-    auto compact = [&] {
-        SubStage sp_comp("overlap.compact");
-        const int g = grid_for(ms, 256);
-        keep_count_kernel<<<g, 256, 0, s>>>(linked, ms, keepc);
-        CURC_LAUNCH_CHECK();
-        exclusive_scan<uint32_t>(keepc, kpos, ms, nullptr, a, s);
-        compact_rows_kernel<<<g, 256, 0, s>>>(suf, sufw, W, mask, words, ms, active, keepc, kpos, suf2, sufw2, mask2);
-        CURC_LAUNCH_CHECK();
-        std::swap(suf, suf2);
-        std::swap(sufw, sufw2);
-        std::swap(mask, mask2);
-        ms = active;
-        CURC_CHECK(cudaMemsetAsync(linked, 0, ms ? ms : 1, s));
-        set_u32_kernel<<<1, 1, 0, s>>>(dcount, ms);
-        CURC_LAUNCH_CHECK();
+    // what the host reads back: list lengths, the room asked for, and the
+    // meetings' starts per offset
+    struct State {
+        uint32_t mp, ms, mp_out, ms_out;
+        unsigned long long used, tally[3];
+        uint32_t start[WALK_MAX_OFFS + 1];
     };
-    for (int off = 1; off < p.max_off && active > 0 && mp > 0; ++off) {
-        if ((off >> 5) >= words) {  // next mask word, for the unlinked suffixes only
-            const uint64_t links = read_scalar(tally + 2, s);
-            active -= uint32_t(links - links_seen);
-            links_seen = links;
-            if (active < ms) compact();
-            if (ms) {
-                SubStage sp_mw("overlap.index_mask");
-                offset_mask_kernel<<<grid_for(ms, 256), 256, 0, s>>>(c, sufw, ms, p.max_off, words, mask);
-                CURC_LAUNCH_CHECK();
+    State* d = a.alloc<State>(1);
+    State h;
+    CURC_CHECK(cudaMemsetAsync(d, 0, sizeof(State), s));
+    select_flagged(sorted, pre_f, pre, m, &d->mp, a, s);
+    select_flagged(sorted, suf_f, suf, m, &d->ms, a, s);
+    read_small(&h, d, 8, s);
+    uint32_t mp = h.mp, ms = h.ms;
+    const uint32_t ms0 = ms;
+    uint64_t active_sum = 0, met = 0;
+    uint32_t passes = 0;
+    const int step0 = ms <= OV_ALL ? p.max_off : p.tune.check_every;
+    int step = step0;
+    if (mp && ms && p.max_off > 1) {
+        uint32_t* pre2 = a.alloc<uint32_t>(mp);
+        uint32_t* suf2 = a.alloc<uint32_t>(ms);
+        Compactor cp(std::max(mp, ms), a, s);
+        const uint32_t cap = uint32_t(std::min<uint64_t>(0xF0000000ull, std::max<uint64_t>(uint64_t(4) << 20, uint64_t(ms) * 2)));
+        uint2* hits = a.alloc<uint2>(cap);
+        OverlapIndex c = {};
+        uint32_t *bits = nullptr, *keys = nullptr, *va = nullptr, *kr = nullptr;
+        uint32_t indexed = 0;  // prefixes in the index (0: none yet)
+        uint64_t bits_cap = 0;
+        auto build_index = [&](int off) {
+            SubStage sp_index("overlap.index");
+            // Buckets: the table's size does not change which prefixes a
+            // suffix meets (equal strings share a bucket whatever its size);
+            // presence bitmaps: 16 bits per prefix for the indexed k-mer, 8
+            // for each further one, fewer where all together would not stay
+            // in L2.
+            int hbits = 10, bbits = 16, xbits = 15;
+            while (hbits < 31 && (4ull << hbits) < uint64_t(mp) * uint64_t(p.tune.table_factor)) ++hbits;
+            while (bbits < 32 && (1ull << bbits) < uint64_t(mp) * uint64_t(p.tune.bitmap_bits)) ++bbits;
+            while (xbits < 31 && (1ull << xbits) < uint64_t(mp) * 8) ++xbits;
+            c = OverlapIndex{};
+            c.db = db;
+            c.W = p.W;
+            c.L = p.L;
+            c.k = p.k;
+            c.kip = p.kip;
+            c.mask = uint32_t((1ull << hbits) - 1);
+            auto further = [&](int pos, int len) {
+                if (len < 12 || c.nq == OV_MAX_Q || pos + len > p.L - off) return;
+                c.qpos[c.nq] = int16_t(pos);
+                c.qlen[c.nq++] = int16_t(len);
+            };
+            further(0, std::min(32, p.kip));
+            for (int q = p.kip + p.k; q + 32 <= p.L - off; q += 32) further(q, 32);
+            auto bitmap_bytes = [&] { return ((1ull << bbits) + (1ull << xbits) * uint64_t(c.nq)) / 8; };
+            while (bitmap_bytes() > OV_BITMAPS && xbits > 20) {
+                --xbits;
+                if (bitmap_bytes() > OV_BITMAPS && (1ull << bbits) > uint64_t(mp) * 8) --bbits;
             }
-            ++words;
-            if (active == 0) break;
+            c.bmask = uint32_t((1ull << bbits) - 1);
+            c.xmask = uint32_t((1ull << xbits) - 1);
+            const uint64_t bwords = (1ull << bbits) / 32, xwords = (1ull << xbits) / 32 * uint64_t(c.nq);
+            // (fewer further k-mers can leave a later index more bits)
+            if (bwords + xwords > bits_cap) bits = a.alloc<uint32_t>(bits_cap = bwords + xwords);
+            if (!indexed) {  // the first index has the most prefixes
+                keys = a.alloc<uint32_t>(mp);
+                va = a.alloc<uint32_t>(mp);
+                kr = a.alloc<uint32_t>((size_t(1) << hbits) + 2);
+            }
+            indexed = mp;
+            c.present = bits;
+            c.extra = bits + bwords;
+            CURC_CHECK(cudaMemsetAsync(bits, 0, (bwords + xwords) * 4, s));
+            CURC_CHECK(cudaMemsetAsync(kr, 0, ((size_t(1) << hbits) + 2) * 4, s));
+            prefix_index_kernel<<<grid_for(mp, 256), 256, 0, s>>>(c, pre, mp, keys, va);
+            CURC_LAUNCH_CHECK();
+            radix_sort_pairs<uint32_t, uint32_t>(keys, va, mp, 0, hbits, a, s);
+            bucket_count_kernel<<<grid_for(mp, 256), 256, 0, s>>>(keys, mp, kr);
+            CURC_LAUNCH_CHECK();
+            exclusive_scan<uint32_t>(kr, kr, (size_t(1) << hbits) + 2, nullptr, a, s);
+            c.va = va;
+            c.kr = kr;
+        };
+        for (int off = 1; off < p.max_off && mp && ms;) {
+            const int noffs = std::min({step, p.max_off - off, WALK_MAX_OFFS}), words = (noffs + 31) / 32;
+            // an index of prefixes of which most are still free serves on: the
+            // walk passes over the others
+            if (!indexed || uint64_t(mp) * 4 < uint64_t(indexed) * 3) build_index(off);
+            auto mk2 = a.mark();
+            SubStage sp_meet("overlap.probe");
+            uint32_t* em = a.alloc<uint32_t>(size_t(words) * ms);
+            uint32_t* ub = a.alloc<uint32_t>(size_t(words) * ms);
+            uint32_t* per = a.alloc<uint32_t>(ms);
+            uint32_t* per_off = a.alloc<uint32_t>(WALK_MAX_OFFS);
+            CURC_CHECK(cudaMemsetAsync(per_off, 0, WALK_MAX_OFFS * 4, s));
+            CURC_CHECK(cudaMemsetAsync(&d->used, 0, 8, s));
+            // long lists fill the device with a thread per suffix
+            const int each = ms > (1u << 18) ? words : 1;
+            meet_kernel<<<dim3(unsigned(div_up(ms, 256)), unsigned(div_up(words, each))), 256,
+                          size_t(256) * (p.W | 1) * 8, s>>>(c, suf, ms, off, noffs, each, hits, cap, &d->used, em, ub,
+                                                            d->tally);
+            CURC_LAUNCH_CHECK();
+            meet_count_kernel<<<resident_grid(meet_count_kernel, 256, ms), 256, 0, s>>>(em, ms, words, per, per_off);
+            CURC_LAUNCH_CHECK();
+            meet_starts_kernel<<<1, 512, 0, s>>>(per_off, noffs, d->start);
+            CURC_LAUNCH_CHECK();
+            exclusive_scan<uint32_t>(per, per, ms, nullptr, a, s);
+            read_small(&h, d, sizeof(State), s);
+            sp_meet.stop();
+            if (h.used > cap) {  // too many for the room: fewer offsets
+                a.release(mk2);
+                step = std::max(1, noffs / 2);
+                continue;
+            }
+            const uint32_t n = h.start[noffs];
+            active_sum += uint64_t(ms) * noffs;
+            met += n;
+            passes += uint32_t(noffs);
+            SubStage sp_walk("overlap.resolve");
+            if (n) {
+                int run_bits = 1, off_bits = 1;
+                while ((1ull << run_bits) < indexed) ++run_bits;
+                while ((1 << off_bits) < noffs) ++off_bits;
+                const int kb = run_bits + off_bits;
+                const Meeting* item =
+                    kb <= 32 ? sorted_meetings<uint32_t>(suf, ms, words, em, ub, hits, per, va, run_bits, kb, n, a, s)
+                             : sorted_meetings<uint64_t>(suf, ms, words, em, ub, hits, per, va, run_bits, kb, n, a, s);
+                walk_stage(item, h.start, d->start, off, noffs, va, &d->used, cap, next, prev, offset, s);
+            }
+            sp_walk.stop();
+            off += noffs;
+            if (off < p.max_off) {  // what is left for the next stage
+                SubStage sp_comp("overlap.compact");
+                cp.run(&d->mp, mp, &d->mp_out, FreeLink{pre, prev}, MoveId{pre, pre2});
+                cp.run(&d->ms, ms, &d->ms_out, FreeLink{suf, next}, MoveId{suf, suf2});
+                CURC_CHECK(cudaMemcpyAsync(&d->mp, &d->mp_out, 8, cudaMemcpyDeviceToDevice, s));
+                std::swap(pre, pre2);
+                std::swap(suf, suf2);
+                read_small(&h, d, 8, s);
+                // where few link, more offsets together waste little
+                const uint64_t linked = ms - h.ms;
+                step *= linked * 16 < ms ? 8 : linked * 4 < ms ? 4 : 2;
+                mp = h.mp;
+                ms = h.ms;
+                if (ms <= OV_ALL) step = p.max_off;
+                sp_comp.stop();
+            }
+            a.release(mk2);
         }
-        ++passes;
-        active_sum += active;  // as of the last check
-        SubStage sp_probe("overlap.probe_resolve");
-        SubStage sp_filter("overlap.filter");
-        cp.run(dcount, ms, dcount + 1,
-               ProbeFilter{linked, mask + uint64_t(off >> 5) * ms, uint32_t(off & 31)}, ProbeListMove{plist});
-        sp_filter.stop();
-        SubStage sp_pk("overlap.probe");
-        probe_kernel<<<gp, PROBE_THREADS, 0, s>>>(c, sufw, plist, dcount + 1, off, run, gnext,
-                                        hlist, hcount + off, tally);
-        CURC_LAUNCH_CHECK();
-        sp_pk.stop();
-        SubStage sp_rk("overlap.resolve");
-        resolve_kernel<<<gr, 512, 0, s>>>(c, suf, sufw, hlist, hcount + off, off, run,
-                                          gnext, linked, tally);
-        CURC_LAUNCH_CHECK();
-        sp_rk.stop();
-        sp_probe.stop();
-        if (off % CHECK_EVERY != 0 && off + 1 < p.max_off) continue;
-        const uint64_t links = read_scalar(tally + 2, s);
-        active -= uint32_t(links - links_seen);
-        links_seen = links;
-        if (active * 2 < ms) compact();
+        cp.check();
     }
-    cp.check();
     if (st) {
-        unsigned long long t[7];
-        read_small(t, tally, 56, s);
+        read_small(&h, d, sizeof(State), s);
         st->passes = passes;
-        st->links = uint32_t(t[2]);
-        st->contested = uint32_t(t[3]);
+        st->links = uint32_t(met);
+        st->contested = 0;
         st->suffixes = ms0;
         st->active_sum = active_sum;
-        st->probes = t[0];
-        st->hits = t[1];
-        st->searched = t[4];
-        st->compares = t[5];
-        st->rows = t[6];
+        st->probes = h.tally[0];
+        st->hits = met;
+        st->searched = h.tally[1];
+        st->compares = h.tally[2];
+        st->rows = h.tally[2];
     }
     a.release(mk);
 }

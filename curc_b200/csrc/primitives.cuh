@@ -117,7 +117,12 @@ struct SubStage {
         if (t) t->end_span(i);
         t = nullptr;
     }
-    ~SubStage() { stop(); }
+    ~SubStage() {
+        try {
+            stop();
+        } catch (...) {  // leaving a scope on an error: that one is reported
+        }
+    }
 };
 
 // out[i] = sum(in[0..i)); optionally *total = sum(in[0..n)) (device pointer).
