@@ -20,6 +20,8 @@
 // index) and are cut in parallel (below); chains are ordered by their first
 // list index with a radix sort and placed by exclusive scans; every read
 // then writes its bases independently.
+#include <mutex>
+
 #include "stages.cuh"
 
 namespace curc {
@@ -386,6 +388,244 @@ __global__ void pack_ref_kernel(const uint8_t* __restrict__ seq, uint64_t len, u
     }
 }
 
+// ---------------------------------------------------------------- short lists
+//
+// Up to ASM_SMALL members by one block: links as list indices in shared
+// memory, ranks by pointer jumping, cycles cut by one thread each, chains
+// placed by a scan over their first list indices.  One launch and one read
+// back, where the general path takes 40 launches and six (0.3 ms for a list of
+// 20 reads, three lists a block).
+constexpr uint32_t ASM_SMALL = 8192;
+constexpr int ASM_THREADS = 1024, ASM_EACH = ASM_SMALL / ASM_THREADS;
+constexpr uint16_t ASM_NONE = 0xFFFFu;
+constexpr size_t asm_small_bytes(uint32_t m) { return size_t(m) * (3 * 2 + 4 + 4 * 2) + 256; }
+
+// out[0] = bases of all chains; *err: a link leaves the list.  place[i] = the
+// first base of member i.
+__global__ void __launch_bounds__(ASM_THREADS) assemble_small_kernel(
+    const uint32_t* __restrict__ ids, uint32_t m, uint32_t n, const uint32_t* __restrict__ next,
+    const uint32_t* __restrict__ prev, const uint16_t* __restrict__ offset, int L, uint8_t is_n,
+    uint32_t* pos_in_ids, DevRecord* __restrict__ rec, uint64_t* __restrict__ place, uint8_t* __restrict__ tail,
+    uint64_t* __restrict__ out, uint32_t* __restrict__ err) {
+    extern __shared__ __align__(16) uint8_t asm_smem[];
+    uint32_t* acc = reinterpret_cast<uint32_t*>(asm_smem);  // bases before this member (later: per first index)
+    uint16_t* nx = reinterpret_cast<uint16_t*>(acc + m);
+    uint16_t* pv = nx + m;
+    uint16_t* off = pv + m;
+    uint16_t* jump = off + m;
+    uint16_t* cnt = jump + m;
+    uint16_t* mn = cnt + m;
+    uint16_t* far = mn + m;
+    __shared__ uint32_t s_warp[32], s_warp2[32];
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5;
+    for (uint32_t i = t; i < m; i += ASM_THREADS) pos_in_ids[ids[i]] = i;
+    __syncthreads();
+    // the member's list index of a linked read
+    auto index = [&](uint32_t x) -> uint16_t {
+        if (x == INVALID) return ASM_NONE;
+        const uint32_t p = x < n ? pos_in_ids[x] : INVALID;
+        if (p >= m || ids[p] != x) {
+            atomicExch(err, 1u);
+            return ASM_NONE;
+        }
+        return uint16_t(p);
+    };
+    for (uint32_t i = t; i < m; i += ASM_THREADS) {
+        const uint32_t x = ids[i];
+        nx[i] = index(next[x]);
+        pv[i] = index(prev[x]);
+        off[i] = nx[i] == ASM_NONE ? 0 : offset[x];
+    }
+    __syncthreads();
+    uint32_t a[ASM_EACH];
+    uint16_t j[ASM_EACH], c[ASM_EACH], lo[ASM_EACH], f[ASM_EACH];
+    // ranks; returns whether this thread saw a cycle
+    auto rank = [&]() -> bool {
+#pragma unroll
+        for (int e = 0; e < ASM_EACH; ++e) {
+            const uint32_t i = t + e * ASM_THREADS;
+            if (i >= m) continue;
+            const uint16_t p = pv[i];
+            jump[i] = p;
+            acc[i] = p == ASM_NONE ? 0 : off[p];
+            cnt[i] = p != ASM_NONE;
+            mn[i] = p == ASM_NONE ? uint16_t(i) : min(uint16_t(i), p);
+            far[i] = p == ASM_NONE ? uint16_t(i) : p;
+        }
+        __syncthreads();
+        for (uint32_t span = 1; span < 2 * m; span *= 2) {
+#pragma unroll
+            for (int e = 0; e < ASM_EACH; ++e) {
+                const uint32_t i = t + e * ASM_THREADS;
+                j[e] = ASM_NONE;
+                if (i >= m || jump[i] == ASM_NONE) continue;
+                const uint32_t p = jump[i];
+                j[e] = uint16_t(p);
+                a[e] = acc[i] + acc[p];
+                c[e] = uint16_t(cnt[i] + cnt[p]);
+                lo[e] = min(mn[i], mn[p]);
+                f[e] = far[p];
+            }
+            bool any = false;
+#pragma unroll
+            for (int e = 0; e < ASM_EACH; ++e) any |= j[e] != ASM_NONE;
+            if (!__syncthreads_or(any)) return false;
+            uint16_t nj[ASM_EACH];
+#pragma unroll
+            for (int e = 0; e < ASM_EACH; ++e) nj[e] = j[e] == ASM_NONE ? ASM_NONE : jump[j[e]];
+            __syncthreads();
+#pragma unroll
+            for (int e = 0; e < ASM_EACH; ++e) {
+                const uint32_t i = t + e * ASM_THREADS;
+                if (j[e] == ASM_NONE) continue;
+                jump[i] = nj[e];
+                acc[i] = a[e];
+                cnt[i] = c[e];
+                mn[i] = lo[e];
+                far[i] = f[e];
+            }
+            __syncthreads();
+        }
+        bool cyc = false;
+#pragma unroll
+        for (int e = 0; e < ASM_EACH; ++e) {
+            const uint32_t i = t + e * ASM_THREADS;
+            if (i < m) cyc |= jump[i] != ASM_NONE;
+        }
+        return cyc;
+    };
+    bool cyc = rank();
+    if (__syncthreads_or(cyc)) {
+        // the cycle's first listed read r walks it from its successor round to
+        // itself and cuts after the first read of largest offset
+#pragma unroll
+        for (int e = 0; e < ASM_EACH; ++e) {
+            const uint32_t r = t + e * ASM_THREADS;
+            if (r >= m || jump[r] == ASM_NONE || mn[r] != r) continue;
+            uint32_t x = nx[r], best = x;
+            for (uint32_t step = 0; step < m && x != r && x < m; ++step) {
+                x = nx[x];
+                if (x < m && off[x] > off[best]) best = x;
+            }
+            if (x != r) {
+                atomicExch(err, 1u);
+                continue;
+            }
+            pv[nx[best]] = ASM_NONE;
+            nx[best] = ASM_NONE;
+        }
+        __syncthreads();
+        cyc = rank();
+        if (__syncthreads_or(cyc)) {
+            if (t == 0) atomicExch(err, 2u);
+            return;
+        }
+    }
+    // what follows needs each member's rank in registers and its chain's first
+    // list index; the shared arrays then hold per first index the chain's
+    // bases and members, and their exclusive scans
+    uint16_t head[ASM_EACH];
+#pragma unroll
+    for (int e = 0; e < ASM_EACH; ++e) {
+        const uint32_t i = t + e * ASM_THREADS;
+        if (i >= m) continue;
+        a[e] = acc[i];
+        c[e] = cnt[i];
+        lo[e] = mn[i];
+        head[e] = far[i];
+    }
+    __syncthreads();
+    uint16_t* key = jump;  // per head: the chain's first list index
+#pragma unroll
+    for (int e = 0; e < ASM_EACH; ++e) {
+        const uint32_t i = t + e * ASM_THREADS;
+        if (i >= m) continue;
+        if (nx[i] == ASM_NONE) key[head[e]] = lo[e];  // the tail's minimum covers the chain
+        acc[i] = 0;
+        cnt[i] = 0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < ASM_EACH; ++e) {
+        const uint32_t i = t + e * ASM_THREADS;
+        if (i < m && nx[i] == ASM_NONE) {
+            acc[lo[e]] = a[e] + uint32_t(L);
+            cnt[lo[e]] = uint16_t(c[e] + 1);
+        }
+    }
+    __syncthreads();
+    // exclusive scans over the list, ASM_EACH consecutive entries per thread
+    uint32_t vb = 0, vc = 0;
+    for (uint32_t i = t * ASM_EACH; i < (t + 1) * ASM_EACH && i < m; ++i) {
+        vb += acc[i];
+        vc += cnt[i];
+    }
+    uint32_t xb = vb, xc = vc;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t yb = __shfl_up_sync(0xFFFFFFFFu, xb, d), yc = __shfl_up_sync(0xFFFFFFFFu, xc, d);
+        if (lane >= uint32_t(d)) {
+            xb += yb;
+            xc += yc;
+        }
+    }
+    if (lane == 31) {
+        s_warp[warp] = xb;
+        s_warp2[warp] = xc;
+    }
+    __syncthreads();
+    uint32_t ob = xb - vb, oc = xc - vc, total = 0;
+    for (uint32_t w = 0; w < 32; ++w) {
+        if (w < warp) {
+            ob += s_warp[w];
+            oc += s_warp2[w];
+        }
+        total += s_warp[w];
+    }
+    for (uint32_t i = t * ASM_EACH; i < (t + 1) * ASM_EACH && i < m; ++i) {
+        const uint32_t wb = acc[i], wc = cnt[i];
+        acc[i] = ob;
+        cnt[i] = uint16_t(oc);
+        ob += wb;
+        oc += wc;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int e = 0; e < ASM_EACH; ++e) {
+        const uint32_t i = t + e * ASM_THREADS;
+        if (i >= m) continue;
+        const uint32_t k = key[head[e]];
+        const uint64_t at = uint64_t(acc[k]) + a[e];
+        DevRecord d;
+        d.read_id = ids[i];
+        d.is_n = is_n;
+        d.strand = 0;
+        d.pad = 0;
+        d.pos = at;
+        rec[uint32_t(cnt[k]) + c[e]] = d;
+        place[i] = at;
+        tail[i] = nx[i] == ASM_NONE;
+    }
+    if (t == 0) out[0] = total;
+}
+
+// Each member writes its bases (a warp per member).
+__global__ void __launch_bounds__(256) place_small_kernel(const uint32_t* __restrict__ ids, uint32_t m,
+                                                          const uint64_t* __restrict__ place,
+                                                          const uint8_t* __restrict__ tail,
+                                                          const uint16_t* __restrict__ offset,
+                                                          const uint64_t* __restrict__ db,
+                                                          const uint8_t* __restrict__ ascii, int L, int W,
+                                                          uint8_t* __restrict__ seq) {
+    const uint32_t i = (blockIdx.x * 256 + threadIdx.x) >> 5;
+    if (i >= m) return;
+    const uint32_t x = ids[i];
+    const int nb = tail[i] ? L : offset[x];
+    uint8_t* out = seq + place[i];
+    for (int j = int(threadIdx.x & 31u); j < nb; j += 32)
+        out[j] = ascii ? ascii[uint64_t(x) * L + j] : uint8_t("ACGT"[code_at(db + uint64_t(x) * W, j)]);
+}
+
 inline int rounds_for(uint32_t m) {
     int r = 1;
     while ((1ull << r) < uint64_t(m) + 1) ++r;
@@ -481,6 +721,46 @@ void pack_ascii_ref(const uint8_t* seq, uint64_t len, uint64_t* packed, cudaStre
     CURC_LAUNCH_CHECK();
 }
 
+namespace {
+void assemble_small(const uint64_t* db, const uint8_t* ascii, int L, int W, const uint32_t* ids, uint32_t m,
+                    uint32_t n, const uint32_t* next, const uint32_t* prev, const uint16_t* offset, bool is_n,
+                    uint32_t* pos_in_ids, Assembled& out, Arena& a, cudaStream_t s) {
+    SubStage sp("assembly.small");
+    static std::mutex mu;
+    static bool done[64] = {};
+    int dev = 0;
+    CURC_CHECK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) throw std::runtime_error("device ordinal out of range");
+    {
+        std::lock_guard<std::mutex> g(mu);
+        if (!done[dev]) {
+            CURC_CHECK(cudaFuncSetAttribute(assemble_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                            int(asm_small_bytes(ASM_SMALL))));
+            done[dev] = true;
+        }
+    }
+    uint64_t* place = a.alloc<uint64_t>(m);
+    uint8_t* tail = a.alloc<uint8_t>(m);
+    uint64_t* res = a.alloc<uint64_t>(2);  // bases, error
+    CURC_CHECK(cudaMemsetAsync(res, 0, 16, s));
+    assemble_small_kernel<<<1, ASM_THREADS, asm_small_bytes(m), s>>>(ids, m, n, next, prev, offset, L, is_n ? 1 : 0,
+                                                                     pos_in_ids, out.records, place, tail, res,
+                                                                     reinterpret_cast<uint32_t*>(res + 1));
+    CURC_LAUNCH_CHECK();
+    uint64_t h[2];
+    read_small(h, res, 16, s);
+    if (uint32_t(h[1]) == 1) throw std::runtime_error("assemble: a chain link leaves the member set");
+    if (h[1]) throw std::runtime_error("assemble: unresolved chain links after cutting cycles");
+    out.len = h[0];
+    out.seq = a.alloc<uint8_t>(out.len + 64);
+    place_small_kernel<<<grid_for(uint64_t(m) * 32, 256), 256, 0, s>>>(ids, m, place, tail, offset, db, ascii, L, W,
+                                                                       out.seq);
+    CURC_LAUNCH_CHECK();
+    out.packed = a.alloc<uint64_t>((out.len + 31) / 32 + 1);
+    pack_ascii_ref(out.seq, out.len, out.packed, s);
+}
+}  // namespace
+
 void assemble(const uint64_t* db, const uint8_t* ascii, int L, int W, const uint32_t* ids, uint32_t m,
               uint32_t n_total, const uint32_t* next, const uint32_t* prev, const uint16_t* offset, bool is_n,
               Assembled& out, Arena& a, cudaStream_t s) {
@@ -495,6 +775,10 @@ void assemble(const uint64_t* db, const uint8_t* ascii, int L, int W, const uint
     }
     const size_t n = n_total;
     uint32_t* pos_in_ids = a.alloc<uint32_t>(n);
+    if (m <= ASM_SMALL) {
+        assemble_small(db, ascii, L, W, ids, m, n_total, next, prev, offset, is_n, pos_in_ids, out, a, s);
+        return;
+    }
     uint32_t* nx = a.alloc<uint32_t>(n);
     uint32_t* pv = a.alloc<uint32_t>(n);
     CURC_CHECK(cudaMemcpyAsync(nx, next, n * 4, cudaMemcpyDeviceToDevice, s));

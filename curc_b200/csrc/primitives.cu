@@ -1005,7 +1005,8 @@ __global__ void scatter_ids_kernel(const uint32_t* __restrict__ vals, const uint
 }
 }  // namespace
 
-void sort_rows(const uint64_t* db, int W, int last_bits, uint32_t* ids, size_t n, Arena& a, cudaStream_t s) {
+void sort_rows(const uint64_t* db, int W, int last_bits, uint32_t* ids, size_t n, Arena& a, cudaStream_t s,
+               int first_bits) {
     // Stable lexicographic order of the rows (compress.cu:1400-1407 under a
     // stable comparison sort; ties keep input order).  First by the first
     // word; then only the runs of rows that share it are ordered by the
@@ -1028,7 +1029,7 @@ void sort_rows(const uint64_t* db, int W, int last_bits, uint32_t* ids, size_t n
         // the first-word sort alone (the tie runs below read a count back to the host)
         SubStage sp("sort_dedupe.first_word");
         gather_words(db, ids, n, W, 0, k0, s);
-        radix_sort_pairs<uint64_t, uint32_t>(k0, ids, n, W == 1 ? 64 - last_bits : 0, 64, a, s);
+        radix_sort_pairs<uint64_t, uint32_t>(k0, ids, n, W == 1 ? 64 - last_bits : 0, first_bits, a, s);
     }
     if (W > 1) {
         uint8_t* large = a.alloc<uint8_t>(n);

@@ -148,8 +148,10 @@ void radix_sort_pairs(K* keys, V* vals, size_t n, int begin_bit, int end_bit, Ar
 // over all words): ids is permuted in place.
 void sort_ids_by_reads(const uint64_t* db, int W, int L, uint32_t* ids, size_t n, Arena& a, cudaStream_t s);
 
-// The same for rows of W words of which the last one's top last_bits count.
-void sort_rows(const uint64_t* rows, int W, int last_bits, uint32_t* ids, size_t n, Arena& a, cudaStream_t s);
+// The same for rows of W words of which the last one's top last_bits count;
+// the first words are below 2^first_bits (fewer passes).
+void sort_rows(const uint64_t* rows, int W, int last_bits, uint32_t* ids, size_t n, Arena& a, cudaStream_t s,
+               int first_bits = 64);
 
 // Gather 64-bit words: out[i] = src[idx[i] * stride + word].
 void gather_words(const uint64_t* src, const uint32_t* idx, size_t n, int stride, int word, uint64_t* out,

@@ -17,13 +17,13 @@
 //
 // B200 design: one thread per probe, the four probes of a segment in
 // adjacent lanes; the 36-mer is compared before the match is extended, and
-// a maximal match met by a run of consecutive segments is extended once; the
-// extensions compare 32 bases per step with XOR and count-leading-zeros
-// instead of one base per step; the triples are ordered with three stable
-// radix passes; the acceptance walk (each decision depends on the end of the
-// previous kept span) is rewritten as a successor chain followed by binary
-// lifting; the map streams and the string compaction are built in parallel
+// a maximal match met by a run of consecutive segments is extended once, by a
+// warp, 1024 bases a step, and gives one triple; the triples are sorted as
+// rows of three words; the acceptance walk (each decision depends on the end
+// of the previous kept span) is walked by one thread for a few triples and
+// rewritten as a successor chain followed by binary lifting for many; the map streams and the string compaction are built in parallel
 // from scans over the kept spans.
+#include <algorithm>
 #include <cstring>
 
 #include "block.cuh"
@@ -89,6 +89,19 @@ __global__ void rm_hash_kernel(const uint64_t* __restrict__ ref, uint64_t count,
 __global__ void rc_ascii_kernel(const uint8_t* __restrict__ in, uint64_t n, uint8_t* __restrict__ out) {
     for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += uint64_t(gridDim.x) * blockDim.x)
         out[i] = uint8_t(comp_char(char(in[n - 1 - i])));
+}
+
+// Reverse complement of a packed string of n bases, and zero words behind it.
+__global__ void rc_packed_kernel(const uint64_t* __restrict__ in, uint64_t n, uint64_t* __restrict__ out,
+                                 uint64_t words) {
+    for (uint64_t w = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; w < words; w += uint64_t(gridDim.x) * blockDim.x) {
+        uint64_t v = 0;
+        if (w * 32 < n) {
+            const int nb = n - w * 32 < 32 ? int(n - w * 32) : 32;
+            v = revcomp_kmer(word_unaligned(in, n - w * 32 - nb, nb), nb) << (64 - 2 * nb);
+        }
+        out[w] = v;
+    }
 }
 
 struct RmIndex {
@@ -157,16 +170,56 @@ __device__ bool probe_candidate(const RmIndex& ix, const uint64_t* dest, uint64_
     return false;
 }
 
+// match_right and match_left by a warp: 1024 bases a step, 32 per lane.
+__device__ __forceinline__ uint64_t match_right_warp(const uint64_t* a, uint64_t ao, const uint64_t* b, uint64_t bo,
+                                                     uint64_t lim) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint64_t k = 0; k < lim; k += 1024) {
+        const uint64_t at = k + 32 * lane;
+        uint32_t eq = 0;  // equal bases of this lane's part; 32 when whole
+        if (at < lim) {
+            const int nb = lim - at < 32 ? int(lim - at) : 32;
+            const uint64_t x = word_unaligned(a, ao + at, nb) ^ word_unaligned(b, bo + at, nb);
+            eq = x ? uint32_t(__clzll(x) - (64 - 2 * nb)) / 2 : uint32_t(nb);
+        }
+        const uint32_t cut = __ballot_sync(0xFFFFFFFFu, eq < 32);
+        if (cut) {
+            const int l = __ffs(cut) - 1;
+            return min(lim, k + 32 * l + __shfl_sync(0xFFFFFFFFu, eq, l));
+        }
+    }
+    return lim;
+}
+__device__ __forceinline__ uint64_t match_left_warp(const uint64_t* a, uint64_t ao, const uint64_t* b, uint64_t bo,
+                                                    uint64_t lim) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint64_t k = 0; k < lim; k += 1024) {
+        const uint64_t at = k + 32 * lane;
+        uint32_t eq = 0;
+        if (at < lim) {
+            const int nb = lim - at < 32 ? int(lim - at) : 32;
+            const uint64_t x = word_unaligned(a, ao - at - nb, nb) ^ word_unaligned(b, bo - at - nb, nb);
+            eq = x ? uint32_t(__ffsll(x) - 1) / 2 : uint32_t(nb);
+        }
+        const uint32_t cut = __ballot_sync(0xFFFFFFFFu, eq < 32);
+        if (cut) {
+            const int l = __ffs(cut) - 1;
+            return min(lim, k + 32 * l + __shfl_sync(0xFFFFFFFFu, eq, l));
+        }
+    }
+    return lim;
+}
+
 // The maximal match through an accepted probe: extended right from the end
-// of the 36-mer and left from its start, as the reference does.
+// of the 36-mer and left from its start, as the reference does.  One warp.
 __device__ Hit extend_full(const RmIndex& ix, const uint64_t* dest, uint64_t dl, uint64_t dpad, uint64_t dpos,
                            uint64_t spos) {
     const uint64_t d0 = dpos + RM_K, s0 = spos + RM_K;
     const uint64_t dlim = d0 <= dl ? dl - d0 : dpad - d0;
     const uint64_t slim = s0 <= ix.rl ? ix.rl - s0 : 0;
-    const uint64_t right = d0 + match_right(dest, d0, ix.ref, s0, min(dlim, slim));
+    const uint64_t right = d0 + match_right_warp(dest, d0, ix.ref, s0, min(dlim, slim));
     const uint64_t lmax = min(dpos, spos);
-    const uint64_t k = match_left(dest, dpos, ix.ref, spos, lmax);
+    const uint64_t k = match_left_warp(dest, dpos, ix.ref, spos, lmax);
     const uint64_t p1 = k < lmax ? dpos - 1 - k : dpos - k;
     const uint64_t p2 = k < lmax ? spos - 1 - k : spos - k;
     return Hit{p2 + 1, right - p1 - 1, p1 + 1};
@@ -208,17 +261,24 @@ __device__ __forceinline__ bool rm_follows(const uint8_t* flag, const ulonglong2
     return c.x + RM_K <= dl && c.y - c.x == p.y - p.x;
 }
 
-// The first segment of each run extends its match once and writes the hit
-// for the whole run.
-__global__ void extend_runs_kernel(RmIndex ix, const uint64_t* __restrict__ dest, uint64_t dl, uint64_t dpad,
-                                   uint64_t segs, const uint8_t* __restrict__ flag,
-                                   const ulonglong2* __restrict__ cand, Hit* __restrict__ hits) {
-    for (uint64_t i = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; i < segs; i += uint64_t(gridDim.x) * blockDim.x) {
-        if (!flag[i] || rm_follows(flag, cand, i, dl)) continue;
-        const Hit h = extend_full(ix, dest, dl, dpad, cand[i].x, cand[i].y);
-        hits[i] = h;
-        for (uint64_t j = i + 1; j < segs && flag[j] && rm_follows(flag, cand, j, dl); ++j) hits[j] = h;
+// lead[j]: segment j accepted and starts a run; *accepted += accepted segments.
+__global__ void __launch_bounds__(256) run_leads_kernel(const uint8_t* __restrict__ flag,
+                                                        const ulonglong2* __restrict__ cand, uint64_t segs, uint64_t dl,
+                                                        uint8_t* __restrict__ lead, uint32_t* __restrict__ accepted) {
+    uint32_t n = 0;
+    for (uint64_t j = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < segs; j += uint64_t(gridDim.x) * blockDim.x) {
+        const bool f = flag[j];
+        n += f;
+        lead[j] = f && !rm_follows(flag, cand, j, dl);
     }
+    block_tally<uint32_t>(n, accepted);
+}
+
+// Beyond the capacity nothing is taken: `last` is the first segment dropped.
+__global__ void drop_leads_kernel(uint8_t* __restrict__ lead, uint64_t segs, const uint32_t* __restrict__ last) {
+    for (uint64_t j = uint64_t(*last) + uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; j < segs;
+         j += uint64_t(gridDim.x) * blockDim.x)
+        lead[j] = 0;
 }
 
 __global__ void probe_ascii_kernel(RmIndex ix, const uint8_t* __restrict__ dest, uint64_t dl, uint64_t dic,
@@ -251,13 +311,12 @@ __global__ void probe_ascii_kernel(RmIndex ix, const uint8_t* __restrict__ dest,
     }
 }
 
-__global__ void gather_hits_kernel(const Hit* __restrict__ in, const uint32_t* __restrict__ sel, uint32_t c,
-                                   uint64_t dl, bool dest_is_ref, Hit* __restrict__ out) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= c) return;
-    Hit h = in[sel[t]];
-    h.dst = dl - (h.dst + h.len);  // back to forward coordinates (compress.cu:903-908)
-    if (dest_is_ref) {             // compress.cu:910-927
+// A hit in forward coordinates (compress.cu:903-908), and for the pseudogenome
+// against itself cut where it overlaps its source (compress.cu:910-927), as a
+// row to sort: (dst, src, len).
+__device__ __forceinline__ void write_row(Hit h, uint64_t dl, bool dest_is_ref, uint64_t* __restrict__ row) {
+    h.dst = dl - (h.dst + h.len);
+    if (dest_is_ref) {
         if (h.src > h.dst) {
             const uint64_t x = h.src;
             h.src = h.dst;
@@ -270,49 +329,83 @@ __global__ void gather_hits_kernel(const Hit* __restrict__ in, const uint32_t* _
             h.dst += margin;
         }
     }
-    out[t] = h;
+    row[0] = h.dst;
+    row[1] = h.src;
+    row[2] = h.len;
 }
 
-__global__ void hit_key_kernel(const Hit* __restrict__ h, const uint32_t* __restrict__ idx, uint32_t c, int field,
-                               uint64_t* __restrict__ key) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= c) return;
-    const Hit x = h[idx[t]];
-    key[t] = field == 0 ? x.len : (field == 1 ? x.src : x.dst);
-}
-
-__global__ void hit_unique_kernel(const Hit* __restrict__ h, const uint32_t* __restrict__ idx, uint32_t c,
-                                  uint8_t* __restrict__ keep, Hit* __restrict__ sorted) {
-    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= c) return;
-    const Hit x = h[idx[t]];
-    sorted[t] = x;
-    bool k = true;
-    if (t > 0) {
-        const Hit y = h[idx[t - 1]];
-        k = !(x.src == y.src && x.len == y.len && x.dst == y.dst);
+// One warp per run: its match, extended once.  Every segment of the run would
+// give the same hit, and equal hits do not change what is kept below, so one
+// per run goes on (a match of 100,000 bases is 8,000 segments).
+__global__ void __launch_bounds__(256) extend_runs_kernel(RmIndex ix, const uint64_t* __restrict__ dest, uint64_t dl,
+                                                          uint64_t dpad, const uint32_t* __restrict__ sel, uint32_t c,
+                                                          const ulonglong2* __restrict__ cand, bool dest_is_ref,
+                                                          uint64_t* __restrict__ rows, uint32_t* __restrict__ idx) {
+    for (uint32_t t = (blockIdx.x * 256 + threadIdx.x) >> 5; t < c; t += gridDim.x * 8) {
+        const ulonglong2 p = cand[sel[t]];
+        const Hit h = extend_full(ix, dest, dl, dpad, p.x, p.y);
+        if ((threadIdx.x & 31u) == 0) {
+            write_row(h, dl, dest_is_ref, rows + uint64_t(t) * 3);
+            idx[t] = t;
+        }
     }
-    keep[t] = k;
 }
 
-__global__ void compact_hits_kernel(const Hit* __restrict__ in, const uint32_t* __restrict__ sel, uint32_t c,
-                                    Hit* __restrict__ out) {
+__global__ void gather_rows3_kernel(const Hit* __restrict__ hits, const uint32_t* __restrict__ sel, uint32_t c,
+                                    uint64_t dl, bool dest_is_ref, uint64_t* __restrict__ rows,
+                                    uint32_t* __restrict__ idx) {
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t < c) out[t] = in[sel[t]];
+    if (t >= c) return;
+    write_row(hits[sel[t]], dl, dest_is_ref, rows + uint64_t(t) * 3);
+    idx[t] = t;
 }
 
-// compress.cu:946-992, the acceptance walk over the sorted distinct hits:
+__global__ void sorted_hits_kernel(const uint64_t* __restrict__ rows, const uint32_t* __restrict__ idx, uint32_t c,
+                                   Hit* __restrict__ out) {
+    const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+    if (t >= c) return;
+    const uint64_t* r = rows + uint64_t(idx[t]) * 3;
+    out[t] = Hit{r[1], r[2], r[0]};
+}
+
+// compress.cu:946-992, the acceptance walk over the sorted hits:
 // a hit starting before the end `pos` of the last kept span is trimmed to
 // start there (or dropped when covered), and kept when 50 or more bases
 // remain; a kept hit sets pos to its end.  Trimming keeps the end, so with
 // end_i = dst_i + len_i, hit i is kept iff len_i >= 50 and end_i >= pos + 50,
-// and then pos = end_i.  The kept hits are therefore the chain
+// and then pos = end_i.  (A hit equal to the one before it is never kept: its
+// end is at most pos, or both fail.)  The kept hits are therefore the chain
 //   start -> nxt(start) -> nxt(nxt(start)) -> ...
 // where nxt(j) is the first i > j with len_i >= 50 and end_i >= end_j + 50
 // (the start has end 0).  nxt is found for every hit at once by descending
 // a sparse table of range maxima of the eligible ends, and the chain is
 // followed by binary lifting, so no step is sequential.  Node c is the
 // start and c + 1 the end of the chain.
+
+// A few hits: the walk itself, by one thread out of shared memory.
+constexpr uint32_t ACCEPT_SMALL = 2048;
+__global__ void __launch_bounds__(256) accept_small_kernel(const Hit* __restrict__ h, uint32_t c,
+                                                           uint8_t* __restrict__ kept, uint64_t* __restrict__ adst,
+                                                           uint64_t* __restrict__ alen) {
+    __shared__ uint64_t dst[ACCEPT_SMALL], len[ACCEPT_SMALL];
+    for (uint32_t i = threadIdx.x; i < c; i += 256) {
+        dst[i] = h[i].dst;
+        len[i] = h[i].len;
+        kept[i] = 0;
+    }
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    uint64_t pos = 0;
+    for (uint32_t i = 0; i < c; ++i) {
+        const uint64_t end = dst[i] + len[i];
+        if (len[i] < uint64_t(RM_MIN) || end < pos + RM_MIN) continue;
+        const uint64_t d = max(dst[i], pos);
+        kept[i] = 1;
+        adst[i] = d;
+        alen[i] = end - d;
+        pos = end;
+    }
+}
 
 // eligible ends: level 0 of the range-maximum table
 __global__ void accept_ends_kernel(const Hit* __restrict__ h, uint32_t c, uint64_t* __restrict__ m0) {
@@ -430,26 +523,56 @@ __global__ void map_len_kernel(const uint32_t* __restrict__ sel, uint32_t K, con
 }
 
 // Each kept span [sd_k, se_k) becomes one '%'; every other symbol moves left
-// by the symbols removed before it.
-__global__ void compact_string_kernel(const uint8_t* __restrict__ in, uint64_t dl, const uint64_t* __restrict__ sd,
-                                      const uint64_t* __restrict__ se, const uint64_t* __restrict__ removed,
-                                      uint64_t kept, uint8_t* __restrict__ out) {
-    for (uint64_t q = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < dl; q += uint64_t(gridDim.x) * blockDim.x) {
-        uint64_t lo = 0, cnt = kept;  // lo = number of spans starting at or before q
+// by the symbols removed before it.  A thread writes 16 bytes: the spans that
+// start in or before them come from one search over the spans' places in the
+// output (sd_k - removed_k), instead of one per symbol.
+__global__ void __launch_bounds__(256) compact_string_kernel(const uint8_t* __restrict__ in, uint64_t out_len,
+                                                             const uint64_t* __restrict__ sd,
+                                                             const uint64_t* __restrict__ se,
+                                                             const uint64_t* __restrict__ removed, uint64_t kept,
+                                                             uint8_t* __restrict__ out) {
+    for (uint64_t o = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) * 16; o < out_len;
+         o += uint64_t(gridDim.x) * blockDim.x * 16) {
+        uint64_t lo = 0, cnt = kept;  // lo = number of spans whose '%' lies before o
         while (cnt > 0) {
             const uint64_t step = cnt / 2, it = lo + step;
-            if (sd[it] <= q) {
+            if (sd[it] - removed[it] < o) {
                 lo = it + 1;
                 cnt -= step + 1;
             } else {
                 cnt = step;
             }
         }
-        if (lo > 0 && q < se[lo - 1]) {
-            if (q == sd[lo - 1]) out[q - removed[lo - 1]] = '%';
-            continue;
+        const int n = out_len - o < 16 ? int(out_len - o) : 16;
+        uint64_t next = lo < kept ? sd[lo] - removed[lo] : ~0ull;  // the next '%'
+        uint64_t shift = removed[lo];                              // input place - output place
+        uint32_t w[4] = {0, 0, 0, 0};
+        if (n == 16 && next >= o + 16) {  // no span: four words, each from two aligned ones
+            const uint64_t q = o + shift;
+            const uint32_t* p = reinterpret_cast<const uint32_t*>(in + (q & ~uint64_t(3)));
+            const uint32_t by = uint32_t(q & 3);
+            uint32_t a = p[0];
+#pragma unroll
+            for (int t = 0; t < 4; ++t) {
+                const uint32_t b = (t < 3 || by) ? p[t + 1] : 0;
+                w[t] = __funnelshift_r(a, b, 8 * by);
+                a = b;
+            }
+        } else {
+            for (int t = 0; t < n; ++t) {
+                uint8_t v;
+                if (o + t == next) {
+                    v = '%';
+                    ++lo;
+                    next = lo < kept ? sd[lo] - removed[lo] : ~0ull;
+                    shift = removed[lo];
+                } else {
+                    v = in[o + t + shift];
+                }
+                w[t / 4] |= uint32_t(v) << (8 * (t % 4));
+            }
         }
-        out[q - removed[lo]] = in[q];
+        *reinterpret_cast<uint4*>(out + o) = make_uint4(w[0], w[1], w[2], w[3]);  // out has 16 bytes to spare
     }
 }
 
@@ -491,10 +614,10 @@ struct RmResult {
     uint64_t len_len = 0;
 };
 
-// One destination (compress.cu:856-993).  `dest` is the ASCII string on the
-// device (forward strand).
-void refmatch_one(const RmIndex& ix, const uint8_t* dest, uint64_t dl, bool has_n, bool dest_is_ref, RmResult& r,
-                  Arena& a, cudaStream_t s) {
+// One destination (compress.cu:856-993): its ASCII string and packed copy on
+// the device (forward strand).
+void refmatch_one(const RmIndex& ix, const uint8_t* dest, const uint64_t* dest_packed, uint64_t dl, bool has_n,
+                  bool dest_is_ref, RmResult& r, Arena& a, cudaStream_t s) {
     r = RmResult{};
     r.seq = dest;  // unchanged unless spans are kept
     r.seq_len = dl;
@@ -503,67 +626,90 @@ void refmatch_one(const RmIndex& ix, const uint8_t* dest, uint64_t dl, bool has_
     if (dic == 0 || ix.rl < uint64_t(RM_K)) return;
     auto mk = a.mark();
     SubStage sp_probe(dest_is_ref ? "refmatch.probe_self" : "refmatch.probe_unmapped");
-    uint8_t* rc = a.alloc<uint8_t>(dl + 64);
-    rc_ascii_kernel<<<grid_for(dl, 256, 8), 256, 0, s>>>(dest, dl, rc);
-    CURC_LAUNCH_CHECK();
     const uint64_t nslots = has_n ? dic : div_up(dic, 4);
     uint8_t* flag = a.alloc<uint8_t>(nslots);
-    Hit* hits = a.alloc<Hit>(nslots);
+    uint32_t* cnt = a.alloc<uint32_t>(4);
+    CURC_CHECK(cudaMemsetAsync(cnt, 0, 16, s));
+    uint32_t* sel = a.alloc<uint32_t>(nslots);
+    uint32_t c = 0;       // hits that go on
+    uint64_t* rows = nullptr;
+    uint32_t* idx = nullptr;
     if (!has_n) {
         const uint64_t words = (dl + 31) / 32 + 8;
         uint64_t* packed = a.alloc<uint64_t>(words);
-        CURC_CHECK(cudaMemsetAsync(packed, 0, words * 8, s));
-        pack_ascii_ref(rc, dl, packed, s);
+        rc_packed_kernel<<<grid_for(words, 256), 256, 0, s>>>(dest_packed, dl, packed, words);
+        CURC_LAUNCH_CHECK();
         const uint64_t dpad = (words - 1) * 32;
         ulonglong2* cand = a.alloc<ulonglong2>(nslots);
         probe_segments_kernel<<<resident_grid(probe_segments_kernel, 256, nslots * 4), 256, 0, s>>>(
             ix, packed, dl, dpad, nslots, dic, dest_is_ref, flag, cand);
         CURC_LAUNCH_CHECK();
-        extend_runs_kernel<<<grid_for(nslots, 256), 256, 0, s>>>(ix, packed, dl, dpad, nslots, flag, cand, hits);
+        uint8_t* lead = a.alloc<uint8_t>(nslots);
+        run_leads_kernel<<<resident_grid(run_leads_kernel, 256, nslots), 256, 0, s>>>(flag, cand, nslots, dl, lead,
+                                                                                      cnt + 1);
+        CURC_LAUNCH_CHECK();
+        select_indices(lead, sel, nslots, cnt, a, s);
+        uint32_t h[2];
+        read_small(h, cnt, 8, s);
+        c = h[0];
+        if (h[1] > cap) {  // capacity: the first accepted segments in probe order
+            if (cap == 0) {
+                c = 0;
+            } else {
+                uint32_t* acc = a.alloc<uint32_t>(h[1]);
+                select_indices(flag, acc, nslots, cnt + 1, a, s);
+                drop_leads_kernel<<<grid_for(nslots, 256), 256, 0, s>>>(lead, nslots, acc + cap);
+                CURC_LAUNCH_CHECK();
+                select_indices(lead, sel, nslots, cnt, a, s);
+                c = read_scalar(cnt, s);
+            }
+        }
+        if (c) {
+            rows = a.alloc<uint64_t>(uint64_t(c) * 3);
+            idx = a.alloc<uint32_t>(c);
+            extend_runs_kernel<<<resident_grid(extend_runs_kernel, 256, uint64_t(c) * 32), 256, 0, s>>>(
+                ix, packed, dl, dpad, sel, c, cand, dest_is_ref, rows, idx);
+            CURC_LAUNCH_CHECK();
+        }
     } else {
+        uint8_t* rc = a.alloc<uint8_t>(dl + 64);
+        rc_ascii_kernel<<<grid_for(dl, 256, 8), 256, 0, s>>>(dest, dl, rc);
+        CURC_LAUNCH_CHECK();
+        Hit* hits = a.alloc<Hit>(nslots);
         CURC_CHECK(cudaMemsetAsync(rc + dl, 0, 64, s));
         probe_ascii_kernel<<<grid_for(nslots, 128), 128, 0, s>>>(ix, rc, dl, dic, flag, hits);
+        CURC_LAUNCH_CHECK();
+        select_indices(flag, sel, nslots, cnt, a, s);
+        c = uint32_t(std::min<uint64_t>(read_scalar(cnt, s), cap));  // the first hits in probe order
+        if (c) {
+            rows = a.alloc<uint64_t>(uint64_t(c) * 3);
+            idx = a.alloc<uint32_t>(c);
+            gather_rows3_kernel<<<grid_for(c, 256), 256, 0, s>>>(hits, sel, c, dl, dest_is_ref, rows, idx);
+            CURC_LAUNCH_CHECK();
+        }
     }
-    CURC_LAUNCH_CHECK();
-    uint32_t* cnt = a.alloc<uint32_t>(4);
-    uint32_t* sel = a.alloc<uint32_t>(nslots);
-    select_indices(flag, sel, nslots, cnt, a, s);
-    uint32_t c = read_scalar(cnt, s);
     sp_probe.stop();
-    if (c > cap) c = uint32_t(cap);  // capacity: the first hits in probe order
     if (c == 0) {
         a.release(mk);
         return;
     }
     SubStage sp_sort("refmatch.sort_unique");
-    Hit* hv = a.alloc<Hit>(c);
-    gather_hits_kernel<<<grid_for(c, 256), 256, 0, s>>>(hits, sel, c, dl, dest_is_ref, hv);
-    CURC_LAUNCH_CHECK();
-    // sort by (dst, src, len): three stable passes, least significant first
-    uint32_t* idx = a.alloc<uint32_t>(c);
-    uint64_t* key = a.alloc<uint64_t>(c);
-    iota(idx, c, s);
-    for (int field = 0; field < 3; ++field) {
-        hit_key_kernel<<<grid_for(c, 256), 256, 0, s>>>(hv, idx, c, field, key);
-        CURC_LAUNCH_CHECK();
-        radix_sort_pairs<uint64_t, uint32_t>(key, idx, c, 0, 64, a, s);
-    }
-    uint8_t* keepf = a.alloc<uint8_t>(c);
-    Hit* sorted = a.alloc<Hit>(c);
-    hit_unique_kernel<<<grid_for(c, 256), 256, 0, s>>>(hv, idx, c, keepf, sorted);
-    CURC_LAUNCH_CHECK();
-    uint32_t* sel2 = a.alloc<uint32_t>(c);
-    select_indices(keepf, sel2, c, cnt + 1, a, s);
-    const uint32_t cu = read_scalar(cnt + 1, s);
+    int dst_bits = 1;
+    while (dst_bits < 64 && (1ull << dst_bits) <= dl) ++dst_bits;
+    sort_rows(rows, 3, 64, idx, c, a, s, dst_bits);  // by (dst, src, len)
+    const uint32_t cu = c;
     Hit* uniq = a.alloc<Hit>(cu);
-    compact_hits_kernel<<<grid_for(cu, 256), 256, 0, s>>>(sorted, sel2, cu, uniq);
+    sorted_hits_kernel<<<grid_for(c, 256), 256, 0, s>>>(rows, idx, c, uniq);
     CURC_LAUNCH_CHECK();
     sp_sort.stop();
     SubStage sp_accept("refmatch.accept");
     uint8_t* keptf = a.alloc<uint8_t>(cu);
     uint64_t* adst = a.alloc<uint64_t>(cu);
     uint64_t* alen = a.alloc<uint64_t>(cu);
-    {
+    if (cu <= ACCEPT_SMALL) {
+        accept_small_kernel<<<1, 256, 0, s>>>(uniq, cu, keptf, adst, alen);
+        CURC_LAUNCH_CHECK();
+    } else {
         int levels = 1;  // range-maximum levels: 2^(levels-1) <= cu
         while ((2ull << (levels - 1)) <= cu) ++levels;
         int lifts = 1;   // lifting levels: 2^lifts > cu
@@ -607,17 +753,18 @@ void refmatch_one(const RmIndex& ix, const uint8_t* dest, uint64_t dl, bool has_
     exclusive_scan<uint32_t>(lsize, lsize, K, cnt + 3, a, s);
     map_len_kernel<<<grid_for(K ? K : 1, 256), 256, 0, s>>>(ksel, K, alen, lsize, mlen);
     CURC_LAUNCH_CHECK();
-    uint64_t total_removed = 0;
-    uint32_t len_bytes = 0;
-    read_small(&total_removed, removed + K, 8, s);
-    read_small(&len_bytes, cnt + 3, 4, s);
+    CURC_CHECK(cudaMemcpyAsync(removed + K + 1, cnt + 3, 4, cudaMemcpyDeviceToDevice, s));
+    uint64_t ends[2] = {0, 0};  // symbols removed; bytes of the lengths (low word)
+    read_small(ends, removed + K, 16, s);
+    const uint64_t total_removed = ends[0];
+    const uint32_t len_bytes = uint32_t(ends[1]);
     uint64_t hi[4] = {K, uint64_t(K) * (std32 ? 4 : 8), 1 + uint64_t(len_bytes), dl - total_removed};
     r.map_off = moff;
     r.off_len = hi[1];
     r.map_len = mlen;
     r.len_len = hi[2];
-    uint8_t* out = a.alloc<uint8_t>(hi[3] + 1);
-    compact_string_kernel<<<grid_for(dl, 256, 8), 256, 0, s>>>(dest, dl, sd, se, removed, hi[0], out);
+    uint8_t* out = a.alloc<uint8_t>(hi[3] + 16);
+    compact_string_kernel<<<grid_for(div_up(hi[3], 16), 256), 256, 0, s>>>(dest, hi[3], sd, se, removed, hi[0], out);
     CURC_LAUNCH_CHECK();
     r.seq = out;
     r.seq_len = hi[3];
@@ -661,17 +808,17 @@ void Block::refmatch_all() {
     }
     // results are copied out right after each destination, before the next
     // one reuses the scratch region
-    refmatch_one(ix, lq.seq, lq.len, false, false, r, arena, s);
+    refmatch_one(ix, lq.seq, lq.packed, lq.len, false, false, r, arena, s);
     keep("unmap_ref", r.seq, r.seq_len);
     keep("unmap_ref_off", r.map_off, r.off_len);
     keep("unmap_ref_len", r.map_len, r.len_len);
     const uint64_t un_len = r.seq_len;
-    refmatch_one(ix, lqn.seq, lqn.len, true, false, r, arena, s);
+    refmatch_one(ix, lqn.seq, lqn.packed, lqn.len, true, false, r, arena, s);
     keep("unmap_n_ref", r.seq, r.seq_len);
     keep("unmap_n_ref_off", r.map_off, r.off_len);
     keep("unmap_n_ref_len", r.map_len, r.len_len);
     const uint64_t unn_len = r.seq_len;
-    refmatch_one(ix, hq.seq, hq.len, false, true, r, arena, s);
+    refmatch_one(ix, hq.seq, hq.packed, hq.len, false, true, r, arena, s);
     keep("ref", r.seq, r.seq_len);
     keep("ref_off", r.map_off, r.off_len);
     keep("ref_len_map", r.map_len, r.len_len);
