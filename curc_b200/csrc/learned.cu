@@ -144,79 +144,49 @@ __global__ void anchors_kernel(const DevRecord* __restrict__ rec, const uint8_t*
 
 // ---------------------------------------------------------------- training
 
-// C[m][n] = sum_k A(m,k) B(k,n) (+ C if acc); A(m,k) = A[m*sam + k*sak],
-// B(k,n) = B[k*sbk + n*sbn].  32x32 tiles, one output per thread, k in
-// order (deterministic).
-__global__ void gemm_kernel(const float* __restrict__ A, const float* __restrict__ B, float* __restrict__ C, int M,
-                            int N, int K, int sam, int sak, int sbk, int sbn, bool acc) {
-    __shared__ float As[32][33], Bs[32][33];
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8 threads, 4 rows each
-    const int n = blockIdx.x * 32 + tx;
-    float sum[4] = {0, 0, 0, 0};
-    for (int k0 = 0; k0 < K; k0 += 32) {
-        for (int r = ty; r < 32; r += 8) {
-            const int mm = blockIdx.y * 32 + r, kk = k0 + tx;
-            As[r][tx] = (mm < M && kk < K) ? A[size_t(mm) * sam + size_t(kk) * sak] : 0.f;
-            const int kb = k0 + r;
-            Bs[r][tx] = (kb < K && n < N) ? B[size_t(kb) * sbk + size_t(n) * sbn] : 0.f;
-        }
-        __syncthreads();
-        for (int kk = 0; kk < 32; ++kk)
-            for (int q = 0; q < 4; ++q) sum[q] += As[ty + 8 * q][kk] * Bs[kk][tx];
-        __syncthreads();
+// A training step is two launches and Adam.  Every sum is one chain of fused
+// multiply-adds in the order of its index (over the 128 inputs of a layer; for
+// a weight's gradient over the whole batch), so that a training run gives the
+// same bits whatever the tiling.  The chains bound the step: 4096 dependent
+// additions of four cycles are 8 us.  With one tiled product per launch, 20
+// launches and three copies a step, a step of 4096 anchors took 1.5 ms on
+// B200; it takes 64 us so (a run of two epochs over 287,000 anchors 208 -> 17
+// ms, of which the host's shuffles are about half).
+
+constexpr int TR_ROWS = 32, TR_S = 132;  // rows per block; padded row of 128 (16-byte reads without conflicts)
+constexpr size_t TR_SMEM = (size_t(2 * HID + OUT + 3 * TR_ROWS) * TR_S + TR_ROWS * OUT) * sizeof(float);
+static_assert(IN == 128 && HID == 128, "one thread tile covers 32 x 128");
+
+// acc[r][c] += sum over k of A[4 ty + r][k] W[tx + 32 c][k], k ascending.
+__device__ __forceinline__ void tile_times_rows(const float* A, const float* W, int tx, int ty, float (&acc)[4][4]) {
+#pragma unroll 4
+    for (int k = 0; k < 128; k += 4) {
+        float4 a[4], w[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const float4*>(A + (4 * ty + r) * TR_S + k);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) w[c] = *reinterpret_cast<const float4*>(W + (tx + 32 * c) * TR_S + k);
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                float v = acc[r][c];
+                v = fmaf(a[r].x, w[c].x, v);
+                v = fmaf(a[r].y, w[c].y, v);
+                v = fmaf(a[r].z, w[c].z, v);
+                acc[r][c] = fmaf(a[r].w, w[c].w, v);
+            }
     }
-    for (int q = 0; q < 4; ++q) {
-        const int mm = blockIdx.y * 32 + ty + 8 * q;
-        if (mm < M && n < N) {
-            float* c = C + size_t(mm) * N + n;
-            *c = acc ? *c + sum[q] : sum[q];
-        }
-    }
 }
 
-void gemm(const float* A, const float* B, float* C, int M, int N, int K, int sam, int sak, int sbk, int sbn, bool acc,
-          cudaStream_t s) {
-    dim3 g((N + 31) / 32, (M + 31) / 32);
-    gemm_kernel<<<g, 256, 0, s>>>(A, B, C, M, N, K, sam, sak, sbk, sbn, acc);
-    CURC_LAUNCH_CHECK();
-}
-
-// dense one-hot inputs of a batch of anchors
-__global__ void inputs_kernel(const Anchor* __restrict__ a, const uint32_t* __restrict__ sel, int B,
-                              float* __restrict__ X) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    float* x = X + size_t(b) * IN;
-    for (int i = 0; i < IN; ++i) x[i] = 0.f;
-    const Anchor an = a[sel ? sel[b] : b];
-    for (int t = 0; t < an.nidx; ++t) x[an.idx[t]] = 1.f;
-}
-
-__global__ void bias_act_kernel(float* __restrict__ H, const float* __restrict__ bias, int B, int N, bool relu) {
-    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= size_t(B) * N) return;
-    float v = H[i] + bias[i % N];
-    H[i] = relu ? fmaxf(v, 0.f) : v;
-}
-
-__global__ void relu_back_kernel(float* __restrict__ dH, const float* __restrict__ H, size_t n) {
-    const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n && H[i] <= 0.f) dH[i] = 0.f;
-}
-
-// Cross-entropy of the base group (when the anchor has a base) and the gap
-// group (when it has a next mismatch); dZ = (softmax - one-hot) / count.
-__global__ void softmax_ce_kernel(const float* __restrict__ Z, const int8_t* __restrict__ tb,
-                                  const int8_t* __restrict__ tg, int B, float inv_n, float* __restrict__ dZ,
-                                  float* __restrict__ loss) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= B) return;
-    const float* z = Z + size_t(b) * OUT;
-    float* d = dZ + size_t(b) * OUT;
+// Softmax cross-entropy of the base group (when the anchor has a base) and
+// the gap group (when it has a next mismatch) of one row; d = (softmax -
+// one-hot) / count.
+__device__ __forceinline__ float softmax_ce(const float* z, int tbase, int tgap, float inv_n, float* d) {
     float l = 0.f;
     for (int g = 0; g < 2; ++g) {
         const int o = g == 0 ? 0 : NB, k = g == 0 ? NB : NG;
-        const int t = g == 0 ? tb[b] : tg[b];
+        const int t = g == 0 ? tbase : tgap;
         if (t < 0) {
             for (int j = 0; j < k; ++j) d[o + j] = 0.f;
             continue;
@@ -228,16 +198,285 @@ __global__ void softmax_ce_kernel(const float* __restrict__ Z, const int8_t* __r
         for (int j = 0; j < k; ++j) d[o + j] = (expf(z[o + j] - mx) / se - (j == t ? 1.f : 0.f)) * inv_n;
         l += (logf(se) + mx - z[o + t]) * inv_n;
     }
-    loss[b] = l;
+    return l;
 }
 
-// out[n] = sum over rows of M (B x N), one thread per column, rows in order
-__global__ void colsum_kernel(const float* __restrict__ M, int B, int N, float* __restrict__ out) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    float s = 0.f;
-    for (int b = 0; b < B; ++b) s += M[size_t(b) * N + n];
-    out[n] = s;
+// Where a step's rows lie in device memory (B rows each).
+struct TrainRows {
+    float *X, *H1, *H2, *dZ, *dH2, *dH1, *loss;
+};
+
+// Forward and backward of 32 rows per block with all weights in shared
+// memory: X (dense from `x`, or the one-hots of the anchors sel lists), H1 =
+// relu(X W1^T + b1), H2 = relu(H1 W2^T + b2), Z = H2 W3^T + b3, softmax
+// cross-entropy, dH2 = dZ W3 and dH1 = dH2 W2 behind their relus.
+__global__ void __launch_bounds__(256) train_rows_kernel(const float* __restrict__ x, const Anchor* __restrict__ anc,
+                                                         const uint32_t* __restrict__ sel,
+                                                         const int8_t* __restrict__ tb, const int8_t* __restrict__ tg,
+                                                         int B, const float* __restrict__ w1,
+                                                         const float* __restrict__ b1, const float* __restrict__ w2,
+                                                         const float* __restrict__ b2, const float* __restrict__ w3,
+                                                         const float* __restrict__ b3, TrainRows out) {
+    extern __shared__ __align__(16) float tr[];
+    float* W1 = tr;
+    float* W2 = W1 + HID * TR_S;
+    float* W3 = W2 + HID * TR_S;
+    float* T0 = W3 + OUT * TR_S;  // X, then dH2
+    float* T1 = T0 + TR_ROWS * TR_S;
+    float* T2 = T1 + TR_ROWS * TR_S;
+    float* Z = T2 + TR_ROWS * TR_S;
+    const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
+    const int row0 = blockIdx.x * TR_ROWS, rows = min(TR_ROWS, B - row0);
+    // weights to shared memory, 16 bytes a load (rows of 128)
+    auto rows_in = [&](const float* src, float* dst, int n) {
+#pragma unroll 8
+        for (int i = tid; i < n * 32; i += 256)
+            *reinterpret_cast<float4*>(dst + (i >> 5) * TR_S + 4 * (i & 31)) =
+                *reinterpret_cast<const float4*>(src + size_t(i) * 4);
+    };
+    rows_in(w1, W1, HID);
+    rows_in(w2, W2, HID);
+    rows_in(w3, W3, OUT);
+    for (int i = tid; i < TR_ROWS * IN; i += 256) {
+        const int r = i >> 7, k = i & 127;
+        T0[r * TR_S + k] = x && r < rows ? x[size_t(row0 + r) * IN + k] : 0.f;
+    }
+    __syncthreads();
+    if (!x && tid < rows) {
+        const Anchor an = anc[sel[row0 + tid]];
+        for (int t = 0; t < an.nidx; ++t) T0[tid * TR_S + an.idx[t]] = 1.f;
+    }
+    __syncthreads();
+    const float inv_n = 1.f / float(B);
+    // rows 4 ty + r and columns tx + 32 c of a tile
+    auto each = [&](auto f) {
+#pragma unroll
+        for (int r = 0; r < 4; ++r)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) f(4 * ty + r, tx + 32 * c, r, c);
+    };
+    {
+        float acc[4][4] = {};
+        tile_times_rows(T0, W1, tx, ty, acc);
+        each([&](int r, int n, int i, int c) {
+            const float v = fmaxf(acc[i][c] + b1[n], 0.f);
+            T1[r * TR_S + n] = v;
+            if (r < rows) {
+                out.H1[size_t(row0 + r) * HID + n] = v;
+                out.X[size_t(row0 + r) * IN + n] = T0[r * TR_S + n];
+            }
+        });
+    }
+    __syncthreads();
+    {
+        float acc[4][4] = {};
+        tile_times_rows(T1, W2, tx, ty, acc);
+        each([&](int r, int n, int i, int c) {
+            const float v = fmaxf(acc[i][c] + b2[n], 0.f);
+            T2[r * TR_S + n] = v;
+            if (r < rows) out.H2[size_t(row0 + r) * HID + n] = v;
+        });
+    }
+    __syncthreads();
+    for (int i = tid; i < TR_ROWS * OUT; i += 256) {
+        const int r = i / OUT, o = i - r * OUT;
+        float v = 0.f;
+#pragma unroll 8
+        for (int k = 0; k < HID; k += 4) {
+            const float4 a = *reinterpret_cast<const float4*>(T2 + r * TR_S + k);
+            const float4 w = *reinterpret_cast<const float4*>(W3 + o * TR_S + k);
+            v = fmaf(a.x, w.x, v);
+            v = fmaf(a.y, w.y, v);
+            v = fmaf(a.z, w.z, v);
+            v = fmaf(a.w, w.w, v);
+        }
+        Z[r * OUT + o] = v + b3[o];
+    }
+    __syncthreads();
+    if (tid < rows) {
+        float z[OUT], d[OUT];
+        for (int o = 0; o < OUT; ++o) z[o] = Z[tid * OUT + o];
+        int ba, ga;
+        if (x) {
+            ba = tb[row0 + tid];
+            ga = tg[row0 + tid];
+        } else {
+            const Anchor* an = anc + sel[row0 + tid];
+            ba = an->tbase;
+            ga = an->tgap;
+        }
+        out.loss[row0 + tid] = softmax_ce(z, ba, ga, inv_n, d);
+        for (int o = 0; o < OUT; ++o) {
+            Z[tid * OUT + o] = d[o];
+            out.dZ[size_t(row0 + tid) * OUT + o] = d[o];
+        }
+    }
+    __syncthreads();
+    {
+        float acc[4][4] = {};
+#pragma unroll 4
+        for (int o = 0; o < OUT; ++o) {
+            float w[4];
+#pragma unroll
+            for (int c = 0; c < 4; ++c) w[c] = W3[o * TR_S + tx + 32 * c];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const float d = Z[(4 * ty + r) * OUT + o];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(d, w[c], acc[r][c]);
+            }
+        }
+        each([&](int r, int n, int i, int c) {
+            const float v = T2[r * TR_S + n] <= 0.f ? 0.f : acc[i][c];
+            T0[r * TR_S + n] = v;
+            if (r < rows) out.dH2[size_t(row0 + r) * HID + n] = v;
+        });
+    }
+    __syncthreads();
+    {
+        float acc[4][4] = {};
+#pragma unroll 4
+        for (int k = 0; k < HID; k += 4) {
+            float4 a[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) a[r] = *reinterpret_cast<const float4*>(T0 + (4 * ty + r) * TR_S + k);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                float w[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c) w[c] = W2[(k + q) * TR_S + tx + 32 * c];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const float d = q == 0 ? a[r].x : q == 1 ? a[r].y : q == 2 ? a[r].z : a[r].w;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) acc[r][c] = fmaf(d, w[c], acc[r][c]);
+                }
+            }
+        }
+        each([&](int r, int n, int i, int c) {
+            if (r < rows) out.dH1[size_t(row0 + r) * HID + n] = T1[r * TR_S + n] <= 0.f ? 0.f : acc[i][c];
+        });
+    }
+}
+
+// Gradients of the weights, G[m][n] = sum over the batch of A[b][m] Bm[b][n],
+// b ascending: 64 threads per 16 x 16 tile, a 2 x 2 patch each (four chains
+// keep the pipeline busy through the four cycles of each addition, and two
+// operands serve two additions each), the rows streamed through eight stages
+// of 32 by asynchronous copies.  What bounds it: shared-memory reads and issue
+// of the two warps a SM has, 14 cycles a row.  Tried and slower: 128 threads
+// with two chains (18 cycles: the operand reads per addition count), and
+// operands stored column by column for 16-byte reads (23).  Behind the tiles'
+// blocks, one block per 32 columns sums a bias gradient the same way.
+constexpr int GR_T = 16, GR_K = 32, GR_STAGES = 8;
+struct GradJob {
+    const float *A, *Bm;  // (B x M), (B x N)
+    float* G;             // M x N
+    int M, N, tiles_n, first;
+};
+struct GradJobs {
+    GradJob w[3];
+    const float* cols[3];  // (B x width): bias gradients
+    float* bias[3];
+    int width[3], first[4];
+};
+
+__device__ __forceinline__ void cp_async16(void* smem, const void* src, bool on) {
+    const uint32_t d = uint32_t(__cvta_generic_to_shared(smem));
+    const int bytes = on ? 16 : 0;  // the rest is zero filled
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(d), "l"(src), "r"(bytes));
+}
+
+__global__ void __launch_bounds__(64) train_grad_kernel(GradJobs jobs, int B) {
+    __shared__ __align__(16) float s_all[2 * GR_STAGES * GR_K * GR_T];
+    float(*sa)[GR_K][GR_T] = reinterpret_cast<float(*)[GR_K][GR_T]>(s_all);
+    float(*sb)[GR_K][GR_T] = sa + GR_STAGES;
+    const int t = threadIdx.x;
+    int blk = blockIdx.x;
+    if (blk >= jobs.first[0]) {  // bias gradients
+        int q = 0;
+        while (q < 2 && blk >= jobs.first[q + 1]) ++q;
+        const int c0 = (blk - jobs.first[q]) * 32, width = jobs.width[q];
+        // stages 32 columns wide in the same memory, loaded by all, added by
+        // one warp (a warp that loads for itself waits a round trip to L2 per
+        // 32 rows)
+        float(*sc)[GR_K][32] = reinterpret_cast<float(*)[GR_K][32]>(s_all);
+        const int steps = (B + GR_K - 1) / GR_K;
+        auto load = [&](int st, int k0) {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int i = t + 64 * e, r = i >> 3, c = (i & 7) * 4;
+                const bool on = k0 + r < B && c0 + c < width;
+                cp_async16(&sc[st][r][c], jobs.cols[q] + (on ? size_t(k0 + r) * width + c0 + c : 0), on);
+            }
+        };
+#pragma unroll
+        for (int i = 0; i < GR_STAGES - 1; ++i) {
+            if (i < steps) load(i, i * GR_K);
+            asm volatile("cp.async.commit_group;");
+        }
+        float v = 0.f;
+        for (int i = 0; i < steps; ++i) {
+            asm volatile("cp.async.wait_group %0;" ::"n"(GR_STAGES - 2));
+            __syncthreads();
+            if (i + GR_STAGES - 1 < steps) load((i + GR_STAGES - 1) % GR_STAGES, (i + GR_STAGES - 1) * GR_K);
+            asm volatile("cp.async.commit_group;");
+            if (t < 32) {  // rows past the batch are zero: they add nothing
+#pragma unroll
+                for (int k = 0; k < GR_K; ++k) v += sc[i % GR_STAGES][k][t];
+            }
+        }
+        if (t < 32 && c0 + t < width) jobs.bias[q][c0 + t] = v;
+        return;
+    }
+    int q = 0;
+    while (q < 2 && blk >= jobs.w[q + 1].first) ++q;
+    const GradJob j = jobs.w[q];
+    blk -= j.first;
+    const int m0 = blk / j.tiles_n * GR_T, n0 = blk % j.tiles_n * GR_T;
+    // stage `st` of rows [k0, k0 + 32): two 16-byte pieces of each operand per thread
+    auto load = [&](int st, int k0) {
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int i = t + 64 * e, r = i >> 2, c = (i & 3) * 4;
+            const bool row = k0 + r < B;
+            const int k = row ? k0 + r : 0;
+            const bool am = row && m0 + c < j.M, bn = row && n0 + c < j.N;  // widths are multiples of 4
+            cp_async16(&sa[st][r][c], j.A + size_t(k) * j.M + (am ? m0 + c : 0), am);
+            cp_async16(&sb[st][r][c], j.Bm + size_t(k) * j.N + (bn ? n0 + c : 0), bn);
+        }
+    };
+    const int steps = (B + GR_K - 1) / GR_K;
+#pragma unroll
+    for (int i = 0; i < GR_STAGES - 1; ++i) {
+        if (i < steps) load(i, i * GR_K);
+        asm volatile("cp.async.commit_group;");
+    }
+    const int pm = (t >> 3) * 2, pn = (t & 7) * 2;
+    float s00 = 0.f, s01 = 0.f, s10 = 0.f, s11 = 0.f;
+    for (int i = 0; i < steps; ++i) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(GR_STAGES - 2));
+        __syncthreads();  // stage i has landed, and stage i - 1 is read
+        if (i + GR_STAGES - 1 < steps) load((i + GR_STAGES - 1) % GR_STAGES, (i + GR_STAGES - 1) * GR_K);
+        asm volatile("cp.async.commit_group;");
+        const int st = i % GR_STAGES;
+#pragma unroll
+        for (int k = 0; k < GR_K; ++k) {  // rows past the batch are zero: they add nothing
+            const float2 a = *reinterpret_cast<const float2*>(&sa[st][k][pm]);
+            const float2 b = *reinterpret_cast<const float2*>(&sb[st][k][pn]);
+            s00 = fmaf(a.x, b.x, s00);
+            s01 = fmaf(a.x, b.y, s01);
+            s10 = fmaf(a.y, b.x, s10);
+            s11 = fmaf(a.y, b.y, s11);
+        }
+    }
+    const int m = m0 + pm, n = n0 + pn;
+    if (m < j.M && n < j.N) {  // patches lie inside or outside whole: sizes are even
+        j.G[size_t(m) * j.N + n] = s00;
+        j.G[size_t(m) * j.N + n + 1] = s01;
+        j.G[size_t(m + 1) * j.N + n] = s10;
+        j.G[size_t(m + 1) * j.N + n + 1] = s11;
+    }
 }
 
 __global__ void adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m1,
@@ -528,6 +767,32 @@ __global__ void __launch_bounds__(TC_ROWS) infer_tc_kernel(const TcModel* __rest
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TC_TMEM_COLS));
 }
 
+// Largest float activations of layers 1 and 2 over the anchors a[0], a[stride],
+// ...: products and sums rounded one by one in index order, as host code rounds
+// them (no fused operations).  One block per anchor, one thread per unit.
+__global__ void __launch_bounds__(HID) calibrate_kernel(const Anchor* __restrict__ a, uint32_t stride,
+                                                        const float* __restrict__ w1, const float* __restrict__ b1,
+                                                        const float* __restrict__ w2, const float* __restrict__ b2,
+                                                        uint32_t* __restrict__ max_bits) {
+    __shared__ float h1[HID];
+    const int h = threadIdx.x;
+    const Anchor& an = a[size_t(blockIdx.x) * stride];
+    float v = b1[h];
+    for (int t = 0; t < an.nidx; ++t) v = __fadd_rn(v, w1[h * IN + an.idx[t]]);
+    v = v > 0.f ? v : 0.f;
+    h1[h] = v;
+    // bits of non-negative floats order as the floats do
+    uint32_t m = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(v));
+    if ((h & 31) == 0) atomicMax(max_bits, m);
+    __syncthreads();
+    v = b2[h];
+#pragma unroll 8
+    for (int t = 0; t < HID; ++t) v = __fadd_rn(v, __fmul_rn(w2[h * HID + t], h1[t]));
+    v = v > 0.f ? v : 0.f;
+    m = __reduce_max_sync(0xFFFFFFFFu, __float_as_uint(v));
+    if ((h & 31) == 0) atomicMax(max_bits + 1, m);
+}
+
 // ---------------------------------------------------------------- host side
 
 struct Trainer {
@@ -573,35 +838,41 @@ struct Trainer {
         fill(oW1, HID, IN);
         fill(oW2, HID, HID);
         fill(oW3, OUT, HID);
-        CURC_CHECK(cudaMemcpy(p, h.data(), NPARAM * 4, cudaMemcpyHostToDevice));
-        CURC_CHECK(cudaMemset(m1, 0, NPARAM * 4));
-        CURC_CHECK(cudaMemset(m2, 0, NPARAM * 4));
+        // on the trainer's stream, which does not wait for the default one
+        CURC_CHECK(cudaMemcpyAsync(p, h.data(), NPARAM * 4, cudaMemcpyHostToDevice, s));
+        CURC_CHECK(cudaMemsetAsync(m1, 0, NPARAM * 4, s));
+        CURC_CHECK(cudaMemsetAsync(m2, 0, NPARAM * 4, s));
+        CURC_CHECK(cudaStreamSynchronize(s));
     }
 
-    // forward + backward on B anchors with dense inputs X; grads to g
-    void step(const float* X, const int8_t* tb, const int8_t* tg, int B, float* H1, float* H2, float* Z, float* dZ,
-              float* dH2, float* dH1, float* lossv) {
-        // forward: H1 = relu(X W1^T + b1), H2 = relu(H1 W2^T + b2), Z = H2 W3^T + b3
-        gemm(X, p + oW1, H1, B, HID, IN, IN, 1, 1, IN, false, s);
-        bias_act_kernel<<<grid_for(size_t(B) * HID, 256), 256, 0, s>>>(H1, p + ob1, B, HID, true);
-        gemm(H1, p + oW2, H2, B, HID, HID, HID, 1, 1, HID, false, s);
-        bias_act_kernel<<<grid_for(size_t(B) * HID, 256), 256, 0, s>>>(H2, p + ob2, B, HID, true);
-        gemm(H2, p + oW3, Z, B, OUT, HID, HID, 1, 1, HID, false, s);
-        bias_act_kernel<<<grid_for(size_t(B) * OUT, 256), 256, 0, s>>>(Z, p + ob3, B, OUT, false);
+    // forward + backward on B rows: dense inputs x with targets tb, tg, or the
+    // anchors sel lists; grads to g
+    void step(const float* x, const uint32_t* sel, const int8_t* tb, const int8_t* tg, int B, const TrainRows& r) {
+        train_rows_kernel<<<(B + TR_ROWS - 1) / TR_ROWS, 256, TR_SMEM, s>>>(x, anc, sel, tb, tg, B, p + oW1, p + ob1,
+                                                                          p + oW2, p + ob2, p + oW3, p + ob3, r);
         CURC_LAUNCH_CHECK();
-        softmax_ce_kernel<<<grid_for(B, 256), 256, 0, s>>>(Z, tb, tg, B, 1.f / float(B), dZ, lossv);
-        CURC_LAUNCH_CHECK();
-        // backward
-        gemm(dZ, H2, g + oW3, OUT, HID, B, 1, OUT, HID, 1, false, s);  // dW3 = dZ^T H2
-        colsum_kernel<<<grid_for(OUT, 128), 128, 0, s>>>(dZ, B, OUT, g + ob3);
-        gemm(dZ, p + oW3, dH2, B, HID, OUT, OUT, 1, HID, 1, false, s);  // dH2 = dZ W3
-        relu_back_kernel<<<grid_for(size_t(B) * HID, 256), 256, 0, s>>>(dH2, H2, size_t(B) * HID);
-        gemm(dH2, H1, g + oW2, HID, HID, B, 1, HID, HID, 1, false, s);  // dW2 = dH2^T H1
-        colsum_kernel<<<grid_for(HID, 128), 128, 0, s>>>(dH2, B, HID, g + ob2);
-        gemm(dH2, p + oW2, dH1, B, HID, HID, HID, 1, HID, 1, false, s);  // dH1 = dH2 W2
-        relu_back_kernel<<<grid_for(size_t(B) * HID, 256), 256, 0, s>>>(dH1, H1, size_t(B) * HID);
-        gemm(dH1, X, g + oW1, HID, IN, B, 1, HID, IN, 1, false, s);  // dW1 = dH1^T X
-        colsum_kernel<<<grid_for(HID, 128), 128, 0, s>>>(dH1, B, HID, g + ob1);
+        GradJobs j;
+        int blk = 0;
+        auto job = [&](int q, const float* A, const float* Bm, float* G, int M, int N) {
+            const int tn = (N + GR_T - 1) / GR_T;
+            j.w[q] = GradJob{A, Bm, G, M, N, tn, blk};
+            blk += tn * ((M + GR_T - 1) / GR_T);
+        };
+        job(0, r.dH1, r.X, g + oW1, HID, IN);   // dW1 = dH1^T X
+        job(1, r.dH2, r.H1, g + oW2, HID, HID);  // dW2 = dH2^T H1
+        job(2, r.dZ, r.H2, g + oW3, OUT, HID);   // dW3 = dZ^T H2
+        auto bias = [&](int q, const float* c, float* o, int width) {
+            j.cols[q] = c;
+            j.bias[q] = o;
+            j.width[q] = width;
+            j.first[q] = blk;
+            blk += (width + 31) / 32;
+        };
+        bias(0, r.dH1, g + ob1, HID);
+        bias(1, r.dH2, g + ob2, HID);
+        bias(2, r.dZ, g + ob3, OUT);
+        j.first[3] = blk;
+        train_grad_kernel<<<blk, 64, 0, s>>>(j, B);
         CURC_LAUNCH_CHECK();
     }
 };
@@ -753,6 +1024,42 @@ std::string encode_stream(const Model& model, Block& b) {
 
 namespace {
 
+// Device memory, pinned memory and events of one call.
+template <class T>
+struct DeviceBuf {
+    T* p = nullptr;
+    explicit DeviceBuf(size_t n) { CURC_CHECK(cudaMalloc(&p, (n ? n : 1) * sizeof(T))); }
+    ~DeviceBuf() { cudaFree(p); }
+    DeviceBuf(const DeviceBuf&) = delete;
+    DeviceBuf& operator=(const DeviceBuf&) = delete;
+};
+template <class T>
+struct PinnedBuf {
+    T* p = nullptr;
+    explicit PinnedBuf(size_t n) {
+        CURC_CHECK(cudaHostAlloc(reinterpret_cast<void**>(&p), n * sizeof(T), cudaHostAllocPortable));
+    }
+    ~PinnedBuf() { cudaFreeHost(p); }
+    PinnedBuf(const PinnedBuf&) = delete;
+    PinnedBuf& operator=(const PinnedBuf&) = delete;
+};
+struct DeviceEvent {
+    cudaEvent_t e = nullptr;
+    DeviceEvent() { CURC_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming)); }
+    ~DeviceEvent() { cudaEventDestroy(e); }
+    DeviceEvent(const DeviceEvent&) = delete;
+    DeviceEvent& operator=(const DeviceEvent&) = delete;
+};
+struct TrainBuffers {
+    DeviceBuf<float> X, H1, H2, dZ, dH2, dH1, loss;
+    explicit TrainBuffers(int B)
+        : X(size_t(B) * IN), H1(size_t(B) * HID), H2(size_t(B) * HID), dZ(size_t(B) * OUT), dH2(size_t(B) * HID),
+          dH1(size_t(B) * HID), loss(B) {
+        CURC_CHECK(cudaFuncSetAttribute(train_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(TR_SMEM)));
+    }
+    TrainRows rows() const { return TrainRows{X.p, H1.p, H2.p, dZ.p, dH2.p, dH1.p, loss.p}; }
+};
+
 template <class F>
 int guarded_learn(curc_learn* L, F&& f) {
     try {
@@ -772,8 +1079,9 @@ int guarded_learn(curc_learn* L, F&& f) {
 }
 
 // Quantises the float parameters (host copy) into the integer model, with
-// activation scales from the largest activations over `calib` anchors.
-void quantise(Trainer& T, const std::vector<float>& P, const std::vector<Anchor>& calib) {
+// activation scales from the largest activations over the calibration anchors
+// (act[0], act[1]; calibrate_kernel).
+void quantise(Trainer& T, const std::vector<float>& P, const float act[2]) {
     auto W1 = [&](int h, int i) { return P[Trainer::oW1 + size_t(h) * IN + i]; };
     auto W2 = [&](int h, int i) { return P[Trainer::oW2 + size_t(h) * HID + i]; };
     auto W3 = [&](int o, int i) { return P[Trainer::oW3 + size_t(o) * HID + i]; };
@@ -785,23 +1093,7 @@ void quantise(Trainer& T, const std::vector<float>& P, const std::vector<Anchor>
     const float sw1 = amax(&P[Trainer::oW1], size_t(HID) * IN) / 127.f;
     const float sw2 = amax(&P[Trainer::oW2], size_t(HID) * HID) / 127.f;
     const float sw3 = amax(&P[Trainer::oW3], size_t(OUT) * HID) / 127.f;
-    // float activations on the calibration set for the activation scales
-    float mx1 = 1e-6f, mx2 = 1e-6f;
-    std::vector<float> h1(HID), h2(HID);
-    for (const Anchor& an : calib) {
-        for (int h = 0; h < HID; ++h) {
-            float v = P[Trainer::ob1 + h];
-            for (int t = 0; t < an.nidx; ++t) v += W1(h, an.idx[t]);
-            h1[h] = std::max(v, 0.f);
-            mx1 = std::max(mx1, h1[h]);
-        }
-        for (int h = 0; h < HID; ++h) {
-            float v = P[Trainer::ob2 + h];
-            for (int t = 0; t < HID; ++t) v += W2(h, t) * h1[t];
-            h2[h] = std::max(v, 0.f);
-            mx2 = std::max(mx2, h2[h]);
-        }
-    }
+    const float mx1 = std::max(1e-6f, act[0]), mx2 = std::max(1e-6f, act[1]);
     const float sa1 = mx1 / 127.f, sa2 = mx2 / 127.f;
     Model& M = T.model;
     auto q8 = [](float v) { return int8_t(std::max(-127.f, std::min(127.f, std::nearbyint(v)))); };
@@ -888,66 +1180,51 @@ int curc_learn_train(curc_learn* L, int epochs, int batch, float lr, uint64_t se
         if (T.n == 0) throw std::runtime_error("learned: no training anchors");
         T.init_params(seed);
         const int B = int(std::min<size_t>(size_t(batch), T.n));
-        float *X, *H1, *H2, *Z, *dZ, *dH2, *dH1, *lossv;
-        int8_t *tb, *tg;
-        uint32_t* sel;
-        CURC_CHECK(cudaMalloc(&X, size_t(B) * IN * 4));
-        CURC_CHECK(cudaMalloc(&H1, size_t(B) * HID * 4));
-        CURC_CHECK(cudaMalloc(&H2, size_t(B) * HID * 4));
-        CURC_CHECK(cudaMalloc(&dH1, size_t(B) * HID * 4));
-        CURC_CHECK(cudaMalloc(&dH2, size_t(B) * HID * 4));
-        CURC_CHECK(cudaMalloc(&Z, size_t(B) * OUT * 4));
-        CURC_CHECK(cudaMalloc(&dZ, size_t(B) * OUT * 4));
-        CURC_CHECK(cudaMalloc(&lossv, size_t(B) * 4));
-        CURC_CHECK(cudaMalloc(&tb, B));
-        CURC_CHECK(cudaMalloc(&tg, B));
-        CURC_CHECK(cudaMalloc(&sel, size_t(B) * 4));
-        std::vector<Anchor> ha(T.n);
-        CURC_CHECK(cudaMemcpy(ha.data(), T.anc, T.n * sizeof(Anchor), cudaMemcpyDeviceToHost));
+        TrainBuffers buf(B);
+        DeviceBuf<uint32_t> sel(T.n);
+        // the order of the anchors per epoch: two host copies, so that one
+        // epoch is shuffled while the last one trains
+        PinnedBuf<uint32_t> pinned(2 * T.n);
         std::vector<uint32_t> order(T.n);
         for (size_t i = 0; i < T.n; ++i) order[i] = uint32_t(i);
         std::mt19937_64 rng(seed);
-        std::vector<int8_t> htb(B), htg(B);
-        float last = 0.f;
         int step = 0;
         const float b1 = 0.9f, b2 = 0.999f;
+        DeviceEvent copied[2];
         for (int e = 0; e < epochs; ++e) {
             std::shuffle(order.begin(), order.end(), rng);
+            uint32_t* host = pinned.p + size_t(e & 1) * T.n;
+            CURC_CHECK(cudaEventSynchronize(copied[e & 1].e));  // its copy of two epochs ago
+            std::copy(order.begin(), order.end(), host);
+            CURC_CHECK(cudaMemcpyAsync(sel.p, host, T.n * 4, cudaMemcpyHostToDevice, T.s));
+            CURC_CHECK(cudaEventRecord(copied[e & 1].e, T.s));
             for (size_t s0 = 0; s0 + size_t(B) <= T.n; s0 += size_t(B)) {
-                for (int b = 0; b < B; ++b) {
-                    htb[b] = ha[order[s0 + b]].tbase;
-                    htg[b] = ha[order[s0 + b]].tgap;
-                }
-                CURC_CHECK(cudaMemcpyAsync(sel, order.data() + s0, size_t(B) * 4, cudaMemcpyHostToDevice, T.s));
-                CURC_CHECK(cudaMemcpyAsync(tb, htb.data(), B, cudaMemcpyHostToDevice, T.s));
-                CURC_CHECK(cudaMemcpyAsync(tg, htg.data(), B, cudaMemcpyHostToDevice, T.s));
-                inputs_kernel<<<grid_for(B, 128), 128, 0, T.s>>>(T.anc, sel, B, X);
-                CURC_LAUNCH_CHECK();
-                T.step(X, tb, tg, B, H1, H2, Z, dZ, dH2, dH1, lossv);
+                T.step(nullptr, sel.p + s0, nullptr, nullptr, B, buf.rows());
                 ++step;
                 adam_kernel<<<grid_for(NPARAM, 256), 256, 0, T.s>>>(
                     T.p, T.g, T.m1, T.m2, NPARAM, lr, b1, b2, 1.f - std::pow(b1, float(step)),
                     1.f - std::pow(b2, float(step)));
                 CURC_LAUNCH_CHECK();
-                CURC_CHECK(cudaStreamSynchronize(T.s));
             }
         }
-        {  // mean loss of the last batch
-            std::vector<float> lv(B);
-            CURC_CHECK(cudaMemcpy(lv.data(), lossv, size_t(B) * 4, cudaMemcpyDeviceToHost));
-            for (float v : lv) last += v;
-        }
-        for (void* q : {(void*)X, (void*)H1, (void*)H2, (void*)dH1, (void*)dH2, (void*)Z, (void*)dZ, (void*)lossv,
-                        (void*)tb, (void*)tg, (void*)sel})
-            cudaFree(q);
-        if (final_loss) *final_loss = last;
         // quantise with up to 4096 anchors for calibration
-        std::vector<float> P(NPARAM);
-        CURC_CHECK(cudaMemcpy(P.data(), T.p, NPARAM * 4, cudaMemcpyDeviceToHost));
-        std::vector<Anchor> calib;
-        for (size_t i = 0; i < ha.size() && calib.size() < 4096; i += std::max<size_t>(1, ha.size() / 4096))
-            calib.push_back(ha[i]);
-        quantise(T, P, calib);
+        const size_t stride = std::max<size_t>(1, T.n / 4096);
+        const uint32_t calib = uint32_t(std::min<size_t>(4096, (T.n + stride - 1) / stride));
+        DeviceBuf<uint32_t> act(2);
+        CURC_CHECK(cudaMemsetAsync(act.p, 0, 8, T.s));
+        calibrate_kernel<<<calib, HID, 0, T.s>>>(T.anc, uint32_t(stride), T.p + Trainer::oW1, T.p + Trainer::ob1,
+                                                 T.p + Trainer::oW2, T.p + Trainer::ob2, act.p);
+        CURC_LAUNCH_CHECK();
+        std::vector<float> P(NPARAM), lv(B);
+        float a2[2];
+        CURC_CHECK(cudaMemcpyAsync(P.data(), T.p, NPARAM * 4, cudaMemcpyDeviceToHost, T.s));
+        CURC_CHECK(cudaMemcpyAsync(lv.data(), buf.loss.p, size_t(B) * 4, cudaMemcpyDeviceToHost, T.s));
+        CURC_CHECK(cudaMemcpyAsync(a2, act.p, 8, cudaMemcpyDeviceToHost, T.s));
+        CURC_CHECK(cudaStreamSynchronize(T.s));
+        float last = 0.f;  // mean loss of the last batch
+        for (float v : lv) last += v;
+        if (final_loss) *final_loss = last;
+        quantise(T, P, a2);
     });
 }
 
@@ -957,33 +1234,21 @@ int curc_learn_grad(curc_learn* L, const float* params, const float* x, const in
     return guarded_learn(L, [&] {
         Trainer& T = L->t;
         const int B = int(n);
-        float *X, *H1, *H2, *Z, *dZ, *dH2, *dH1, *lossv;
-        int8_t *dtb, *dtg;
-        CURC_CHECK(cudaMalloc(&X, size_t(B) * IN * 4));
-        CURC_CHECK(cudaMalloc(&H1, size_t(B) * HID * 4));
-        CURC_CHECK(cudaMalloc(&H2, size_t(B) * HID * 4));
-        CURC_CHECK(cudaMalloc(&dH1, size_t(B) * HID * 4));
-        CURC_CHECK(cudaMalloc(&dH2, size_t(B) * HID * 4));
-        CURC_CHECK(cudaMalloc(&Z, size_t(B) * OUT * 4));
-        CURC_CHECK(cudaMalloc(&dZ, size_t(B) * OUT * 4));
-        CURC_CHECK(cudaMalloc(&lossv, size_t(B) * 4));
-        CURC_CHECK(cudaMalloc(&dtb, B));
-        CURC_CHECK(cudaMalloc(&dtg, B));
-        CURC_CHECK(cudaMemcpy(T.p, params, NPARAM * 4, cudaMemcpyHostToDevice));
-        CURC_CHECK(cudaMemcpy(X, x, size_t(B) * IN * 4, cudaMemcpyHostToDevice));
-        CURC_CHECK(cudaMemcpy(dtb, tb, B, cudaMemcpyHostToDevice));
-        CURC_CHECK(cudaMemcpy(dtg, tg, B, cudaMemcpyHostToDevice));
-        T.step(X, dtb, dtg, B, H1, H2, Z, dZ, dH2, dH1, lossv);
-        CURC_CHECK(cudaStreamSynchronize(T.s));
+        TrainBuffers buf(B);
+        DeviceBuf<float> X(size_t(B) * IN);
+        DeviceBuf<int8_t> dtb(B), dtg(B);
+        CURC_CHECK(cudaMemcpyAsync(T.p, params, NPARAM * 4, cudaMemcpyHostToDevice, T.s));
+        CURC_CHECK(cudaMemcpyAsync(X.p, x, size_t(B) * IN * 4, cudaMemcpyHostToDevice, T.s));
+        CURC_CHECK(cudaMemcpyAsync(dtb.p, tb, B, cudaMemcpyHostToDevice, T.s));
+        CURC_CHECK(cudaMemcpyAsync(dtg.p, tg, B, cudaMemcpyHostToDevice, T.s));
+        T.step(X.p, nullptr, dtb.p, dtg.p, B, buf.rows());
         std::vector<float> lv(B);
-        CURC_CHECK(cudaMemcpy(lv.data(), lossv, size_t(B) * 4, cudaMemcpyDeviceToHost));
+        CURC_CHECK(cudaMemcpyAsync(lv.data(), buf.loss.p, size_t(B) * 4, cudaMemcpyDeviceToHost, T.s));
+        CURC_CHECK(cudaMemcpyAsync(grads, T.g, NPARAM * 4, cudaMemcpyDeviceToHost, T.s));
+        CURC_CHECK(cudaStreamSynchronize(T.s));
         float l = 0.f;
         for (float v : lv) l += v;
         *loss = l;
-        CURC_CHECK(cudaMemcpy(grads, T.g, NPARAM * 4, cudaMemcpyDeviceToHost));
-        for (void* q : {(void*)X, (void*)H1, (void*)H2, (void*)dH1, (void*)dH2, (void*)Z, (void*)dZ, (void*)lossv,
-                        (void*)dtb, (void*)dtg})
-            cudaFree(q);
     });
 }
 
