@@ -943,20 +943,60 @@ void infer(const Model& model, const Anchor* a, uint32_t n, uint16_t* fq, Arena&
     if (read_scalar(err, s)) throw std::runtime_error("learned: tensor-core wait timed out");
 }
 
+// What the range coder needs of an anchor, 16 bytes: the cumulative count and
+// frequency of its base (frequency 0: none) and of its gap bin, the gap, and
+// where it lies.  The frequencies of the other outcomes stay on the device
+// (an anchor and its 20 frequencies are 76 bytes, and went to the host through
+// pageable memory: most of the time of a stream).
+struct __align__(16) CodedAnchor {
+    uint16_t bcum, bfreq, gcum, gfreq, gap, gmax;
+    uint8_t tgap, strand;  // tgap NO_GAP: no next mismatch
+    uint16_t start;        // 1: a record's first anchor
+};
+constexpr uint8_t NO_GAP = 255;
+
+__global__ void coded_anchors_kernel(const Anchor* __restrict__ a, const uint16_t* __restrict__ fq, uint32_t n,
+                                     CodedAnchor* __restrict__ out) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const Anchor& x = a[i];
+    const uint16_t* f = fq + size_t(i) * OUT;
+    CodedAnchor c = {0, 0, 0, 0, x.gap, x.gmax, NO_GAP, x.strand, uint16_t(x.tbase < 0)};
+    if (x.tbase >= 0) {
+        for (int j = 0; j < x.tbase; ++j) c.bcum = uint16_t(c.bcum + f[j]);
+        c.bfreq = f[x.tbase];
+    }
+    if (x.tgap >= 0) {
+        for (int j = 0; j < x.tgap; ++j) c.gcum = uint16_t(c.gcum + f[NB + j]);
+        c.gfreq = f[NB + x.tgap];
+        c.tgap = uint8_t(x.tgap);
+    }
+    out[i] = c;
+}
+
 // The learned stream of a block (its anchors listed and the network run on
 // the GPU, the range coding on the host, chunks of records in parallel).
 std::string encode_stream(const Model& model, Block& b) {
     const int L = b.p.L;
+    const bool verbose = std::getenv("CURC_VERBOSE") != nullptr;
     auto mk = b.arena.mark();
+    struct Pinned {  // given back when the stream is made
+        PinnedArena& p;
+        PinnedArena::Mark m;
+        ~Pinned() { p.release(m); }
+    } pinned{b.pinned, b.pinned.mark()};
     uint32_t na = 0;
     Anchor* a = block_anchors(b, b.arena, &na);
     uint16_t* fq = b.arena.alloc<uint16_t>(size_t(na ? na : 1) * OUT);
     infer(model, a, na, fq, b.arena, b.stream);
-    std::vector<Anchor> ha(na);
-    std::vector<uint16_t> hf(size_t(na) * OUT);
+    const CodedAnchor* ha = nullptr;
     if (na) {
-        CURC_CHECK(cudaMemcpyAsync(ha.data(), a, size_t(na) * sizeof(Anchor), cudaMemcpyDeviceToHost, b.stream));
-        CURC_CHECK(cudaMemcpyAsync(hf.data(), fq, hf.size() * 2, cudaMemcpyDeviceToHost, b.stream));
+        CodedAnchor* dc = b.arena.alloc<CodedAnchor>(na);
+        coded_anchors_kernel<<<grid_for(na, 256), 256, 0, b.stream>>>(a, fq, na, dc);
+        CURC_LAUNCH_CHECK();
+        CodedAnchor* host = reinterpret_cast<CodedAnchor*>(b.pinned.alloc(size_t(na) * sizeof(CodedAnchor)));
+        CURC_CHECK(cudaMemcpyAsync(host, dc, size_t(na) * sizeof(CodedAnchor), cudaMemcpyDeviceToHost, b.stream));
+        ha = host;
     }
     CURC_CHECK(cudaStreamSynchronize(b.stream));
     b.arena.release(mk);
@@ -964,7 +1004,7 @@ std::string encode_stream(const Model& model, Block& b) {
     std::vector<size_t> cut{0};
     uint32_t recs = 0;
     for (size_t k = 0; k < na; ++k)
-        if (ha[k].tbase < 0 && k > 0 && ++recs % CHUNK_RECORDS == 0) cut.push_back(k);
+        if (ha[k].start && k > 0 && ++recs % CHUNK_RECORDS == 0) cut.push_back(k);
     cut.push_back(na);
     const int nc = int(cut.size()) - 1;
     std::vector<std::string> chunks(nc);
@@ -976,27 +1016,22 @@ std::string encode_stream(const Model& model, Block& b) {
         double cb[3] = {0, 0, 0};
         int q = -1;  // the anchor's offset along the read, in pseudogenome order
         for (size_t k = cut[c]; k < cut[c + 1]; ++k) {
-            const Anchor& x = ha[k];
-            const uint16_t* f = &hf[k * OUT];
-            if (x.tbase < 0) q = -1;  // a record's start anchor
-            if (x.tbase >= 0) {
-                uint32_t cum = 0;
-                for (int j = 0; j < x.tbase; ++j) cum += f[j];
-                enc.encode(cum, f[x.tbase], TOTAL);
-                cb[0] -= std::log2(double(f[x.tbase]) / TOTAL);
+            const CodedAnchor& x = ha[k];
+            if (x.start) q = -1;  // a record's start anchor
+            if (x.bfreq) {
+                enc.encode(x.bcum, x.bfreq, TOTAL);
+                if (verbose) cb[0] -= std::log2(double(x.bfreq) / TOTAL);
             }
-            if (x.tgap >= 0) {
-                uint32_t cum = 0;
-                for (int j = 0; j < x.tgap; ++j) cum += f[NB + j];
-                enc.encode(cum, f[NB + x.tgap], TOTAL);
-                cb[1] -= std::log2(double(f[NB + x.tgap]) / TOTAL);
+            if (x.tgap != NO_GAP) {
+                enc.encode(x.gcum, x.gfreq, TOTAL);
+                if (verbose) cb[1] -= std::log2(double(x.gfreq) / TOTAL);
                 const int lo = gap_bin_lo(x.tgap);
                 const int hi = std::min(gap_bin_lo(x.tgap + 1), int(x.gmax) + 1);
                 const int bc = bin_context(q, L, x.strand);
                 uint32_t oc, of, ot;
                 bins.lookup(bc, x.tgap, x.gap - lo, hi - lo, oc, of, ot);
                 enc.encode(oc, of, ot);
-                cb[2] -= std::log2(double(of) / ot);
+                if (verbose) cb[2] -= std::log2(double(of) / ot);
                 bins.update(bc, x.tgap, x.gap - lo);
                 q += 1 + x.gap;
             }
@@ -1005,7 +1040,7 @@ std::string encode_stream(const Model& model, Block& b) {
 #pragma omp critical
         for (int q = 0; q < 3; ++q) bits[q] += cb[q];
     }
-    if (std::getenv("CURC_VERBOSE"))
+    if (verbose)
         std::fprintf(stderr, "curc: learned bytes: bases %.0f, gap bins %.0f, offsets in bins %.0f (%u anchors)\n",
                      bits[0] / 8, bits[1] / 8, bits[2] / 8, na);
     std::string s;

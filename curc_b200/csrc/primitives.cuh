@@ -71,6 +71,14 @@ public:
     PinnedArena& operator=(PinnedArena&& o) noexcept;
     uint8_t* alloc(size_t bytes);
     void reset();
+    // Marks let a call give back what it took.
+    struct Mark { size_t chunk, used; };
+    Mark mark() const { return {cur_, cur_ < chunks_.size() ? chunks_[cur_].used : 0}; }
+    void release(const Mark& m) {
+        for (size_t i = m.chunk + 1; i < chunks_.size(); ++i) chunks_[i].used = 0;
+        cur_ = m.chunk;
+        if (cur_ < chunks_.size()) chunks_[cur_].used = m.used;
+    }
 
 private:
     struct Chunk { uint8_t* base; size_t size, used; };
