@@ -483,7 +483,14 @@ void select_indices(const uint8_t* flags, uint32_t* out, size_t n, uint32_t* cou
 // ---------------------------------------------------------------- radix sort
 
 namespace {
-constexpr int RS_THREADS = 256, RS_ROUNDS = 16, RS_TILE = RS_THREADS * RS_ROUNDS, RS_WARPS = RS_THREADS / 32;
+constexpr int RS_THREADS = 256, RS_WARPS = RS_THREADS / 32;
+// Items per thread of a pass, and of a pass over few items.
+constexpr int RS_ROUNDS = 16, RS_ROUNDS_FEW = 4, RS_TILE = RS_THREADS * RS_ROUNDS;
+// Few: less than one full tile per SM.  A tile of 4 rounds is ranked in a
+// quarter of the time and the SMs are not idle; with more items its longer
+// look-back and shorter runs cost more than that gives.  Sort of 50k reads
+// 0.167 -> 0.11 ms, 200k 0.19 -> 0.155, 700k and more unchanged or slower.
+constexpr size_t RS_FEW = size_t(SM_COUNT_B200) * RS_TILE;
 
 template <class K>
 __device__ __forceinline__ uint32_t digit_of(K k, int shift, uint32_t mask) {
@@ -539,20 +546,20 @@ __device__ __forceinline__ uint32_t rs_scan256(uint32_t v, uint32_t* wsum) {
     return before + x - v;
 }
 
-// Items of one tile in registers, 16 rounds of 32 consecutive items per warp,
+// Items of one tile in registers, R rounds of 32 consecutive items per warp,
 // each ranked among the warp's earlier items of its digit with match_any and
 // warp-private digit counters (no block barrier inside).
-template <class K, class V>
+template <class K, class V, int R>
 struct RsTile {
-    K k[RS_ROUNDS];
-    V v[RS_ROUNDS];
-    uint32_t rk[RS_ROUNDS];
+    K k[R];
+    V v[R];
+    uint32_t rk[R];
     __device__ __forceinline__ void rank(uint32_t items, int shift, uint32_t mask, uint32_t* cnt) {
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
         const uint32_t lt_mask = (1u << lane) - 1u;
 #pragma unroll
-        for (int r = 0; r < RS_ROUNDS; ++r) {
-            const uint32_t t = uint32_t(warp) * (RS_TILE / RS_WARPS) + r * 32 + lane;
+        for (int r = 0; r < R; ++r) {
+            const uint32_t t = uint32_t(warp) * (R * 32) + r * 32 + lane;
             const bool valid = t < items;
             const uint32_t d = valid ? digit_of(k[r], shift, mask) : 256u;
             const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
@@ -576,16 +583,17 @@ struct RsTile {
 // coalesce.  One launch and one read and write of the items per pass; with a
 // histogram, a scan and a scatter launch per pass a sort of a few thousand
 // items took 360 us, all of it launches (B200, 64-bit keys).
-template <class K, class V>
+template <class K, class V, int R>
 __global__ void __launch_bounds__(RS_THREADS) rs_pass_kernel(const K* __restrict__ kin, const V* __restrict__ vin,
                                                              K* __restrict__ kout, V* __restrict__ vout, size_t n,
                                                              int shift, uint32_t mask,
                                                              const uint32_t* __restrict__ hist,
                                                              unsigned long long* __restrict__ st, uint32_t tiles,
                                                              uint32_t* __restrict__ err) {
+    constexpr int TILE = RS_THREADS * R;
     extern __shared__ __align__(16) uint8_t rs_smem[];
     K* sk = reinterpret_cast<K*>(rs_smem);
-    V* sv = reinterpret_cast<V*>(rs_smem + sizeof(K) * RS_TILE);
+    V* sv = reinterpret_cast<V*>(rs_smem + sizeof(K) * TILE);
     __shared__ uint32_t gbase[256], tstart[256];
     __shared__ uint32_t wcnt[RS_WARPS][256];
     __shared__ uint32_t wsum[RS_WARPS], s_tile;
@@ -596,12 +604,12 @@ __global__ void __launch_bounds__(RS_THREADS) rs_pass_kernel(const K* __restrict
     const uint32_t digit_start = rs_scan256(hist[tid], wsum);
     __syncthreads();
     const uint32_t tile = s_tile;
-    const size_t base = size_t(tile) * RS_TILE;
-    const uint32_t items = uint32_t(min(size_t(RS_TILE), n - base));
-    RsTile<K, V> T;
+    const size_t base = size_t(tile) * TILE;
+    const uint32_t items = uint32_t(min(size_t(TILE), n - base));
+    RsTile<K, V, R> T;
 #pragma unroll
-    for (int r = 0; r < RS_ROUNDS; ++r) {
-        const uint32_t t = uint32_t(warp) * (RS_TILE / RS_WARPS) + r * 32 + lane;
+    for (int r = 0; r < R; ++r) {
+        const uint32_t t = uint32_t(warp) * (R * 32) + r * 32 + lane;
         T.k[r] = t < items ? kin[base + t] : K{};
         T.v[r] = (t < items && vin) ? vin[base + t] : V{};
     }
@@ -620,8 +628,8 @@ __global__ void __launch_bounds__(RS_THREADS) rs_pass_kernel(const K* __restrict
     tstart[tid] = rs_scan256(mine, wsum);
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < RS_ROUNDS; ++r) {
-        const uint32_t t = uint32_t(warp) * (RS_TILE / RS_WARPS) + r * 32 + lane;
+    for (int r = 0; r < R; ++r) {
+        const uint32_t t = uint32_t(warp) * (R * 32) + r * 32 + lane;
         if (t < items) {
             const uint32_t d = digit_of(T.k[r], shift, mask);
             const uint32_t lp = tstart[d] + wcnt[warp][d] + T.rk[r];
@@ -663,7 +671,8 @@ __global__ void __launch_bounds__(RS_THREADS) rs_single_kernel(K* __restrict__ k
     __shared__ uint32_t wcnt[RS_WARPS][256];
     __shared__ uint32_t wsum[RS_WARPS];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    RsTile<K, V> T;
+    constexpr int R = RS_ROUNDS;
+    RsTile<K, V, R> T;
     const int np = dg.passes();
     for (int p = 0; p < np; ++p) {
         const int shift = dg.shift(p);
@@ -671,8 +680,8 @@ __global__ void __launch_bounds__(RS_THREADS) rs_single_kernel(K* __restrict__ k
 #pragma unroll
         for (int w = 0; w < RS_WARPS; ++w) wcnt[w][tid] = 0;
 #pragma unroll
-        for (int r = 0; r < RS_ROUNDS; ++r) {
-            const uint32_t t = uint32_t(warp) * (RS_TILE / RS_WARPS) + r * 32 + lane;
+        for (int r = 0; r < R; ++r) {
+            const uint32_t t = uint32_t(warp) * (R * 32) + r * 32 + lane;
             T.k[r] = t < n ? (p ? sk[t] : keys[t]) : K{};
             T.v[r] = (t < n && vals) ? (p ? sv[t] : vals[t]) : V{};
         }
@@ -689,8 +698,8 @@ __global__ void __launch_bounds__(RS_THREADS) rs_single_kernel(K* __restrict__ k
         tstart[tid] = rs_scan256(mine, wsum);
         __syncthreads();
 #pragma unroll
-        for (int r = 0; r < RS_ROUNDS; ++r) {
-            const uint32_t t = uint32_t(warp) * (RS_TILE / RS_WARPS) + r * 32 + lane;
+        for (int r = 0; r < R; ++r) {
+            const uint32_t t = uint32_t(warp) * (R * 32) + r * 32 + lane;
             if (t < n) {
                 const uint32_t d = digit_of(T.k[r], shift, mask);
                 const uint32_t lp = tstart[d] + wcnt[warp][d] + T.rk[r];
@@ -721,7 +730,7 @@ void rs_prepare() {
     if (dev < 0 || dev >= 64) throw std::runtime_error("device ordinal out of range");
     std::lock_guard<std::mutex> g(mu);
     if (!done[dev]) {
-        CURC_CHECK(cudaFuncSetAttribute(rs_pass_kernel<K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        CURC_CHECK(cudaFuncSetAttribute(rs_pass_kernel<K, V, RS_ROUNDS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         int(rs_smem_bytes<K, V>())));
         CURC_CHECK(cudaFuncSetAttribute(rs_single_kernel<K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         int(rs_smem_bytes<K, V>())));
@@ -744,7 +753,9 @@ void radix_sort_pairs(K* keys, V* vals, size_t n, int begin_bit, int end_bit, Ar
     auto m = a.mark();
     K* kalt = a.alloc<K>(n);
     V* valt = vals ? a.alloc<V>(n) : nullptr;
-    const uint32_t tiles = uint32_t(div_up(n, RS_TILE));
+    const bool few = n < RS_FEW;
+    const uint32_t tile = few ? RS_THREADS * RS_ROUNDS_FEW : RS_TILE;
+    const uint32_t tiles = uint32_t(div_up(n, tile));
     const int np = dg.passes();
     // per pass: 256 states per tile and the tile counter; then the counts
     const size_t pass_words = size_t(tiles) * 256 + 1;
@@ -759,7 +770,8 @@ void radix_sort_pairs(K* keys, V* vals, size_t n, int begin_bit, int end_bit, Ar
     for (int p = 0; p < np; ++p) {
         K* ko = (kc == keys) ? kalt : keys;
         V* vo = vals ? ((vc == vals) ? valt : vals) : nullptr;
-        rs_pass_kernel<K, V><<<tiles, RS_THREADS, rs_smem_bytes<K, V>(), s>>>(
+        auto pass = few ? rs_pass_kernel<K, V, RS_ROUNDS_FEW> : rs_pass_kernel<K, V, RS_ROUNDS>;
+        pass<<<tiles, RS_THREADS, (sizeof(K) + sizeof(V)) * size_t(tile), s>>>(
             kc, vc, ko, vo, n, dg.shift(p), dg.mask(p), hist + p * 256, st + pass_words * p, tiles, a.wait_error());
         CURC_LAUNCH_CHECK();
         kc = ko;

@@ -44,3 +44,14 @@ def test_blocks_of_long_runs(ctx, n):
     ctx.block_run(reads)
     bad = [nm for nm, dt in STAGE_RESULTS.items() if not np.array_equal(ctx.get(nm, dt), ora.get(nm, dt))]
     assert not bad, bad
+
+
+@pytest.mark.parametrize("n", [148 * 4096 - 1, 148 * 4096])
+def test_few_or_many_items(ctx, n):
+    """On both sides of the size from which the sort's passes take full tiles."""
+    L = 40
+    rng = np.random.default_rng(n)
+    reads = np.ascontiguousarray(synth.ACGT[rng.integers(0, 4, size=(n, L))])
+    reads[::5] = reads[0]
+    ctx.block_run(reads)
+    assert np.array_equal(ctx.get("sorted_ids", np.uint32), np.argsort(reads.view(f"S{L}").ravel(), kind="stable"))
