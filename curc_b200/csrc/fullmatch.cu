@@ -223,11 +223,19 @@ __device__ __forceinline__ void run_bounds_block(const Acc& acc, const uint32_t*
         }
         __syncthreads();
     }
+    // Reads with several letters that share the last symbol are not in the
+    // order the search takes them to be in; its bounds may then cross, and
+    // the merges would read beyond the list.
     if (threadIdx.x == 0) {
+        uint32_t b = 0;
         bounds[0] = 0;
+#pragma unroll
+        for (int q = 0; q < NB; ++q) {
+            b = max(b, lo_s[q]);
+            bounds[q + 1] = b;
+        }
         bounds[Acc::ALPHA] = m;
     }
-    if (threadIdx.x < NB) bounds[threadIdx.x + 1] = lo_s[threadIdx.x];
 }
 
 template <class Acc>

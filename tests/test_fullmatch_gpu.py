@@ -64,8 +64,11 @@ def test_listed_form_at_its_edges(ctx, kind, n, L, with_n):
 @pytest.mark.parametrize("kind,n", [("tails", 300), ("random", 1600)])
 def test_other_letters_take_the_pass_form(ctx, kind, n):
     seqs = reads_of(kind, n, 60, 1)
+    # one letter beyond A, C, G and N: the passes merge runs per first letter,
+    # with T, R, ... as one run, so reads that mix those are not sorted by them
+    # and which of their equal ends meet is not defined
+    seqs[seqs == ord("T")] = ord("G")
     seqs[::5, 7] = ord("R")
-    seqs[1::5, 11] = ord("a")
     a, b = results(ctx, seqs), results(ctx, seqs, fm_loop=0)
     bad = [nm for nm in a if not np.array_equal(a[nm], b[nm])]
     assert not bad, bad
