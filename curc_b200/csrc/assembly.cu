@@ -642,7 +642,6 @@ struct RankScratch {
     SubTotal* tot;
     RankState* A;
     RankState* B;
-    uint32_t* counts;  // [0] rulers, [1] unreached, [2] active
     uint32_t epoch;    // walks so far (loc is zeroed once, so 0 is never current)
 };
 
@@ -655,32 +654,33 @@ uint32_t rank_members(const uint32_t* ids, uint32_t m, uint32_t n, const uint32_
     const uint8_t* promote = nullptr;
     uint32_t nr = 0;
     SubStage sp_walk("assembly.walk");
-    CURC_CHECK(cudaMemsetAsync(k.counts + 3, 0, 4, s));
+    // per attempt: rulers, unreached, a link out of the set
+    uint32_t* counts = a.zeros<uint32_t>(2 * 3, s);
     chain_nodes_kernel<<<resident_grid(chain_nodes_kernel, 256, n), 256, 0, s>>>(n, pos_in_ids, nx, offset, k.node);
     CURC_LAUNCH_CHECK();
     for (int attempt = 0; attempt < 2; ++attempt) {
         const uint32_t epoch = ++k.epoch;
         ruler_flags_kernel<<<g, 256, 0, s>>>(ids, m, pv, promote, k.flags);
         CURC_LAUNCH_CHECK();
-        select_flagged(ids, k.flags, k.rul, m, k.counts, a, s);
+        select_flagged(ids, k.flags, k.rul, m, counts, a, s);
         if (attempt) {  // clear the ruler marks of the first attempt
             chain_nodes_kernel<<<resident_grid(chain_nodes_kernel, 256, n), 256, 0, s>>>(n, pos_in_ids, nx, offset,
                                                                                           k.node);
             CURC_LAUNCH_CHECK();
         }
-        CURC_CHECK(cudaMemsetAsync(k.counts + 1, 0, 4, s));
-        nr = read_scalar(k.counts, s);
+        nr = read_scalar(counts, s);
         ruler_index_kernel<<<grid_for(nr, 256), 256, 0, s>>>(k.rul, nr, k.node);
         CURC_LAUNCH_CHECK();
         ruler_walk_kernel<<<resident_grid(ruler_walk_kernel, 256, nr), 256, 0, s>>>(k.rul, nr, m, n, epoch, k.node,
-                                                                                    k.loc, k.tot, k.counts + 3);
+                                                                                    k.loc, k.tot, counts + 2);
         CURC_LAUNCH_CHECK();
         unreached_kernel<<<resident_grid(unreached_kernel, 256, m), 256, 0, s>>>(m, epoch, k.loc, k.flags,
-                                                                                  k.counts + 1);
+                                                                                  counts + 1);
         CURC_LAUNCH_CHECK();
-        uint32_t hc[4];
-        read_small(hc, k.counts, 16, s);
-        if (hc[3]) throw std::runtime_error("assemble: a chain link leaves the member set");
+        uint32_t hc[3];
+        read_small(hc, counts, 12, s);
+        counts += 3;
+        if (hc[2]) throw std::runtime_error("assemble: a chain link leaves the member set");
         if (hc[1] == 0) break;
         if (attempt == 1) throw std::runtime_error("assemble: reads left unranked after promoting cycle rulers");
         CURC_CHECK(cudaMemsetAsync(k.promote, 0, m, s));
@@ -699,13 +699,13 @@ uint32_t rank_members(const uint32_t* ids, uint32_t m, uint32_t n, const uint32_
     // converged states changes nothing)
     const int R = rounds_for(nr);
     const int gs = resident_grid(rank_step_kernel, 512, nr);
+    uint32_t* active = a.zeros<uint32_t>(R, s);  // per round
     for (int t = 0; t < R; ++t) {
-        CURC_CHECK(cudaMemsetAsync(k.counts + 2, 0, 4, s));
-        rank_step_kernel<<<gs, 512, 0, s>>>(nr, A, B, k.counts + 2);
+        rank_step_kernel<<<gs, 512, 0, s>>>(nr, A, B, active + t);
         CURC_LAUNCH_CHECK();
         std::swap(A, B);
         if (t % 4 != 3 && t + 1 < R) continue;
-        left = read_scalar(k.counts + 2, s);
+        left = read_scalar(active + t, s);
         if (left == 0) break;
     }
     member_state_kernel<<<g, 256, 0, s>>>(m, k.rul, k.loc, A, st);
@@ -741,8 +741,7 @@ void assemble_small(const uint64_t* db, const uint8_t* ascii, int L, int W, cons
     }
     uint64_t* place = a.alloc<uint64_t>(m);
     uint8_t* tail = a.alloc<uint8_t>(m);
-    uint64_t* res = a.alloc<uint64_t>(2);  // bases, error
-    CURC_CHECK(cudaMemsetAsync(res, 0, 16, s));
+    uint64_t* res = a.zeros<uint64_t>(2, s);  // bases, error
     assemble_small_kernel<<<1, ASM_THREADS, asm_small_bytes(m), s>>>(ids, m, n, next, prev, offset, L, is_n ? 1 : 0,
                                                                      pos_in_ids, out.records, place, tail, res,
                                                                      reinterpret_cast<uint32_t*>(res + 1));
@@ -790,8 +789,7 @@ void assemble(const uint64_t* db, const uint8_t* ascii, int L, int W, const uint
     SubStage sp_rank("assembly.ranking");
     RankScratch k;
     k.node = a.alloc<ChainNode>(n);
-    k.loc = a.alloc<SubPos>(m);
-    CURC_CHECK(cudaMemsetAsync(k.loc, 0, size_t(m) * sizeof(SubPos), s));
+    k.loc = a.zeros<SubPos>(m, s);
     k.epoch = 0;
     k.flags = a.alloc<uint8_t>(m);
     k.promote = a.alloc<uint8_t>(m);
@@ -799,7 +797,6 @@ void assemble(const uint64_t* db, const uint8_t* ascii, int L, int W, const uint
     k.tot = a.alloc<SubTotal>(m);
     k.A = a.alloc<RankState>(m);
     k.B = a.alloc<RankState>(m);
-    k.counts = a.alloc<uint32_t>(4);
     RankState* R = a.alloc<RankState>(m);
     uint32_t left = rank_members(ids, m, n_total, nx, pv, offset, pos_in_ids, k, R, a, s);
     if (left) {
@@ -812,13 +809,13 @@ void assemble(const uint64_t* db, const uint8_t* ascii, int L, int W, const uint
         uint32_t* leader_of_head = a.alloc<uint32_t>(n);
         unsigned long long* best = a.alloc<unsigned long long>(n);
         CURC_CHECK(cudaMemsetAsync(best, 0, n * sizeof(unsigned long long), s));
-        CURC_CHECK(cudaMemsetAsync(k.counts + 3, 0, 4, s));
-        cycle_open_kernel<<<g, 256, 0, s>>>(ids, m, R, cyc, nx, pv, leader_of_head, k.counts + 3);
+        uint32_t* cut = a.zeros<uint32_t>(2, s);  // members on cycles, a cycle that does not close
+        cycle_open_kernel<<<g, 256, 0, s>>>(ids, m, R, cyc, nx, pv, leader_of_head, cut + 1);
         CURC_LAUNCH_CHECK();
         uint32_t* cidx = a.alloc<uint32_t>(m);
-        select_indices(cyc, cidx, m, k.counts + 2, a, s);
+        select_indices(cyc, cidx, m, cut, a, s);
         uint32_t hc[2];
-        read_small(hc, k.counts + 2, 8, s);
+        read_small(hc, cut, 8, s);
         if (hc[1]) throw std::runtime_error("assemble: broken cycle");
         const uint32_t mc = hc[0];
         const int gc = grid_for(mc, 256);
@@ -831,8 +828,7 @@ void assemble(const uint64_t* db, const uint8_t* ascii, int L, int W, const uint
         CURC_CHECK(cudaMemsetAsync(all, 1, mc, s));
         RankScratch kc;
         kc.node = k.node;
-        kc.loc = a.alloc<SubPos>(mc);
-        CURC_CHECK(cudaMemsetAsync(kc.loc, 0, size_t(mc) * sizeof(SubPos), s));
+        kc.loc = a.zeros<SubPos>(mc, s);
         kc.epoch = 0;
         kc.flags = a.alloc<uint8_t>(mc);
         kc.promote = a.alloc<uint8_t>(mc);
@@ -840,7 +836,6 @@ void assemble(const uint64_t* db, const uint8_t* ascii, int L, int W, const uint
         kc.tot = a.alloc<SubTotal>(mc);
         kc.A = a.alloc<RankState>(mc);
         kc.B = a.alloc<RankState>(mc);
-        kc.counts = a.alloc<uint32_t>(4);
         RankState* T = a.alloc<RankState>(mc);
         if (rank_members(cids, mc, n_total, nx, pv, offset, pos_in_cyc, kc, T, a, s))
             throw std::runtime_error("assemble: cycle still closed after its temporary cut");
@@ -869,7 +864,9 @@ void assemble(const uint64_t* db, const uint8_t* ascii, int L, int W, const uint
     uint32_t* hkey = a.alloc<uint32_t>(nh);
     gather_heads_kernel<<<grid_for(nh, 256), 256, 0, s>>>(heads, nh, key, hkey);
     CURC_LAUNCH_CHECK();
-    radix_sort_pairs<uint32_t, uint32_t>(hkey, heads, nh, 0, 32, a, s);
+    int key_bits = 1;  // a key is a list index
+    while (key_bits < 32 && (1ull << key_bits) < m) ++key_bits;
+    radix_sort_pairs<uint32_t, uint32_t>(hkey, heads, nh, 0, key_bits, a, s);
     uint64_t* chain_bases = a.alloc<uint64_t>(n);
     uint32_t* chain_members = a.alloc<uint32_t>(n);
     tail_sizes_kernel<<<g, 256, 0, s>>>(ids, m, nx, R, L, chain_bases, chain_members);

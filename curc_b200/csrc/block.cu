@@ -71,8 +71,8 @@ void Block::run(const uint8_t* d_seq, uint64_t n_reads, int L, bool po, bool pe)
     cudaEvent_t ev0 = run_ev.a, ev1 = run_ev.b;
     CURC_CHECK(cudaEventRecord(ev0, s));
     uint32_t* counts = arena.alloc<uint32_t>(16);
-    uint32_t* err = arena.alloc<uint32_t>(1);
-    CURC_CHECK(cudaMemsetAsync(err, 0, 4, s));
+    arena.clear_zeros(s);
+    uint32_t* err = arena.zeros<uint32_t>(1, s);
 
     // a1
     T.begin("pack");
@@ -103,9 +103,7 @@ void Block::run(const uint8_t* d_seq, uint64_t n_reads, int L, bool po, bool pe)
     next = arena.alloc<uint32_t>(n ? n : 1);
     prev = arena.alloc<uint32_t>(n ? n : 1);
     offset = arena.alloc<uint16_t>(n ? n : 1);
-    fill<uint32_t>(next, INVALID, n, s);
-    fill<uint32_t>(prev, INVALID, n, s);
-    fill<uint16_t>(offset, INVALOFF, n, s);
+    unlinked(next, prev, offset, n, s);
     sorted = arena.alloc<uint32_t>(m ? m : 1);
     if (m) CURC_CHECK(cudaMemcpyAsync(sorted, reads_id, size_t(m) * 4, cudaMemcpyDeviceToDevice, s));
     {
@@ -133,8 +131,7 @@ void Block::run(const uint8_t* d_seq, uint64_t n_reads, int L, bool po, bool pe)
 
     // a6 (compress.cu:1576-1591)
     T.begin("full_match");
-    fm_tally = arena.alloc<unsigned long long>(3);
-    CURC_CHECK(cudaMemsetAsync(fm_tally, 0, 3 * sizeof(unsigned long long), s));
+    fm_tally = arena.zeros<unsigned long long>(3, s);
     {
         auto mk = arena.mark();
         uint8_t* pf = arena.alloc<uint8_t>(n_ref ? n_ref : 1);
@@ -179,8 +176,7 @@ void Block::run(const uint8_t* d_seq, uint64_t n_reads, int L, bool po, bool pe)
     mo.mm = arena.alloc<uint8_t>(U + NN + 1);
     mo.strand = arena.alloc<uint8_t>(U + NN + 1);
     mo.pos = arena.alloc<uint64_t>(U + NN + 1);
-    mo.tally = arena.alloc<unsigned long long>(6);
-    CURC_CHECK(cudaMemsetAsync(mo.tally, 0, 6 * sizeof(unsigned long long), s));
+    mo.tally = arena.zeros<unsigned long long>(6, s);
     map_reads(p, hq.packed, hq.len, udb, U, nreads, NN, mo, arena, s);
     T.end();
     if (keep_intermediates) {

@@ -342,8 +342,7 @@ void Block::emit(StageTimer& T) {
     const int L = p.L, W = p.W;
     const uint32_t tot = U + NN;
     uint32_t* counts = arena.alloc<uint32_t>(8);
-    uint32_t* err = arena.alloc<uint32_t>(2);
-    CURC_CHECK(cudaMemsetAsync(err, 0, 8, s));
+    uint32_t* err = arena.zeros<uint32_t>(2, s);
 
     // ---- mapped records and unmapped lists (compress.cu:524-594)
     T.begin("emit");
@@ -423,7 +422,6 @@ void Block::emit(StageTimer& T) {
     // ---- mismatches (compress.cu:1815-1886)
     uint32_t* base_idx = arena.alloc<uint32_t>(Tn + 1);
     uint32_t* mis32 = arena.alloc<uint32_t>(Tn + 1);
-    CURC_CHECK(cudaMemsetAsync(mis32, 0, size_t(Tn + 1) * 4, s));
     widen_u8(smis, mis32, Tn, s);
     uint32_t* nbases_dev = counts + 3;
     exclusive_scan<uint32_t>(mis32, base_idx, Tn, nbases_dev, arena, s);
@@ -433,8 +431,7 @@ void Block::emit(StageTimer& T) {
     mbase = arena.alloc<uint8_t>(nbases ? nbases : 1);
     // classes
     const int maxm = p.max_mm;
-    uint32_t* chist = arena.alloc<uint32_t>(maxm + 2);
-    CURC_CHECK(cudaMemsetAsync(chist, 0, size_t(maxm + 2) * 4, s));
+    uint32_t* chist = arena.zeros<uint32_t>(maxm + 2, s);
     if (Tn) {
         class_hist_kernel<<<resident_grid(class_hist_kernel, 256, Tn), 256, 0, s>>>(smis, Tn, maxm + 2, chist);
         CURC_LAUNCH_CHECK();
@@ -478,8 +475,7 @@ void Block::emit(StageTimer& T) {
         CURC_LAUNCH_CHECK();
     }
     // context recode (compress.cu:1889-1929)
-    unsigned long long* chh = arena.alloc<unsigned long long>(20);
-    CURC_CHECK(cudaMemsetAsync(chh, 0, 20 * 8, s));
+    unsigned long long* chh = arena.zeros<unsigned long long>(20, s);
     uint8_t* rank = arena.alloc<uint8_t>(20);
     char* table = arena.alloc<char>(16);
     if (nbases) {
@@ -508,17 +504,12 @@ void Block::emit(StageTimer& T) {
         uint32_t* nx = arena.alloc<uint32_t>(n_ug);
         uint32_t* pv = arena.alloc<uint32_t>(n_ug);
         uint16_t* of = arena.alloc<uint16_t>(n_ug);
-        fill<uint32_t>(nx, INVALID, n_ug, s);
-        fill<uint32_t>(pv, INVALID, n_ug, s);
-        fill<uint16_t>(of, INVALOFF, n_ug, s);
         uint32_t* seqids = arena.alloc<uint32_t>(n_ug);
-        iota(seqids, n_ug, s);
         {
             auto mk = arena.mark();
             uint32_t* pre = arena.alloc<uint32_t>(n_ug);
             uint32_t* suf = arena.alloc<uint32_t>(n_ug);
-            iota(pre, n_ug, s);
-            iota(suf, n_ug, s);
+            unlinked(nx, pv, of, n_ug, s, seqids, pre, suf);
             full_match_packed(p, ldb, pre, suf, n_ug, nx, pv, of, arena, s);
             arena.release(mk);
         }

@@ -867,13 +867,12 @@ void full_match_events(const Acc& acc, uint32_t* pre, uint32_t* suf, uint32_t cn
         // prefix, so that 3% of the strings that meet none pass
         int bbits = 15;
         while (bbits < 32 && (1ull << bbits) < uint64_t(m) * 32) ++bbits;
-        uint32_t* bits = a.alloc<uint32_t>((1ull << bbits) / 32);
+        uint32_t* bits = a.zeros<uint32_t>((1ull << bbits) / 32, s);
         const uint32_t bmask = uint32_t((1ull << bbits) - 1);
         const uint32_t nw = uint32_t(div_up(m, 32));
         uint32_t* em = a.alloc<uint32_t>(size_t(words) * m);
         uint32_t* ub = a.alloc<uint32_t>(size_t(words) * m);
         uint32_t* count = a.alloc<uint32_t>(size_t(words) * 32 * nw);
-        CURC_CHECK(cudaMemsetAsync(bits, 0, (1ull << bbits) / 8, s));
         const State init{0, 0, m, {0, 0}};
         CURC_CHECK(cudaMemcpyAsync(st, &init, sizeof(init), cudaMemcpyHostToDevice, s));
         fm_prefix_kernel<Acc><<<grid_for(m, 256), 256, 0, s>>>(acc, pl, m, pk, fk, bits, bmask);
@@ -995,9 +994,7 @@ void sort_ids_by_ascii(const uint8_t* reads, int L, uint32_t* ids, uint32_t m, A
 void full_match_ascii(const BlockParams& p, const uint8_t* reads, uint32_t* ids, uint32_t m, uint32_t n_total,
                       uint32_t* next, uint32_t* prev, uint16_t* offset, Arena& a, cudaStream_t s) {
     // compress.cu:1179-1210: sort, duplicate links, prefix/suffix lists
-    fill<uint32_t>(next, INVALID, n_total, s);
-    fill<uint32_t>(prev, INVALID, n_total, s);
-    fill<uint16_t>(offset, INVALOFF, n_total, s);
+    unlinked(next, prev, offset, n_total, s);
     if (m == 0) return;
     sort_ids_by_ascii(reads, p.L, ids, m, a, s);
     if (m > 1) {
@@ -1011,8 +1008,7 @@ void full_match_ascii(const BlockParams& p, const uint8_t* reads, uint32_t* ids,
     CURC_LAUNCH_CHECK();
     uint32_t* pre = a.alloc<uint32_t>(m);
     uint32_t* suf = a.alloc<uint32_t>(m);
-    uint32_t* counts = a.alloc<uint32_t>(3);  // ends of each kind, other symbols seen
-    CURC_CHECK(cudaMemsetAsync(counts + 2, 0, 4, s));
+    uint32_t* counts = a.zeros<uint32_t>(3, s);  // ends of each kind, other symbols seen
     other_symbols_kernel<<<resident_grid(other_symbols_kernel, 256, uint64_t(m) * p.L), 256, 0, s>>>(reads, p.L, ids, m,
                                                                                                   counts + 2);
     CURC_LAUNCH_CHECK();

@@ -340,14 +340,25 @@ inline int log2_exact(uint32_t x) {
     return b;
 }
 
+// Every read unmapped: one mismatch more than allowed.
+__global__ void unmapped_kernel(uint8_t* __restrict__ mm, uint8_t* __restrict__ strand, uint64_t* __restrict__ pos,
+                                uint32_t n, uint8_t beyond) {
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    mm[i] = beyond;
+    strand[i] = 0;
+    pos[i] = 0;
+}
+
 }  // namespace
 
 void map_reads(const BlockParams& p, const uint64_t* ref, uint64_t ref_len, const uint64_t* udb, uint32_t U,
                const uint8_t* ndb, uint32_t NN, MapOut& out, Arena& a, cudaStream_t s) {
     const uint32_t total = U + NN;
-    fill<uint8_t>(out.mm, uint8_t(p.max_mm + 1), total, s);
-    fill<uint8_t>(out.strand, 0, total, s);
-    fill<uint64_t>(out.pos, 0, total, s);
+    if (total) {
+        unmapped_kernel<<<grid_for(total, 256), 256, 0, s>>>(out.mm, out.strand, out.pos, total, uint8_t(p.max_mm + 1));
+        CURC_LAUNCH_CHECK();
+    }
     const int k = BlockParams::k1, step = BlockParams::ref_step;
     if (total == 0 || ref_len < uint64_t(k)) return;
     const uint64_t index_count = (ref_len - k + 1 + step - 1) / step;

@@ -390,9 +390,8 @@ void overlap_link(const BlockParams& p, const uint64_t* db, const uint32_t* sort
         unsigned long long used, tally[3];
         uint32_t start[WALK_MAX_OFFS + 1];
     };
-    State* d = a.alloc<State>(1);
-    State h;
-    CURC_CHECK(cudaMemsetAsync(d, 0, sizeof(State), s));
+    State* d = a.zeros<State>(1, s);
+    State h{};
     select_flagged(sorted, pre_f, pre, m, &d->mp, a, s);
     select_flagged(sorted, suf_f, suf, m, &d->ms, a, s);
     read_small(&h, d, 8, s);
@@ -476,9 +475,8 @@ void overlap_link(const BlockParams& p, const uint64_t* db, const uint32_t* sort
             uint32_t* em = a.alloc<uint32_t>(size_t(words) * ms);
             uint32_t* ub = a.alloc<uint32_t>(size_t(words) * ms);
             uint32_t* per = a.alloc<uint32_t>(ms);
-            uint32_t* per_off = a.alloc<uint32_t>(WALK_MAX_OFFS);
-            CURC_CHECK(cudaMemsetAsync(per_off, 0, WALK_MAX_OFFS * 4, s));
-            CURC_CHECK(cudaMemsetAsync(&d->used, 0, 8, s));
+            uint32_t* per_off = a.zeros<uint32_t>(WALK_MAX_OFFS, s);
+            if (h.used) CURC_CHECK(cudaMemsetAsync(&d->used, 0, 8, s));
             // long lists fill the device with a thread per suffix
             const int each = ms > (1u << 18) ? words : 1;
             meet_kernel<<<dim3(unsigned(div_up(ms, 256)), unsigned(div_up(words, each))), 256,

@@ -23,6 +23,31 @@ uint64_t launches() { return g_launches.load(); }
 Arena::~Arena() {
     for (auto& c : chunks_) cudaFree(c.base);
     if (wait_error_) cudaFree(wait_error_);
+    if (zero_) cudaFree(zero_);
+}
+
+void Arena::clear_zeros(cudaStream_t s) {
+    zero_used_ = ZERO_POOL;
+    if (!zero_ && cudaMalloc(&zero_, ZERO_POOL) != cudaSuccess) {
+        cudaGetLastError();  // no room: pieces are cleared one by one
+        zero_ = nullptr;
+        return;
+    }
+    CURC_CHECK(cudaMemsetAsync(zero_, 0, ZERO_POOL, s));
+    zero_used_ = 0;
+    zero_stream_ = s;
+}
+
+void* Arena::zero_bytes(size_t bytes, cudaStream_t s) {
+    const size_t take = (bytes + 255) & ~size_t(255);
+    if (take <= ZERO_PIECE && zero_used_ + take <= ZERO_POOL && s == zero_stream_) {
+        void* p = zero_ + zero_used_;
+        zero_used_ += take;
+        return p;
+    }
+    void* p = alloc_bytes(bytes);
+    CURC_CHECK(cudaMemsetAsync(p, 0, bytes, s));
+    return p;
 }
 
 uint32_t* Arena::wait_error() {
@@ -124,6 +149,9 @@ void Arena::reset() {
 }
 
 void Arena::trim() {
+    if (zero_) CURC_CHECK(cudaFree(zero_));
+    zero_ = nullptr;
+    zero_used_ = ZERO_POOL;
     for (auto& c : chunks_) CURC_CHECK(cudaFree(c.base));
     chunks_.clear();
     cur_ = 0;
@@ -378,9 +406,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(const T* in, T* out,
 
 // Zeroed tile states and counter of a one-pass kernel.
 unsigned long long* look_states(size_t tiles, Arena& a, cudaStream_t s) {
-    unsigned long long* st = a.alloc<unsigned long long>(tiles + 1);
-    CURC_CHECK(cudaMemsetAsync(st, 0, (tiles + 1) * sizeof(unsigned long long), s));
-    return st;
+    return a.zeros<unsigned long long>(tiles + 1, s);
 }
 }  // namespace
 
@@ -759,9 +785,8 @@ void radix_sort_pairs(K* keys, V* vals, size_t n, int begin_bit, int end_bit, Ar
     const int np = dg.passes();
     // per pass: 256 states per tile and the tile counter; then the counts
     const size_t pass_words = size_t(tiles) * 256 + 1;
-    unsigned long long* st = a.alloc<unsigned long long>(pass_words * np + size_t(np) * 128);
+    unsigned long long* st = a.zeros<unsigned long long>(pass_words * np + size_t(np) * 128, s);
     uint32_t* hist = reinterpret_cast<uint32_t*>(st + pass_words * np);
-    CURC_CHECK(cudaMemsetAsync(st, 0, (pass_words * np + size_t(np) * 128) * sizeof(unsigned long long), s));
     rs_hist_kernel<K><<<unsigned(std::min<size_t>(div_up(n, RS_THREADS * 8), size_t(SM_COUNT_B200) * 8)), RS_THREADS, 0,
                         s>>>(keys, n, dg, hist);
     CURC_LAUNCH_CHECK();
@@ -808,6 +833,18 @@ __global__ void iota_kernel(uint32_t* p, size_t n) {
         p[i] = uint32_t(i);
 }
 
+__global__ void unlinked_kernel(uint32_t* next, uint32_t* prev, uint16_t* offset, size_t n, uint32_t* ids0,
+                                uint32_t* ids1, uint32_t* ids2) {
+    for (size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += size_t(gridDim.x) * blockDim.x) {
+        next[i] = INVALID;
+        prev[i] = INVALID;
+        offset[i] = INVALOFF;
+        if (ids0) ids0[i] = uint32_t(i);
+        if (ids1) ids1[i] = uint32_t(i);
+        if (ids2) ids2[i] = uint32_t(i);
+    }
+}
+
 int persistent_grid(size_t n) {
     size_t g = div_up(n, 256);
     return int(std::max<size_t>(1, std::min<size_t>(g, size_t(SM_COUNT_B200) * 16)));
@@ -827,6 +864,13 @@ void fill(T* p, T v, size_t n, cudaStream_t s) {
     fill_kernel<T><<<persistent_grid(n), 256, 0, s>>>(p, v, n);
     CURC_LAUNCH_CHECK();
 }
+void unlinked(uint32_t* next, uint32_t* prev, uint16_t* offset, size_t n, cudaStream_t s, uint32_t* ids0,
+              uint32_t* ids1, uint32_t* ids2) {
+    if (n == 0) return;
+    unlinked_kernel<<<persistent_grid(n), 256, 0, s>>>(next, prev, offset, n, ids0, ids1, ids2);
+    CURC_LAUNCH_CHECK();
+}
+
 template void fill<uint8_t>(uint8_t*, uint8_t, size_t, cudaStream_t);
 template void fill<uint16_t>(uint16_t*, uint16_t, size_t, cudaStream_t);
 template void fill<uint32_t>(uint32_t*, uint32_t, size_t, cudaStream_t);
@@ -1044,10 +1088,8 @@ void sort_rows(const uint64_t* db, int W, int last_bits, uint32_t* ids, size_t n
         radix_sort_pairs<uint64_t, uint32_t>(k0, ids, n, W == 1 ? 64 - last_bits : 0, first_bits, a, s);
     }
     if (W > 1) {
-        uint8_t* large = a.alloc<uint8_t>(n);
-        uint32_t* cnt = a.alloc<uint32_t>(2);
-        CURC_CHECK(cudaMemsetAsync(large, 0, n, s));
-        CURC_CHECK(cudaMemsetAsync(cnt, 0, 8, s));
+        uint8_t* large = a.zeros<uint8_t>(n, s);
+        uint32_t* cnt = a.zeros<uint32_t>(2, s);
         order_runs_kernel<<<grid_for(n, 256), 256, 0, s>>>(db, W, ids, k0, uint32_t(n), large, cnt);
         CURC_LAUNCH_CHECK();
         const uint32_t m = read_scalar(cnt, s);

@@ -38,6 +38,16 @@ public:
     uint32_t* wait_error();
     // Throws when a host copy of it (4 bytes) is set, and clears it.
     void check_waits(const void* copy, cudaStream_t s);
+    // Zeroed scratch of a run.  clear_zeros() clears a pool once, at the
+    // start of a run; zeros() takes pieces of it, each handed out once per
+    // clearing.  What does not fit there, or is asked for on another stream,
+    // is allocated and cleared by itself: a small memset costs 6 us between
+    // two kernels (2 us and the gaps around it), and a block of 100k pairs
+    // had 119 of them in 7 ms.
+    void clear_zeros(cudaStream_t s);
+    void* zero_bytes(size_t bytes, cudaStream_t s);
+    template <class T>
+    T* zeros(size_t n, cudaStream_t s) { return static_cast<T*>(zero_bytes(n * sizeof(T), s)); }
     size_t high_water() const { return high_water_; }
     size_t in_use() const;
 
@@ -53,6 +63,13 @@ private:
     size_t chunk_;
     size_t high_water_ = 0;
     uint32_t* wait_error_ = nullptr;
+    // 16 MiB clear in 3 us and hold the tile states of every sort of a block
+    // of some 100k reads; a piece of 4 MiB or more is long enough to be
+    // cleared by itself
+    static constexpr size_t ZERO_POOL = size_t(16) << 20, ZERO_PIECE = size_t(4) << 20;
+    char* zero_ = nullptr;
+    size_t zero_used_ = ZERO_POOL;  // nothing clear yet
+    cudaStream_t zero_stream_ = nullptr;
 };
 
 // Growable pinned host memory, bump allocated, reset per block; results are
@@ -167,6 +184,11 @@ void gather_words(const uint64_t* src, const uint32_t* idx, size_t n, int stride
 
 template <class T>
 void fill(T* p, T v, size_t n, cudaStream_t s);
+
+// The links of n unlinked reads (next, prev, offset), and up to three lists
+// of their numbers (null: none).
+void unlinked(uint32_t* next, uint32_t* prev, uint16_t* offset, size_t n, cudaStream_t s, uint32_t* ids0 = nullptr,
+              uint32_t* ids1 = nullptr, uint32_t* ids2 = nullptr);
 
 void iota(uint32_t* p, size_t n, cudaStream_t s);
 

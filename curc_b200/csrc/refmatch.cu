@@ -628,8 +628,7 @@ void refmatch_one(const RmIndex& ix, const uint8_t* dest, const uint64_t* dest_p
     SubStage sp_probe(dest_is_ref ? "refmatch.probe_self" : "refmatch.probe_unmapped");
     const uint64_t nslots = has_n ? dic : div_up(dic, 4);
     uint8_t* flag = a.alloc<uint8_t>(nslots);
-    uint32_t* cnt = a.alloc<uint32_t>(4);
-    CURC_CHECK(cudaMemsetAsync(cnt, 0, 16, s));
+    uint32_t* cnt = a.zeros<uint32_t>(4, s);
     uint32_t* sel = a.alloc<uint32_t>(nslots);
     uint32_t c = 0;       // hits that go on
     uint64_t* rows = nullptr;
