@@ -21,6 +21,22 @@ struct HostBuf {
 
 struct Block {
     cudaStream_t stream = nullptr;
+    // Results leave on a stream of their own while the run goes on (send):
+    // `made`, the device has them; `sent`, they are in host memory.
+    cudaStream_t copy_stream = nullptr;
+    cudaEvent_t made = nullptr, sent = nullptr;
+    struct Piece {
+        const uint8_t* dev;
+        uint8_t* host;
+        uint32_t bytes;
+    };
+    static constexpr size_t SEND_SMALL = size_t(32) << 10;
+    static constexpr int SEND_PIECES = 32;
+    struct Pieces {
+        Piece p[SEND_PIECES];
+    };
+    std::vector<Piece> small;                       // results kept since the last send
+    std::vector<std::pair<HostBuf, const uint8_t*>> large;
     Arena arena;
     bool keep_intermediates = true;
     Tuning tune;  // launch and table choices for the next runs (no effect on results)
@@ -55,8 +71,16 @@ struct Block {
     PinnedArena pinned;
     std::map<std::string, float> stage_ms;
 
-    Block() { CURC_CHECK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking)); }
+    Block() {
+        CURC_CHECK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
+        CURC_CHECK(cudaStreamCreateWithFlags(&copy_stream, cudaStreamNonBlocking));
+        CURC_CHECK(cudaEventCreateWithFlags(&made, cudaEventDisableTiming));
+        CURC_CHECK(cudaEventCreateWithFlags(&sent, cudaEventDisableTiming));
+    }
     ~Block() {
+        if (made) cudaEventDestroy(made);
+        if (sent) cudaEventDestroy(sent);
+        if (copy_stream) cudaStreamDestroy(copy_stream);
         if (stream) cudaStreamDestroy(stream);
     }
     Block(const Block&) = delete;
@@ -68,17 +92,30 @@ struct Block {
     // a12 on the three pseudogenomes; fills the ref / map streams
     void refmatch_all();
 
-    // D2H copy of a device array into pinned staging (async on the stream)
+    // A device array as a result: room in pinned staging, filled by the next
+    // send() and there when the run returns.  The array stays as it is until
+    // then, or until wait_sent().
     template <class T>
     void keep(const std::string& name, const T* dev, size_t count) {
         HostBuf b;
         b.size = count * sizeof(T);
         if (count) {
             uint8_t* p = pinned.alloc(b.size);
-            CURC_CHECK(cudaMemcpyAsync(p, dev, b.size, cudaMemcpyDeviceToHost, stream));
             b.ptr = p;
+            const uint8_t* d = reinterpret_cast<const uint8_t*>(dev);
+            if (b.size <= SEND_SMALL) small.push_back(Piece{d, p, uint32_t(b.size)});
+            else large.push_back({b, d});
         }
         host[name] = std::move(b);
+    }
+    // Queues what was kept, as the stream's work so far leaves it.
+    void send();
+    // Later work of the stream waits for all that was sent.
+    void wait_sent();
+    // Kept and sent, and unchanged until it has left.
+    void send_now() {
+        send();
+        wait_sent();
     }
     void put(const std::string& name, std::vector<uint8_t>&& v) {
         HostBuf b;

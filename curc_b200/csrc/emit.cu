@@ -494,6 +494,28 @@ void Block::emit(StageTimer& T) {
         if (he[0]) throw std::runtime_error("emit: mismatch count disagrees with mapping");
         if (he[1]) throw std::runtime_error("emit: unexpected symbol in a mismatch");
     }
+    // what is ready leaves while the unmapped pseudogenomes are assembled
+    keep("strand", strand, Tn);
+    keep("mis_cnt", smis, Tn);
+    keep("mis_base", mbase, nbases);
+    keep("decoder_table", table, 16);
+    keep("read_off", read_off, p.preserve_order ? 0 : Tn);
+    {
+        // per-class offset streams: consecutive slices of off_all
+        keep("mis_off", off_all, class_elems);
+        const HostBuf all = host["mis_off"];
+        host.erase("mis_off");
+        uint64_t b = 0;
+        for (int mm = 1; mm <= p.max_mm; ++mm) {
+            HostBuf h;
+            const uint64_t ne = uint64_t(class_count[mm]) * class_width(mm);
+            h.size = ne * sizeof(uint16_t);
+            if (ne) h.ptr = all.ptr + b * sizeof(uint16_t);
+            host["mis_off_" + std::to_string(mm)] = h;
+            b += ne;
+        }
+    }
+    send();
     T.end();
 
     // ---- a11: unmapped pseudogenomes (compress.cu:1649-1728)
@@ -548,39 +570,24 @@ void Block::emit(StageTimer& T) {
             pe_order + Tn + lq.n_records, id_to_pos);
         CURC_LAUNCH_CHECK();
     }
-    T.end();
-
     // ---- host copies of the streams
-    keep("strand", strand, Tn);
-    keep("mis_cnt", smis, Tn);
-    keep("mis_base", mbase, nbases);
-    keep("decoder_table", table, 16);
     if (!p.preserve_order) {
-        keep("read_off", read_off, Tn);
         keep("unmap_read_off", uoff, lq.n_records);
         keep("unmap_n_read_off", unoff, lqn.n_records);
         keep("pe_order", pe_order, pe_total);
         keep("id_to_pos", id_to_pos, 0);
     } else {
-        keep("read_off", read_off, 0);
         keep("unmap_read_off", uoff, 0);
         keep("unmap_n_read_off", unoff, 0);
         keep("pe_order", pe_order, 0);
         keep("id_to_pos", id_to_pos, n);
     }
-    {
-        // per-class offset streams: consecutive slices of off_all
-        uint64_t b = 0;
-        for (int mm = 1; mm <= p.max_mm; ++mm) {
-            const uint64_t ne = uint64_t(class_count[mm]) * class_width(mm);
-            keep("mis_off_" + std::to_string(mm), off_all + b, ne);
-            b += ne;
-        }
-    }
     if (keep_intermediates) {
         keep("unmap_seq", lq.seq, lq.len);
         keep("unmap_n_seq", lqn.seq, lqn.len);
     }
+    send();
+    T.end();
 
     // ---- a12: reverse-complement repeat removal
     T.begin("refmatch");

@@ -603,8 +603,8 @@ inline int log2_ceil(uint32_t x) {
     return b;
 }
 
-// Device views of one destination's results (valid until the arena region
-// is reused: the caller copies them out before the next destination).
+// Device views of one destination's results (valid as long as the arena
+// region that the caller marked).
 struct RmResult {
     const uint8_t* seq = nullptr;
     uint64_t seq_len = 0;
@@ -624,6 +624,13 @@ void refmatch_one(const RmIndex& ix, const uint8_t* dest, const uint64_t* dest_p
     const uint64_t dic = dl >= uint64_t(RM_K) ? (dl - RM_K + 1 + RM_DEST_STEP - 1) / RM_DEST_STEP : 0;
     const uint64_t cap = uint64_t(double(dic) * (dest_is_ref ? 0.2 : 0.21));
     if (dic == 0 || ix.rl < uint64_t(RM_K)) return;
+    // Results, below the scratch so that they stay while the next destination
+    // reuses it (they are still on their way to the host): kept spans do not
+    // overlap and have 50 bases or more, and a length takes at most 10 bytes.
+    const uint64_t most = std::min(cap, dl / RM_MIN);
+    uint8_t* moff = a.alloc<uint8_t>(most * 8 + 8);
+    uint8_t* mlen = a.alloc<uint8_t>(most * 10 + 16);
+    uint8_t* out = a.alloc<uint8_t>(dl + 16);
     auto mk = a.mark();
     SubStage sp_probe(dest_is_ref ? "refmatch.probe_self" : "refmatch.probe_unmapped");
     const uint64_t nslots = has_n ? dic : div_up(dic, 4);
@@ -741,8 +748,6 @@ void refmatch_one(const RmIndex& ix, const uint8_t* dest, const uint64_t* dest_p
     uint64_t* se = a.alloc<uint64_t>(K + 1);
     uint64_t* removed = a.alloc<uint64_t>(K + 2);
     uint32_t* lsize = a.alloc<uint32_t>(K + 1);
-    uint8_t* moff = a.alloc<uint8_t>(uint64_t(K) * 8 + 8);
-    uint8_t* mlen = a.alloc<uint8_t>(uint64_t(K) * 10 + 16);
     if (K) {
         kept_spans_kernel<<<grid_for(K, 256), 256, 0, s>>>(ksel, K, uniq, adst, alen, std32, sd, se, removed, lsize,
                                                             moff);
@@ -762,7 +767,6 @@ void refmatch_one(const RmIndex& ix, const uint8_t* dest, const uint64_t* dest_p
     r.off_len = hi[1];
     r.map_len = mlen;
     r.len_len = hi[2];
-    uint8_t* out = a.alloc<uint8_t>(hi[3] + 16);
     compact_string_kernel<<<grid_for(div_up(hi[3], 16), 256), 256, 0, s>>>(dest, hi[3], sd, se, removed, hi[0], out);
     CURC_LAUNCH_CHECK();
     r.seq = out;
@@ -805,22 +809,24 @@ void Block::refmatch_all() {
     } else {
         ix.rl = 0;  // no index: every pseudogenome is kept as assembled
     }
-    // results are copied out right after each destination, before the next
-    // one reuses the scratch region
+    // each destination's results leave while the next one is searched
     refmatch_one(ix, lq.seq, lq.packed, lq.len, false, false, r, arena, s);
     keep("unmap_ref", r.seq, r.seq_len);
     keep("unmap_ref_off", r.map_off, r.off_len);
     keep("unmap_ref_len", r.map_len, r.len_len);
+    send();
     const uint64_t un_len = r.seq_len;
     refmatch_one(ix, lqn.seq, lqn.packed, lqn.len, true, false, r, arena, s);
     keep("unmap_n_ref", r.seq, r.seq_len);
     keep("unmap_n_ref_off", r.map_off, r.off_len);
     keep("unmap_n_ref_len", r.map_len, r.len_len);
+    send();
     const uint64_t unn_len = r.seq_len;
     refmatch_one(ix, hq.seq, hq.packed, hq.len, false, true, r, arena, s);
     keep("ref", r.seq, r.seq_len);
     keep("ref_off", r.map_off, r.off_len);
     keep("ref_len_map", r.map_len, r.len_len);
+    send();
     const uint64_t main_len = r.seq_len;
     arena.release(mk);
     const uint64_t sizes[6] = {hq.len, lq.len, lqn.len, main_len, un_len, unn_len};
