@@ -492,7 +492,6 @@ void full_match_passes(const Acc& acc, uint32_t* pre, uint32_t* suf, uint32_t cn
             if (h[0] == 0 || h[1] == 0) break;
         }
     }
-    cp.check();
     a.release(mk);
 }
 
@@ -903,7 +902,6 @@ void full_match_events(const Acc& acc, uint32_t* pre, uint32_t* suf, uint32_t cn
         m = h.len_out[0];
         hi = low - 1;
     }
-    cp.check();
     if (hi >= 1 && m > 0) small(pl, sl, m, acc.L - hi, true);
     a.release(mk);
 }

@@ -530,7 +530,6 @@ void overlap_link(const BlockParams& p, const uint64_t* db, const uint32_t* sort
             }
             a.release(mk2);
         }
-        cp.check();
     }
     if (st) {
         read_small(&h, d, sizeof(State), s);
