@@ -10,6 +10,8 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
+#include <mutex>
+#include <stdexcept>
 
 #include "common.cuh"
 
@@ -163,19 +165,109 @@ static __device__ __forceinline__ void walk_offset(const Meeting* __restrict__ i
     }
 }
 
+// A run of up to FEW suffixes and FEW prefixes, by the thread of its first
+// meeting: its reads, which do not depend on the links and are loaded ahead
+// of the barrier.  ns = 0: not a run's first meeting; np = 0: a longer run.
+constexpr uint32_t FEW = 4;
+struct Ahead {
+    uint32_t s[FEW], p[FEW];
+    uint32_t ns, np;
+};
+__device__ __forceinline__ Ahead look_ahead(const Meeting* __restrict__ item, uint32_t a, uint32_t e, uint32_t i,
+                                            const uint32_t* __restrict__ pre) {
+    Ahead h;
+    h.ns = h.np = 0;
+    if (i >= e) return h;
+    const Meeting it = item[i];
+    if (i > a && item[i - 1].lo == it.lo) return h;
+    h.s[0] = it.s;
+    h.p[0] = it.p;
+    h.ns = 1;
+#pragma unroll
+    for (uint32_t k = 1; k <= FEW; ++k) {
+        if (h.ns < k || i + k >= e) continue;
+        const Meeting m = item[i + k];
+        if (m.lo != it.lo) continue;
+        h.ns = k + 1;
+        if (k < FEW) h.s[k] = m.s;
+    }
+    if (h.ns > FEW || it.hi - it.lo > FEW) return h;
+    h.np = it.hi - it.lo;
+#pragma unroll
+    for (uint32_t k = 1; k < FEW; ++k)
+        if (k < h.np) h.p[k] = pre[it.lo + k];
+    return h;
+}
+
+// The same with the runs read ahead (h: this thread's first): one thread per
+// run of few, whose links are loaded together and paired in registers, longer
+// runs by a warp.  Where the overlap stage walks thousands of meetings an
+// offset, mostly of runs of one to three, a thread's chain of ten dependent
+// loads was what an offset took; where an offset has few meetings, as in the
+// full match, the plain form is the shorter one.
+static __device__ __forceinline__ void walk_offset_ahead(const Meeting* __restrict__ item, uint32_t a, uint32_t e,
+                                                   uint32_t threads, uint32_t me, Ahead h,
+                                                   const uint32_t* __restrict__ pre, int off, uint32_t* next,
+                                                   uint32_t* prev, uint16_t* offset) {
+    for (uint32_t i0 = a;;) {  // the same trip count for a whole warp
+        if (h.np) {
+            uint32_t fs = 0, fp = 0;  // free suffixes and prefixes
+#pragma unroll
+            for (uint32_t k = 0; k < FEW; ++k) {
+                if (k < h.ns && ld_l2(next + h.s[k]) == INVALID) fs |= 1u << k;
+                if (k < h.np && ld_l2(prev + h.p[k]) == INVALID) fp |= 1u << k;
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < FEW; ++k) {
+                if (!(fs >> k & 1u)) continue;
+                bool open = true;
+#pragma unroll
+                for (uint32_t q = 0; q < FEW; ++q)
+                    if (open && (fp >> q & 1u) && h.p[q] != h.s[k]) {
+                        open = false;
+                        fp &= ~(1u << q);
+                        next[h.s[k]] = h.p[q];
+                        prev[h.p[q]] = h.s[k];
+                        offset[h.s[k]] = uint16_t(off);
+                    }
+            }
+        }
+        uint32_t todo = __ballot_sync(0xFFFFFFFFu, h.ns && !h.np);
+        while (todo) {
+            const int l = __ffs(todo) - 1;
+            todo &= todo - 1;
+            const uint32_t ii = i0 + me - (threadIdx.x & 31u) + l;
+            const Meeting it = item[ii];
+            walk_run_warp(item, ii, e, pre, it.lo, it.hi, off, next, prev, offset);
+        }
+        i0 += threads;
+        if (i0 >= e) return;
+        h = look_ahead(item, a, e, i0 + me, pre);
+    }
+}
+
 // One offset by a whole grid.
 static __global__ void __launch_bounds__(256) walk_one_kernel(const Meeting* __restrict__ item, uint32_t a, uint32_t e,
                                                               int off, const uint32_t* __restrict__ pre, uint32_t* next,
                                                               uint32_t* prev, uint16_t* offset) {
-    walk_offset(item, a, e, gridDim.x * 256, blockIdx.x * 256 + threadIdx.x, pre, off, next, prev, offset);
+    const uint32_t me = blockIdx.x * 256 + threadIdx.x;
+    if (a < e)
+        walk_offset_ahead(item, a, e, gridDim.x * 256, me, look_ahead(item, a, e, a + me, pre), pre, off, next, prev,
+                          offset);
 }
 
 // The walk: offset after offset, one thread per run of equal suffix strings
 // (long runs: a warp).  Runs of one offset share no read, so an offset's runs
 // are independent; a barrier over the cluster separates the offsets.  One
 // cluster suffices: an offset has few meetings (thousands at most where a
-// list has 400,000 entries), and its time is the latency of two dependent
-// loads and the barrier.
+// list has 400,000 entries), and its time is the latency of its dependent
+// loads, the sectors that 8 or 16 SMs can ask for, and the barrier.  With
+// AHEAD the next offset's runs are read between the barrier's two halves.
+// Overlap stage on B200, 8 blocks plain, 16 blocks plain, 16 with AHEAD: 100k
+// pairs 0.64, 0.44, 0.37 ms; 700k reads of 251 1.00, 0.90, 0.75; 8M of 250
+// 3.22, 2.56, 2.09 (blocks of 256 or 1024 threads: slower, as is AHEAD in one
+// block: 64 offsets of 83 meetings 0.133 -> 0.158).
+template <bool AHEAD>
 static __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(const Meeting* __restrict__ item,
                                                                    const uint32_t* __restrict__ start_in, int off0,
                                                                    int noffs, const uint32_t* __restrict__ pre,
@@ -193,30 +285,49 @@ static __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(const Meeting
         tally[1] += start[noffs];
         tally[2] += start[noffs];
     }
-    for (int o = 0; o < noffs; ++o) {
-        const uint32_t a = start[o], e = start[o + 1];
-        if (a == e) continue;
-        walk_offset(item, a, e, threads, me, pre, off0 + o, next, prev, offset);
+    auto skip = [&](int o) {  // the next offset with meetings
+        while (o < noffs && start[o] == start[o + 1]) ++o;
+        return o;
+    };
+    int o = skip(0);
+    if (o == noffs) return;
+    Ahead h;
+    if (AHEAD) h = look_ahead(item, start[o], start[o + 1], start[o] + me, pre);
+    for (;;) {
+        if (AHEAD) walk_offset_ahead(item, start[o], start[o + 1], threads, me, h, pre, off0 + o, next, prev, offset);
+        else walk_offset(item, start[o], start[o + 1], threads, me, pre, off0 + o, next, prev, offset);
+        o = skip(o + 1);
+        if (o == noffs) return;
         if (gridDim.x > 1) {
-            asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            if (AHEAD) h = look_ahead(item, start[o], start[o + 1], start[o] + me, pre);
+            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
         } else {
             __syncthreads();
         }
     }
 }
 
-
-// Walks the meetings of offsets [off0, off0 + noffs), noffs <= WALK_MAX_OFFS;
-// start (device) holds the first item of each offset and the end of the last.
-inline void walk_meetings(const Meeting* item, const uint32_t* start, int off0, int noffs, const uint32_t* pre,
-                          const unsigned long long* used, uint32_t cap, uint32_t entries, uint32_t* next,
-                          uint32_t* prev, uint16_t* offset, unsigned long long* tally, cudaStream_t s) {
+// The launch, with clusters of 16 allowed (once per device).
+template <bool AHEAD>
+static void walk_launch(unsigned blocks, const Meeting* item, const uint32_t* start, int off0, int noffs,
+                        const uint32_t* pre, const unsigned long long* used, uint32_t cap, uint32_t* next,
+                        uint32_t* prev, uint16_t* offset, unsigned long long* tally, cudaStream_t s) {
+    static std::mutex mu;
+    static bool done[64] = {};
+    int dev = 0;
+    CURC_CHECK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) throw std::runtime_error("device ordinal out of range");
+    {
+        std::lock_guard<std::mutex> g(mu);
+        if (!done[dev]) {
+            CURC_CHECK(cudaFuncSetAttribute(walk_kernel<AHEAD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            done[dev] = true;
+        }
+    }
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeClusterDimension;
-    // short lists meet a few hundred at a time: one block, whose barrier is
-    // cheaper than the cluster's
-    const unsigned blocks = entries > 16384 ? 8 : 1;
     at.val.clusterDim.x = blocks;
     at.val.clusterDim.y = at.val.clusterDim.z = 1;
     cfg.gridDim = dim3(blocks);
@@ -224,16 +335,29 @@ inline void walk_meetings(const Meeting* item, const uint32_t* start, int off0, 
     cfg.stream = s;
     cfg.attrs = &at;
     cfg.numAttrs = 1;
-    CURC_CHECK(cudaLaunchKernelEx(&cfg, walk_kernel, item, start, off0, noffs, pre, used, cap, next, prev, offset,
-                                  tally));
+    CURC_CHECK(cudaLaunchKernelEx(&cfg, walk_kernel<AHEAD>, item, start, off0, noffs, pre, used, cap, next, prev,
+                                  offset, tally));
     CURC_LAUNCH_CHECK();
+}
+constexpr unsigned WALK_CLUSTER = 16;
+
+// Walks the meetings of offsets [off0, off0 + noffs), noffs <= WALK_MAX_OFFS;
+// start (device) holds the first item of each offset and the end of the last.
+static inline void walk_meetings(const Meeting* item, const uint32_t* start, int off0, int noffs, const uint32_t* pre,
+                                 const unsigned long long* used, uint32_t cap, uint32_t entries, uint32_t* next,
+                                 uint32_t* prev, uint16_t* offset, unsigned long long* tally, cudaStream_t s) {
+    // short lists meet a few hundred at a time: one block, whose barrier is
+    // cheaper than the cluster's (50k reads, 2,048 to 4,096 ends: full match
+    // 0.33 against 0.36 ms; 100k reads, more ends: 0.60 against 0.53)
+    walk_launch<false>(entries > 4096 ? WALK_CLUSTER : 1, item, start, off0, noffs, pre, used, cap, next, prev, offset,
+                       tally, s);
 }
 
 // The same with the starts known to the host: an offset with many meetings is
 // walked by a grid of its own (one launch each, no barrier), the others
 // between them by one cluster.
 constexpr uint32_t WALK_GRID = 32768;
-inline void walk_stage(const Meeting* item, const uint32_t* host_start, const uint32_t* start, int off0, int noffs,
+static inline void walk_stage(const Meeting* item, const uint32_t* host_start, const uint32_t* start, int off0, int noffs,
                        const uint32_t* pre, const unsigned long long* used, uint32_t cap, uint32_t* next,
                        uint32_t* prev, uint16_t* offset, cudaStream_t s) {
     for (int o = 0; o < noffs;) {
@@ -251,8 +375,11 @@ inline void walk_stage(const Meeting* item, const uint32_t* host_start, const ui
             most = std::max(most, host_start[e + 1] - host_start[e]);
             ++e;
         }
-        if (host_start[e] != host_start[o])
-            walk_meetings(item, start + o, off0 + o, e - o, pre, used, cap, most * 8, next, prev, offset, nullptr, s);
+        if (host_start[e] != host_start[o]) {
+            const bool many = most > 2048;
+            (many ? walk_launch<true> : walk_launch<false>)(many ? WALK_CLUSTER : 1, item, start + o, off0 + o, e - o, pre,
+                                                            used, cap, next, prev, offset, nullptr, s);
+        }
         o = e;
     }
 }
