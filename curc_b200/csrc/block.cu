@@ -101,26 +101,17 @@ void Block::run(const uint8_t* d_seq, uint64_t n_reads, int L, bool po, bool pe)
         cudaStream_t s;
         ~Sent() { cudaStreamSynchronize(s); }
     } sent_guard{copy_stream};
-    StageTimer T{stream, {}, {}};
+    StageTimer T(stream, events);
     struct TimerScope {
         explicit TimerScope(StageTimer* t) { active_timer() = t; }
         ~TimerScope() { active_timer() = nullptr; }
     } timer_scope(&T);
     cudaStream_t s = stream;
     const int W = p.W;
-    struct RunEvents {  // released on every exit from the run
-        cudaEvent_t a = nullptr, b = nullptr;
-        ~RunEvents() {
-            if (a) cudaEventDestroy(a);
-            if (b) cudaEventDestroy(b);
-        }
-    } run_ev;
-    CURC_CHECK(cudaEventCreate(&run_ev.a));
-    CURC_CHECK(cudaEventCreate(&run_ev.b));
-    cudaEvent_t ev0 = run_ev.a, ev1 = run_ev.b;
-    CURC_CHECK(cudaEventRecord(ev0, s));
+    const cudaEvent_t ev0 = T.mark();
     uint32_t* counts = arena.alloc<uint32_t>(16);
     arena.clear_zeros(s);
+    T.part();
     uint32_t* err = arena.zeros<uint32_t>(1, s);
 
     // a1
@@ -246,6 +237,7 @@ void Block::run(const uint8_t* d_seq, uint64_t n_reads, int L, bool po, bool pe)
     uint8_t* waits = pinned.alloc(sizeof(uint32_t));
     small.push_back(Piece{reinterpret_cast<const uint8_t*>(arena.wait_error()), waits, sizeof(uint32_t)});
     send_now();
+    const cudaEvent_t ev1 = events.take();
     CURC_CHECK(cudaEventRecord(ev1, s));
     T.collect(stage_ms);
     CURC_CHECK(cudaStreamSynchronize(s));

@@ -25,6 +25,7 @@ struct Block {
     // `made`, the device has them; `sent`, they are in host memory.
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t made = nullptr, sent = nullptr;
+    EventPool events;
     struct Piece {
         const uint8_t* dev;
         uint8_t* host;

@@ -243,28 +243,30 @@ void PinnedArena::reset() {
 
 // ---------------------------------------------------------------- stage timer
 
-size_t StageTimer::begin_span(const std::string& name) {
-    Span sp{name, nullptr, nullptr};
-    CURC_CHECK(cudaEventCreate(&sp.a));
-    CURC_CHECK(cudaEventCreate(&sp.b));
-    CURC_CHECK(cudaEventRecord(sp.a, s));
-    ev.push_back(sp);
-    return ev.size() - 1;
+cudaEvent_t StageTimer::mark() {
+    // (another thread's launches only make it record once more)
+    if (!last_ || launches() != last_launches_) {
+        last_launches_ = launches();
+        last_ = pool_.take();
+        CURC_CHECK(cudaEventRecord(last_, s_));
+    }
+    return last_;
 }
 
-void StageTimer::end_span(size_t i) { CURC_CHECK(cudaEventRecord(ev[i].b, s)); }
+size_t StageTimer::begin_span(const std::string& name) {
+    ev_.push_back(Span{name, mark(), nullptr});
+    return ev_.size() - 1;
+}
 
 void StageTimer::collect(std::map<std::string, float>& out) {
-    CURC_CHECK(cudaStreamSynchronize(s));
-    for (auto& e : ev) {
+    CURC_CHECK(cudaStreamSynchronize(s_));
+    for (auto& e : ev_) {
         float ms = 0;
-        CURC_CHECK(cudaEventElapsedTime(&ms, e.a, e.b));
+        if (e.a != e.b) CURC_CHECK(cudaEventElapsedTime(&ms, e.a, e.b));
         out[e.name] += ms;
-        cudaEventDestroy(e.a);
-        cudaEventDestroy(e.b);
     }
-    ev.clear();
-    open.clear();
+    ev_.clear();
+    open_.clear();
 }
 
 StageTimer*& active_timer() {

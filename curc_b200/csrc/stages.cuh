@@ -13,11 +13,10 @@ namespace curc {
 std::string& ctxless_error();
 
 // Launch and table choices that change no result (the autotuner's knobs):
-// the overlap index's bucket table size as a multiple of the prefix count
-// (the reference's get_hash_size is factor 1; equal strings share a bucket
-// whatever the size), bits of the prefix presence bitmap per prefix, how
-// many overlap passes run between host reads of the link count, and the
-// threads per block of the mapping kernel (one warp per read).
+// the overlap index's bucket table size in quarters of the prefix count
+// (equal strings share a bucket whatever the size), bits of the prefix
+// presence bitmap per prefix, the offsets of the overlap's first stage on a
+// long list, and the threads per block of the mapping kernel.
 struct Tuning {
     int table_factor = 4, bitmap_bits = 16, check_every = 8, map_threads = 128;
     int fm_loop = 1;  // full match: 0 a pass of launches per offset, 1 and 2 meetings listed at once

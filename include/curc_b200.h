@@ -101,14 +101,14 @@ int curc_ctx_keep_intermediates(curc_ctx* ctx, int keep);
 int curc_ctx_trim(curc_ctx* ctx);
 
 /* Autotuner (no counterpart in the reference).  Knobs, in this order: the
- * overlap index's bucket table size as a multiple of the prefix count
- * {1, 2, 4, 8}, presence-bitmap bits per prefix {8, 16, 32}, overlap passes
- * between host reads of the link count {2, 4, 8, 16}, threads per block of
+ * overlap index's bucket table size in quarters of the prefix count
+ * {1, 2, 4, 8}, presence-bitmap bits per prefix {8, 16, 32}, offsets of the
+ * overlap's first stage on a long list {2, 4, 8, 16}, threads per block of
  * the mapping kernel {64, 128, 256}, and the form of the full match: a pass
  * of launches per offset, queued from the host (0), or every meeting of a
  * suffix with prefixes listed at once and walked offset by offset (1; 2 is
- * the same).  None changes any result: every stream
- * is the same under every setting; only the time does.  curc_autotune runs
+ * the same).  None changes any result: every stream is the same under every
+ * setting; only the time does.  curc_autotune runs
  * the given block (device memory) under the candidates one knob at a time,
  * keeps the fastest, and sets it on the context; with cache_path, choices
  * are read from and saved to that file per (read length, read count rounded
