@@ -6,6 +6,7 @@
 #include <string>
 
 #include <mutex>
+#include <set>
 
 #include "primitives.cuh"
 
@@ -272,6 +273,17 @@ void StageTimer::collect(std::map<std::string, float>& out) {
 StageTimer*& active_timer() {
     thread_local StageTimer* t = nullptr;
     return t;
+}
+
+void allow_large_clusters(const void* kernel) {
+    static std::mutex mu;
+    static std::set<std::pair<int, const void*>> done;
+    int dev = 0;
+    CURC_CHECK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> g(mu);
+    if (done.count({dev, kernel})) return;
+    CURC_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    done.insert({dev, kernel});
 }
 
 // ---------------------------------------------------------------- scan

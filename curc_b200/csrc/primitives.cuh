@@ -180,6 +180,28 @@ struct SubStage {
     }
 };
 
+// Clusters of more than 8 blocks are not portable: allowed for `kernel` on
+// the current device, once.
+void allow_large_clusters(const void* kernel);
+
+// Launches one cluster of `blocks` (at most 16) blocks.
+template <class... P, class... Q>
+void launch_cluster(void (*kernel)(P...), unsigned blocks, unsigned threads, cudaStream_t s, Q... args) {
+    if (blocks > 8) allow_large_clusters(reinterpret_cast<const void*>(kernel));
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = blocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    CURC_CHECK(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+    CURC_LAUNCH_CHECK();
+}
+
 // out[i] = sum(in[0..i)); optionally *total = sum(in[0..n)) (device pointer).
 // In-place (out == in) is allowed.
 template <class T>

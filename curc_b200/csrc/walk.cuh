@@ -10,10 +10,9 @@
 #include <cuda_runtime.h>
 #include <algorithm>
 #include <cstdint>
-#include <mutex>
-#include <stdexcept>
 
 #include "common.cuh"
+#include "primitives.cuh"
 
 namespace curc {
 
@@ -308,37 +307,6 @@ static __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(const Meeting
     }
 }
 
-// The launch, with clusters of 16 allowed (once per device).
-template <bool AHEAD>
-static void walk_launch(unsigned blocks, const Meeting* item, const uint32_t* start, int off0, int noffs,
-                        const uint32_t* pre, const unsigned long long* used, uint32_t cap, uint32_t* next,
-                        uint32_t* prev, uint16_t* offset, unsigned long long* tally, cudaStream_t s) {
-    static std::mutex mu;
-    static bool done[64] = {};
-    int dev = 0;
-    CURC_CHECK(cudaGetDevice(&dev));
-    if (dev < 0 || dev >= 64) throw std::runtime_error("device ordinal out of range");
-    {
-        std::lock_guard<std::mutex> g(mu);
-        if (!done[dev]) {
-            CURC_CHECK(cudaFuncSetAttribute(walk_kernel<AHEAD>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-            done[dev] = true;
-        }
-    }
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at;
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = blocks;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.gridDim = dim3(blocks);
-    cfg.blockDim = dim3(WALK_THREADS);
-    cfg.stream = s;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    CURC_CHECK(cudaLaunchKernelEx(&cfg, walk_kernel<AHEAD>, item, start, off0, noffs, pre, used, cap, next, prev,
-                                  offset, tally));
-    CURC_LAUNCH_CHECK();
-}
 constexpr unsigned WALK_CLUSTER = 16;
 
 // Walks the meetings of offsets [off0, off0 + noffs), noffs <= WALK_MAX_OFFS;
@@ -349,8 +317,8 @@ static inline void walk_meetings(const Meeting* item, const uint32_t* start, int
     // short lists meet a few hundred at a time: one block, whose barrier is
     // cheaper than the cluster's (50k reads, 2,048 to 4,096 ends: full match
     // 0.33 against 0.36 ms; 100k reads, more ends: 0.60 against 0.53)
-    walk_launch<false>(entries > 4096 ? WALK_CLUSTER : 1, item, start, off0, noffs, pre, used, cap, next, prev, offset,
-                       tally, s);
+    launch_cluster(walk_kernel<false>, entries > 4096 ? WALK_CLUSTER : 1, WALK_THREADS, s, item, start, off0, noffs, pre,
+                   used, cap, next, prev, offset, tally);
 }
 
 // The same with the starts known to the host: an offset with many meetings is
@@ -377,8 +345,8 @@ static inline void walk_stage(const Meeting* item, const uint32_t* host_start, c
         }
         if (host_start[e] != host_start[o]) {
             const bool many = most > 2048;
-            (many ? walk_launch<true> : walk_launch<false>)(many ? WALK_CLUSTER : 1, item, start + o, off0 + o, e - o, pre,
-                                                            used, cap, next, prev, offset, nullptr, s);
+            launch_cluster(many ? walk_kernel<true> : walk_kernel<false>, many ? WALK_CLUSTER : 1, WALK_THREADS, s, item,
+                           start + o, off0 + o, e - o, pre, used, cap, next, prev, offset, nullptr);
         }
         o = e;
     }
