@@ -69,8 +69,8 @@ def parse():
                          "scale, one block at a time against the batched drain, default against autotuned "
                          "launch choices, streams compared; each prints one JSON line")
     ap.add_argument("--fm-loop", type=int, default=None, choices=[0, 1, 2],
-                    help="full-match pass loop: 0 a launch per kernel, 1 one CUDA graph, 2 one persistent "
-                         "cooperative kernel (default: the library's)")
+                    help="full match: 0 pass by pass, 1 or 2 the meetings of many offsets listed at once "
+                         "(default: the library's)")
     ap.add_argument("--large-reads", type=int, default=40_000_000)
     ap.add_argument("--batched-blocks", type=int, default=16)
     ap.add_argument("--batched-scale", type=float, default=0.1)
@@ -150,16 +150,16 @@ def pack_bytes(n, L):
     return n * (L + 8 * ((L + 31) // 32) + 1)
 
 
-# Algorithmic bytes of the overlap probe kernel (its launches over all
-# passes), with one 32-byte sector per random access: per listed suffix its
-# k-mer (32); per bucket searched the bucket range (32); per prefix
-# comparison the prefix entry (32) and the prefix's row (32 * ceil(8W/32),
-# counted as rows read); per hit the run slot (32).  Counts come from the
+# Algorithmic bytes of the overlap meetings (sub-stage overlap.probe), with one
+# 32-byte sector per random access: each suffix's row once; per bucket searched
+# its range (32); per prefix comparison the prefix entry (32) and its row
+# (32 * ceil(8W/32)); per meeting its run (8) and its place in the masks (8).
+# The presence bitmaps stay in L2 and are not counted.  Counts come from the
 # kernel's own counters.
 def probe_bytes(st, L):
     row = 32 * -(-8 * ((L + 31) // 32) // 32)
-    return (32 * st["overlap_probes"] + 32 * st["overlap_searched"] + 32 * st["overlap_compares"]
-            + row * st.get("overlap_rows", 0) + 32 * st["overlap_hits"])
+    return (8 * ((L + 31) // 32) * st["overlap_suffixes"] + 32 * st["overlap_searched"]
+            + (32 + row) * st["overlap_compares"] + 16 * st["overlap_hits"])
 
 
 # Algorithmic bytes of the first-word read sort (sub-stage sort_dedupe.radix):
@@ -175,42 +175,31 @@ def sort_lower_bound_bytes(m, L):
     return m * (8 * ((L + 31) // 32) + 8)
 
 
-# Algorithmic bytes of the overlap resolve kernel (its launches over all
-# passes): per hit its 16-byte record, its run slot (32), the prefix id and
-# the prefix's predecessor (32 each) and one prefix row (32 * ceil(8W/32));
-# per link 10 bytes of next/prev/offset and the bucket's free word (32).
+# Algorithmic bytes of ordering and walking the meetings (sub-stage
+# overlap.resolve): per meeting its 8-byte key and value written and read by
+# each of four sort passes, its 16-byte item written and read, and the link
+# words of its suffix and prefix (32 each).
 def resolve_bytes(st, L):
-    row = 32 * -(-8 * ((L + 31) // 32) // 32)
-    return st["overlap_hits"] * (16 + 32 + 64 + row) + st["overlap_links"] * (10 + 32)
+    return st["overlap_links"] * (4 * 16 + 32 + 64)
 
 
 # Algorithmic bytes of the mapping kernels (forward and reverse complement):
-# per read searched its packed row (8W); per k-mer probe the bucket range,
-# one 32-byte sector; per candidate its pos_array slot (32) and the
-# pseudogenome window, 32 * (ceil((2L + 62) / 256) + 1).
+# per read searched its packed row (8W); per k-mer probe the bucket's slot,
+# one 32-byte sector; per candidate compared the pseudogenome window,
+# 32 * (ceil((2L + 62) / 256) + 1).
 def map_bytes(st, L, strand):
     win = 32 * (-(-(2 * L + 62) // 256) + 1)
     return (st[f"map_reads_{strand}"] * 8 * ((L + 31) // 32) + st[f"map_probes_{strand}"] * 32
-            + st[f"map_candidates_{strand}"] * (32 + win))
+            + st[f"map_candidates_{strand}"] * win)
 
 
-# Algorithmic bytes of the full-match pass loop (stage a6), per list entry
-# per pass, from the loop's own counters: a suffix entry has its 32-base key
-# gathered (one 32-byte sector of its row), moves through two merge levels
-# (12 bytes read and 12 written each), is read once by the pairing (12) and
-# is compacted (4 read, its link word's sector 32, 4 written); a prefix
-# entry is compacted with its key (12 read, link sector 32, 12 written).
-# The pairing's binary searches over the prefix keys are not counted, so
-# this is a lower bound.
+# Algorithmic bytes of the full match (stage a6), per meeting of a suffix with
+# a run of prefixes, from the walk's own counters: its 16-byte item written and
+# read, and the link words of its suffix and prefix (32 each).  Listing the
+# meetings (a look into L2-resident bitmaps per suffix and offset) and sorting
+# the two lists are not counted, so this is a lower bound.
 def full_match_bytes(st):
-    return st.get("fm_suffix_entries", 0) * (32 + 2 * 24 + 12 + 40) + st.get("fm_prefix_entries", 0) * 56
-
-
-# DRAM bytes per listed suffix of the probe kernel, from ncu
-# (dram__bytes_read.sum + dram__bytes_write.sum over its 96 launches) on the
-# 2M-pair case of the same generator: 5.767e9 bytes / 20.21e6 probes.  The
-# traffic of a launch at full size is this times its probes.
-PROBE_DRAM_BYTES_PER_PROBE = 5.767e9 / 20.207e6
+    return st.get("fm_suffix_entries", 0) * (32 + 64)
 
 
 STAT_NAMES = ["reads", "non_n", "n_reads", "pseudogenome_reads", "unmatched", "mapped", "unmapped",
@@ -257,7 +246,7 @@ def reduce_max(values, world, device="cpu"):
 
 def run_ours(a, rank, world):
     import torch
-    from curc_b200 import Context, kernel_launches
+    from curc_b200 import Context, CurcError, kernel_launches
 
     dev = int(os.environ.get("LOCAL_RANK", 0))
     torch.cuda.set_device(dev)
@@ -285,12 +274,11 @@ def run_ours(a, rank, world):
         dev_step()
     stage_names = ["pack", "sort_dedupe", "overlap", "chain_filter", "full_match", "assembly", "mapping", "emit",
                    "unmapped_refs", "refmatch"]
-    sub_names = ["pack.kernel", "sort_dedupe.first_word", "sort_dedupe.radix", "overlap.index", "overlap.index_sort", "overlap.index_mask",
-                 "overlap.probe_resolve", "overlap.filter", "overlap.probe", "overlap.resolve", "overlap.compact",
-                 "full_match.resort", "full_match.groups", "full_match.compact", "full_match.graph", "assembly.ranking", "assembly.walk", "assembly.jump",
-                 "assembly.order_place", "mapping.index_fwd", "mapping.map_fwd", "mapping.index_rc", "mapping.map_rc",
-                 "refmatch.index", "refmatch.probe_unmapped", "refmatch.probe_self", "refmatch.sort_unique",
-                 "refmatch.accept"]
+    sub_names = ["pack.kernel", "sort_dedupe.first_word", "sort_dedupe.radix", "overlap.index", "overlap.probe",
+                 "overlap.resolve", "overlap.compact", "assembly.small", "assembly.ranking", "assembly.walk",
+                 "assembly.jump", "assembly.order_place", "mapping.index_fwd", "mapping.map_fwd", "mapping.index_rc",
+                 "mapping.map_rc", "refmatch.index", "refmatch.probe_unmapped", "refmatch.probe_self",
+                 "refmatch.sort_unique", "refmatch.accept"]
     stage_tot = {k: 0.0 for k in stage_names}
     sub_tot = {}
     l0 = kernel_launches()
@@ -349,7 +337,11 @@ def run_ours(a, rank, world):
         batched = batched_vs_plain(ctx, a)
     cli = None
     if not a.no_cli and world == 1:
-        cli = cli_measure(ctx, w, a, dev)
+        try:
+            cli = cli_measure(ctx, w, a, dev)
+        except CurcError as e:
+            if "built without" not in str(e):
+                raise  # without the reference's coders there is no archive to write
     res = dict(bases=bases, n=n, L=L, step_s=step_s, e2e_s=e2e_s, wall=wall, launches=launches, stats=stats,
                stage_ms={k: v / a.steps for k, v in stage_tot.items()},
                substage_ms={k: round(v / a.steps, 3) for k, v in sub_tot.items()}, clocks=clocks.summary(),
@@ -626,9 +618,8 @@ def run_large(a):
         out["block_stats"] = block_stats(ctx)
         out["substage_ms"] = {k: round(ctx.stage_ms(k), 3) for k in
                               ["mapping.index_fwd", "mapping.map_fwd", "mapping.index_rc", "mapping.map_rc",
-                               "overlap.index", "overlap.index_mask", "overlap.filter", "overlap.probe",
-                               "overlap.resolve", "overlap.compact", "refmatch.index", "refmatch.probe_self",
-                               "refmatch.sort_unique", "refmatch.accept", "full_match.graph",
+                               "overlap.index", "overlap.probe", "overlap.resolve", "overlap.compact",
+                               "refmatch.index", "refmatch.probe_self", "refmatch.sort_unique", "refmatch.accept",
                                "assembly.ranking", "assembly.order_place"]
                               if _has_stage(ctx, k)}
         pack_ms = stage["pack"]
@@ -870,13 +861,11 @@ def main():
                                     "api": "curc_batch_submit/curc_batch_drain from pinned host memory, streams "
                                            "back to the host, no stream coders",
                                     "one_call_per_step": r["bases"] * world / r["e2e_plain_s"] / 1e6},
-        "roofline": {"kernel": "probe_kernel (overlap passes, stage a4; the memory-bound kernel with the largest share of the launch list: map_kernel<0> has a slightly larger share but is issue-bound, see roofline_map)",
+        "roofline": {"kernel": "meetings of the overlap stage (a4, sub-stage overlap.probe: meet_kernel, its counts and starts; the largest sub-stage)",
                      "bound": "hbm", "achieved": probe_ach, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                      "frac": probe_ach / peak if probe_ach else None,
-                     "traffic": PROBE_DRAM_BYTES_PER_PROBE * st["overlap_probes"] / passes,
-                     "algorithmic_bytes_per_launch": probe_bytes(st, r["L"]) / passes, "launches": passes,
-                     "ms_per_launch": probe_ms / passes,
-                     "traffic_source": "ncu dram bytes per probe on the 2M-pair case, times this launch's probes"},
+                     "traffic": None, "algorithmic_bytes": probe_bytes(st, r["L"]), "offsets": passes,
+                     "ms": probe_ms},
         "roofline_pack": {"kernel": "pack_kernel (stage a1, sub-stage pack.kernel)", "bound": "hbm",
                           "achieved": achieved, "peak": peak,
                           "peak_kind": peak_kind, "unit": "GB/s", "frac": achieved / peak if achieved else None,
@@ -888,12 +877,11 @@ def main():
                                                        (sub["sort_dedupe.first_word"] / 1000.0) / 1e9 / peak)
                                if sub.get("sort_dedupe.first_word") else None,
                                "whole_sort_ms": sub.get("sort_dedupe.radix")}),
-        "roofline_resolve": roof("resolve_kernel (overlap passes, stage a4)", resolve_bytes(st, r["L"]),
-                                 sub.get("overlap.resolve", 0.0), passes),
-        "roofline_full_match": roof("full-match pass loop (stage a6: key gather, two merge levels, pairing, "
-                                    "two compactions per pass; one CUDA graph, or per-launch with --fm-loop 0)",
-                                    full_match_bytes(st), r["stage_ms"].get("full_match", 0.0),
-                                    max(1, st.get("fm_passes", 0)), {"passes": st.get("fm_passes", 0)}),
+        "roofline_resolve": roof("ordering and walk of the meetings (overlap, stage a4, sub-stage overlap.resolve)",
+                                 resolve_bytes(st, r["L"]), sub.get("overlap.resolve", 0.0), 1),
+        "roofline_full_match": roof("full match (stage a6: lists sorted, meetings listed and walked)",
+                                    full_match_bytes(st), r["stage_ms"].get("full_match", 0.0), 1,
+                                    {"passes": st.get("fm_passes", 0)}),
         "roofline_map": roof("map_kernel forward + reverse complement (stage a9)",
                              map_bytes(st, r["L"], "fwd") + map_bytes(st, r["L"], "rc"),
                              sub.get("mapping.map_fwd", 0.0) + sub.get("mapping.map_rc", 0.0), 2),
