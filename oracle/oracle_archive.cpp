@@ -508,13 +508,19 @@ int oracle_block_get(void* hv, const char* name, const void** ptr, uint64_t* byt
 }
 
 // Codes the block into the reference block layout; returns its size and a
-// malloc'd buffer in *out (free with oracle_buf_free).
+// malloc'd buffer in *out (free with oracle_buf_free); 0 and null on an error.
 uint64_t oracle_block_encode(void* hv, const char* tmpdir, const char* bsc, char** out) {
-    auto* h = static_cast<Handle*>(hv);
-    std::string b = oracle::encode_block(h->p, h->s, tmpdir, bsc);
-    *out = static_cast<char*>(std::malloc(b.size() ? b.size() : 1));
-    std::memcpy(*out, b.data(), b.size());
-    return b.size();
+    *out = nullptr;
+    try {
+        auto* h = static_cast<Handle*>(hv);
+        std::string b = oracle::encode_block(h->p, h->s, tmpdir, bsc);
+        *out = static_cast<char*>(std::malloc(b.size() ? b.size() : 1));
+        std::memcpy(*out, b.data(), b.size());
+        return b.size();
+    } catch (const std::exception& e) {
+        std::fprintf(stderr, "oracle: %s\n", e.what());
+        return 0;
+    }
 }
 
 void oracle_buf_free(char* p) { std::free(p); }
