@@ -8,6 +8,7 @@
 #include <mutex>
 #include <set>
 
+#include "lookback.cuh"
 #include "primitives.cuh"
 
 namespace curc {
@@ -23,7 +24,6 @@ uint64_t launches() { return g_launches.load(); }
 
 Arena::~Arena() {
     for (auto& c : chunks_) cudaFree(c.base);
-    if (wait_error_) cudaFree(wait_error_);
     if (zero_) cudaFree(zero_);
 }
 
@@ -49,22 +49,6 @@ void* Arena::zero_bytes(size_t bytes, cudaStream_t s) {
     void* p = alloc_bytes(bytes);
     CURC_CHECK(cudaMemsetAsync(p, 0, bytes, s));
     return p;
-}
-
-uint32_t* Arena::wait_error() {
-    if (!wait_error_) {
-        CURC_CHECK(cudaMalloc(&wait_error_, sizeof(uint32_t)));
-        CURC_CHECK(cudaMemset(wait_error_, 0, sizeof(uint32_t)));
-    }
-    return wait_error_;
-}
-
-void Arena::check_waits(const void* copy, cudaStream_t s) {
-    uint32_t e;
-    std::memcpy(&e, copy, sizeof(e));
-    if (!e) return;
-    CURC_CHECK(cudaMemsetAsync(wait_error(), 0, sizeof(uint32_t), s));
-    throw std::runtime_error("a tile's bounded wait ran out");
 }
 
 void* Arena::alloc_bytes(size_t bytes) {
@@ -319,60 +303,11 @@ __device__ T block_exclusive_sum(T v, T* block_total) {
     return warp_prefix + x - v;
 }
 
-// One-pass scans: tiles are taken in order from a counter, publish their
-// sum, and find the sum before them by looking back over the tiles before
-// (whose blocks have started, since the counter is in order).  A state is a
-// 62-bit value under two flag bits: 1, the tile's own sum; 2, the sum up to
-// and with the tile.  Waits are bounded: one that runs out sets *err, which
-// the block run checks before it returns results (Arena::check_waits).
-constexpr uint32_t LOOK_WAIT_LIMIT = 1u << 22;
-constexpr uint64_t LOOK_SUM = 1ull << 62, LOOK_INCL = 2ull << 62, LOOK_VALUE = LOOK_SUM - 1;
-
-__device__ __forceinline__ uint64_t look_wait(unsigned long long* st, uint32_t* err) {
-    uint64_t v;
-    uint32_t spins = 0;
-    for (;;) {
-        v = *reinterpret_cast<volatile unsigned long long*>(st);
-        if (v >> 62) return v;
-        if (++spins >= LOOK_WAIT_LIMIT) {
-            atomicExch(err, 1u);
-            return LOOK_INCL;  // void, and *err says so; no later tile waits on this one
-        }
-        __nanosleep(32);
-    }
-}
-
-// Warp 0, all lanes: publishes the tile's sum and returns the sum of the
-// tiles before it (32 predecessors per step).
-__device__ __forceinline__ uint64_t look_back(unsigned long long* st, uint32_t tile, uint64_t sum, uint32_t* err) {
-    const uint32_t lane = threadIdx.x & 31u;
-    if (tile == 0) {
-        if (lane == 0) atomicExch(&st[0], LOOK_INCL | (sum & LOOK_VALUE));
-        return 0;
-    }
-    if (lane == 0) atomicExch(&st[tile], LOOK_SUM | (sum & LOOK_VALUE));
-    uint64_t before = 0;
-    for (int64_t top = int64_t(tile) - 1;; top -= 32) {
-        const int64_t j = top - int64_t(lane);
-        const uint64_t v = j >= 0 ? look_wait(&st[j], err) : LOOK_INCL;
-        __syncwarp();
-        // the nearest lane with an inclusive sum ends the search
-        const uint32_t inc = __ballot_sync(0xFFFFFFFFu, (v >> 62) == 2);
-        const int stop = inc ? __ffs(inc) - 1 : 32;
-        uint64_t add = int(lane) <= stop ? v & LOOK_VALUE : 0;
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) add += __shfl_xor_sync(0xFFFFFFFFu, add, d);
-        before += add;
-        if (inc) break;
-    }
-    if (lane == 0) atomicExch(&st[tile], LOOK_INCL | ((before + sum) & LOOK_VALUE));
-    return before;
-}
-
-// st: one state per tile and, behind them, the tile counter (all zero).
+// One-pass scan (lookback.cuh).  st: one state per tile and, behind them, the
+// tile counter (all zero).
 template <class T>
 __global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(const T* in, T* out, size_t n, T* total,
-                                                            unsigned long long* st, uint32_t tiles, uint32_t* err) {
+                                                            unsigned long long* st, uint32_t tiles) {
     __shared__ T sm[SCAN_TILE];
     __shared__ uint32_t s_tile;
     __shared__ uint64_t s_before;
@@ -397,7 +332,12 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(const T* in, T* out,
     T run = block_exclusive_sum(tsum, &btotal);
     if (tiles > 1) {
         if (threadIdx.x < 32) {
-            const uint64_t before = look_back(st, tile, uint64_t(btotal), err);
+            const uint64_t before = look_back(LookOnce{}, st, tile, uint64_t(btotal), in == out, [&](uint32_t j) {
+                uint64_t c = 0;
+                for (int i = int(threadIdx.x); i < SCAN_TILE; i += 32)  // an earlier tile is full
+                    c += __ldcg(in + size_t(j) * SCAN_TILE + i);
+                return warp_sum(c);
+            });
             if (threadIdx.x == 0) s_before = before;
         }
         __syncthreads();
@@ -433,8 +373,7 @@ void exclusive_scan(const T* in, T* out, size_t n, T* total, Arena& a, cudaStrea
     const size_t tiles = div_up(n, SCAN_TILE);
     auto m = a.mark();
     unsigned long long* st = tiles > 1 ? look_states(tiles, a, s) : nullptr;
-    scan_kernel<T><<<unsigned(tiles), SCAN_THREADS, 0, s>>>(in, out, n, total, st, uint32_t(tiles),
-                                                            tiles > 1 ? a.wait_error() : nullptr);
+    scan_kernel<T><<<unsigned(tiles), SCAN_THREADS, 0, s>>>(in, out, n, total, st, uint32_t(tiles));
     CURC_LAUNCH_CHECK();
     a.release(m);
 }
@@ -453,7 +392,7 @@ static_assert(SEL_THREADS == SCAN_THREADS, "block_exclusive_sum");
 template <class T, bool kIndices>
 __global__ void __launch_bounds__(SEL_THREADS) select_kernel(const T* __restrict__ in, const uint8_t* __restrict__ flags,
                                                              size_t n, T* __restrict__ out, uint32_t* __restrict__ count,
-                                                             unsigned long long* st, uint32_t tiles, uint32_t* err) {
+                                                             unsigned long long* st, uint32_t tiles) {
     __shared__ uint32_t s_tile;
     __shared__ uint64_t s_before;
     if (threadIdx.x == 0) s_tile = tiles > 1 ? uint32_t(atomicAdd(&st[tiles], 1ull)) : 0;
@@ -475,7 +414,11 @@ __global__ void __launch_bounds__(SEL_THREADS) select_kernel(const T* __restrict
     uint64_t pos = block_exclusive_sum<uint32_t>(__popc(keep), &total);
     if (tiles > 1) {
         if (threadIdx.x < 32) {
-            const uint64_t before = look_back(st, tile, total, err);
+            const uint64_t before = look_back(LookOnce{}, st, tile, total, false, [&](uint32_t j) {
+                uint64_t c = 0;
+                for (int i = int(threadIdx.x); i < SEL_TILE; i += 32) c += flags[size_t(j) * SEL_TILE + i] != 0;
+                return warp_sum(c);
+            });
             if (threadIdx.x == 0) s_before = before;
         }
         __syncthreads();
@@ -500,8 +443,7 @@ void select_impl(const T* in, const uint8_t* flags, T* out, size_t n, uint32_t* 
     auto m = a.mark();
     const size_t tiles = div_up(n, SEL_TILE);
     unsigned long long* st = tiles > 1 ? look_states(tiles, a, s) : nullptr;
-    select_kernel<T, kIndices><<<unsigned(tiles), SEL_THREADS, 0, s>>>(in, flags, n, out, count, st, uint32_t(tiles),
-                                                                       tiles > 1 ? a.wait_error() : nullptr);
+    select_kernel<T, kIndices><<<unsigned(tiles), SEL_THREADS, 0, s>>>(in, flags, n, out, count, st, uint32_t(tiles));
     CURC_LAUNCH_CHECK();
     a.release(m);
 }
@@ -614,6 +556,15 @@ struct RsTile {
     }
 };
 
+// Items of digit d in a tile not heard from (lookback.cuh), by one thread.
+template <class K>
+__device__ __noinline__ uint32_t rs_count_digit(const K* __restrict__ keys, int items, int shift, uint32_t mask,
+                                                uint32_t d) {
+    uint32_t c = 0;
+    for (int i = 0; i < items; ++i) c += digit_of(keys[i], shift, mask) == d;
+    return c;
+}
+
 // One pass: tiles are taken in order from a counter; each ranks its items,
 // publishes its count of every digit, reorders itself by digit in shared
 // memory and, thread d for digit d, looks back over the tiles before it for
@@ -628,8 +579,7 @@ __global__ void __launch_bounds__(RS_THREADS) rs_pass_kernel(const K* __restrict
                                                              K* __restrict__ kout, V* __restrict__ vout, size_t n,
                                                              int shift, uint32_t mask,
                                                              const uint32_t* __restrict__ hist,
-                                                             unsigned long long* __restrict__ st, uint32_t tiles,
-                                                             uint32_t* __restrict__ err) {
+                                                             unsigned long long* __restrict__ st, uint32_t tiles) {
     constexpr int TILE = RS_THREADS * R;
     extern __shared__ __align__(16) uint8_t rs_smem[];
     K* sk = reinterpret_cast<K*>(rs_smem);
@@ -664,7 +614,8 @@ __global__ void __launch_bounds__(RS_THREADS) rs_pass_kernel(const K* __restrict
         mine += c;
     }
     unsigned long long* state = st + size_t(tile) * 256 + tid;
-    atomicExch(state, (tile == 0 ? LOOK_INCL : LOOK_SUM) | mine);
+    const LookOnce look;
+    atomicExch(state, look.make(tile == 0 ? 2 : 1, mine));
     tstart[tid] = rs_scan256(mine, wsum);
     __syncthreads();
 #pragma unroll
@@ -681,13 +632,16 @@ __global__ void __launch_bounds__(RS_THREADS) rs_pass_kernel(const K* __restrict
     uint64_t before = 0;
     if (tile > 0) {
         unsigned long long* p = state;
-        for (uint32_t j = tile; j > 0; --j) {
+        uint32_t spins = LOOK_SPINS;
+        for (uint32_t j = tile; j > 0;) {
             p -= 256;
-            const uint64_t v = look_wait(p, err);
-            before += v & LOOK_VALUE;
-            if ((v >> 62) == 2) break;
+            --j;
+            const uint64_t v = look_wait(look, p, spins);
+            if (look.flag(v)) before += look.sum(v);
+            else before += rs_count_digit(kin + size_t(j) * TILE, TILE, shift, mask, uint32_t(tid));
+            if (look.flag(v) == 2) break;
         }
-        atomicExch(state, LOOK_INCL | (before + mine));
+        atomicExch(state, look.make(2, before + mine));
     }
     gbase[tid] = digit_start + uint32_t(before) - tstart[tid];
     __syncthreads();
@@ -811,7 +765,7 @@ void radix_sort_pairs(K* keys, V* vals, size_t n, int begin_bit, int end_bit, Ar
         V* vo = vals ? ((vc == vals) ? valt : vals) : nullptr;
         auto pass = few ? rs_pass_kernel<K, V, RS_ROUNDS_FEW> : rs_pass_kernel<K, V, RS_ROUNDS>;
         pass<<<tiles, RS_THREADS, (sizeof(K) + sizeof(V)) * size_t(tile), s>>>(
-            kc, vc, ko, vo, n, dg.shift(p), dg.mask(p), hist + p * 256, st + pass_words * p, tiles, a.wait_error());
+            kc, vc, ko, vo, n, dg.shift(p), dg.mask(p), hist + p * 256, st + pass_words * p, tiles);
         CURC_LAUNCH_CHECK();
         kc = ko;
         vc = vo;

@@ -33,11 +33,6 @@ public:
     // Frees every chunk (nothing may be in use: the stream work that used
     // them must have completed; cudaFree waits for the device).
     void trim();
-    // Device error word of the one-pass kernels that take their scratch here
-    // (a wait on another tile that ran out), zero unless one did.
-    uint32_t* wait_error();
-    // Throws when a host copy of it (4 bytes) is set, and clears it.
-    void check_waits(const void* copy, cudaStream_t s);
     // Zeroed scratch of a run.  clear_zeros() clears a pool once, at the
     // start of a run; zeros() takes pieces of it, each handed out once per
     // clearing.  What does not fit there, or is asked for on another stream,
@@ -62,7 +57,6 @@ private:
     size_t cur_ = 0;
     size_t chunk_;
     size_t high_water_ = 0;
-    uint32_t* wait_error_ = nullptr;
     // 16 MiB clear in 3 us and hold the tile states of every sort of a block
     // of some 100k reads; a piece of 4 MiB or more is long enough to be
     // cleared by itself
