@@ -19,12 +19,21 @@ constexpr int CP_THREADS = 512;
 constexpr int CP_ITEMS = 8;
 constexpr uint32_t CP_TILE = CP_THREADS * CP_ITEMS;
 
+// Items kept of a tile not heard from (an earlier one is full).
+template <class Keep>
+__device__ __forceinline__ uint64_t kept_in_tile(const Keep& keep, uint32_t j) {
+    uint64_t c = 0;
+#pragma unroll 1
+    for (uint32_t i = threadIdx.x; i < CP_TILE; i += 32) c += keep(j * CP_TILE + i) ? 1 : 0;  // warp 0
+    return warp_sum(c);
+}
+
 // keep(i) -> bool for item i < n; move(i, dst) places kept item i at dst.
 // Each thread takes CP_ITEMS consecutive items; one block scan ranks them.
 // The grid covers *n_dev items; keep() gives the same for an item whenever it
 // is asked.
 template <class Keep, class Move>
-__global__ void __launch_bounds__(CP_THREADS) compact_kernel(const uint32_t* __restrict__ n_dev,
+__global__ void __launch_bounds__(CP_THREADS, 4) compact_kernel(const uint32_t* __restrict__ n_dev,
                                                              uint32_t* __restrict__ n_out, Keep keep, Move move,
                                                              unsigned long long* tiles, uint32_t* counter,
                                                              uint32_t base, uint32_t epoch) {
@@ -63,9 +72,7 @@ __global__ void __launch_bounds__(CP_THREADS) compact_kernel(const uint32_t* __r
     const uint32_t rank = before + incl - mine;
     if (warp == 0) {
         const uint32_t excl = uint32_t(look_back(LookEpoch{epoch}, tiles, tile, local, false, [&](uint32_t j) {
-            uint64_t c = 0;
-            for (uint32_t i = lane; i < CP_TILE; i += 32) c += keep(j * CP_TILE + i) ? 1 : 0;  // an earlier tile is full
-            return warp_sum(c);
+            return kept_in_tile(keep, j);
         }));
         if (lane == 0) {
             s_excl = excl;

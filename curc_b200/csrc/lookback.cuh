@@ -5,8 +5,8 @@
 // with itself as soon as it knows it; the next tiles add up what they find.
 //
 // Waits are bounded, and none can fail: a tile that has waited LOOK_SPINS
-// times adds the items of the tiles it has not heard from up itself, from the
-// kernel's input.  (It never came to that in any measurement: a block that
+// reads for another waits no more, and adds up the items of the tiles it has
+// not heard from itself, from the kernel's input.  (It never came to that in any measurement: a block that
 // has started publishes within microseconds, and a wait lasts 0.1 s.)
 #pragma once
 #include <cuda_runtime.h>
@@ -14,7 +14,7 @@
 
 namespace curc {
 
-// Reads of one thread, over all of its tile's waits, before it counts itself.
+// Reads of a state before its tile is not waited for any longer.
 #ifndef CURC_LOOK_SPINS
 #define CURC_LOOK_SPINS (1u << 22)
 #endif
@@ -55,6 +55,35 @@ __device__ __forceinline__ uint64_t look_wait(const S& S_, const unsigned long l
     }
 }
 
+// Sum of a value over the warp's lanes.
+__device__ __forceinline__ uint64_t warp_sum(uint64_t v) {
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, d);
+    return v;
+}
+
+// The rest of a look-back without waits: the sum of the tiles up to and with
+// `top`, one after another; those not heard from are counted.  Out of line, to
+// keep its registers out of the kernels.
+template <class S, class Count>
+__device__ __noinline__ uint64_t look_on(S S_, unsigned long long* st, uint32_t top, bool in_place, Count count) {
+    uint64_t before = 0;
+    for (uint32_t j = top;; --j) {
+        uint32_t spins = 0;
+        uint64_t v = __shfl_sync(0xFFFFFFFFu, look_wait(S_, &st[j], spins), 0);
+        if (!S_.flag(v)) {
+            const uint64_t own = count(j);
+            if (in_place) {  // it holds if the tile is silent still
+                __threadfence();
+                v = __shfl_sync(0xFFFFFFFFu, look_wait(S_, &st[j], spins), 0);
+            }
+            if (!S_.flag(v)) v = S_.make(1, own);
+        }
+        before += S_.sum(v);
+        if (S_.flag(v) == 2 || j == 0) return before;
+    }
+}
+
 // One warp, all lanes: publishes the tile's sum and returns the sum of the
 // tiles before it (32 predecessors per step).  count(j), called by all lanes,
 // is tile j's sum from the input.  in_place: the kernel overwrites its input
@@ -70,42 +99,24 @@ __device__ __forceinline__ uint64_t look_back(const S& S_, unsigned long long* s
     }
     if (tile == 0) return 0;
     uint64_t before = 0;
-    uint32_t spins = LOOK_SPINS;
     for (int64_t top = int64_t(tile) - 1;; top -= 32) {
         const int64_t j = top - int64_t(lane);
         uint64_t v = S_.make(2, 0);  // lanes past tile 0 add nothing
+        uint32_t spins = LOOK_SPINS;
         if (j >= 0) v = look_wait(S_, &st[j], spins);
         __syncwarp();
-        uint32_t silent = __ballot_sync(0xFFFFFFFFu, S_.flag(v) == 0);
-        while (silent) {
-            const int l = __ffs(silent) - 1;
-            silent &= silent - 1;
-            const uint64_t own = count(uint32_t(top - l));
-            if (in_place) __threadfence();
-            if (int(lane) == l) {
-                v = *reinterpret_cast<const volatile unsigned long long*>(&st[j]);
-                if (!S_.flag(v)) v = S_.make(1, own);
-            }
+        if (__any_sync(0xFFFFFFFFu, S_.flag(v) == 0)) {
+            before += look_on(S_, st, uint32_t(top), in_place, count);
+            break;
         }
-        __syncwarp();
         // the nearest lane with an inclusive sum ends the search
         const uint32_t inc = __ballot_sync(0xFFFFFFFFu, S_.flag(v) == 2);
         const int stop = inc ? __ffs(inc) - 1 : 32;
-        uint64_t add = int(lane) <= stop ? S_.sum(v) : 0;
-#pragma unroll
-        for (int d = 16; d > 0; d >>= 1) add += __shfl_xor_sync(0xFFFFFFFFu, add, d);
-        before += add;
+        before += warp_sum(int(lane) <= stop ? S_.sum(v) : 0);
         if (inc) break;
     }
     if (lane == 0) atomicExch(&st[tile], S_.make(2, before + sum));
     return before;
-}
-
-// Sum of a value over the warp's lanes.
-__device__ __forceinline__ uint64_t warp_sum(uint64_t v) {
-#pragma unroll
-    for (int d = 16; d > 0; d >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, d);
-    return v;
 }
 
 }  // namespace curc

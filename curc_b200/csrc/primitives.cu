@@ -303,10 +303,19 @@ __device__ T block_exclusive_sum(T v, T* block_total) {
     return warp_prefix + x - v;
 }
 
+// Sum of a tile not heard from (lookback.cuh).  An earlier tile is full.
+template <class T>
+__device__ __forceinline__ uint64_t scan_tile_sum(const T* in) {
+    uint64_t c = 0;
+#pragma unroll 1
+    for (int i = int(threadIdx.x); i < SCAN_TILE; i += 32) c += __ldcg(in + i);
+    return warp_sum(c);
+}
+
 // One-pass scan (lookback.cuh).  st: one state per tile and, behind them, the
 // tile counter (all zero).
 template <class T>
-__global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(const T* in, T* out, size_t n, T* total,
+__global__ void __launch_bounds__(SCAN_THREADS, sizeof(T) == 4 ? 6 : 5) scan_kernel(const T* in, T* out, size_t n, T* total,
                                                             unsigned long long* st, uint32_t tiles) {
     __shared__ T sm[SCAN_TILE];
     __shared__ uint32_t s_tile;
@@ -333,10 +342,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) scan_kernel(const T* in, T* out,
     if (tiles > 1) {
         if (threadIdx.x < 32) {
             const uint64_t before = look_back(LookOnce{}, st, tile, uint64_t(btotal), in == out, [&](uint32_t j) {
-                uint64_t c = 0;
-                for (int i = int(threadIdx.x); i < SCAN_TILE; i += 32)  // an earlier tile is full
-                    c += __ldcg(in + size_t(j) * SCAN_TILE + i);
-                return warp_sum(c);
+                return scan_tile_sum(in + size_t(j) * SCAN_TILE);
             });
             if (threadIdx.x == 0) s_before = before;
         }
@@ -387,10 +393,17 @@ namespace {
 constexpr int SEL_THREADS = 256, SEL_ITEMS = 16, SEL_TILE = SEL_THREADS * SEL_ITEMS;
 static_assert(SEL_THREADS == SCAN_THREADS, "block_exclusive_sum");
 
+__device__ __forceinline__ uint64_t flagged_in_tile(const uint8_t* flags) {
+    uint64_t c = 0;
+#pragma unroll 1
+    for (int i = int(threadIdx.x); i < SEL_TILE; i += 32) c += flags[i] != 0;
+    return warp_sum(c);
+}
+
 // One-pass stable compaction (tile states as in scan_kernel); thread t owns
 // the tile's items [16 t, 16 t + 16).
 template <class T, bool kIndices>
-__global__ void __launch_bounds__(SEL_THREADS) select_kernel(const T* __restrict__ in, const uint8_t* __restrict__ flags,
+__global__ void __launch_bounds__(SEL_THREADS, 8) select_kernel(const T* __restrict__ in, const uint8_t* __restrict__ flags,
                                                              size_t n, T* __restrict__ out, uint32_t* __restrict__ count,
                                                              unsigned long long* st, uint32_t tiles) {
     __shared__ uint32_t s_tile;
@@ -415,9 +428,7 @@ __global__ void __launch_bounds__(SEL_THREADS) select_kernel(const T* __restrict
     if (tiles > 1) {
         if (threadIdx.x < 32) {
             const uint64_t before = look_back(LookOnce{}, st, tile, total, false, [&](uint32_t j) {
-                uint64_t c = 0;
-                for (int i = int(threadIdx.x); i < SEL_TILE; i += 32) c += flags[size_t(j) * SEL_TILE + i] != 0;
-                return warp_sum(c);
+                return flagged_in_tile(flags + size_t(j) * SEL_TILE);
             });
             if (threadIdx.x == 0) s_before = before;
         }
@@ -556,13 +567,25 @@ struct RsTile {
     }
 };
 
-// Items of digit d in a tile not heard from (lookback.cuh), by one thread.
+// Items of digit d in the tiles before tile j + 1, by one thread that no longer
+// waits (lookback.cuh): those of tiles not heard from are counted.  p: tile
+// j's state of the digit.
 template <class K>
-__device__ __noinline__ uint32_t rs_count_digit(const K* __restrict__ keys, int items, int shift, uint32_t mask,
-                                                uint32_t d) {
-    uint32_t c = 0;
-    for (int i = 0; i < items; ++i) c += digit_of(keys[i], shift, mask) == d;
-    return c;
+__device__ __noinline__ uint64_t rs_look_on(const K* __restrict__ keys, uint32_t j, int items, int shift, uint32_t mask,
+                                            uint32_t d, const unsigned long long* p) {
+    const LookOnce look;
+    uint64_t before = 0;
+    for (;; p -= 256, --j) {
+        uint32_t spins = 0;
+        const uint64_t v = look_wait(look, p, spins);
+        if (look.flag(v)) {
+            before += look.sum(v);
+        } else {
+            const K* k = keys + size_t(j) * items;
+            for (int i = 0; i < items; ++i) before += digit_of(k[i], shift, mask) == d;
+        }
+        if (look.flag(v) == 2 || j == 0) return before;
+    }
 }
 
 // One pass: tiles are taken in order from a counter; each ranks its items,
@@ -632,13 +655,15 @@ __global__ void __launch_bounds__(RS_THREADS) rs_pass_kernel(const K* __restrict
     uint64_t before = 0;
     if (tile > 0) {
         unsigned long long* p = state;
-        uint32_t spins = LOOK_SPINS;
-        for (uint32_t j = tile; j > 0;) {
+        for (uint32_t j = tile; j > 0; --j) {
             p -= 256;
-            --j;
+            uint32_t spins = LOOK_SPINS;
             const uint64_t v = look_wait(look, p, spins);
-            if (look.flag(v)) before += look.sum(v);
-            else before += rs_count_digit(kin + size_t(j) * TILE, TILE, shift, mask, uint32_t(tid));
+            if (look.flag(v) == 0) {
+                before += rs_look_on(kin, j - 1, TILE, shift, mask, uint32_t(tid), p);
+                break;
+            }
+            before += look.sum(v);
             if (look.flag(v) == 2) break;
         }
         atomicExch(state, look.make(2, before + mine));
