@@ -896,24 +896,48 @@ __global__ void run_number_kernel(const uint32_t* __restrict__ excl, const uint3
 // their remaining words, ties by position (stable).  The thread at a run's
 // start orders runs of up to RUN_THREAD rows by insertion; a warp orders
 // runs of up to 32, each lane ranking its row against the others' words by
-// shuffles (rows of up to 16 words) or loads; longer runs are flagged for
-// the radix path, and *any_large counts their rows.  Most runs have two or
-// three rows (reads that start at one place), so a warp per run left most
-// lanes idle.
-constexpr uint32_t RUN_THREAD = 4;
+// shuffles (rows of up to 16 words) or loads; the rows of longer runs are
+// flagged for the radix path, each by its own thread, and *any_large counts
+// them.  Most runs have two or three rows (reads that start at one place), so
+// a warp per run left most lanes idle; and a run may be the whole list (reads
+// behind one primer), which one warp took 8 ms a million rows to flag, 32 rows
+// a step (sort of 4M such reads of 64 bp 33.1 -> 1.69 ms, B200).
+constexpr uint32_t RUN_THREAD = 4, RUN_WARP = 32;
+
+// Whether row i lies in a run of more than RUN_WARP rows.  Most rows of
+// such a run have RUN_WARP equal ones to one side, the others half as many.
+__device__ __forceinline__ bool in_long_run(const uint64_t* __restrict__ k0, uint32_t i, uint32_t n, uint64_t v) {
+    constexpr uint32_t H = RUN_WARP / 2;
+    if ((i >= RUN_WARP && k0[i - RUN_WARP] == v) || (n - i > RUN_WARP && k0[i + RUN_WARP] == v)) return true;
+    if (!(i >= H && k0[i - H] == v) && !(n - i > H && k0[i + H] == v)) return false;
+    // equal rows before and behind, fewer than RUN_WARP of each, by bisection
+    uint32_t b = 0, f = 0;
+#pragma unroll
+    for (uint32_t d = H; d > 0; d >>= 1) {
+        if (i >= b + d && k0[i - b - d] == v) b += d;
+        if (n - i > f + d && k0[i + f + d] == v) f += d;
+    }
+    return b + f + 1 > RUN_WARP;
+}
 __global__ void __launch_bounds__(256) order_runs_kernel(const uint64_t* __restrict__ db, int W,
                                                          uint32_t* __restrict__ ids,
                                                          const uint64_t* __restrict__ k0, uint32_t n,
                                                          uint8_t* __restrict__ large, uint32_t* __restrict__ any_large) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31u;
-    uint32_t len = 0;  // of the run that starts here (up to 33), else 0
-    if (i + 1 < n) {
+    uint32_t len = 0;  // of the run that starts here, if a thread or warp orders it
+    bool flag = false;
+    if (i < n) {
         const uint64_t v = k0[i];
-        if (k0[i + 1] == v && (i == 0 || k0[i - 1] != v)) {
+        const bool behind = i + 1 < n && k0[i + 1] == v, before = i > 0 && k0[i - 1] == v;
+        flag = (behind || before) && in_long_run(k0, i, n, v);
+        large[i] = flag;
+        if (!flag && behind && !before) {
             len = 2;
-            while (len <= 32 && i + len < n && k0[i + len] == v) ++len;
+            while (len < RUN_WARP && i + len < n && k0[i + len] == v) ++len;
         }
     }
+    const uint32_t flagged = __popc(__ballot_sync(0xFFFFFFFFu, flag));
+    if (flagged && lane == 0) atomicAdd(any_large, flagged);
     if (len >= 2 && len <= RUN_THREAD) {
         uint32_t id[RUN_THREAD];
 #pragma unroll
@@ -950,19 +974,6 @@ __global__ void __launch_bounds__(256) order_runs_kernel(const uint64_t* __restr
         const int l = __ffs(todo) - 1;
         todo &= todo - 1;
         const uint32_t p0 = __shfl_sync(0xFFFFFFFFu, i, l), m = __shfl_sync(0xFFFFFFFFu, len, l);
-        if (m > 32) {  // flag the whole run
-            const uint64_t v = k0[p0];
-            uint32_t rows = 0;
-            for (uint32_t t = p0 + lane;; t += 32) {
-                const bool in = t < n && k0[t] == v;
-                if (in) large[t] = 1;
-                const uint32_t c = __popc(__ballot_sync(0xFFFFFFFFu, in));
-                rows += c;
-                if (c < 32) break;
-            }
-            if (lane == 0) atomicAdd(any_large, rows);
-            continue;
-        }
         const uint32_t id = lane < m ? ids[p0 + lane] : 0;
         uint32_t rank = 0;
         if (W <= 16) {
@@ -1081,7 +1092,7 @@ void sort_rows(const uint64_t* db, int W, int last_bits, uint32_t* ids, size_t n
         radix_sort_pairs<uint64_t, uint32_t>(k0, ids, n, W == 1 ? 64 - last_bits : 0, first_bits, a, s);
     }
     if (W > 1) {
-        uint8_t* large = a.zeros<uint8_t>(n, s);
+        uint8_t* large = a.alloc<uint8_t>(n);
         uint32_t* cnt = a.zeros<uint32_t>(2, s);
         order_runs_kernel<<<grid_for(n, 256), 256, 0, s>>>(db, W, ids, k0, uint32_t(n), large, cnt);
         CURC_LAUNCH_CHECK();
