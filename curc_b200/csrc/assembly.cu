@@ -244,7 +244,8 @@ __global__ void __launch_bounds__(512) rank_rounds_kernel(uint32_t n, RankState*
             out[x] = st;
         }
         block_tally<uint32_t>(still, active + t);
-        asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+        cluster_arrive();
+        cluster_wait();
         const uint32_t left = __ldcg(active + t);  // the same for every thread
         if (left == 0 || t + 1 == rounds) {
             if (me == 0) {

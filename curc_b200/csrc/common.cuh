@@ -168,6 +168,12 @@ __device__ __forceinline__ int cmp_span(const uint64_t* a, uint32_t aoff, const 
     return 0;
 }
 
+// The two halves of the cluster's barrier, with what was written before it
+// visible behind it.  Each thread arrives by itself (not the .aligned form,
+// which needs the whole warp together): the callers come from branches.
+__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release;" ::: "memory"); }
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire;" ::: "memory"); }
+
 inline int grid_for(uint64_t n, int block, int per_thread = 1) {
     uint64_t g = div_up(n, uint64_t(block) * per_thread);
     if (g < 1) g = 1;

@@ -298,9 +298,9 @@ static __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(const Meeting
         o = skip(o + 1);
         if (o == noffs) return;
         if (gridDim.x > 1) {
-            asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+            cluster_arrive();
             if (AHEAD) h = look_ahead(item, start[o], start[o + 1], start[o] + me, pre);
-            asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+            cluster_wait();
         } else {
             __syncthreads();
         }
