@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(512) rank_rounds_kernel(uint32_t n, RankState*
         const RankState* in = t & 1 ? B : A;
         RankState* out = t & 1 ? A : B;
         uint32_t still = 0;
-        for (uint32_t x = me; x < n; x += RANK_BLOCKS * 512) {
+        for (uint32_t x = me; x < n; x += gridDim.x * 512) {
             RankState st = ld_state(in + x);
             if (st.jump != INVALID) {
                 const RankState a = ld_state(in + st.jump);

@@ -168,6 +168,12 @@ __device__ __forceinline__ int cmp_span(const uint64_t* a, uint32_t aoff, const 
     return 0;
 }
 
+// `most` blocks (a power of two) halved until `held` of them fit.
+inline unsigned cluster_fit(unsigned most, unsigned held) {
+    while (most > 1 && most > held) most /= 2;
+    return most;
+}
+
 // The two halves of the cluster's barrier, with what was written before it
 // visible behind it.  Each thread arrives by itself (not the .aligned form,
 // which needs the whole warp together): the callers come from branches.

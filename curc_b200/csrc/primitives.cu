@@ -6,7 +6,6 @@
 #include <string>
 
 #include <mutex>
-#include <set>
 
 #include "lookback.cuh"
 #include "primitives.cuh"
@@ -259,15 +258,24 @@ StageTimer*& active_timer() {
     return t;
 }
 
-void allow_large_clusters(const void* kernel) {
+unsigned cluster_blocks(const void* kernel, unsigned most, unsigned threads) {
+    if (most == 1) return 1;
     static std::mutex mu;
-    static std::set<std::pair<int, const void*>> done;
+    static std::map<std::pair<int, const void*>, int> held;  // the largest the device can hold
     int dev = 0;
     CURC_CHECK(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> g(mu);
-    if (done.count({dev, kernel})) return;
-    CURC_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    done.insert({dev, kernel});
+    int& h = held[{dev, kernel}];
+    if (h == 0) {
+        CURC_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(16);
+        cfg.blockDim = dim3(threads);
+        int n = 0;
+        CURC_CHECK(cudaOccupancyMaxPotentialClusterSize(&n, kernel, &cfg));
+        h = std::max(1, n);
+    }
+    return cluster_fit(most, unsigned(h));
 }
 
 // ---------------------------------------------------------------- scan

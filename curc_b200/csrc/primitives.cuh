@@ -174,14 +174,17 @@ struct SubStage {
     }
 };
 
-// Clusters of more than 8 blocks are not portable: allowed for `kernel` on
-// the current device, once.
-void allow_large_clusters(const void* kernel);
+// Blocks of a cluster of `kernel` on the current device: `most` (a power of
+// two, at most 16), or the largest half of it that the device can hold (more
+// than 8 are not portable; a partition of a device may have no group of SMs
+// for 16).
+unsigned cluster_blocks(const void* kernel, unsigned most, unsigned threads);
 
-// Launches one cluster of `blocks` (at most 16) blocks.
+// Launches one cluster of at most `most` blocks; the kernel reads how many
+// there are.
 template <class... P, class... Q>
-void launch_cluster(void (*kernel)(P...), unsigned blocks, unsigned threads, cudaStream_t s, Q... args) {
-    if (blocks > 8) allow_large_clusters(reinterpret_cast<const void*>(kernel));
+void launch_cluster(void (*kernel)(P...), unsigned most, unsigned threads, cudaStream_t s, Q... args) {
+    const unsigned blocks = cluster_blocks(reinterpret_cast<const void*>(kernel), most, threads);
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at;
     at.id = cudaLaunchAttributeClusterDimension;

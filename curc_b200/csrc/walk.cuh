@@ -297,13 +297,10 @@ static __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(const Meeting
         else walk_offset(item, start[o], start[o + 1], threads, me, pre, off0 + o, next, prev, offset);
         o = skip(o + 1);
         if (o == noffs) return;
-        if (gridDim.x > 1) {
-            cluster_arrive();
-            if (AHEAD) h = look_ahead(item, start[o], start[o + 1], start[o] + me, pre);
-            cluster_wait();
-        } else {
-            __syncthreads();
-        }
+        if (gridDim.x > 1) cluster_arrive();
+        if (AHEAD) h = look_ahead(item, start[o], start[o + 1], start[o] + me, pre);
+        if (gridDim.x > 1) cluster_wait();
+        else __syncthreads();
     }
 }
 
