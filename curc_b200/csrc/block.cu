@@ -95,12 +95,19 @@ void Block::run(const uint8_t* d_seq, uint64_t n_reads, int L, bool po, bool pe)
     host.clear();
     stage_ms.clear();
     pinned.reset();
+    pending.clear();
     small.clear();
     large.clear();
     struct Sent {  // no copy outlives the run, however it ends
-        cudaStream_t s;
-        ~Sent() { cudaStreamSynchronize(s); }
-    } sent_guard{copy_stream};
+        Block& b;
+        bool done = false;
+        ~Sent() {
+            cudaStreamSynchronize(b.copy_stream);
+            if (done) return;
+            cudaStreamSynchronize(b.stream);
+            b.drop_pending();
+        }
+    } sent_guard{*this};
     StageTimer T(stream, events);
     struct TimerScope {
         explicit TimerScope(StageTimer* t) { active_timer() = t; }
@@ -233,11 +240,14 @@ void Block::run(const uint8_t* d_seq, uint64_t n_reads, int L, bool po, bool pe)
     }
 
     emit(T);
-    send_now();
+    send();
+    wait_sent();
     const cudaEvent_t ev1 = events.take();
     CURC_CHECK(cudaEventRecord(ev1, s));
     T.collect(stage_ms);
     CURC_CHECK(cudaStreamSynchronize(s));
+    sent_guard.done = true;
+    pending.clear();
     float total = 0;
     CURC_CHECK(cudaEventElapsedTime(&total, ev0, ev1));
     stage_ms["total"] = total;

@@ -38,6 +38,7 @@ struct Block {
     };
     std::vector<Piece> small;                       // results kept since the last send
     std::vector<std::pair<HostBuf, const uint8_t*>> large;
+    std::vector<std::string> pending;               // names given since the last send_now()
     Arena arena;
     bool keep_intermediates = true;
     Tuning tune;  // launch and table choices for the next runs (no effect on results)
@@ -107,7 +108,19 @@ struct Block {
             if (b.size <= SEND_SMALL) small.push_back(Piece{d, p, uint32_t(b.size)});
             else large.push_back({b, d});
         }
+        name_result(name, std::move(b));
+    }
+    void name_result(const std::string& name, HostBuf&& b) {
         host[name] = std::move(b);
+        pending.push_back(name);
+    }
+    // A run that ends early has the results that send_now() completed, and no
+    // others.
+    void drop_pending() {
+        for (const auto& n : pending) host.erase(n);
+        pending.clear();
+        small.clear();
+        large.clear();
     }
     // Queues what was kept, as the stream's work so far leaves it.
     void send();
@@ -117,13 +130,14 @@ struct Block {
     void send_now() {
         send();
         wait_sent();
+        pending.clear();
     }
     void put(const std::string& name, std::vector<uint8_t>&& v) {
         HostBuf b;
         b.own = std::move(v);
         b.ptr = b.own.data();
         b.size = b.own.size();
-        host[name] = std::move(b);
+        name_result(name, std::move(b));
     }
 };
 

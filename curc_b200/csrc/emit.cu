@@ -511,7 +511,7 @@ void Block::emit(StageTimer& T) {
             const uint64_t ne = uint64_t(class_count[mm]) * class_width(mm);
             h.size = ne * sizeof(uint16_t);
             if (ne) h.ptr = all.ptr + b * sizeof(uint16_t);
-            host["mis_off_" + std::to_string(mm)] = h;
+            name_result("mis_off_" + std::to_string(mm), std::move(h));
             b += ne;
         }
     }

@@ -210,7 +210,7 @@ int curc_decompress_file(const char* archive_path, const char* out_prefix, const
  * "mis_base", "read_off", "ref", ... and the stage intermediates
  * "sorted_ids", "next", "prev", "offset", "hq_seq", ...).  The pointer stays
  * valid until the next run or destroy.  Returns CURC_ERR_ARG for an unknown
- * name. */
+ * name; after a run that failed, the streams are unknown. */
 int curc_block_get(curc_ctx* ctx, const char* name, const void** ptr, uint64_t* bytes);
 
 /* Batched path: blocks queued on a context and run by several block
