@@ -119,7 +119,7 @@ void run_staged(BatchWorker& w, const BatchItem& it, int wi, std::chrono::steady
     Block& blk = *w.blk;
     CURC_CHECK(cudaEventSynchronize(w.landed));
     const double tl = batch_verbose() ? ms_since(t0) : 0;
-    blk.arena.reset();
+    blk.restart();
     blk.run(w.dev, it.n, it.L, it.po, it.pe);
     if (batch_verbose())
         std::fprintf(stderr, "curc: batch block %u pipeline %d: reads landed %.1f, done %.1f ms (device %.1f)\n",

@@ -413,7 +413,7 @@ int curc_block_run_device(curc_ctx* ctx, const char* seqs_dev, uint64_t n, uint1
     if (ctx)
         if (const int rc = curc::ctx_wait(ctx)) return rc;
     return guarded(ctx, [&] {
-        ctx->block->arena.reset();
+        ctx->block->restart();
         ctx->block->run(reinterpret_cast<const uint8_t*>(seqs_dev), n, read_len, preserve_order != 0,
                         paired_end != 0);
     });
@@ -426,7 +426,7 @@ int curc_block_run(curc_ctx* ctx, const char* seqs, uint64_t n, uint16_t read_le
         if (const int rc = curc::ctx_wait(ctx)) return rc;
     return guarded(ctx, [&] {
         curc::Block& b = *ctx->block;
-        b.arena.reset();
+        b.restart();
         const size_t bytes = size_t(n) * read_len;
         uint8_t* d = b.arena.alloc<uint8_t>(bytes + 16);
         CURC_CHECK(cudaMemcpyAsync(d, seqs, bytes, cudaMemcpyHostToDevice, b.stream));
@@ -460,7 +460,7 @@ int curc_ctx_trim(curc_ctx* ctx) {
     return guarded(ctx, [&] {
         CURC_CHECK(cudaStreamSynchronize(ctx->block->stream));
         if (ctx->batch) ctx->batch->pool.clear();  // the extra pipelines, input slots and staging
-        ctx->block->arena.trim();
+        ctx->block->trim();
     });
 }
 

@@ -88,6 +88,20 @@ struct Block {
     Block(const Block&) = delete;
     Block& operator=(const Block&) = delete;
 
+    // The last block's records and pseudogenome, which the learned coder reads,
+    // lie in the arena: they are gone once its memory starts anew.
+    void forget() {
+        n_records = 0;
+        hq = Assembled{};
+    }
+    void restart() {
+        forget();
+        arena.reset();
+    }
+    void trim() {
+        forget();
+        arena.trim();
+    }
     void run(const uint8_t* d_seq, uint64_t n_reads, int L, bool po, bool pe);
     // a10-a12: stream emission, unmapped pseudogenomes, repeat removal
     void emit(StageTimer& T);

@@ -202,7 +202,7 @@ private:
     };
     // the device side of the current block: its input in the arena
     void open_device_block() {
-        blk_->arena.reset();
+        blk_->restart();
         dev_ = blk_->arena.alloc<uint8_t>(max_bytes_ + 16);
         cap_ = max_bytes_;
         off_ = 0;

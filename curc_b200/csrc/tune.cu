@@ -156,7 +156,7 @@ int curc_autotune(curc_ctx* ctx, const char* seqs_dev, uint64_t n, uint16_t read
             blk.tune = t;
             float best = 1e30f;
             for (int r = 0; r < 2; ++r) {
-                blk.arena.reset();  // the input is the caller's memory, not the arena's
+                blk.restart();  // the input is the caller's memory, not the arena's
                 blk.run(reinterpret_cast<const uint8_t*>(seqs_dev), n, read_len, preserve_order != 0,
                         paired_end != 0);
                 best = std::min(best, blk.stage_ms.at(stage));
