@@ -180,7 +180,7 @@ def sort_lower_bound_bytes(m, L):
 # each of four sort passes, its 16-byte item written and read, and the link
 # words of its suffix and prefix (32 each).
 def resolve_bytes(st, L):
-    return st["overlap_links"] * (4 * 16 + 32 + 64)
+    return st["overlap_hits"] * (4 * 16 + 32 + 64)
 
 
 # Algorithmic bytes of the mapping kernels (forward and reverse complement):
@@ -199,7 +199,7 @@ def map_bytes(st, L, strand):
 # meetings (a look into L2-resident bitmaps per suffix and offset) and sorting
 # the two lists are not counted, so this is a lower bound.
 def full_match_bytes(st):
-    return st.get("fm_suffix_entries", 0) * (32 + 64)
+    return st.get("fm_meetings", 0) * (32 + 64)
 
 
 STAT_NAMES = ["reads", "non_n", "n_reads", "pseudogenome_reads", "unmatched", "mapped", "unmapped",
@@ -207,7 +207,7 @@ STAT_NAMES = ["reads", "non_n", "n_reads", "pseudogenome_reads", "unmatched", "m
               "overlap_suffixes", "overlap_active_sum", "overlap_probes", "overlap_hits",
               "overlap_searched", "overlap_compares", "overlap_links", "map_reads_fwd", "map_probes_fwd",
               "map_candidates_fwd", "map_reads_rc", "map_probes_rc", "map_candidates_rc", "overlap_rows",
-              "fm_passes", "fm_suffix_entries", "fm_prefix_entries"]
+              "fm_offsets", "fm_meetings", "fm_runs_met"]
 
 
 def block_stats(ctx):
@@ -881,7 +881,7 @@ def main():
                                  resolve_bytes(st, r["L"]), sub.get("overlap.resolve", 0.0), 1),
         "roofline_full_match": roof("full match (stage a6: lists sorted, meetings listed and walked)",
                                     full_match_bytes(st), r["stage_ms"].get("full_match", 0.0), 1,
-                                    {"passes": st.get("fm_passes", 0)}),
+                                    {"passes": st.get("fm_offsets", 0)}),
         "roofline_map": roof("map_kernel forward + reverse complement (stage a9)",
                              map_bytes(st, r["L"], "fwd") + map_bytes(st, r["L"], "rc"),
                              sub.get("mapping.map_fwd", 0.0) + sub.get("mapping.map_rc", 0.0), 2),

@@ -727,6 +727,7 @@ __global__ void __launch_bounds__(FM_SMALL) fm_small_kernel(Acc acc, const uint3
         if (t < n) me = suf[t];
     }
     int passes = 0;
+    uint32_t met = 0;
     for (int off = off0; off < acc.L; ++off) {
         ++passes;
         uint32_t lo = INVALID;
@@ -752,7 +753,9 @@ __global__ void __launch_bounds__(FM_SMALL) fm_small_kernel(Acc acc, const uint3
             if (b < n && at == 0) lo = b;
             run[t] = lo;
         }
-        if (!__syncthreads_or(lo != INVALID)) continue;
+        const int here = __syncthreads_count(lo != INVALID && !sdone[t]);
+        if (here == 0) continue;
+        met += uint32_t(here);
         if (t < n && lo != INVALID && (t == 0 || run[t - 1] != lo)) {
             const int len = acc.L - off;
             const uint64_t k = acc.key(me, off);
@@ -785,8 +788,8 @@ __global__ void __launch_bounds__(FM_SMALL) fm_small_kernel(Acc acc, const uint3
     }
     if (tally && t == 0) {
         tally[0] += uint32_t(passes);
-        tally[1] += uint64_t(passes) * n;
-        tally[2] += uint64_t(passes) * n;
+        tally[1] += met;
+        tally[2] += met;
     }
 }
 

@@ -387,7 +387,7 @@ void overlap_link(const BlockParams& p, const uint64_t* db, const uint32_t* sort
     // meetings' starts per offset
     struct State {
         uint32_t mp, ms, mp_out, ms_out;
-        unsigned long long used, tally[3];
+        unsigned long long used, tally[3], walked[2];
         uint32_t start[WALK_MAX_OFFS + 1];
     };
     State* d = a.zeros<State>(1, s);
@@ -398,6 +398,7 @@ void overlap_link(const BlockParams& p, const uint64_t* db, const uint32_t* sort
     uint32_t mp = h.mp, ms = h.ms;
     const uint32_t ms0 = ms;
     uint64_t active_sum = 0, met = 0;
+    uint64_t listed[3] = {0, 0, 0}, voided[3] = {0, 0, 0};  // the tally so far, and of listings that were repeated
     uint32_t passes = 0;
     const int step0 = ms <= OV_ALL ? p.max_off : p.tune.check_every;
     int step = step0;
@@ -493,8 +494,11 @@ void overlap_link(const BlockParams& p, const uint64_t* db, const uint32_t* sort
             if (h.used > cap) {  // too many for the room: fewer offsets
                 a.release(mk2);
                 step = std::max(1, noffs / 2);
+                for (int q = 0; q < 3; ++q) voided[q] += h.tally[q] - listed[q];
+                std::copy(h.tally, h.tally + 3, listed);
                 continue;
             }
+            std::copy(h.tally, h.tally + 3, listed);
             const uint32_t n = h.start[noffs];
             active_sum += uint64_t(ms) * noffs;
             met += n;
@@ -508,7 +512,7 @@ void overlap_link(const BlockParams& p, const uint64_t* db, const uint32_t* sort
                 const Meeting* item =
                     kb <= 32 ? sorted_meetings<uint32_t>(suf, ms, words, em, ub, hits, per, va, run_bits, kb, n, a, s)
                              : sorted_meetings<uint64_t>(suf, ms, words, em, ub, hits, per, va, run_bits, kb, n, a, s);
-                walk_stage(item, h.start, d->start, off, noffs, va, &d->used, cap, next, prev, offset, s);
+                walk_stage(item, h.start, d->start, off, noffs, va, &d->used, cap, next, prev, offset, d->walked, s);
             }
             sp_walk.stop();
             off += noffs;
@@ -534,15 +538,14 @@ void overlap_link(const BlockParams& p, const uint64_t* db, const uint32_t* sort
     if (st) {
         read_small(&h, d, sizeof(State), s);
         st->passes = passes;
-        st->links = uint32_t(met);
-        st->contested = 0;
+        st->links = h.walked[0];
+        st->contested = h.walked[1];
         st->suffixes = ms0;
         st->active_sum = active_sum;
-        st->probes = h.tally[0];
+        st->probes = h.tally[0] - voided[0];
         st->hits = met;
-        st->searched = h.tally[1];
-        st->compares = h.tally[2];
-        st->rows = h.tally[2];
+        st->searched = h.tally[1] - voided[1];
+        st->compares = h.tally[2] - voided[2];
     }
     a.release(mk);
 }

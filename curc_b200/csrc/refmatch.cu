@@ -858,14 +858,14 @@ void Block::refmatch_all() {
     put("sizes", std::vector<uint8_t>(reinterpret_cast<const uint8_t*>(sizes),
                                       reinterpret_cast<const uint8_t*>(sizes) + sizeof(sizes)));
     // block statistics: reads, non-N reads, N reads, pseudogenome reads,
-    // unmatched, mapped, unmapped (non-N, N), overlap passes, contested
-    // suffixes, records, mismatches; overlap suffixes, and summed over the
-    // passes: unlinked suffixes, suffixes probed, probes that met a prefix,
-    // probes that searched a bucket, prefix comparisons; overlap links; for
-    // the mapping, forward then reverse complement: reads searched, k-mer
-    // probes listed, candidate windows compared; prefix rows the probes read;
-    // full-match passes with both lists non-empty, and over them the summed
-    // suffix and prefix list lengths
+    // unmatched, mapped, unmapped (non-N, N); overlap: offsets passed, free
+    // suffixes of runs that two or more of them met; records, mismatches;
+    // overlap again: suffixes, and summed over the offsets free suffixes, their
+    // k-mers found in the presence bitmap, meetings with a run of prefixes,
+    // buckets searched, prefix rows compared; links made; mapping, forward then
+    // reverse complement: reads searched, k-mer probes listed, candidate windows
+    // compared; prefix rows read (as many as compared); full match: offsets
+    // passed, and meetings, twice (MapOut::tally, full_match_packed)
     unsigned long long mt[6] = {0, 0, 0, 0, 0, 0}, ft[3] = {0, 0, 0};
     if (mo.tally) read_small(mt, mo.tally, sizeof(mt), s);
     if (fm_tally) read_small(ft, fm_tally, sizeof(ft), s);
@@ -873,7 +873,7 @@ void Block::refmatch_all() {
                                 n_ug,       n_un,        ostats.passes, ostats.contested, n_records, n_mis,
                                 ostats.suffixes, ostats.active_sum, ostats.probes, ostats.hits, ostats.searched,
                                 ostats.compares, ostats.links, mt[0], mt[1], mt[2], mt[3], mt[4], mt[5],
-                                ostats.rows, ft[0], ft[1], ft[2]};
+                                ostats.compares, ft[0], ft[1], ft[2]};
     put("stats", std::vector<uint8_t>(reinterpret_cast<const uint8_t*>(stats),
                                       reinterpret_cast<const uint8_t*>(stats) + sizeof(stats)));
 }

@@ -72,9 +72,13 @@ void gather_ascii_rows(const uint8_t* seq, const uint32_t* ids, uint32_t m, int 
 // ---- a2..a5 (overlap.cu)
 void dedupe_links(const uint64_t* db, int W, const uint32_t* sorted, uint32_t m, uint32_t* next, uint32_t* prev,
                   uint16_t* offset, cudaStream_t s);
+// Offsets passed, links made, suffixes of runs that two or more free suffixes
+// met at one offset, suffixes; summed over the offsets: free suffixes, their
+// k-mers found in the presence bitmap, meetings, buckets searched, prefix
+// rows read and compared there.
 struct OverlapStats {
-    uint32_t passes = 0, links = 0, contested = 0, suffixes = 0;
-    uint64_t active_sum = 0, probes = 0, hits = 0, searched = 0, compares = 0, rows = 0;  // summed over passes
+    uint64_t passes = 0, links = 0, contested = 0, suffixes = 0;
+    uint64_t active_sum = 0, probes = 0, hits = 0, searched = 0, compares = 0;
 };
 void overlap_link(const BlockParams& p, const uint64_t* db, const uint32_t* sorted, uint32_t m, uint32_t* next,
                   uint32_t* prev, uint16_t* offset, Arena& a, cudaStream_t s, OverlapStats* st = nullptr);
@@ -86,8 +90,8 @@ void chain_filter(uint32_t n, const uint32_t* sorted, uint32_t m, uint32_t* next
 
 // ---- a6/a7 (fullmatch.cu)
 // Packed reads: prefix/suffix lists are consumed (scratch).  tally (device,
-// 3 counters, optional): offsets passed, and the suffix and prefix list
-// entries examined there (in the listed form: the meetings).
+// 3 counters, optional): offsets passed, and the meetings of a suffix with a
+// run of prefixes there, twice (pass form: the lengths of the two lists).
 void full_match_packed(const BlockParams& p, const uint64_t* db, uint32_t* pre, uint32_t* suf, uint32_t cnt,
                        uint32_t* next, uint32_t* prev, uint16_t* offset, Arena& a, cudaStream_t s,
                        unsigned long long* tally = nullptr);

@@ -36,18 +36,34 @@ struct __align__(16) Meeting {
 
 __device__ __forceinline__ uint32_t ld_l2(const uint32_t* p) { return __ldcg(p); }
 
+// What a walk did, where it is counted: links made, and the free suffixes of
+// runs that two or more of them met.
+struct Walked {
+    uint32_t links = 0, contested = 0;
+    __device__ __forceinline__ void met(uint32_t free_members) { contested += free_members > 1 ? free_members : 0; }
+};
+
 // The suffixes of one run (items [i, e) with the same lo, in order) each take
 // the first free prefix that is not themselves, as the reference's merge of
 // the run does (its rotation puts a prefix that meets itself back in front).
-// One thread.
-__device__ __forceinline__ void walk_run(const Meeting* __restrict__ item, uint32_t i, uint32_t e,
-                                        const uint32_t* __restrict__ pre, uint32_t q0, uint32_t hi, int off,
-                                        uint32_t* next, uint32_t* prev, uint16_t* offset) {
+// One thread.  Returns the free suffixes it met from item `from` on; they are
+// all met only where that is counted.
+template <bool COUNT>
+__device__ __forceinline__ uint32_t walk_run(const Meeting* __restrict__ item, uint32_t i, uint32_t e,
+                                             const uint32_t* __restrict__ pre, uint32_t q0, uint32_t hi, int off,
+                                             uint32_t* next, uint32_t* prev, uint16_t* offset, uint32_t from,
+                                             Walked& w) {
     const uint32_t lo = item[i].lo;
+    uint32_t met = 0;
+    bool any = true;  // a free prefix was left
     for (; i < e && item[i].lo == lo; ++i) {
         const uint32_t s = item[i].s;
         if (ld_l2(next + s) != INVALID) continue;
-        bool any = false;  // a free prefix was left
+        if (COUNT) {
+            met += i >= from;
+            if (!any) continue;
+        }
+        any = false;
         for (uint32_t q = q0; q < hi; ++q) {
             const uint32_t p = pre[q];
             if (ld_l2(prev + p) != INVALID) {
@@ -59,41 +75,50 @@ __device__ __forceinline__ void walk_run(const Meeting* __restrict__ item, uint3
             next[s] = p;
             prev[p] = s;
             offset[s] = uint16_t(off);
+            if (COUNT) ++w.links;
             break;
         }
-        if (!any) return;
+        if (!COUNT && !any) return met;
     }
+    return met;
 }
 
 // The same by a whole warp, for long runs: free suffixes and free prefixes
 // are taken 32 at a time and paired in order; where a read would meet itself
-// the rest of the run is walked by one lane.
-static __device__ void walk_run_warp(const Meeting* __restrict__ item, uint32_t i, uint32_t e, const uint32_t* __restrict__ pre,
-                             uint32_t q, uint32_t hi, int off, uint32_t* next, uint32_t* prev, uint16_t* offset) {
+// the rest of the run is walked by one lane.  Lane 0 counts.
+template <bool COUNT>
+static __device__ void walk_run_warp(const Meeting* __restrict__ item, uint32_t i, uint32_t e,
+                                     const uint32_t* __restrict__ pre, uint32_t q, uint32_t hi, int off, uint32_t* next,
+                                     uint32_t* prev, uint16_t* offset, Walked& w) {
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t lo = item[i].lo;
     uint32_t sm = 0, pm = 0;          // free entries of the current 32 items / prefixes
     uint32_t ib = i, qb = q;          // where the next 32 start
     uint32_t s = 0, p = 0;            // this lane's entries
-    bool more_s = true;
-    for (;;) {
-        while (sm == 0) {
-            if (!more_s) return;
+    uint32_t met = 0;
+    bool more_s = true, more_p = true;
+    while (more_p) {
+        while (sm == 0 && more_s) {
             const uint32_t t = ib + lane;
             const bool in = t < e && item[t].lo == lo;
             const uint32_t all = __ballot_sync(0xFFFFFFFFu, in);
             s = in ? item[t].s : 0;
             sm = __ballot_sync(0xFFFFFFFFu, in && ld_l2(next + s) == INVALID);
+            if (COUNT) met += __popc(sm);
             ib += 32;
             more_s = all == 0xFFFFFFFFu;
         }
-        while (pm == 0) {
-            if (qb >= hi) return;
+        if (sm == 0) break;
+        while (pm == 0 && qb < hi) {
             const uint32_t t = qb + lane;
             const bool in = t < hi;
             p = in ? pre[t] : 0;
             pm = __ballot_sync(0xFFFFFFFFu, in && ld_l2(prev + p) == INVALID);
             qb += 32;
+        }
+        if (pm == 0) {
+            more_p = false;
+            break;
         }
         const int n = min(__popc(sm), __popc(pm));
         // lane k < n pairs the k-th free suffix with the k-th free prefix
@@ -108,15 +133,26 @@ static __device__ void walk_run_warp(const Meeting* __restrict__ item, uint32_t 
             offset[S] = uint16_t(off);
         }
         __syncwarp();
+        if (COUNT && lane == 0) w.links += uint32_t(good);
         if (self) {
-            if (lane == 0) walk_run(item, ib - 32, e, pre, qb - 32, hi, off, next, prev, offset);
+            if (lane == 0) met += walk_run<COUNT>(item, ib - 32, e, pre, qb - 32, hi, off, next, prev, offset, ib, w);
             __syncwarp();
-            return;
+            more_s = false;
+            break;
         }
         for (int k = 0; k < n; ++k) {  // the n lowest of each are used up
             sm &= sm - 1;
             pm &= pm - 1;
         }
+    }
+    if (COUNT) {
+        for (; more_s; ib += 32) {  // no prefix is left for these
+            const uint32_t t = ib + lane;
+            const bool in = t < e && item[t].lo == lo;
+            more_s = __ballot_sync(0xFFFFFFFFu, in) == 0xFFFFFFFFu;
+            met += __popc(__ballot_sync(0xFFFFFFFFu, in && ld_l2(next + item[t].s) == INVALID));
+        }
+        if (lane == 0) w.met(met);
     }
 }
 
@@ -125,9 +161,11 @@ constexpr int WALK_MAX_OFFS = 512;
 
 // The meetings [a, e) of one offset by `threads` threads, of which this is
 // number me: one thread per run, long runs by a warp.
+template <bool COUNT>
 static __device__ __forceinline__ void walk_offset(const Meeting* __restrict__ item, uint32_t a, uint32_t e,
                                                    uint32_t threads, uint32_t me, const uint32_t* __restrict__ pre,
-                                                   int off, uint32_t* next, uint32_t* prev, uint16_t* offset) {
+                                                   int off, uint32_t* next, uint32_t* prev, uint16_t* offset,
+                                                   Walked& w) {
     for (uint32_t i0 = a; i0 < e; i0 += threads) {  // the same trip count for a whole warp
         const uint32_t i = i0 + me;
         bool long_run = false;
@@ -144,12 +182,17 @@ static __device__ __forceinline__ void walk_offset(const Meeting* __restrict__ i
                             next[it.s] = it.p;
                             prev[it.p] = it.s;
                             offset[it.s] = uint16_t(off);
+                            if (COUNT) ++w.links;
                         }
                     }
                 } else {
                     // more than a few members or prefixes: by the whole warp
                     long_run = it.hi - it.lo > 8 || (i + 8 < e && item[i + 8].lo == it.lo);
-                    if (!long_run) walk_run(item, i, e, pre, it.lo, it.hi, off, next, prev, offset);
+                    if (!long_run) {
+                        const uint32_t met =
+                            walk_run<COUNT>(item, i, e, pre, it.lo, it.hi, off, next, prev, offset, i, w);
+                        if (COUNT) w.met(met);
+                    }
                 }
             }
         }
@@ -159,7 +202,7 @@ static __device__ __forceinline__ void walk_offset(const Meeting* __restrict__ i
             todo &= todo - 1;
             const uint32_t ii = __shfl_sync(0xFFFFFFFFu, i, l), lo = __shfl_sync(0xFFFFFFFFu, it.lo, l),
                            hi = __shfl_sync(0xFFFFFFFFu, it.hi, l);
-            walk_run_warp(item, ii, e, pre, lo, hi, off, next, prev, offset);
+            walk_run_warp<COUNT>(item, ii, e, pre, lo, hi, off, next, prev, offset, w);
         }
     }
 }
@@ -204,10 +247,11 @@ __device__ __forceinline__ Ahead look_ahead(const Meeting* __restrict__ item, ui
 // offset, mostly of runs of one to three, a thread's chain of ten dependent
 // loads was what an offset took; where an offset has few meetings, as in the
 // full match, the plain form is the shorter one.
+template <bool COUNT>
 static __device__ __forceinline__ void walk_offset_ahead(const Meeting* __restrict__ item, uint32_t a, uint32_t e,
-                                                   uint32_t threads, uint32_t me, Ahead h,
-                                                   const uint32_t* __restrict__ pre, int off, uint32_t* next,
-                                                   uint32_t* prev, uint16_t* offset) {
+                                                         uint32_t threads, uint32_t me, Ahead h,
+                                                         const uint32_t* __restrict__ pre, int off, uint32_t* next,
+                                                         uint32_t* prev, uint16_t* offset, Walked& w) {
     for (uint32_t i0 = a;;) {  // the same trip count for a whole warp
         if (h.np) {
             uint32_t fs = 0, fp = 0;  // free suffixes and prefixes
@@ -216,6 +260,7 @@ static __device__ __forceinline__ void walk_offset_ahead(const Meeting* __restri
                 if (k < h.ns && ld_l2(next + h.s[k]) == INVALID) fs |= 1u << k;
                 if (k < h.np && ld_l2(prev + h.p[k]) == INVALID) fp |= 1u << k;
             }
+            if (COUNT) w.met(__popc(fs));
 #pragma unroll
             for (uint32_t k = 0; k < FEW; ++k) {
                 if (!(fs >> k & 1u)) continue;
@@ -228,6 +273,7 @@ static __device__ __forceinline__ void walk_offset_ahead(const Meeting* __restri
                         next[h.s[k]] = h.p[q];
                         prev[h.p[q]] = h.s[k];
                         offset[h.s[k]] = uint16_t(off);
+                        if (COUNT) ++w.links;
                     }
             }
         }
@@ -237,7 +283,7 @@ static __device__ __forceinline__ void walk_offset_ahead(const Meeting* __restri
             todo &= todo - 1;
             const uint32_t ii = i0 + me - (threadIdx.x & 31u) + l;
             const Meeting it = item[ii];
-            walk_run_warp(item, ii, e, pre, it.lo, it.hi, off, next, prev, offset);
+            walk_run_warp<COUNT>(item, ii, e, pre, it.lo, it.hi, off, next, prev, offset, w);
         }
         i0 += threads;
         if (i0 >= e) return;
@@ -245,14 +291,25 @@ static __device__ __forceinline__ void walk_offset_ahead(const Meeting* __restri
     }
 }
 
+// A warp's counts to counts[0] (links) and counts[1] (contested).
+__device__ __forceinline__ void add_walked(const Walked& w, unsigned long long* counts) {
+    const uint32_t l = __reduce_add_sync(0xFFFFFFFFu, w.links), c = __reduce_add_sync(0xFFFFFFFFu, w.contested);
+    if ((threadIdx.x & 31u) != 0) return;
+    if (l) atomicAdd(counts, static_cast<unsigned long long>(l));
+    if (c) atomicAdd(counts + 1, static_cast<unsigned long long>(c));
+}
+
 // One offset by a whole grid.
 static __global__ void __launch_bounds__(256) walk_one_kernel(const Meeting* __restrict__ item, uint32_t a, uint32_t e,
                                                               int off, const uint32_t* __restrict__ pre, uint32_t* next,
-                                                              uint32_t* prev, uint16_t* offset) {
+                                                              uint32_t* prev, uint16_t* offset,
+                                                              unsigned long long* __restrict__ counts) {
     const uint32_t me = blockIdx.x * 256 + threadIdx.x;
+    Walked w;
     if (a < e)
-        walk_offset_ahead(item, a, e, gridDim.x * 256, me, look_ahead(item, a, e, a + me, pre), pre, off, next, prev,
-                          offset);
+        walk_offset_ahead<true>(item, a, e, gridDim.x * 256, me, look_ahead(item, a, e, a + me, pre), pre, off, next,
+                                prev, offset, w);
+    add_walked(w, counts);
 }
 
 // The walk: offset after offset, one thread per run of equal suffix strings
@@ -266,24 +323,27 @@ static __global__ void __launch_bounds__(256) walk_one_kernel(const Meeting* __r
 // pairs 0.64, 0.44, 0.37 ms; 700k reads of 251 1.00, 0.90, 0.75; 8M of 250
 // 3.22, 2.56, 2.09 (blocks of 256 or 1024 threads: slower, as is AHEAD in one
 // block: 64 offsets of 83 meetings 0.133 -> 0.158).
-template <bool AHEAD>
+// COUNT: links and contested suffixes go to counts; else counts, if given, are
+// the full match's (offsets passed, and twice the meetings).
+template <bool AHEAD, bool COUNT>
 static __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(const Meeting* __restrict__ item,
                                                                    const uint32_t* __restrict__ start_in, int off0,
                                                                    int noffs, const uint32_t* __restrict__ pre,
                                                                    const unsigned long long* __restrict__ used,
                                                                    uint32_t cap, uint32_t* next, uint32_t* prev,
                                                                    uint16_t* offset,
-                                                                   unsigned long long* __restrict__ tally) {
+                                                                   unsigned long long* __restrict__ counts) {
     __shared__ uint32_t start[WALK_MAX_OFFS + 1];
     if (*used > cap) return;  // the listing is incomplete: the caller repeats it
     for (int o = threadIdx.x; o <= noffs; o += WALK_THREADS) start[o] = start_in[o];
     __syncthreads();
     const uint32_t threads = gridDim.x * WALK_THREADS, me = blockIdx.x * WALK_THREADS + threadIdx.x;
-    if (tally && me == 0) {
-        tally[0] += uint32_t(noffs);
-        tally[1] += start[noffs];
-        tally[2] += start[noffs];
+    if (!COUNT && counts && me == 0) {
+        counts[0] += uint32_t(noffs);
+        counts[1] += start[noffs];
+        counts[2] += start[noffs];
     }
+    Walked w;
     auto skip = [&](int o) {  // the next offset with meetings
         while (o < noffs && start[o] == start[o + 1]) ++o;
         return o;
@@ -293,15 +353,18 @@ static __global__ void __launch_bounds__(WALK_THREADS) walk_kernel(const Meeting
     Ahead h;
     if (AHEAD) h = look_ahead(item, start[o], start[o + 1], start[o] + me, pre);
     for (;;) {
-        if (AHEAD) walk_offset_ahead(item, start[o], start[o + 1], threads, me, h, pre, off0 + o, next, prev, offset);
-        else walk_offset(item, start[o], start[o + 1], threads, me, pre, off0 + o, next, prev, offset);
+        if (AHEAD)
+            walk_offset_ahead<COUNT>(item, start[o], start[o + 1], threads, me, h, pre, off0 + o, next, prev, offset, w);
+        else
+            walk_offset<COUNT>(item, start[o], start[o + 1], threads, me, pre, off0 + o, next, prev, offset, w);
         o = skip(o + 1);
-        if (o == noffs) return;
+        if (o == noffs) break;
         if (gridDim.x > 1) cluster_arrive();
         if (AHEAD) h = look_ahead(item, start[o], start[o + 1], start[o] + me, pre);
         if (gridDim.x > 1) cluster_wait();
         else __syncthreads();
     }
+    if (COUNT) add_walked(w, counts);
 }
 
 constexpr unsigned WALK_CLUSTER = 16;
@@ -314,7 +377,7 @@ static inline void walk_meetings(const Meeting* item, const uint32_t* start, int
     // short lists meet a few hundred at a time: one block, whose barrier is
     // cheaper than the cluster's (50k reads, 2,048 to 4,096 ends: full match
     // 0.33 against 0.36 ms; 100k reads, more ends: 0.60 against 0.53)
-    launch_cluster(walk_kernel<false>, entries > 4096 ? WALK_CLUSTER : 1, WALK_THREADS, s, item, start, off0, noffs, pre,
+    launch_cluster(walk_kernel<false, false>, entries > 4096 ? WALK_CLUSTER : 1, WALK_THREADS, s, item, start, off0, noffs, pre,
                    used, cap, next, prev, offset, tally);
 }
 
@@ -324,12 +387,12 @@ static inline void walk_meetings(const Meeting* item, const uint32_t* start, int
 constexpr uint32_t WALK_GRID = 32768;
 static inline void walk_stage(const Meeting* item, const uint32_t* host_start, const uint32_t* start, int off0, int noffs,
                        const uint32_t* pre, const unsigned long long* used, uint32_t cap, uint32_t* next,
-                       uint32_t* prev, uint16_t* offset, cudaStream_t s) {
+                       uint32_t* prev, uint16_t* offset, unsigned long long* counts, cudaStream_t s) {
     for (int o = 0; o < noffs;) {
         const uint32_t n = host_start[o + 1] - host_start[o];
         if (n > WALK_GRID) {
             walk_one_kernel<<<resident_grid(walk_one_kernel, 256, n), 256, 0, s>>>(
-                item, host_start[o], host_start[o + 1], off0 + o, pre, next, prev, offset);
+                item, host_start[o], host_start[o + 1], off0 + o, pre, next, prev, offset, counts);
             CURC_LAUNCH_CHECK();
             ++o;
             continue;
@@ -342,8 +405,8 @@ static inline void walk_stage(const Meeting* item, const uint32_t* host_start, c
         }
         if (host_start[e] != host_start[o]) {
             const bool many = most > 2048;
-            launch_cluster(many ? walk_kernel<true> : walk_kernel<false>, many ? WALK_CLUSTER : 1, WALK_THREADS, s, item,
-                           start + o, off0 + o, e - o, pre, used, cap, next, prev, offset, nullptr);
+            launch_cluster(many ? walk_kernel<true, true> : walk_kernel<false, true>, many ? WALK_CLUSTER : 1,
+                           WALK_THREADS, s, item, start + o, off0 + o, e - o, pre, used, cap, next, prev, offset, counts);
         }
         o = e;
     }

@@ -58,7 +58,7 @@ void walks(Arena& a, uint32_t reads, int noffs, uint32_t per_off, bool ahead) {
         uint32_t* nx = up(a, std::vector<uint32_t>(reads, INVALID));
         uint32_t* pv = up(a, std::vector<uint32_t>(reads, INVALID));
         uint16_t* of = up(a, std::vector<uint16_t>(reads, INVALOFF));
-        launch_cluster(ahead ? walk_kernel<true> : walk_kernel<false>, blocks, WALK_THREADS, s, di, ds, 1, noffs, dp,
+        launch_cluster(ahead ? walk_kernel<true, false> : walk_kernel<false, false>, blocks, WALK_THREADS, s, di, ds, 1, noffs, dp,
                        used, 1u, nx, pv, of, nullptr);
         const auto n = down(nx, reads), p = down(pv, reads);
         const auto o = down(of, reads);
