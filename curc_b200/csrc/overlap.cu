@@ -466,8 +466,11 @@ void overlap_link(const BlockParams& p, const uint64_t* db, const uint32_t* sort
             c.va = va;
             c.kr = kr;
         };
+        double asked = 0;  // the room that the last listing asked for, per suffix and offset
         for (int off = 1; off < p.max_off && mp && ms;) {
-            const int noffs = std::min({step, p.max_off - off, WALK_MAX_OFFS}), words = (noffs + 31) / 32;
+            int noffs = std::min({step, p.max_off - off, WALK_MAX_OFFS});
+            if (asked * ms * noffs > 0.9 * cap) noffs = std::max(1, int(0.9 * cap / (asked * ms)));
+            const int words = (noffs + 31) / 32;
             // an index of prefixes of which most are still free serves on: the
             // walk passes over the others
             if (!indexed || uint64_t(mp) * 4 < uint64_t(indexed) * 3) build_index(off);
@@ -491,6 +494,7 @@ void overlap_link(const BlockParams& p, const uint64_t* db, const uint32_t* sort
             exclusive_scan<uint32_t>(per, per, ms, nullptr, a, s);
             read_small(&h, d, sizeof(State), s);
             sp_meet.stop();
+            asked = double(h.used) / (double(ms) * noffs);
             if (h.used > cap) {  // too many for the room: fewer offsets
                 a.release(mk2);
                 step = std::max(1, noffs / 2);
