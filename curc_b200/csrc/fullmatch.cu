@@ -22,11 +22,16 @@
 // reads.  One sort of the suffix list by reversed reads therefore makes each
 // run contiguous and ordered at every offset.
 //
+// Other letters.  The ASCII buckets are of A, C, G, N and T, so a string with
+// another letter among its first three meets nothing; further on, other
+// letters are symbols like any.  In byte order the listed form needs nothing
+// more for them than that rule.
+//
 // The launch-per-kernel form that re-sorts at every offset
-// (full_match_passes) remains for reads with symbols other than A, C, G, N
-// and T, whose partition classes do not follow their byte order, and as
-// tune.fm_loop 0.  There (1) is a tree of parallel stable pairwise merges
-// of the per-symbol runs (merge path).
+// (full_match_passes) remains as tune.fm_loop 0 for reads of those five
+// letters.  There (1) is a tree of parallel stable pairwise merges of the
+// per-symbol runs (merge path), whose last class would hold T and every other
+// letter unsorted.
 #include <algorithm>
 
 #include "compact.cuh"
@@ -58,6 +63,8 @@ struct PackedAcc {
         return reverse_bases(word_at(db + uint64_t(a) * W, uint32_t(end - nb), nb));
     }
     __device__ __forceinline__ int rwords() const { return W; }
+    // whether the string from pos on can be met
+    __device__ __forceinline__ bool bucketed(uint32_t, int) const { return true; }
     // hash of the FK <= FK_MAX symbols from pos
     static constexpr int FK_MAX = 32;
     __device__ __forceinline__ uint64_t fhash(uint32_t a, int pos, int fk) const {
@@ -72,10 +79,22 @@ struct PackedAcc {
     };
 };
 
+__device__ __forceinline__ bool other_letter(uint8_t c) {
+    return c != 'A' && c != 'C' && c != 'G' && c != 'N' && c != 'T';
+}
+
 struct AsciiAcc {
     const uint8_t* r;
     int W, L;  // W unused
+    bool other;  // the reads hold letters beyond A, C, G, N and T
     static constexpr int ALPHA = 5;
+    __device__ __forceinline__ bool bucketed(uint32_t a, int pos) const {
+        if (!other) return true;
+        const uint8_t* x = r + uint64_t(a) * L;
+        for (int i = pos; i < pos + 3 && i < L; ++i)
+            if (other_letter(x[i])) return false;
+        return true;
+    }
     __device__ __forceinline__ int cmp(uint32_t a, int aoff, uint32_t b, int boff, int len) const {
         const uint8_t* x = r + uint64_t(a) * L + aoff;
         const uint8_t* y = r + uint64_t(b) * L + boff;
@@ -83,7 +102,7 @@ struct AsciiAcc {
             if (x[i] != y[i]) return x[i] < y[i] ? -1 : 1;
         return 0;
     }
-    // partition symbols of compress.cu:1238-1249: A, C, G, N, everything else
+    // partition symbols of compress.cu:1238-1249: A, C, G, N, T
     __device__ __forceinline__ int sym(uint32_t a, int pos) const {
         switch (r[uint64_t(a) * L + pos]) {
             case 'A': return 0;
@@ -223,17 +242,10 @@ __device__ __forceinline__ void run_bounds_block(const Acc& acc, const uint32_t*
         }
         __syncthreads();
     }
-    // Reads with several letters that share the last symbol are not in the
-    // order the search takes them to be in; its bounds may then cross, and
-    // the merges would read beyond the list.
     if (threadIdx.x == 0) {
-        uint32_t b = 0;
         bounds[0] = 0;
 #pragma unroll
-        for (int q = 0; q < NB; ++q) {
-            b = max(b, lo_s[q]);
-            bounds[q + 1] = b;
-        }
+        for (int q = 0; q < NB; ++q) bounds[q + 1] = lo_s[q];
         bounds[Acc::ALPHA] = m;
     }
 }
@@ -513,6 +525,7 @@ __global__ void fm_prefix_kernel(Acc acc, const uint32_t* __restrict__ pre, uint
 template <class Acc>
 __device__ __forceinline__ bool fm_run(const Acc& acc, const uint32_t* pre, const uint64_t* pk, uint32_t mp,
                                        uint32_t s, int off, uint32_t& lo_out, uint32_t& hi_out) {
+    if (!acc.bucketed(s, off)) return false;
     const int len = acc.L - off;
     const uint64_t k = acc.key(s, off);
     auto pcmp = [&](uint32_t i) { return cmp_keyed(acc, pk[i], pre[i], 0, k, s, off, len); };
@@ -736,7 +749,7 @@ __global__ void __launch_bounds__(FM_SMALL) fm_small_kernel(Acc acc, const uint3
             const int len = acc.L - off;
             const uint64_t k = acc.key(me, off);
             const uint32_t h = fm_small_bit<Acc>(k);
-            const bool maybe = len < FS || (bits[h >> 5] >> (h & 31) & 1u);
+            const bool maybe = (len < FS || (bits[h >> 5] >> (h & 31) & 1u)) && acc.bucketed(me, off);
             uint32_t b = 0, c = maybe ? n : 0;
             int at = 1;
             while (c > 0) {
@@ -945,8 +958,7 @@ __global__ void other_symbols_kernel(const uint8_t* __restrict__ r, int L, const
     for (uint64_t t = uint64_t(blockIdx.x) * blockDim.x + threadIdx.x; t < uint64_t(m) * L;
          t += uint64_t(gridDim.x) * blockDim.x) {
         const uint32_t i = uint32_t(t / L), b = uint32_t(t - uint64_t(i) * L);
-        const uint8_t c = r[uint64_t(ids[i]) * L + b];
-        if (c != 'A' && c != 'C' && c != 'G' && c != 'N' && c != 'T') *other = 1;
+        if (other_letter(r[uint64_t(ids[i]) * L + b])) *other = 1;
     }
 }
 
@@ -1036,8 +1048,8 @@ void full_match_ascii(const BlockParams& p, const uint8_t* reads, uint32_t* ids,
     select_flagged(ids, sf, suf, m, counts + 1, a, s);
     uint32_t h[3];
     read_small(h, counts, 12, s);
-    full_match_loop(AsciiAcc{reads, 0, p.L}, pre, suf, h[0], next, prev, offset, p.tune.fm_loop == 0 || h[2] != 0,
-                    nullptr, a, s);
+    full_match_loop(AsciiAcc{reads, 0, p.L, h[2] != 0}, pre, suf, h[0], next, prev, offset,
+                    p.tune.fm_loop == 0 && h[2] == 0, nullptr, a, s);
     a.release(mk);
 }
 
