@@ -173,7 +173,7 @@ int curc_autotune(curc_ctx* ctx, const char* seqs_dev, uint64_t n, uint16_t read
                               {&Tuning::bitmap_bits, {8, 16, 32}, "overlap"},
                               {&Tuning::check_every, {4, 8, 16}, "overlap"},
                               {&Tuning::map_threads, {64, 128, 256}, "mapping"},
-                              {&Tuning::fm_loop, {0, 1, 2}, "full_match"}};
+                              {&Tuning::fm_loop, {0, 1}, "full_match"}};  // (2 is 1)
         for (const Knob& k : knobs) {
             float tbest = 1e30f;
             int vbest = best.*(k.field);
