@@ -160,31 +160,13 @@ __device__ __forceinline__ int cmp_keyed(const Acc& acc, uint64_t ka, uint32_t a
     return acc.cmp(a, aoff + Acc::KS, b, boff + Acc::KS, len - Acc::KS);
 }
 
-// Keys of the list entries [t0, m) step ts at offset off.  With sym_count
-// (2-bit reads only), also how many entries have each base at off-1: the
-// list is sorted by read[off-1, L), so these counts give the base runs'
-// bounds.  Each thread counts in four 16-bit fields (a resident grid leaves
-// it far fewer than 65536 entries), then one atomic per block and base
-// (every thread of the block calls this).
-template <class Acc>
-__device__ __forceinline__ void list_keys_range(const Acc& acc, const uint32_t* __restrict__ ids, uint32_t m, int off,
-                                                uint64_t* __restrict__ key, uint32_t* __restrict__ sym_count,
-                                                uint32_t t0, uint32_t ts) {
-    uint64_t c = 0;
-    for (uint32_t i = t0; i < m; i += ts) {
-        const uint32_t id = ids[i];
-        key[i] = acc.key(id, off);
-        if constexpr (Acc::ALPHA == 4)
-            if (sym_count) c += 1ull << (16 * acc.sym(id, off - 1));
-    }
-    if constexpr (Acc::ALPHA == 4)
-        if (sym_count)
-            for (int b = 0; b < 4; ++b) block_tally<uint32_t>(uint32_t(c >> (16 * b)) & 0xFFFFu, sym_count + b);
-}
-
-// With tally: one thread adds the pass to the counters (passes with both
-// lists non-empty, their suffix and prefix entries; mp_dev is the prefix
-// list's length).
+// Keys of the list entries at offset off.  With sym_count (2-bit reads only),
+// also how many entries have each base at off-1: the list is sorted by
+// read[off-1, L), so these counts give the base runs' bounds.  Each thread
+// counts in four 16-bit fields (a resident grid leaves it far fewer than 65536
+// entries), then one atomic per block and base.  With tally: one thread adds
+// the pass to the counters (passes with both lists non-empty, their suffix and
+// prefix entries; mp_dev is the prefix list's length).
 template <class Acc>
 __global__ void list_keys_kernel(Acc acc, const uint32_t* __restrict__ ids, const uint32_t* __restrict__ m_dev,
                                  int off, uint64_t* __restrict__ key, uint32_t* __restrict__ sym_count,
@@ -198,7 +180,16 @@ __global__ void list_keys_kernel(Acc acc, const uint32_t* __restrict__ ids, cons
             tally[2] += mp;
         }
     }
-    list_keys_range(acc, ids, m, off, key, sym_count, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    uint64_t c = 0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < m; i += gridDim.x * blockDim.x) {
+        const uint32_t id = ids[i];
+        key[i] = acc.key(id, off);
+        if constexpr (Acc::ALPHA == 4)
+            if (sym_count) c += 1ull << (16 * acc.sym(id, off - 1));
+    }
+    if constexpr (Acc::ALPHA == 4)
+        if (sym_count)
+            for (int b = 0; b < 4; ++b) block_tally<uint32_t>(uint32_t(c >> (16 * b)) & 0xFFFFu, sym_count + b);
 }
 
 // bounds[c] = first index whose symbol at off-1 is >= c (the list is
@@ -206,10 +197,11 @@ __global__ void list_keys_kernel(Acc acc, const uint32_t* __restrict__ ids, cons
 // narrows all boundaries at once, 64 threads each: every round samples 64
 // evenly spaced positions of the boundary's interval, so a few rounds of
 // independent loads replace a chain of ~log2(m) dependent ones.
-// (One block of at least 256 threads; every thread calls it.)
 template <class Acc>
-__device__ __forceinline__ void run_bounds_block(const Acc& acc, const uint32_t* __restrict__ suf, uint32_t m, int off,
-                                                 uint32_t* __restrict__ bounds) {
+__global__ void __launch_bounds__(256) run_bounds_kernel(Acc acc, const uint32_t* __restrict__ suf,
+                                                         const uint32_t* __restrict__ m_dev, int off,
+                                                         uint32_t* __restrict__ bounds) {
+    const uint32_t m = *m_dev;
     constexpr int NB = Acc::ALPHA - 1;  // boundaries to find: symbols 1 .. ALPHA-1 (at most 4)
     constexpr uint32_t S = 64;          // samples per boundary and round
     __shared__ uint32_t lo_s[4], hi_s[4];
@@ -250,13 +242,6 @@ __device__ __forceinline__ void run_bounds_block(const Acc& acc, const uint32_t*
     }
 }
 
-template <class Acc>
-__global__ void __launch_bounds__(256) run_bounds_kernel(Acc acc, const uint32_t* __restrict__ suf,
-                                                         const uint32_t* __restrict__ m_dev, int off,
-                                                         uint32_t* __restrict__ bounds) {
-    run_bounds_block(acc, suf, *m_dev, off, bounds);
-}
-
 // Stable merge of the symbol runs by read[off, L), as a tree of pairwise
 // merges of adjacent runs (level l merges groups of 2^l runs; ties go to the
 // lower run, as in the reference's stable merges), each
@@ -268,12 +253,14 @@ __global__ void __launch_bounds__(256) run_bounds_kernel(Acc acc, const uint32_t
 // reads themselves only when the first key symbols are equal.
 constexpr int MP_ITEMS = 8;
 
-// Outputs [t0, m) step ts (in units of MP_ITEMS).
+// bounds: the run bounds (ALPHA + 1 entries), or with `counts` the number of
+// entries per symbol, from which the bounds are summed.
 template <class Acc>
-__device__ __forceinline__ void merge_level_range(const Acc& acc, int off, const uint32_t* __restrict__ in,
-                                                  const uint64_t* __restrict__ ink, uint32_t* __restrict__ out,
-                                                  uint64_t* __restrict__ outk, const uint32_t* __restrict__ bounds,
-                                                  bool counts, uint32_t m, int width, uint64_t t0, uint64_t ts) {
+__global__ void merge_level_kernel(Acc acc, int off, const uint32_t* __restrict__ in, const uint64_t* __restrict__ ink,
+                                   uint32_t* __restrict__ out, uint64_t* __restrict__ outk,
+                                   const uint32_t* __restrict__ bounds, bool counts, const uint32_t* __restrict__ m_dev,
+                                   int width) {
+    const uint32_t m = *m_dev;
     uint32_t bd[Acc::ALPHA + 1];
     if (counts) {
         bd[0] = 0;
@@ -290,8 +277,8 @@ __device__ __forceinline__ void merge_level_range(const Acc& acc, int off, const
     auto cmp_at = [&](uint32_t x, uint32_t y) {
         return cmp_keyed(acc, ink[x], in[x], off, ink[y], in[y], off, len);
     };
-    const uint64_t stride = ts * MP_ITEMS;
-    for (uint64_t d0 = t0 * MP_ITEMS; d0 < m; d0 += stride) {
+    const uint64_t stride = uint64_t(gridDim.x) * blockDim.x * MP_ITEMS;
+    for (uint64_t d0 = (uint64_t(blockIdx.x) * blockDim.x + threadIdx.x) * MP_ITEMS; d0 < m; d0 += stride) {
         const uint32_t dend = uint32_t(min(uint64_t(m), d0 + MP_ITEMS));
         uint32_t d = uint32_t(d0);
         int k = 0;
@@ -323,17 +310,6 @@ __device__ __forceinline__ void merge_level_range(const Acc& acc, int off, const
             }
         }
     }
-}
-
-// bounds: the run bounds (ALPHA + 1 entries), or with `counts` the number of
-// entries per symbol, from which the bounds are summed.
-template <class Acc>
-__global__ void merge_level_kernel(Acc acc, int off, const uint32_t* __restrict__ in, const uint64_t* __restrict__ ink,
-                                   uint32_t* __restrict__ out, uint64_t* __restrict__ outk,
-                                   const uint32_t* __restrict__ bounds, bool counts, const uint32_t* __restrict__ m_dev,
-                                   int width) {
-    merge_level_range(acc, off, in, ink, out, outk, bounds, counts, *m_dev, width,
-                      uint64_t(blockIdx.x) * blockDim.x + threadIdx.x, uint64_t(gridDim.x) * blockDim.x);
 }
 
 // One thread per run of equal suffix strings: the reference's bucket merge

@@ -158,8 +158,7 @@ StageTimer*& active_timer();
 struct SubStage {
     StageTimer* t;
     size_t i = 0;
-    // on = false: no span (launches being captured into a graph)
-    explicit SubStage(const char* name, bool on = true) : t(on ? active_timer() : nullptr) {
+    explicit SubStage(const char* name) : t(active_timer()) {
         if (t) i = t->begin_span(name);
     }
     void stop() {
