@@ -150,8 +150,10 @@ __global__ void anchors_kernel(const DevRecord* __restrict__ rec, const uint8_t*
 // same bits whatever the tiling.  The chains bound the step: 4096 dependent
 // additions of four cycles are 8 us.  With one tiled product per launch, 20
 // launches and three copies a step, a step of 4096 anchors took 1.5 ms on
-// B200; it takes 64 us so (a run of two epochs over 287,000 anchors 208 -> 17
-// ms, of which the host's shuffles are about half).
+// B200; it takes 66 us so (rows 28, gradients 35, Adam 4.5).  Two epochs over
+// 287,000 anchors, 208 -> 16 to 17 ms, are 138 steps, 9.1 ms, behind which the
+// host's shuffles (0.7 ms an epoch) hide, and 6.6 ms that a call takes whatever
+// its epochs (parameters drawn on the host, buffers, quantisation).
 
 constexpr int TR_ROWS = 32, TR_S = 132;  // rows per block; padded row of 128 (16-byte reads without conflicts)
 constexpr size_t TR_SMEM = (size_t(2 * HID + OUT + 3 * TR_ROWS) * TR_S + TR_ROWS * OUT) * sizeof(float);

@@ -296,9 +296,12 @@ __device__ __forceinline__ void map_read(const MapIndex& ix, const uint64_t* __r
 }
 
 // Warps take reads in turn (a resident grid, so that no warp waits for its
-// block's slowest read).  What bounds it: random sectors, at 3.3 TB/s of DRAM
-// reads, and behind them issue slots.  Six blocks of 256 threads a SM (42
-// registers) hide more of the loads than five without the limit; eight spill.
+// block's slowest read).  What bounds it: random sectors (2M pairs of 150 bp:
+// 3.3 TB/s of DRAM traffic forward, 2.5 reverse complement), and behind them
+// issue slots.  The bound of 42 registers (it takes 40, and spills 12 bytes in
+// the reverse-complement form) holds 1536 threads a SM, 12 blocks of the
+// default 128; that hides more of the loads than 1280 threads without it, and
+// 2048 spill.
 // Measured on B200, forward and reverse complement together, against a bucket
 // range, a position and a window load per candidate: 8M reads of 250 bp
 // 60 -> 35.8 ms, 10M pairs of 150 bp 15.5 -> 9.6 ms with the index.  Tried and

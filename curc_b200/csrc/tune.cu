@@ -1,13 +1,13 @@
 // Autotuner for the launch and table choices that change no result (no
 // counterpart in the reference, whose launch shapes are Thrust defaults).
 //
-// Knobs (struct Tuning): the overlap index's bucket table size as a multiple
-// of the prefix count, bits of the prefix presence bitmap per prefix, overlap
-// passes between host reads of the link count, threads per block of the
-// mapping kernel, and the form of the full-match pass loop (a launch per
-// kernel, one graph, or one persistent kernel).  None of them changes which prefixes a suffix meets, the
-// order candidates are visited in, or any stream: the tests compare every
-// stage result and stream under each setting.  The k-mer length and the
+// Knobs (struct Tuning): the overlap index's bucket table size in quarters of
+// the prefix count, bits of the prefix presence bitmap per prefix, offsets of
+// the overlap's first stage on a long list, threads per block of the mapping
+// kernel, and the form of the full match (meetings of many offsets listed at
+// once, or a pass of launches per offset).  None of them changes which
+// prefixes a suffix meets, the order candidates are visited in, or any stream:
+// the tests compare every stage result and stream under each setting.  The k-mer length and the
 // other derived parameters (preprocess.cpp:295-313) are part of the format
 // and are never tuned.
 //

@@ -96,8 +96,9 @@ int curc_ctx_keep_intermediates(curc_ctx* ctx, int keep);
 /* Frees the device memory a context keeps between blocks: its pipeline's
  * arena and the extra pipelines, input slots and pinned staging of the
  * batched path (they are made again on the next run or drain).  Results of
- * the last run stay readable.  CURC_ERR_STATE while blocks are queued.  No
- * reference counterpart. */
+ * the last run stay readable; the learned coder, which reads the last block
+ * on the device, finds none until the next run.  CURC_ERR_STATE while blocks
+ * are queued.  No reference counterpart. */
 int curc_ctx_trim(curc_ctx* ctx);
 
 /* Autotuner (no counterpart in the reference).  Knobs, in this order: the
