@@ -859,7 +859,8 @@ void Block::refmatch_all() {
                                       reinterpret_cast<const uint8_t*>(sizes) + sizeof(sizes)));
     // block statistics: reads, non-N reads, N reads, pseudogenome reads,
     // unmatched, mapped, unmapped (non-N, N); overlap: offsets passed, free
-    // suffixes of runs that two or more of them met; records, mismatches;
+    // suffixes of runs with a free prefix that two or more of them met at one
+    // offset; records, mismatches;
     // overlap again: suffixes, and summed over the offsets free suffixes, their
     // k-mers found in the presence bitmap, meetings with a run of prefixes,
     // buckets searched, prefix rows compared; links made; mapping, forward then

@@ -72,8 +72,8 @@ void gather_ascii_rows(const uint8_t* seq, const uint32_t* ids, uint32_t m, int 
 // ---- a2..a5 (overlap.cu)
 void dedupe_links(const uint64_t* db, int W, const uint32_t* sorted, uint32_t m, uint32_t* next, uint32_t* prev,
                   uint16_t* offset, cudaStream_t s);
-// Offsets passed, links made, suffixes of runs that two or more free suffixes
-// met at one offset, suffixes; summed over the offsets: free suffixes, their
+// Offsets passed, links made, free suffixes of runs with a free prefix that two
+// or more of them met at one offset, suffixes; summed over the offsets: free suffixes, their
 // k-mers found in the presence bitmap, meetings, buckets searched, prefix
 // rows read and compared there.
 struct OverlapStats {

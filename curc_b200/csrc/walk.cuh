@@ -37,7 +37,7 @@ struct __align__(16) Meeting {
 __device__ __forceinline__ uint32_t ld_l2(const uint32_t* p) { return __ldcg(p); }
 
 // What a walk did, where it is counted: links made, and the free suffixes of
-// runs that two or more of them met.
+// runs with a free prefix that two or more of them met.
 struct Walked {
     uint32_t links = 0, contested = 0;
     __device__ __forceinline__ void met(uint32_t free_members) { contested += free_members > 1 ? free_members : 0; }
@@ -46,8 +46,8 @@ struct Walked {
 // The suffixes of one run (items [i, e) with the same lo, in order) each take
 // the first free prefix that is not themselves, as the reference's merge of
 // the run does (its rotation puts a prefix that meets itself back in front).
-// One thread.  Returns the free suffixes it met from item `from` on; they are
-// all met only where that is counted.
+// One thread.  Returns the free suffixes it met from item `from` on, where that
+// is counted: all of them, unless there was no free prefix to begin with.
 template <bool COUNT>
 __device__ __forceinline__ uint32_t walk_run(const Meeting* __restrict__ item, uint32_t i, uint32_t e,
                                              const uint32_t* __restrict__ pre, uint32_t q0, uint32_t hi, int off,
@@ -55,7 +55,7 @@ __device__ __forceinline__ uint32_t walk_run(const Meeting* __restrict__ item, u
                                              Walked& w) {
     const uint32_t lo = item[i].lo;
     uint32_t met = 0;
-    bool any = true;  // a free prefix was left
+    bool any = true, had = false;  // a free prefix was left; there was one
     for (; i < e && item[i].lo == lo; ++i) {
         const uint32_t s = item[i].s;
         if (ld_l2(next + s) != INVALID) continue;
@@ -78,7 +78,8 @@ __device__ __forceinline__ uint32_t walk_run(const Meeting* __restrict__ item, u
             if (COUNT) ++w.links;
             break;
         }
-        if (!COUNT && !any) return met;
+        had |= any;
+        if (!any && (!COUNT || !had)) return 0;
     }
     return met;
 }
@@ -96,8 +97,8 @@ static __device__ void walk_run_warp(const Meeting* __restrict__ item, uint32_t 
     uint32_t ib = i, qb = q;          // where the next 32 start
     uint32_t s = 0, p = 0;            // this lane's entries
     uint32_t met = 0;
-    bool more_s = true, more_p = true;
-    while (more_p) {
+    bool more_s = true, had = false;  // had: there was a free prefix
+    for (;;) {
         while (sm == 0 && more_s) {
             const uint32_t t = ib + lane;
             const bool in = t < e && item[t].lo == lo;
@@ -117,9 +118,10 @@ static __device__ void walk_run_warp(const Meeting* __restrict__ item, uint32_t 
             qb += 32;
         }
         if (pm == 0) {
-            more_p = false;
+            if (COUNT && !had) return;
             break;
         }
+        had = true;
         const int n = min(__popc(sm), __popc(pm));
         // lane k < n pairs the k-th free suffix with the k-th free prefix
         const int ks = int(lane) < n ? int(__fns(sm, 0, int(lane) + 1)) : 0;
@@ -146,12 +148,22 @@ static __device__ void walk_run_warp(const Meeting* __restrict__ item, uint32_t 
         }
     }
     if (COUNT) {
-        for (; more_s; ib += 32) {  // no prefix is left for these
-            const uint32_t t = ib + lane;
-            const bool in = t < e && item[t].lo == lo;
-            more_s = __ballot_sync(0xFFFFFFFFu, in) == 0xFFFFFFFFu;
-            met += __popc(__ballot_sync(0xFFFFFFFFu, in && ld_l2(next + item[t].s) == INVALID));
+        uint32_t left = 0;  // free suffixes for which no prefix is left, eight a lane at a time
+        for (; more_s; ib += 256) {
+            uint32_t sv[8], in = 0;
+#pragma unroll
+            for (uint32_t k = 0; k < 8; ++k) {
+                const uint32_t t = ib + 32 * k + lane;
+                const bool is = t < e && item[t].lo == lo;
+                sv[k] = is ? item[t].s : 0;
+                in |= uint32_t(is) << k;
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < 8; ++k)
+                if (in >> k & 1u) left += ld_l2(next + sv[k]) == INVALID;
+            more_s = __all_sync(0xFFFFFFFFu, in >> 7);
         }
+        met += __reduce_add_sync(0xFFFFFFFFu, left);
         if (lane == 0) w.met(met);
     }
 }
@@ -260,7 +272,7 @@ static __device__ __forceinline__ void walk_offset_ahead(const Meeting* __restri
                 if (k < h.ns && ld_l2(next + h.s[k]) == INVALID) fs |= 1u << k;
                 if (k < h.np && ld_l2(prev + h.p[k]) == INVALID) fp |= 1u << k;
             }
-            if (COUNT) w.met(__popc(fs));
+            if (COUNT && fp) w.met(__popc(fs));
 #pragma unroll
             for (uint32_t k = 0; k < FEW; ++k) {
                 if (!(fs >> k & 1u)) continue;
