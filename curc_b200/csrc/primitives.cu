@@ -578,15 +578,15 @@ struct RsTile {
 // waits (lookback.cuh): those of tiles not heard from are counted.  p: tile
 // j's state of the digit.
 template <class K>
-__device__ __noinline__ uint64_t rs_look_on(const K* __restrict__ keys, uint32_t j, int items, int shift, uint32_t mask,
+__device__ __noinline__ uint32_t rs_look_on(const K* __restrict__ keys, uint32_t j, int items, int shift, uint32_t mask,
                                             uint32_t d, const unsigned long long* p) {
     const LookOnce look;
-    uint64_t before = 0;
+    uint32_t before = 0;
     for (;; p -= 256, --j) {
         uint32_t spins = 0;
         const uint64_t v = look_wait(look, p, spins);
         if (look.flag(v)) {
-            before += look.sum(v);
+            before += uint32_t(look.sum(v));
         } else {
             const K* k = keys + size_t(j) * items;
             for (int i = 0; i < items; ++i) before += digit_of(k[i], shift, mask) == d;
@@ -659,23 +659,22 @@ __global__ void __launch_bounds__(RS_THREADS) rs_pass_kernel(const K* __restrict
         }
     }
     // items of digit tid in the tiles before this one
-    uint64_t before = 0;
+    uint32_t before = 0;
     if (tile > 0) {
-        unsigned long long* p = state;
-        for (uint32_t j = tile; j > 0; --j) {
+        const unsigned long long* p = state;
+        uint32_t j = tile;
+        uint64_t v;
+        do {  // as far as tile 0, whose sum is inclusive
             p -= 256;
+            --j;
             uint32_t spins = LOOK_SPINS;
-            const uint64_t v = look_wait(look, p, spins);
-            if (look.flag(v) == 0) {
-                before += rs_look_on(kin, j - 1, TILE, shift, mask, uint32_t(tid), p);
-                break;
-            }
-            before += look.sum(v);
-            if (look.flag(v) == 2) break;
-        }
+            v = look_wait(look, p, spins);
+            before += uint32_t(look.sum(v));
+        } while (look.flag(v) == 1);
+        if (look.flag(v) == 0) before += rs_look_on(kin, j, TILE, shift, mask, uint32_t(tid), p);
         atomicExch(state, look.make(2, before + mine));
     }
-    gbase[tid] = digit_start + uint32_t(before) - tstart[tid];
+    gbase[tid] = digit_start + before - tstart[tid];
     __syncthreads();
     // the tile in digit order: runs of one digit go to consecutive places
     for (uint32_t p = tid; p < items; p += RS_THREADS) {
