@@ -169,7 +169,7 @@ __device__ __forceinline__ void map_read(const MapIndex& ix, const uint64_t* __r
     }
     for (uint32_t t = lane; t < SEEN; t += 32) seen[t] = ~0ull;
     __syncwarp();
-    const int probes = (L - k) / BlockParams::read_step + 1;
+    const int probes = L < k ? 0 : (L - k) / BlockParams::read_step + 1;
     int best = init;  // smallest count met so far (the same in every lane)
     uint64_t best_pos = 0;
     bool done = false;
